@@ -40,6 +40,7 @@
 #include "host_util.h"
 #include "ptx.cuh"
 #include "split3.cuh"
+#include "w8_gemm.h"
 
 namespace tb {
 
@@ -54,22 +55,6 @@ constexpr int THREADS_WIDE = 32 * (2 + EPI_WARPS_WIDE);
 constexpr int DYN_SMEM_MAX = 226 * 1024;  // 227 KB per CTA minus 1 KB left for static shared memory
 constexpr int CORESIDENT_SMEM = 112 * 1024;  // dynamic shared memory of a CTA when two share an SM (228 KB)
 constexpr int MAX_SPLITS = 8;             // portable cluster size
-
-// EPI_GEGLU_PACKED: one weight matrix whose 128-row tiles hold 64 gate rows followed by the 64
-// up rows of the same channels; the tile yields 64 output channels gelu(gate) * up.
-// EPI_QKV_ROPE: packed q/k/v projection whose 128-row tiles hold 64 head dimensions followed by
-// their rotate-half partners (d, d + D/2); the tile is rotated and stored as q rows / cache rows.
-enum : int { EPI_NONE = 0, EPI_GELU = 1, EPI_RESIDUAL = 2, EPI_GEGLU = 3, EPI_GEGLU_PACKED = 4, EPI_QKV_ROPE = 5 };
-
-struct RopeEpi {
-  const int* pos;              // [M] position of every token row
-  const __nv_bfloat16* cos;    // [max_pos][D]
-  const __nv_bfloat16* sin;
-  __nv_bfloat16* q;            // [M][H*D]
-  __nv_bfloat16* kcache;       // [B][G][Lcap][D]
-  __nv_bfloat16* vcache;
-  int L, H, G, D, Lcap, key_off;
-};
 
 struct GemmParams {
   int M, N, K;
@@ -96,8 +81,6 @@ struct GemmParams {
   float dn_inv_w, dn_eps;
   const float* bias_f32;  // consumer: [N] fp32 bias in weight-row order, or NULL
   int merge;     // 1: the planes are one UMMA of N = np*bt whose column groups the epilogue adds
-  int pair;      // 1: CTA pairs (cluster of 2 along the channel tiles) run one UMMA of M = 256; each CTA
-                 // loads its own weight tile and half of the activation planes (tm_w1 = half-tile map)
   int epi;
   int pdl;
   float out_scale;   // 2^-x_shift: undoes the power-of-two pre-scale of the activation planes
@@ -125,7 +108,7 @@ struct __align__(8) Barriers {
   uint64_t full[MAX_STAGES];
   uint64_t empty[MAX_STAGES];
   uint64_t tmem_full;
-  uint64_t mma_done;  // every tensor-core instruction this CTA (or its pair) issued has retired
+  uint64_t mma_done;  // every tensor-core instruction this CTA issued has retired
   uint32_t tmem_base;
   volatile int abort;
 };
@@ -148,8 +131,6 @@ __device__ __forceinline__ void fail(Barriers* b, int* status, int code) {
 
 // Bounded for two CTAs per SM: multi-wave full-K launches run with a shallow ring so that one
 // tile's epilogue overlaps the other's main loop (register budget 64K / 640 threads).
-// PAIR: the CTA-pair form (cta_group::2 instructions oblige every launch of a kernel that holds
-// them to use clusters of two, so it is an instantiation of its own).
 // EW: epilogue warps.  A split-K CTA has the SM to itself and a long serial epilogue per thread
 // (accumulator groups to push, rows to finish): sixteen warps halve both.
 // rsqrt(mean(x^2) + eps) of token row m from the producer's per-channel-tile partial sums (fixed order).
@@ -168,7 +149,7 @@ __device__ __forceinline__ float deferred_rstd(const GemmParams& p, int m) {
   return rsqrtf(t * p.dn_inv_w + p.dn_eps);
 }
 
-template <bool PAIR, int EW = EPI_WARPS>
+template <int EW>
 __global__ void __launch_bounds__(32 * (2 + EW), EW == EPI_WARPS ? 2 : 1)
 w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                const __grid_constant__ CUtensorMap tm_x, const GemmParams p) {
@@ -180,24 +161,22 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   const int warp = tid >> 5;
   const int lane = tid & 31;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  constexpr int KID = PAIR ? 2 : (EW == EPI_WARPS ? 0 : 1);
+  constexpr int KID = EW == EPI_WARPS ? 0 : 1;
   if (tid == 0) dbg_stage(p.dbg, KID, 0);
 
   const int ns = p.nstages;
-  const int x_bytes = PAIR ? p.np * p.bt * 64 : p.np * p.bt * 128;  // np planes of bt rows x 128 bytes (a pair: half each)
+  const int x_bytes = p.np * p.bt * 128;              // np planes of bt rows x 128 bytes
   const int x_off = p.nw * W_TILE_BYTES;              // activation planes follow the weight tile(s)
   const int stage_bytes = x_off + x_bytes;
 
-  // A pair is two neighbouring channel tiles; pairs lie along x of the grid (and of the cluster).
-  const int t_tile = PAIR ? blockIdx.y : blockIdx.x, n_tile = PAIR ? blockIdx.x : blockIdx.y, split = blockIdx.z;
-  const uint32_t pair_rank = PAIR ? cluster_ctarank() : 0u;  // 0 issues the pair's UMMAs
+  const int t_tile = blockIdx.x, n_tile = blockIdx.y, split = blockIdx.z;
   const int kb0 = split * p.kb_per_split;
   const int nkb = min(p.kb_total, kb0 + p.kb_per_split) - kb0;
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_w0);
-    if (p.nw == 2 || PAIR) tma_prefetch_desc(&tm_w1);
-    if (!PAIR) tma_prefetch_desc(&tm_x);
+    if (p.nw == 2) tma_prefetch_desc(&tm_w1);
+    tma_prefetch_desc(&tm_x);
     for (int i = 0; i < MAX_STAGES; ++i) {
       mbar_init(&bars.full[i], 1);
       mbar_init(&bars.empty[i], 1);
@@ -207,35 +186,22 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     bars.abort = 0;
     fence_barrier_init();
     // Weights depend on nothing that runs before this kernel: request the first stages now,
-    // before the rest of the CTA has even finished its set-up.  (A pair first has to know that
-    // the partner's barriers exist: it requests them after the cluster has met.)
-    if (!PAIR) {
-      const int pre = min(ns, nkb);
-      for (int i = 0; i < pre; ++i) {
-        uint8_t* st = smem + i * stage_bytes;
-        mbar_arrive_expect_tx(&bars.full[i], stage_bytes);
-        const int k0 = (kb0 + i) * BK;
-        tma_load_2d(st, &tm_w0, &bars.full[i], k0, n_tile * BN);
-        if (p.nw == 2) tma_load_2d(st + W_TILE_BYTES, &tm_w1, &bars.full[i], k0, n_tile * BN);
-      }
+    // before the rest of the CTA has even finished its set-up.
+    const int pre = min(ns, nkb);
+    for (int i = 0; i < pre; ++i) {
+      uint8_t* st = smem + i * stage_bytes;
+      mbar_arrive_expect_tx(&bars.full[i], stage_bytes);
+      const int k0 = (kb0 + i) * BK;
+      tma_load_2d(st, &tm_w0, &bars.full[i], k0, n_tile * BN);
+      if (p.nw == 2) tma_load_2d(st + W_TILE_BYTES, &tm_w1, &bars.full[i], k0, n_tile * BN);
     }
   }
   if (warp == 1) {
-    if (PAIR) {
-      tmem_alloc_pair(&bars.tmem_base, p.tmem_cols);
-      tmem_relinquish_pair();
-    } else {
-      tmem_alloc(&bars.tmem_base, p.tmem_cols);
-      tmem_relinquish();
-    }
+    tmem_alloc(&bars.tmem_base, p.tmem_cols);
+    tmem_relinquish();
   }
   tc_fence_before();
-  if (PAIR) {
-    __syncwarp();
-    cluster_sync_all();
-  } else {
-    __syncthreads();
-  }
+  __syncthreads();
   tc_fence_after();
   if (tid == 0) dbg_stage(p.dbg, KID, 1);
   const uint32_t tmem = bars.tmem_base;
@@ -265,47 +231,6 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       // this grid is running; they still wait for this grid to complete before touching its output.
       if (p.pdl) pdl_launch_dependents();
       const int pre = min(ns, nkb);
-      if (PAIR) {
-        // CTA pair: both CTAs load their own weight tile and their half of the activation planes
-        // (three boxes of bt/2 token rows of one plane); every byte is credited to the full
-        // barrier of the even-ranked CTA, which issues the UMMAs for both.
-        const int hrows = p.bt >> 1;
-        auto pair_stage = [&](int i, bool weights, bool acts) {
-          uint8_t* st = smem + (i % ns) * stage_bytes;
-          const uint32_t bar = dsmem_addr(smem_u32(&bars.full[i % ns]), 0);
-          const int k0 = (kb0 + i) * BK;
-          if (weights) {
-            if (pair_rank == 0) mbar_arrive_expect_tx(&bars.full[i % ns], 2 * stage_bytes);
-            tma_load_2d_pair(st, &tm_w0, bar, k0, n_tile * BN);
-          }
-          if (acts) {
-            for (int j = 0; j < p.np; ++j) {
-              const int u = static_cast<int>(pair_rank) * p.np + j;  // half-plane index 0 .. 2 np - 1
-              tma_load_3d_pair(st + x_off + j * hrows * 128, &tm_w1, bar, k0, t_tile * p.bt + (u & 1) * hrows, u >> 1);
-            }
-          }
-        };
-        for (int i = 0; i < pre; ++i) pair_stage(i, true, false);
-        if (p.pdl) pdl_wait();
-        dbg_stage(p.dbg, KID, 2);
-        for (int i = 0; i < pre; ++i) pair_stage(i, false, true);
-        int armed = pre;
-        for (int i = pre; i < nkb; ++i) {
-          if (!wait_or_abort(&bars.empty[i % ns], ((i / ns) & 1) ^ 1, &bars.abort)) {
-            fail(&bars, p.status, TYBOK_DEV_TIMEOUT_PRODUCER);
-            break;
-          }
-          pair_stage(i, true, true);
-          armed = i + 1;
-        }
-        // Unwinding (completion is observed through the issuing CTA's barriers only): the even CTA
-        // waits for the newest copy of every stage it armed; the pair leaves together at the
-        // closing cluster barrier.
-        if (bars.abort && pair_rank == 0)
-          for (int i = max(0, armed - ns); i < armed; ++i) mbar_wait(&bars.full[i % ns], (i / ns) & 1);
-        issued = 0;
-        ok = true;
-      } else {
       // The weight tiles of the first stages were requested during set-up; the activation planes
       // are requested once the programmatic dependency has resolved.
       if (p.pdl) pdl_wait();
@@ -328,8 +253,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         tma_load_3d(st + x_off, &tm_x, &bars.full[s], k0, t_tile * p.bt, 0);
         issued = i + 1;
       }
-      }
-      if (!PAIR && (!ok || bars.abort)) {
+      if (!ok || bars.abort) {
         // Unwinding: do not leave the CTA while its own bulk copies may still land in its
         // shared memory. Wait (bounded) for the newest copy of every stage.
         for (int i = max(0, issued - ns); i < issued; ++i) mbar_wait(&bars.full[i % ns], (i / ns) & 1);
@@ -344,13 +268,12 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     // instead of 12 instructions per weight tile and K block.  Larger tiles issue one UMMA per
     // plane into the same accumulator.
     const int mma_n = p.merge ? p.np * p.bt : p.bt;
-    const uint32_t idesc = p.np == 2 ? idesc_e4m3_e4m3_f32(PAIR ? 2 * BN : BN, mma_n) : idesc_e4m3_e5m2_f32(PAIR ? 2 * BN : BN, mma_n);
-    const int nkb_mma = (PAIR && pair_rank != 0) ? 0 : nkb;  // the odd CTA of a pair issues nothing
+    const uint32_t idesc = p.np == 2 ? idesc_e4m3_e4m3_f32(BN, mma_n) : idesc_e4m3_e5m2_f32(BN, mma_n);
     const uint64_t desc_const = smem_desc_sw128(0);
     const uint32_t plane16 = static_cast<uint32_t>(p.bt * 128) >> 4;  // plane pitch in 16-byte units
     const int acc_cols = p.merge ? p.np * p.bt : p.bt;
     bool ok = true;
-    for (int i = 0; i < nkb_mma; ++i) {
+    for (int i = 0; i < nkb; ++i) {
       const int s = i % ns;
       const long long c0 = tr ? clock64() : 0;
       const bool ready = wait_or_abort(&bars.full[s], (i / ns) & 1, &bars.abort);
@@ -371,10 +294,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           for (int j = 0; j < 4; ++j) {  // K = 32 per instruction: 32 bytes = 2 sixteen-byte units
             const uint64_t a_desc = desc_const | (w16 + j * 2);
             const uint64_t b_desc = desc_const | (x16 + j * 2);
-            if (leader) {
-              if (PAIR) umma_ss_f8_pair(d_addr, a_desc, b_desc, idesc, (i > 0 || j > 0) ? 1u : 0u);
-              else umma_ss_f8(d_addr, a_desc, b_desc, idesc, (i > 0 || j > 0) ? 1u : 0u);
-            }
+            if (leader) umma_ss_f8(d_addr, a_desc, b_desc, idesc, (i > 0 || j > 0) ? 1u : 0u);
           }
         } else {
           for (int pl = 0; pl < p.np; ++pl) {
@@ -387,25 +307,15 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           }
         }
       }
-      if (leader) {  // frees the stage (in both CTAs of a pair) once these MMAs have read it
-        if (PAIR) tc_commit_pair(&bars.empty[s], 3);
-        else tc_commit(&bars.empty[s]);
-      }
+      if (leader) tc_commit(&bars.empty[s]);  // frees the stage once these MMAs have read it
       __syncwarp();
     }
-    if (ok && leader && nkb_mma > 0) {
-      if (PAIR) tc_commit_pair(&bars.tmem_full, 3);
-      else tc_commit(&bars.tmem_full);
-    }
+    if (ok && leader) tc_commit(&bars.tmem_full);
     if (tr && leader) tr[3] = clock64();
     // Whatever happened above, and whatever the other warps decide: this warp frees the tensor
-    // memory at the end, so it first sees every instruction it issued retire (in a pair the even
-    // CTA's commit arrives in both CTAs).  On the normal path this completes together with
+    // memory at the end, so it first sees every instruction it issued retire.  On the normal path this completes together with
     // tmem_full; the warp has nothing else to do until the CTA meets.
-    if (leader && (!PAIR || pair_rank == 0)) {
-      if (PAIR) tc_commit_pair(&bars.mma_done, 3);
-      else tc_commit(&bars.mma_done);
-    }
+    if (leader) tc_commit(&bars.mma_done);
     __syncwarp();
     if (!mbar_wait(&bars.mma_done, 0) && lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
   } else {
@@ -724,17 +634,10 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
 
   if (tr && tid == 64) tr[7] = clock64();
   // After the meeting point nobody touches another CTA's shared memory: CTAs leave on their own.
-  if (PAIR) {  // tensor memory of a pair is released together, once both CTAs have read theirs
-    tc_fence_before();
-    __syncwarp();
-    cluster_sync_all();
-  } else {
-    __syncthreads();
-  }
+  __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    if (PAIR) tmem_dealloc_pair(tmem, p.tmem_cols);
-    else tmem_dealloc(tmem, p.tmem_cols);
+    tmem_dealloc(tmem, p.tmem_cols);
   }
   if (tid == 0) dbg_stage(p.dbg, KID, 4);
 }
@@ -769,7 +672,7 @@ __global__ void split3_kernel(const __nv_bfloat16* __restrict__ x, long long ldx
 
 // ------------------------------------------------------------------------------------ host
 struct Plan {
-  int bt, t_tiles, n_tiles, splits, kb_total, kb_per_split, nstages, smem_bytes, tmem_cols, merge, stage_off, pair;
+  int bt, t_tiles, n_tiles, splits, kb_total, kb_per_split, nstages, smem_bytes, tmem_cols, merge, stage_off;
 };
 
 static int round_up(int a, int b) { return (a + b - 1) / b * b; }
@@ -781,7 +684,7 @@ static int max_active_clusters(int splits) {
   static int cached[MAX_SPLITS + 1] = {};
   if (splits <= 1) return 1 << 30;
   if (cached[splits] == 0) {
-    cudaFuncSetAttribute(w8_gemm_kernel<false, EPI_WARPS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX);
+    cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(1, 1, splits);
     cfg.blockDim = dim3(THREADS_WIDE);
@@ -794,7 +697,7 @@ static int max_active_clusters(int splits) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, w8_gemm_kernel<false, EPI_WARPS_WIDE>, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, w8_gemm_kernel<EPI_WARPS_WIDE>, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = host::sm_count() / (2 * splits);  // conservative guess
     }
@@ -818,14 +721,9 @@ static bool make_plan(int M, int N, int K, int nw, int force_bt, int force_split
     const int n_tiles = (N + BN - 1) / BN;
     long long best_cost = 0;
     bt = 0;
-    // Two planes: np * bt <= 256 allows token tiles up to 128 (caps 128 / 112 / 96 / 80 / 64).  Their
-    // cost model knows the two launch forms: up to 2 * SMs tiles run one CTA per SM in whole waves; from
-    // there on (CTA pairs, two CTAs per SM, one tile's epilogue under the other's main loop) CTAs start
-    // as others finish, a "wave" of 2 * SMs tiles costs 1.5 single waves and fractions of it count.
-    // Measured against forced tiles of 64 .. 128 the pick is within a few percent of the best from 544
-    // tokens up; between 256 and 800 tokens with short K the spread between tiles is inside the noise.
+    // Two planes: np * bt <= 256 allows token tiles up to 128 (caps 128 / 112 / 96 / 80 / 64).
+    // (More tiles than SMs only reach this plan with a folded norm or a forced tile: see w8_gemm_pair.cu.)
     const int caps3[5] = {80, 64, 0, 0, 0}, caps2[5] = {128, 112, 96, 80, 64};
-    double best2 = 0.0;
     for (int ci = 0; ci < 5; ++ci) {
       const int cap = np == 2 ? caps2[ci] : caps3[ci];
       if (cap == 0) break;
@@ -833,17 +731,9 @@ static bool make_plan(int M, int N, int K, int nw, int force_bt, int force_split
       const int tiles = (M + cap - 1) / cap;
       const int cand = round_up((M + tiles - 1) / tiles, 16);
       const long long ctas = static_cast<long long>((M + cand - 1) / cand) * n_tiles;
-      if (np == 2) {
-        const bool multi = ctas >= 2 * sms && nw == 1;
-        const double waves = multi ? std::max(1.0, static_cast<double>(ctas) / (2.0 * sms)) * 1.5
-                                   : static_cast<double>((ctas + sms - 1) / sms);
-        const double cost = waves * (cand + 24);
-        if (bt == 0 || cost < best2) { bt = cand; best2 = cost; }
-      } else {
-        const long long waves = (ctas + sms - 1) / sms;
-        const long long cost = waves * (cand + 24);
-        if (bt == 0 || cost < best_cost) { bt = cand; best_cost = cost; }
-      }
+      const long long waves = (ctas + sms - 1) / sms;
+      const long long cost = waves * (cand + 24);
+      if (bt == 0 || cost < best_cost) { bt = cand; best_cost = cost; }
     }
   }
   if (bt % 16 != 0 || bt < 16 || bt > max_bt) return false;
@@ -862,13 +752,7 @@ static bool make_plan(int M, int N, int K, int nw, int force_bt, int force_split
     while (splits > 1 && tiles > max_active_clusters(splits)) --splits;
   }
   splits = std::max(1, std::min(std::min(splits, MAX_SPLITS), pl.kb_total));
-  // Multi-wave full-K launches run as CTA pairs (one UMMA of 256 weight rows per two CTAs): each
-  // CTA then loads half of the activation planes, a third less shared-memory fill per MMA and a
-  // third stage in the same shared memory (4146 x 3072 x 14336: 503 -> 409 us; 544 x 32768 x 2048:
-  // unchanged; single-wave launches lose a microsecond to the pair's set-up, so they stay single).
-  pl.pair = (splits == 1 && nw == 1 && np * bt <= 256 && pl.n_tiles % 2 == 0 &&
-             pl.t_tiles * pl.n_tiles >= 2 * host::sm_count()) ? 1 : 0;
-  const int stage_bytes = pl.pair ? W_TILE_BYTES + np * bt * 64 : nw * W_TILE_BYTES + np * bt * 128;
+  const int stage_bytes = nw * W_TILE_BYTES + np * bt * 128;
   for (;; --splits) {  // fewer splits if the split-K staging tile does not fit beside the ring
     pl.kb_per_split = (pl.kb_total + splits - 1) / splits;
     pl.splits = (pl.kb_total + pl.kb_per_split - 1) / pl.kb_per_split;  // no empty split
@@ -952,18 +836,24 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   if (!make_plan(M, N, K, nw, force_bt, force_splits, pl, np))
     return host::fail(TYBOK_ERR_ARG, "w8 gemm: unsupported token tile (multiple of 16, <= 256, <= 128 when gated)");
   if (force_splits > MAX_SPLITS) return host::fail(TYBOK_ERR_ARG, "w8 gemm: at most 8 K splits (cluster size)");
-  if ((pl.pair ? pl.t_tiles : pl.n_tiles) > 65535) return host::fail(TYBOK_ERR_ARG, "w8 gemm: grid too large");
+  if (pl.n_tiles > 65535) return host::fail(TYBOK_ERR_ARG, "w8 gemm: grid too large");
   if (check_only) return TYBOK_OK;  // every argument check has passed; nothing was launched
+  if (force_bt <= 0 && force_splits <= 0 && !fold && gemm_pair_suits(M, N, nw, np)) {
+    GemmCall c{};
+    c.planes = planes; c.np = np; c.row_scale = row_scale; c.w0 = w0; c.w1 = w1; c.s0 = s0; c.s1 = s1;
+    c.bias = static_cast<const __nv_bfloat16*>(bias); c.y = static_cast<__nv_bfloat16*>(y); c.ldy = ldy;
+    c.y_planes = static_cast<uint8_t*>(y_planes); c.M = M; c.N = N; c.K = K; c.n_out = n_out; c.epi = epi;
+    c.res = static_cast<const __nv_bfloat16*>(res); c.ldres = ldres; c.gate = gate; c.ldgate = ldgate;
+    c.rows_per_gate = rows_per_gate; c.gate_bf16 = gate_bf16; c.out_scale = row_scale ? 1.0f : ldexpf(1.0f, -x_shift);
+    c.plane_scale = ldexpf(1.0f, out_shift); c.rope = rope; c.status = status; c.stream = stream;
+    return launch_gemm_pair(c);
+  }
 
   CUtensorMap tm_w0, tm_w1, tm_x;
   if (int rc = host::tensor_map_2d(&tm_w0, w0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, N, K, BK, BN)) return rc;
   tm_w1 = tm_w0;
   if (nw == 2)
     if (int rc = host::tensor_map_2d(&tm_w1, w1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, N, K, BK, BN)) return rc;
-  if (pl.pair)  // half-plane boxes of the activation planes: bt/2 token rows of one plane
-    if (int rc = host::tensor_map_3d(&tm_w1, planes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, M, np, K,
-                                     static_cast<uint64_t>(M) * K, BK, pl.bt / 2, 1))
-      return rc;
   if (int rc = host::tensor_map_3d(&tm_x, planes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, M, np, K,
                                    static_cast<uint64_t>(M) * K, BK, pl.bt, np))
     return rc;
@@ -971,7 +861,7 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.n_out = n_out;
   p.bt = pl.bt; p.nw = nw; p.splits = pl.splits; p.kb_total = pl.kb_total; p.kb_per_split = pl.kb_per_split;
-  p.nstages = pl.nstages; p.tmem_cols = pl.tmem_cols; p.merge = pl.merge; p.pair = pl.pair; p.stage_off = pl.stage_off; p.epi = epi; p.pdl = host::pdl_enabled() ? 1 : 0;
+  p.nstages = pl.nstages; p.tmem_cols = pl.tmem_cols; p.merge = pl.merge; p.stage_off = pl.stage_off; p.epi = epi; p.pdl = host::pdl_enabled() ? 1 : 0;
   p.np = np; p.row_scale = row_scale;
   p.out_scale = row_scale ? 1.0f : ldexpf(1.0f, -x_shift);
   p.plane_scale = ldexpf(1.0f, out_shift);
@@ -994,17 +884,16 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   static bool attr_set[64] = {};
   const int dev = host::current_device();
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(w8_gemm_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) != cudaSuccess ||
-        cudaFuncSetAttribute(w8_gemm_kernel<false, EPI_WARPS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) != cudaSuccess ||
-        cudaFuncSetAttribute(w8_gemm_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) != cudaSuccess)
+    if (cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) != cudaSuccess ||
+        cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) != cudaSuccess)
       return host::fail_cuda("cudaFuncSetAttribute(w8_gemm_kernel)");
     attr_set[dev] = true;
   }
 
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = pl.pair ? dim3(pl.n_tiles, pl.t_tiles, 1) : dim3(pl.t_tiles, pl.n_tiles, pl.splits);
+  cfg.gridDim = dim3(pl.t_tiles, pl.n_tiles, pl.splits);
   // sixteen epilogue warps wherever a CTA has its SM to itself: split-K, and full-K grids of one wave
-  const bool wide = !pl.pair && (pl.splits > 1 || pl.t_tiles * pl.n_tiles <= host::sm_count());
+  const bool wide = pl.splits > 1 || pl.t_tiles * pl.n_tiles <= host::sm_count();
   cfg.blockDim = dim3(wide ? THREADS_WIDE : THREADS);
   cfg.dynamicSmemBytes = pl.smem_bytes;
   cfg.stream = stream;
@@ -1015,18 +904,16 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
     attr[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
   }
-  if (pl.splits > 1 || pl.pair) {
+  if (pl.splits > 1) {
     attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = pl.pair ? 2 : 1;
+    attr[na].val.clusterDim.x = 1;
     attr[na].val.clusterDim.y = 1;
-    attr[na].val.clusterDim.z = pl.pair ? 1 : pl.splits;
+    attr[na].val.clusterDim.z = pl.splits;
     ++na;
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  if ((pl.pair         ? cudaLaunchKernelEx(&cfg, w8_gemm_kernel<true>, tm_w0, tm_w1, tm_x, p)
-       : wide          ? cudaLaunchKernelEx(&cfg, w8_gemm_kernel<false, EPI_WARPS_WIDE>, tm_w0, tm_w1, tm_x, p)
-                       : cudaLaunchKernelEx(&cfg, w8_gemm_kernel<false>, tm_w0, tm_w1, tm_x, p)) != cudaSuccess)
+  if (cudaLaunchKernelEx(&cfg, wide ? w8_gemm_kernel<EPI_WARPS_WIDE> : w8_gemm_kernel<EPI_WARPS>, tm_w0, tm_w1, tm_x, p) != cudaSuccess)
     return host::fail_cuda("launch w8_gemm_kernel");
   host::count_launch();
   return TYBOK_OK;
