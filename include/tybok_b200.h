@@ -170,6 +170,10 @@ int tybok_rmsnorm(const void* x, int64_t ldx, const float* weight, const float* 
  * 392-397 and wan_base.py:131-148.  Outputs as tybok_rmsnorm. */
 int tybok_layernorm_modulate(const void* x, int64_t ldx, const void* shift, const void* scale, int M, int W, float eps,
                              void* y, int64_t ldy, void* y_planes, int out_shift, void* stream);
+/* The same with one shift / scale row (row stride ldmod elements, a multiple of 8) per group of rows_per_group token rows. */
+int tybok_layernorm_modulate_groups(const void* x, int64_t ldx, const void* shift, const void* scale, int64_t ldmod,
+                                    int rows_per_group, int M, int W, float eps, void* y, int64_t ldy, void* y_planes,
+                                    int out_shift, void* stream);
 
 /* Per-step tail of the action-expert loop, one launch: final AdaRMS norm (scale/shift from
  * mod[g, 0:2W]) -> fp32 out-projection [A=32, W] -> x_t += dt * v (fp32, in place) -> next
@@ -260,6 +264,19 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
                     void* out_planes, int out_shift, int B, int L, int H, int G, int D, int Lk, int Lcap, float scale,
                     void* workspace, size_t workspace_bytes, int* status_word, void* stream);
 size_t tybok_attention_workspace_bytes(int B, int L, int H, int Lk);
+
+/* Attention of one sequence at head_dim 128 whose first n_rows keys / values lie token-major, as a host framework keeps
+ * them: k_rows / v_rows [n_rows][H*D] bf16, read in place.  With Lk > n_rows the keys from block b = n_rows / 128 on
+ * (128 keys per block) come head-major from k_tail / v_tail [H][tail_cap][D], finite, tail_cap >= Lk - 128 b; their first
+ * n_rows % 128 rows repeat the last rows of k_rows / v_rows (tybok_kv_rows_to_heads).  Same arithmetic, in the same
+ * order, as tybok_attention over one head-major copy of all keys.  Takes the per-layer K/V that the reference's runner
+ * is handed (tybok/policies/fastwam/models/fused_action.py:318-357). */
+int tybok_attention_rows(const void* q, const void* k_rows, const void* v_rows, int n_rows, const void* k_tail, const void* v_tail,
+                         int tail_cap, const void* key_valid, void* out, void* out_planes, int out_shift, int L, int H, int D,
+                         int Lk, float scale, int* status_word, void* stream);
+/* Rows [row0, row0 + n) of token-major K and V [rows][H*D] -> rows 0..n-1 of head-major [H][cap][D] (D % 8 == 0). */
+int tybok_kv_rows_to_heads(const void* k_rows, const void* v_rows, int row0, int n, void* k_out, void* v_out, int cap, int H, int D,
+                           void* stream);
 
 /* tybok_w8x3_geglu on ONE packed weight matrix [2*I, K]: every block of 128 rows holds the 64
  * gate rows of channels 64j..64j+63 followed by their 64 up rows (scale_packed [2*I] likewise),

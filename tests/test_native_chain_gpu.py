@@ -1,0 +1,79 @@
+"""The native chains at the sizes where they branch: token-major keys with and without a partial last block (bit-equal to
+one head-major copy), blocks on either side of the two-plane threshold, the batched FFN tail against one call per element."""
+
+import pytest
+import torch
+
+from tybok_b200.shapes import DIT_TINY
+from tybok_b200.weights import quantize_dit_block, quantize_w8, random_dit_block_params
+
+pytestmark = pytest.mark.gpu
+
+
+def _rnd(g, *shape, std=1.0):
+    return torch.empty(*shape, device="cuda").normal_(0, std, generator=g).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("m", [1, 50, 128, 200])
+@pytest.mark.parametrize("lv", [1, 127, 128, 129, 300])
+def test_token_major_keys_equal_one_head_major_copy(m, lv):
+    from tybok_b200 import ops
+    from tybok_b200.dit import DiTBlock, DiTDenoiser
+
+    s = DIT_TINY
+    g = torch.Generator(device="cuda").manual_seed(m * 1000 + lv)
+    params = quantize_dit_block(random_dit_block_params(s, seed=3, device="cuda"))
+    den = DiTDenoiser([params], s)
+    blk = den.blocks[0]
+    a, c = s.heads * s.head_dim, 140
+    x, vk, vv, ck, cv = _rnd(g, 1, m, s.hidden), _rnd(g, 1, lv, a), _rnd(g, 1, lv, a), _rnd(g, 1, c, a), _rnd(g, 1, c, a)
+    t_mod = _rnd(g, 1, 6, s.hidden, std=0.5)
+    freqs = torch.polar(torch.ones(m, s.head_dim // 2, dtype=torch.float64), torch.arange(m, dtype=torch.float64)[:, None] * 0.01
+                        + torch.zeros(m, s.head_dim // 2, dtype=torch.float64))[:, None, :].cuda()
+    mask = torch.ones(c, dtype=torch.bool)
+    mask[-9:-2] = False
+    got = den.run_action_layers(x, t_mod, freqs, [{"k": vk, "v": vv}], [(ck, cv)], mask.cuda())
+    kc, vc = blk.store_context_kv(vk, vv)
+    pad = torch.zeros(1, s.heads, m, s.head_dim, dtype=torch.bfloat16, device="cuda")
+    cache = (torch.cat([kc, pad], 2).contiguous(), torch.cat([vc, pad], 2).contiguous())
+    f = freqs.reshape(m, -1).to(torch.complex64)
+    want = blk.forward(x[0], blk.modulations(t_mod), f.real.float().contiguous(), f.imag.float().contiguous(), cache, lv,
+                       blk.store_context_kv(ck, cv), mask[None].to(torch.uint8).cuda())
+    ops.check_status()
+    assert torch.equal(got[0], want)
+    if m == 50:  # an unaligned, non-contiguous caller tensor gives the same
+        odd = torch.cat([_rnd(g, 1, lv, 1), vk], dim=2)[:, :, 1:]
+        again = den.run_action_layers(x, t_mod, freqs, [{"k": odd, "v": vv}], [(ck, cv)], mask.cuda())
+        assert torch.equal(again, got)
+
+
+@pytest.mark.parametrize("b,s,rows", [(1, 7, "one"), (2, 64, "each"), (3, 43, "mixed"), (2, 515, "each")])
+def test_batched_ffn_tail_equals_one_call_per_element(b, s, rows):
+    from tybok_b200 import ops
+    from tybok_b200.hooks import make_fused_ffn_tail
+
+    h, f = 256, 640
+    g = torch.Generator(device="cuda").manual_seed(s)
+
+    class Lin:
+        def __init__(self, n, k):
+            self.weight, self.weight_scale = quantize_w8(_rnd(g, n, k, std=0.02))
+            self.bias = _rnd(g, n)
+
+    class Blk:
+        ffn = [Lin(f, h), None, Lin(h, f)]
+
+    fn = make_fused_ffn_tail(Blk)
+    x, table = _rnd(g, b, s, h), _rnd(g, b, 6, h, std=0.5)
+    mods = [table[:, i : i + 1] for i in (3, 4, 5)]
+    if rows == "one":
+        mods = [m[0, 0] for m in mods]
+    elif rows == "mixed":
+        mods[1] = mods[1][:1]
+    y = fn(x, *mods)
+    ops.check_status()
+    assert y.shape == x.shape
+    for i in range(b):
+        one = [m if m.dim() == 1 else m[min(i, m.shape[0] - 1)] for m in mods]
+        ref = fn(x[i], *one)
+        assert float((y[i].float() - ref.float()).norm() / ref.float().norm()) <= 2e-3

@@ -45,6 +45,11 @@ SIGNATURES = {
     "tybok_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                 c_int, c_int, c_int, c_int, ctypes.c_float, c_void_p, c_size_t, c_void_p, c_void_p]),
     "tybok_attention_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
+    "tybok_attention_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                     c_int, c_int, c_int, c_int, c_int, ctypes.c_float, c_void_p, c_void_p]),
+    "tybok_kv_rows_to_heads": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
+    "tybok_layernorm_modulate_groups": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_i64, c_int, c_int, c_int, ctypes.c_float,
+                                                c_void_p, c_i64, c_void_p, c_int, c_void_p]),
     "tybok_w8x3_geglu_packed": (
         c_int,
         [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_i64, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
@@ -137,6 +142,23 @@ def load() -> ctypes.CDLL:
         fn.argtypes = argtypes
     _lib = lib
     return lib
+
+
+_native = None
+
+
+def native():
+    """The ``_native`` extension: the host path from torch tensors to the C ABI without Python or the
+    torch dispatcher between two launches.  Built beside the library; there is no fallback either."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from . import _native as mod
+        except ImportError as e:
+            raise ImportError("tybok_b200/_native.so is missing or stale: build it with `python -m tybok_b200.build`") from e
+        _native = mod
+    return _native
 
 
 def check(rc: int, what: str) -> None:

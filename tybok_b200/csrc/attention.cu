@@ -214,6 +214,21 @@ __global__ void __launch_bounds__(512) qknorm_rope_store_kernel(const QkNormPara
   if (threadIdx.x == 0) dbg_stage(p.dbg, 7, 4);
 }
 
+// Rows [row0, row0 + n) of token-major keys and values [rows][H*D] into rows 0..n-1 of head-major ones [H][cap][D].
+__global__ void __launch_bounds__(256) kv_rows_to_heads_kernel(const uint4* __restrict__ k, const uint4* __restrict__ v, uint4* k_out,
+                                                               uint4* v_out, int row0, int n, int H, int vec, int cap, int pdl) {
+  if (pdl) pdl_launch_dependents();
+  if (pdl) pdl_wait();
+  const int per_row = H * vec, total = n * per_row;  // vec: 16-byte vectors of one head
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const int r = i / per_row, c = i - r * per_row, h = c / vec;
+    const long long src = static_cast<long long>(row0 + r) * per_row + c;
+    const long long dst = (static_cast<long long>(h) * cap + r) * vec + (c - h * vec);
+    k_out[dst] = k[src];
+    v_out[dst] = v[src];
+  }
+}
+
 struct AttnParams {
   int B, L, H, G, Lk, Lcap;
   int nsplit;
@@ -227,6 +242,8 @@ struct AttnParams {
   uint8_t* ws;       // [CTA][AT_WS_PER_CTA] exchange workspace (nsplit > 1)
   int q_rows;        // query rows per bulk copy: 128, or 64 when all real rows fit (the rest of the tile is never read back)
   int dsplit;        // 1, or 2: two CTAs per (query tile, key block), each producing half of the output columns
+  int nb_rows;       // key-loop form: the first nb_rows key blocks come from token-major rows [Lk][G*D], the others from
+                     // the head-major caches (whose key 0 is then the first key of block nb_rows); 0 = all from the caches
   long long* trace;  // tuning aid: [CTA][16] SM-clock samples, NULL in production
   int* dbg;          // debugging aid: stage counters, NULL in production
 };
@@ -836,7 +853,8 @@ struct __align__(8) PrefillBars {
 template <int HD>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
-                         const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
+                         const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kr,
+                         const __grid_constant__ CUtensorMap tm_vr, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ PrefillBars bars;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -913,13 +931,17 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       for (int j = 0; j < nkb; ++j) {
         const int s = j & 1;
         const uint32_t par = ((j >> 1) & 1) ^ 1;  // the ring slot's previous use
-        const int krow = (b * p.G + g) * p.Lcap + j * PF_BK;
+        const bool rows = j < p.nb_rows;
+        const CUtensorMap* mk = rows ? &tm_kr : &tm_k;
+        const CUtensorMap* mv = rows ? &tm_vr : &tm_v;
+        const int kcol = rows ? g * HD : 0;
+        const int krow = rows ? b * p.Lk + j * PF_BK : (b * p.G + g) * p.Lcap + (j - p.nb_rows) * PF_BK;
         if (j >= 2 && !at_wait(&bars.k_empty[s], par, &bars.abort)) break;
         mbar_arrive_expect_tx(&bars.k_full[s], PF_KV);
-        for (int c = 0; c < NCH; ++c) tma_load_2d(sk + s * PF_KV + c * PF_KCHUNK, &tm_k, &bars.k_full[s], c * 64, krow);
+        for (int c = 0; c < NCH; ++c) tma_load_2d(sk + s * PF_KV + c * PF_KCHUNK, mk, &bars.k_full[s], kcol + c * 64, krow);
         if (j >= 2 && !at_wait(&bars.v_empty[s], par, &bars.abort)) break;
         mbar_arrive_expect_tx(&bars.v_full[s], PF_KV);
-        for (int c = 0; c < NCH; ++c) tma_load_2d(sv + s * PF_KV + c * PF_KCHUNK, &tm_v, &bars.v_full[s], c * 64, krow);
+        for (int c = 0; c < NCH; ++c) tma_load_2d(sv + s * PF_KV + c * PF_KCHUNK, mv, &bars.v_full[s], kcol + c * 64, krow);
       }
     }
   } else if (warp == 1) {
@@ -1397,10 +1419,101 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  if (cudaLaunchKernelEx(&cfg, prefill ? (D == 128 ? attention_prefill_kernel<128> : attention_prefill_kernel<256>)
-                                       : push ? attention_kernel<true> : attention_kernel<false>,
-                         tm_q, tm_k, tm_v, p) != cudaSuccess)
+  cudaError_t e;
+  if (prefill)
+    e = cudaLaunchKernelEx(&cfg, D == 128 ? attention_prefill_kernel<128> : attention_prefill_kernel<256>, tm_q, tm_k, tm_v, tm_k, tm_v, p);
+  else
+    e = cudaLaunchKernelEx(&cfg, push ? attention_kernel<true> : attention_kernel<false>, tm_q, tm_k, tm_v, p);
+  if (e != cudaSuccess)
     return host::fail_cuda("launch attention_kernel");
+  host::count_launch();
+  return TYBOK_OK;
+}
+
+int tybok_attention_rows(const void* q, const void* k_rows, const void* v_rows, int n_rows, const void* k_tail, const void* v_tail,
+                         int tail_cap, const void* key_valid, void* out, void* out_planes, int out_shift, int L, int H, int D,
+                         int Lk, float scale, int* status_word, void* stream) {
+  using namespace tb;
+  if (!q || !k_rows || !v_rows || (!out && !out_planes)) return host::fail(TYBOK_ERR_ARG, "attention_rows: null pointer argument");
+  if (D != 128) return host::fail(TYBOK_ERR_ARG, "attention_rows: head_dim must be 128");
+  if (L <= 0 || H <= 0 || n_rows <= 0 || Lk < n_rows || Lk > PF_MAX_KEYS)
+    return host::fail(TYBOK_ERR_ARG, "attention_rows: bad shape (0 < n_rows <= Lk <= 8192)");
+  constexpr int BK = pf_bk(128);
+  const int nb = Lk > n_rows ? n_rows / BK : (n_rows + BK - 1) / BK;  // blocks that lie in the rows
+  if (Lk > n_rows && (!k_tail || !v_tail || tail_cap < Lk - nb * BK))
+    return host::fail(TYBOK_ERR_ARG, "attention_rows: the tail must hold every key from the last whole block of rows on");
+  if ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k_rows) | reinterpret_cast<uintptr_t>(v_rows) |
+       reinterpret_cast<uintptr_t>(k_tail) | reinterpret_cast<uintptr_t>(v_tail) | reinterpret_cast<uintptr_t>(out) |
+       reinterpret_cast<uintptr_t>(out_planes)) & 15)
+    return host::fail(TYBOK_ERR_ARG, "attention_rows: tensors must be 16-byte aligned");
+  if (out_shift < -60 || out_shift > 60) return host::fail(TYBOK_ERR_ARG, "attention_rows: exponent shift out of range");
+  if (int rc = host::require_sm100()) return rc;
+  CUtensorMap tm_q, tm_k, tm_v, tm_kr, tm_vr;
+  const uint64_t hd = static_cast<uint64_t>(H) * D;
+  const CUtensorMapDataType bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  if (int rc = host::tensor_map_2d(&tm_q, q, bf, 2, hd, L, hd * 2, 64, AT_BQ)) return rc;
+  if (int rc = host::tensor_map_2d(&tm_kr, k_rows, bf, 2, hd, n_rows, hd * 2, 64, BK)) return rc;
+  if (int rc = host::tensor_map_2d(&tm_vr, v_rows, bf, 2, hd, n_rows, hd * 2, 64, BK)) return rc;
+  tm_k = tm_kr;
+  tm_v = tm_vr;
+  if (Lk > n_rows) {
+    const uint64_t rows = static_cast<uint64_t>(H) * tail_cap;
+    if (int rc = host::tensor_map_2d(&tm_k, k_tail, bf, 2, D, rows, D * 2, 64, BK)) return rc;
+    if (int rc = host::tensor_map_2d(&tm_v, v_tail, bf, 2, D, rows, D * 2, 64, BK)) return rc;
+  }
+  AttnParams p{};
+  p.B = 1; p.L = L; p.H = H; p.G = H; p.Lk = Lk; p.Lcap = tail_cap; p.nsplit = 1; p.nb_rows = nb;
+  p.scale_log2e = scale * 1.4426950408889634f;
+  p.key_valid = static_cast<const uint8_t*>(key_valid);
+  p.out = static_cast<__nv_bfloat16*>(out); p.out_planes = static_cast<uint8_t*>(out_planes); p.plane_scale = ldexpf(1.0f, out_shift);
+  p.status = status_word; p.pdl = host::pdl_enabled() ? 1 : 0; p.q_rows = AT_BQ; p.dsplit = 1;
+  p.trace = host::trace_buffer(); p.dbg = host::counter_buffer();
+  static bool attr_set[64] = {};
+  const int dev = host::current_device();
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
+    if (cudaFuncSetAttribute(attention_prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem(128)) != cudaSuccess)
+      return host::fail_cuda("cudaFuncSetAttribute(attention_prefill_kernel)");
+    attr_set[dev] = true;
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((L + AT_BQ - 1) / AT_BQ, H, 1);
+  cfg.blockDim = dim3(AT_THREADS);
+  cfg.dynamicSmemBytes = pf_smem(128);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = p.pdl;
+  if (cudaLaunchKernelEx(&cfg, attention_prefill_kernel<128>, tm_q, tm_k, tm_v, tm_kr, tm_vr, p) != cudaSuccess)
+    return host::fail_cuda("launch attention_prefill_kernel");
+  host::count_launch();
+  return TYBOK_OK;
+}
+
+int tybok_kv_rows_to_heads(const void* k_rows, const void* v_rows, int row0, int n, void* k_out, void* v_out, int cap, int H, int D,
+                           void* stream) {
+  using namespace tb;
+  if (!k_rows || !v_rows || !k_out || !v_out) return host::fail(TYBOK_ERR_ARG, "kv_rows_to_heads: null pointer argument");
+  if (row0 < 0 || n <= 0 || n > cap || H <= 0 || D <= 0 || D % 8 != 0) return host::fail(TYBOK_ERR_ARG, "kv_rows_to_heads: bad shape");
+  if ((reinterpret_cast<uintptr_t>(k_rows) | reinterpret_cast<uintptr_t>(v_rows) | reinterpret_cast<uintptr_t>(k_out) |
+       reinterpret_cast<uintptr_t>(v_out)) & 15)
+    return host::fail(TYBOK_ERR_ARG, "kv_rows_to_heads: tensors must be 16-byte aligned");
+  if (int rc = host::require_sm100()) return rc;
+  cudaLaunchConfig_t cfg{};
+  const int total = n * H * (D / 8);
+  cfg.gridDim = dim3(std::min((total + 255) / 256, 4 * host::sm_count()));
+  cfg.blockDim = dim3(256);
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = host::pdl_enabled() ? 1 : 0;
+  if (cudaLaunchKernelEx(&cfg, kv_rows_to_heads_kernel, static_cast<const uint4*>(k_rows), static_cast<const uint4*>(v_rows),
+                         static_cast<uint4*>(k_out), static_cast<uint4*>(v_out), row0, n, H, D / 8, cap, host::pdl_enabled() ? 1 : 0) !=
+      cudaSuccess)
+    return host::fail_cuda("launch kv_rows_to_heads_kernel");
   host::count_launch();
   return TYBOK_OK;
 }

@@ -1,0 +1,85 @@
+// Shared by the sources of the tybok_b200._native extension: the host path from torch tensors to the C ABI without
+// Python or the torch dispatcher in between.  A chain of launches (an FFN, a block, a decoder stack) is one call here.
+#pragma once
+
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/extension.h>
+
+#include <optional>
+#include <string>
+#include <vector>
+
+#include "../../../include/tybok_b200.h"
+
+namespace tbn {
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+// Exponent shifts of the activation planes per producer (planes hold value * 2^shift).
+constexpr int SHIFT_NORMED = 4;  // normalised activations, O(1)
+constexpr int SHIFT_ATTN = 6;    // attention outputs: convex combinations of value rows
+constexpr int SHIFT_FFN = 4;     // FFN intermediates
+constexpr int SHIFT_FOLD = 0;    // residual stream times (1 + scale), not normalised
+// From this many token rows a GEMM fed by a norm takes two e4m3 planes with a per-row scale.
+constexpr int TWO_PLANE_MIN_TOKENS = 128;
+
+[[noreturn]] void raise_status(int rc, const char* what);
+inline void check(int rc, const char* what) {
+  if (rc != 0) raise_status(rc, what);
+}
+[[noreturn]] inline void type_error(const std::string& m) { throw py::type_error(m); }
+[[noreturn]] inline void value_error(const std::string& m) { throw py::value_error(m); }
+void require_cuda(const Tensor& t, const char* what);  // NotImplementedError for anything else
+
+int* status_ptr(int device);  // per-device status word (created once, kept)
+
+inline void* stream_of(const Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.get_device()).stream(); }
+inline void* ptr(const Tensor& t) { return t.data_ptr(); }
+inline void* ptr(const OptTensor& t) { return t ? t->data_ptr() : nullptr; }
+inline const float* f32(const Tensor& t) { return static_cast<const float*>(t.data_ptr()); }
+inline bool is_bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16; }
+
+// [rows, width] view of x with unit inner stride.
+Tensor rows_of(const Tensor& x);
+
+// An e4m3 weight [n, k] with its fp32 scale [n] and optional bf16 bias [n].
+struct W8 {
+  Tensor w, s;
+  OptTensor b;
+  int n = 0, k = 0;
+  const void* wp() const { return w.data_ptr(); }
+  const float* sp() const { return f32(s); }
+  const void* bp() const { return b ? b->data_ptr() : nullptr; }
+};
+W8 w8_of(const py::handle& t, const char* what);  // (weight, scale[, bias])
+
+// One allocation per chain, carved into 256-byte aligned pieces; stream-ordered like any torch allocation.
+class Arena {
+ public:
+  size_t add(size_t bytes) {
+    const size_t at = size_;
+    size_ += (bytes + 255) & ~size_t(255);
+    return at;
+  }
+  void allocate(const Tensor& like) {
+    buf_ = at::empty({static_cast<int64_t>(size_ ? size_ : 1)}, like.options().dtype(at::kByte));
+    base_ = static_cast<char*>(buf_.data_ptr());
+  }
+  void* at(size_t offset) const { return base_ + offset; }
+  const Tensor& tensor() const { return buf_; }
+
+ private:
+  size_t size_ = 0;
+  Tensor buf_;
+  char* base_ = nullptr;
+};
+
+void bind_ops(py::module_& m);
+void bind_dit(py::module_& m);
+void bind_gemma(py::module_& m);
+
+}  // namespace tbn

@@ -25,7 +25,7 @@ struct NormParams {
   long long ldx;
   const float* weight;  // [W] or NULL
   const float* mod;     // [groups, ldmod] or NULL; scale at [0,W), shift at [W,2W)
-  const __nv_bfloat16* ln_scale;  // [W] bf16: LayerNorm + modulate form when set
+  const __nv_bfloat16* ln_scale;  // [W] bf16: LayerNorm + modulate form when set (one row per group at stride ldmod)
   const __nv_bfloat16* ln_shift;  // [W] bf16
   int ln_affine;  // 1: ln_scale / ln_shift are an affine LayerNorm's weight / bias, y = bf16(LN(x) * w + b) in fp32
   long long ldmod;
@@ -128,8 +128,9 @@ __global__ void __launch_bounds__(128) rmsnorm_kernel(const NormParams p) {
         if (p.ln_scale) {
           // modulate(LN(x)) with every step rounded to bf16, as the reference's bf16 tensor ops
           // do: n = bf16(LN), t = bf16(1 + scale), out = bf16(bf16(n * t) + shift).
-          const uint4 rs = *reinterpret_cast<const uint4*>(p.ln_scale + c * 8);
-          const uint4 rh = *reinterpret_cast<const uint4*>(p.ln_shift + c * 8);
+          const long long go = static_cast<long long>(m / p.rows_per_group) * p.ldmod;
+          const uint4 rs = *reinterpret_cast<const uint4*>(p.ln_scale + go + c * 8);
+          const uint4 rh = *reinterpret_cast<const uint4*>(p.ln_shift + go + c * 8);
           const __nv_bfloat16* ps = reinterpret_cast<const __nv_bfloat16*>(&rs);
           const __nv_bfloat16* ph = reinterpret_cast<const __nv_bfloat16*>(&rh);
           if (p.ln_affine) {  // fp32 statistics and fp32 affine, one rounding (wan_base.py:141-148)
@@ -793,6 +794,15 @@ int tybok_layernorm_modulate(const void* x, int64_t ldx, const void* shift, cons
   return tb::launch_norm(x, ldx, nullptr, nullptr, 0, 1, scale, shift, M, W, eps, y, ldy, y_planes, out_shift, stream);
 }
 
+
+int tybok_layernorm_modulate_groups(const void* x, int64_t ldx, const void* shift, const void* scale, int64_t ldmod,
+                                    int rows_per_group, int M, int W, float eps, void* y, int64_t ldy, void* y_planes,
+                                    int out_shift, void* stream) {
+  if (!shift || !scale) return tb::host::fail(TYBOK_ERR_ARG, "layernorm_modulate: null shift/scale");
+  if (((reinterpret_cast<uintptr_t>(shift) | reinterpret_cast<uintptr_t>(scale)) & 15) || ldmod % 8 != 0 || rows_per_group <= 0)
+    return tb::host::fail(TYBOK_ERR_ARG, "layernorm_modulate: shift/scale rows must be 16-byte aligned, rows_per_group positive");
+  return tb::launch_norm(x, ldx, nullptr, nullptr, ldmod, rows_per_group, scale, shift, M, W, eps, y, ldy, y_planes, out_shift, stream);
+}
 
 int tybok_layernorm_affine(const void* x, int64_t ldx, const void* weight, const void* bias, int M, int W, float eps,
                            void* y, int64_t ldy, void* y_planes, int out_shift, void* stream) {

@@ -22,7 +22,7 @@ from __future__ import annotations
 
 import torch
 
-from . import ops
+from . import _lib, ops
 from .shapes import DiTShape
 from .weights import quantize_w8
 
@@ -157,6 +157,11 @@ class DiTBlock:
         self.ffn = DiTFFN(g("ffn.0.weight"), g("ffn.0.bias"), g("ffn.2.weight"), g("ffn.2.bias"), device=device, rank=rank,
                           world=world, group=group, eps=eps, up_scale=params.get("ffn.0.scale_weight"),
                           down_scale=params.get("ffn.2.scale_weight"))
+        # the block's launches as one native call; a sharded FFN keeps its collective, and so its steps, in Python
+        whole = world == 1
+        self._chain = _lib.native().DitBlock(self.heads, self.hd, eps, self.qkv, self.o, self.cross_q, self.cross_o,
+                                             self.ffn.up if whole else None, self.ffn.down if whole else None, self.norm_q,
+                                             self.norm_k, self.cross_norm_q, *self.norm3)
 
     def modulations(self, t_mod: torch.Tensor) -> torch.Tensor:
         """``modulation + t_mod`` -> six contiguous bf16 rows ``[6, H]``: shift / scale / gate of the
@@ -190,29 +195,24 @@ class DiTBlock:
         ``(K, V)`` ``[1, heads, Lcap, D]`` whose first ``key_off`` rows hold earlier keys / values
         (this block's own are appended there); ``cross_cache`` from ``context_cache`` with
         ``ctx_valid`` uint8 ``[1, C]`` (``None`` skips the cross-attention, dit_block.py:385-390)."""
-        s = x.shape[0]
-        a, hd = self.attn_dim, self.hd
-        hp, rs = _ln_planes(x, mods[0], mods[1], self.eps)
-        qkv, _ = _gemm(hp, rs, *self.qkv)
-        q = ops.qknorm_rope_store(qkv, q_off=0, k_off=a, v_off=2 * a, norm_q=self.norm_q, norm_k=self.norm_k, eps=self.eps,
-                                  cos=cos, sin=sin, k_cache=self_cache[0], v_cache=self_cache[1], heads=self.heads,
-                                  head_dim=hd, key_off=key_off)
-        _, ap = ops.attention(q, self_cache[0], self_cache[1], None, tokens=s, keys=key_off + s, scale=hd**-0.5,
-                              out_bf16=False, out_planes=True, out_shift=SHIFT_ATTN)
-        x, _ = ops.w8x3_linear(ap, SHIFT_ATTN, *self.o, epilogue=ops.EPI_RESIDUAL, residual=x, gate=mods[2:3],
-                               rows_per_gate=s)
-        if cross_cache is not None:
-            if s >= TWO_PLANE_MIN_TOKENS:
-                cp, rs = ops.norm_planes2(x, ops.NORM_LN_AFFINE, *self.norm3, eps=self.eps)
-            else:
-                cp, rs = ops.layernorm_affine(x, *self.norm3, eps=self.eps, out_shift=SHIFT_IN)[1], None
-            qc, _ = _gemm(cp, rs, *self.cross_q)
-            qc = ops.qknorm_rope_store(qc, q_off=0, norm_q=self.cross_norm_q, eps=self.eps, heads=self.heads, head_dim=hd)
-            lc = ctx_valid.shape[1] if ctx_valid is not None else cross_cache[0].shape[2]
-            _, cap = ops.attention(qc, cross_cache[0], cross_cache[1], ctx_valid, tokens=s, keys=lc, scale=hd**-0.5,
-                                   out_bf16=False, out_planes=True, out_shift=SHIFT_ATTN)
-            x, _ = ops.w8x3_linear(cap, SHIFT_ATTN, *self.cross_o, epilogue=ops.EPI_RESIDUAL, residual=x)
-        return self.ffn(x, mods[3], mods[4], mods[5])
+        return self._forward(x, mods, cos, sin, *self_cache, key_off, None, None, *(cross_cache or (None, None)), ctx_valid)
+
+    def _forward(self, x, mods, cos, sin, k_cache, v_cache, key_off, k_rows, v_rows, cross_k, cross_v, ctx_valid):
+        """The native chain; earlier keys / values either in the caches or as token-major rows
+        ``[L, heads*D]`` read in place (``k_cache`` / ``v_cache`` are then the tail, see ``tybok_attention_rows``)."""
+        y = self._chain.forward(x, mods, cos, sin, k_cache, v_cache, key_off, k_rows, v_rows, cross_k, cross_v,
+                                ctx_valid if cross_k is not None else None)
+        return y if self.ffn.world == 1 else self.ffn(y, mods[3], mods[4], mods[5])
+
+
+def _token_rows(t: torch.Tensor, width: int) -> torch.Tensor:
+    """``[1, L, width]`` (or ``[L, width]``) keys or values as contiguous bf16 rows ``[L, width]``; a view whenever the
+    caller's tensor already is that."""
+    if t.dtype != torch.bfloat16 or not t.is_contiguous():
+        t = t.to(torch.bfloat16).contiguous()
+    if t.data_ptr() & 15:
+        t = t.clone()
+    return t.view(-1, width)
 
 
 def rotary_parts(freqs: torch.Tensor, device) -> tuple[torch.Tensor, torch.Tensor]:
@@ -248,18 +248,31 @@ class DiTDenoiser:
     def step(self, x: torch.Tensor, t_mod: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
         """All blocks on ``x [S, H]`` for one modulation table ``t_mod [6, H]``.  Every block's own
         keys / values are consumed inside the block, so one cache pair serves the whole stack."""
+        return self._stack(x, self._all_modulations(t_mod[None])[0], cos, sin)
+
+    def _all_modulations(self, t_mods: torch.Tensor) -> torch.Tensor:
+        """``modulation + t_mod`` of every step and block in one launch: bf16 ``[steps, blocks, 6, H]``."""
+        table = torch.stack([blk.modulation for blk in self.blocks])
+        return table[None] + t_mods.reshape(t_mods.shape[0], 1, 6, -1).to(torch.bfloat16)
+
+    def _stack(self, x: torch.Tensor, mods: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
         cache = self._cache(x.shape[0])
         for i, blk in enumerate(self.blocks):
-            x = blk.forward(x, blk.modulations(t_mod), cos, sin, cache, 0, None if self._cross is None else self._cross[i],
-                            self._ctx_valid)
+            x = blk.forward(x, mods[i], cos, sin, cache, 0, None if self._cross is None else self._cross[i], self._ctx_valid)
         return x
 
     @torch.no_grad()
     def denoise(self, x: torch.Tensor, t_mods: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, deltas) -> torch.Tensor:
         """``len(deltas)`` denoise steps over token space: ``x <- x + stack(x, t_mods[s]) * delta_s``
         in bf16 (the scheduler's update, tybok/policies/fastwam/models/fastwam.py:68-73)."""
+        if not self.blocks or len(deltas) == 0:
+            for delta in deltas:  # an empty stack is the identity
+                x = x + x * float(torch.tensor(float(delta), dtype=x.dtype))
+            return x
+        mods = self._all_modulations(torch.stack([t_mods[s].reshape(6, -1) for s in range(len(deltas))]))
         for s, delta in enumerate(deltas):
-            x = x + self.step(x, t_mods[s], cos, sin) * torch.tensor(float(delta), dtype=x.dtype, device=x.device)
+            # the step size in the stream's own precision, as a host scalar: no copy to the device, no wait for it
+            x = x + self._stack(x, mods[s], cos, sin) * float(torch.tensor(float(delta), dtype=x.dtype))
         return x
 
     @torch.no_grad()
@@ -269,7 +282,8 @@ class DiTDenoiser:
         ``t_mod [1, 6, H]``, ``freqs`` complex ``[M, 1, d/2]``, per layer ``video_kv[i] = {"k", "v"}``
         ``[1, L_video, heads*D]`` (keys / values every action token also attends to) and
         ``cross_kv[i] = (k, v)`` ``[1, C, heads*D]`` with qk-norm applied, ``context_mask`` bool ``[C]``
-        -> ``[1, M, H]``.  The caller's tensors are copied once per call into head-major caches."""
+        -> ``[1, M, H]``.  The caller's keys and values are read where they lie (head_dim 128); only the rows of a
+        last partial block of 128 keys are copied, in front of the layer's own."""
         n = len(self.blocks)
         if len(video_kv) != n or len(cross_kv) != n:
             raise ValueError(f"video/cross KV layer counts {len(video_kv)}/{len(cross_kv)} != {n}")
@@ -281,11 +295,20 @@ class DiTDenoiser:
         m = x.shape[0]
         cos, sin = rotary_parts(freqs, self.device)
         valid = context_mask.reshape(1, -1).to(self.device, torch.uint8).contiguous()
+        mods = self._all_modulations(t_mod.reshape(1, 6, -1))[0]
+        tail = None
         for i, blk in enumerate(self.blocks):
-            lv = video_kv[i]["k"].shape[-2]
-            kc, vc = blk.store_context_kv(video_kv[i]["k"], video_kv[i]["v"])  # [1, heads, Lv, D]
-            pad = torch.zeros(1, blk.heads, m, blk.hd, dtype=torch.bfloat16, device=self.device)
-            cache = (torch.cat([kc, pad], dim=2).contiguous(), torch.cat([vc, pad], dim=2).contiguous())
-            cross = blk.store_context_kv(*cross_kv[i])
-            x = blk.forward(x, blk.modulations(t_mod), cos, sin, cache, lv, cross, valid)
+            vk, vv = video_kv[i]["k"], video_kv[i]["v"]
+            lv = vk.shape[-2]
+            if blk.hd != 128 or lv == 0:  # one head-major copy
+                kc, vc = blk.store_context_kv(vk, vv)  # [1, heads, Lv, D]
+                pad = torch.zeros(1, blk.heads, m, blk.hd, dtype=torch.bfloat16, device=self.device)
+                cache = (torch.cat([kc, pad], dim=2).contiguous(), torch.cat([vc, pad], dim=2).contiguous())
+                x = blk.forward(x, mods[i], cos, sin, cache, lv, blk.store_context_kv(*cross_kv[i]), valid)
+                continue
+            if tail is None:  # zeroed once: whatever lies past a layer's own keys stays finite
+                cap = (127 + m + 127) // 128 * 128
+                tail = torch.zeros(2, blk.heads, cap, blk.hd, dtype=torch.bfloat16, device=self.device)
+            rows = lambda t, a=blk.attn_dim: _token_rows(t, a)  # noqa: E731
+            x = blk._forward(x, mods[i], cos, sin, tail[0], tail[1], 0, rows(vk), rows(vv), rows(cross_kv[i][0]), rows(cross_kv[i][1]), valid)
         return x[None]

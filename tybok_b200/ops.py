@@ -79,21 +79,13 @@ _L.define("w8x3_qkv_rope_adarms(Tensor u_planes, int shift, Tensor ss_part, floa
 NORM_RMS, NORM_ADARMS, NORM_LN_MODULATE, NORM_LN_AFFINE = 0, 1, 2, 3
 EPI_GEGLU_PACKED = 4
 
-_status: dict[int, torch.Tensor] = {}
-
-
 def _dev_index(device: torch.device) -> int:
     return device.index if device.index is not None else torch.cuda.current_device()
 
 
 def status_word(device: torch.device) -> torch.Tensor:
     """Per-device int32 that kernels set when one of their bounded waits runs out."""
-    idx = _dev_index(device)
-    word = _status.get(idx)
-    if word is None:
-        word = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", idx))
-        _status[idx] = word
-    return word
+    return _lib.native().status_word(_dev_index(device))
 
 
 def check_status(device: torch.device | None = None) -> None:
@@ -249,24 +241,7 @@ def _rope_store_cuda(qkv, pos, cos, sin, k_cache, v_cache, heads, key_off):
 
 
 def _attention_cuda(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift):
-    lib = _lib.load()
-    b, g, lcap, d = k_cache.shape
-    if q.dtype != torch.bfloat16 or q.dim() != 2 or not q.is_contiguous() or q.shape[0] != b * tokens:
-        raise TypeError("attention: q must be contiguous bf16 [B*L, H*D]")
-    h = q.shape[1] // d
-    if key_valid is not None and (key_valid.dtype != torch.uint8 or key_valid.shape != (b, keys)
-                                  or not key_valid.is_contiguous()):
-        raise TypeError("attention: key_valid must be contiguous uint8 [B, Lk]")
-    y, yp = _outputs(b * tokens, h * d, q.device, out_bf16, out_planes)
-    # head_dim 128 always takes the key-loop kernel, which exchanges nothing
-    need = 0 if d == 128 else int(lib.tybok_attention_workspace_bytes(b, int(tokens), h, int(keys)))
-    ws = torch.empty(need, dtype=torch.uint8, device=q.device) if need else None
-    rc = lib.tybok_attention(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), _ptr(key_valid),
-                             y.data_ptr() if out_bf16 else None, yp.data_ptr() if out_planes else None, int(out_shift),
-                             b, int(tokens), h, g, d, int(keys), lcap, float(scale), _ptr(ws), need,
-                             status_word(q.device).data_ptr(), _stream(q))
-    _lib.check(rc, "tybok_attention")
-    return y, yp
+    return _lib.native().attention(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
 
 
 def _layernorm_modulate_cuda(x, shift, scale, eps, out_bf16, out_planes, out_shift):
@@ -535,10 +510,8 @@ def w8x3_geglu_packed(planes, shift, w8_packed, scale_packed, *, out_bf16=True, 
 
 def w8a16_linear(x, w8, scale, bias=None, *, epilogue=EPI_NONE, residual=None, gate=None, rows_per_gate=1,
                  token_tile=0, splits=0, shift=DEFAULT_SHIFT) -> torch.Tensor:
-    """``epilogue(x @ (w8*scale).T + bias)`` for bf16 ``x``: ``split3`` then ``w8x3_linear``."""
-    y, _ = w8x3_linear(split3(x, shift), shift, w8, scale, bias, epilogue=epilogue, residual=residual, gate=gate,
-                       rows_per_gate=rows_per_gate, token_tile=token_tile, splits=splits)
-    return y.reshape(*x.shape[:-1], w8.shape[0])
+    """``epilogue(x @ (w8*scale).T + bias)`` for bf16 ``x``: ``split3`` then ``w8x3_linear``, as one native call."""
+    return _lib.native().w8a16_linear(x, w8, scale, bias, epilogue, residual, gate, rows_per_gate, token_tile, splits, shift)
 
 
 def w8a16_geglu(x, w8_gate, scale_gate, w8_up, scale_up, *, token_tile=0, splits=0, shift=DEFAULT_SHIFT):
@@ -565,8 +538,7 @@ def attention(q, k_cache, v_cache, key_valid=None, *, tokens, keys, scale, out_b
               out_shift=DEFAULT_SHIFT):
     """GQA attention over the first ``keys`` cache rows; returns ``(out_bf16, out_planes)``; see
     ``tybok_attention``."""
-    return torch.ops.tybok_b200.attention(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes,
-                                          out_shift)
+    return _lib.native().attention(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
 
 
 def layernorm_modulate(x, shift, scale, *, eps=1e-6, out_bf16=False, out_planes=True, out_shift=DEFAULT_SHIFT):

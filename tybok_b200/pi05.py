@@ -23,19 +23,13 @@ import math
 import torch
 import torch.nn.functional as F  # noqa: N812
 
-from . import ops
+from . import _lib, ops
 from .shapes import GemmaSpec, PI05Shape
 from .weights import EXPERT, PROJECTOR, VISION, VLM, quantize_w8
 
-#: Exponent shifts of the activation planes per producer (planes hold value * 2**shift and are
-#: exact for |value * 2**shift| in [2**-7, 57344]).
-SHIFT_NORMED = 4  # RMS-normalised activations, O(1)
-SHIFT_ATTN = 6  # attention outputs (convex combinations of V rows)
-SHIFT_FFN = 4  # gelu(gate) * up
-SHIFT_FOLD = 0  # residual stream times (1 + scale), not normalised: exact from 2^-7 to 57344
 #: From this many token rows a GEMM fed by a norm takes its activations as two e4m3 planes with a
 #: per-row power-of-two scale (a third less tensor work, token tiles to 128); below it the GEMMs are
-#: bound by launch latency and keep the three-plane form.
+#: bound by launch latency and keep the three-plane form.  (The rule itself is in csrc/host/native.h.)
 TWO_PLANE_MIN_TOKENS = 128
 
 
@@ -132,6 +126,9 @@ class PI05Model:
         self.embed_scale = torch.tensor(shape.vlm.width**0.5, dtype=self.embed.dtype, device=dev)
         self.vlm_layers = _pack_decoder(params, VLM, shape.vlm, False, dev)
         self.exp_layers = _pack_decoder(params, EXPERT, shape.expert, True, dev)
+        # each decoder stack as one native call: its launches follow one another without Python in between
+        self._vlm = self._stack(shape.vlm, self.vlm_layers, adarms=False)
+        self._expert = self._stack(shape.expert, self.exp_layers, adarms=True)
         self.final_norm = (params[f"{EXPERT}.norm.dense.weight"].to(dev).float(),
                            params[f"{EXPERT}.norm.dense.bias"].to(dev).float())
         f32 = lambda n: params[n].to(dev).float()  # noqa: E731
@@ -140,8 +137,17 @@ class PI05Model:
         self.time_in = (f32("time_mlp_in.weight"), f32("time_mlp_in.bias"))
         self.time_out = (f32("time_mlp_out.weight"), f32("time_mlp_out.bias"))
         self.cos, self.sin = _rope_table(shape.vlm.head_dim, shape.prefix_len + shape.chunk + 8, dev)
-        self._cache_by_batch: dict[int, list] = {}
+        self._cache_by_batch: dict[int, tuple] = {}
         self._precompute_step_constants()
+
+    @staticmethod
+    def _stack(spec: GemmaSpec, layers: list[_Layer], adarms: bool):
+        rows = []
+        for lay in layers:
+            gate_up, up = (lay.gate_up, None) if lay.gate_up is not None else (lay.gate, lay.up)
+            norms = (None, None) if adarms else (lay.norm_in, lay.norm_post)
+            rows.append((lay.qkv_paired, lay.o, gate_up, up, lay.down, *norms))
+        return _lib.native().GemmaStack(spec.width, spec.num_heads, spec.num_kv_heads, spec.head_dim, rows)
 
     # ------------------------------------------------------------------ constants
     def _adarms_cond(self, times: torch.Tensor) -> torch.Tensor:
@@ -300,122 +306,39 @@ class PI05Model:
 
     # ------------------------------------------------------------------ decoder pieces
     def _caches(self, b: int):
-        """Per-layer K/V caches ``[B, G, prefix_len + chunk, D]`` (zero-initialised once per batch
+        """Per-layer K and V caches ``[B, G, prefix_len + chunk, D]``, as two lists (zero-initialised once per batch
         size): the prefill writes keys [0, Lp), every expert layer-step rewrites [Lp, Lp + L)."""
         c = self._cache_by_batch.get(b)
         if c is None:
             s = self.shape
             lcap = s.prefix_len + s.chunk
-            mk = lambda: torch.zeros(b, s.vlm.num_kv_heads, lcap, s.vlm.head_dim, dtype=torch.bfloat16,  # noqa: E731
-                                     device=self.device)
-            c = [(mk(), mk()) for _ in range(s.vlm.depth)]
+            mk = lambda: [torch.zeros(b, s.vlm.num_kv_heads, lcap, s.vlm.head_dim, dtype=torch.bfloat16, device=self.device)  # noqa: E731
+                          for _ in range(s.vlm.depth)]
+            c = (mk(), mk())
             self._cache_by_batch[b] = c
         return c
 
-    def _layer(self, spec, lay: _Layer, x, b, l, pos, cache, key_off, key_valid, mods):
-        """One decoder layer on ``x [B*L, W]`` bf16 (layers.py:268-308). ``mods`` is None for the
-        VLM (plain norms) or ``(mod_in, mod_post)`` ``[1, 3W]`` AdaRMS modulations.  ``cache`` is
-        this layer's ``(K, V)`` cache; the layer appends its keys at ``key_off``."""
-        w = spec.width
-        m = x.shape[0]
-        two = m >= TWO_PLANE_MIN_TOKENS and lay.gate_up is not None
-        gate_in = gate_post = None
-        if mods is not None:
-            gate_in, gate_post = mods[0][:, 2 * w :], mods[1][:, 2 * w :]
-
-        def norm(which):
-            """This layer's input (0) or post-attention (1) norm -> the activation form the next GEMM takes."""
-            if two:
-                if mods is None:
-                    return ops.norm_planes2(x, ops.NORM_RMS, lay.norm_in if which == 0 else lay.norm_post)
-                return ops.norm_planes2(x, ops.NORM_ADARMS, mods[which], rows_per_group=m)
-            if mods is None:
-                return ops.rmsnorm(x, weight=lay.norm_in if which == 0 else lay.norm_post, out_shift=SHIFT_NORMED)[1], None
-            return ops.rmsnorm(x, mod=mods[which], rows_per_group=m, out_shift=SHIFT_NORMED)[1], None
-
-        xp, rs = norm(0)
-        if two:
-            q = ops.w8x2_qkv_rope(xp, rs, *lay.qkv_paired, pos, self.cos, self.sin, cache[0], cache[1],
-                                  heads=spec.num_heads, key_off=key_off)
-        else:
-            q = ops.w8x3_qkv_rope(xp, SHIFT_NORMED, *lay.qkv_paired, pos, self.cos, self.sin, cache[0], cache[1],
-                                  heads=spec.num_heads, key_off=key_off)
-        _, ap = ops.attention(q, cache[0], cache[1], key_valid, tokens=l, keys=key_off + l,
-                              scale=spec.head_dim**-0.5, out_bf16=False, out_planes=True, out_shift=SHIFT_ATTN)
-        x, _ = ops.w8x3_linear(ap, SHIFT_ATTN, *lay.o, epilogue=ops.EPI_RESIDUAL, residual=x, gate=gate_in,
-                               rows_per_gate=m)
-        xp, rs = norm(1)
-        if two:
-            _, hp = ops.w8x2_gemm(xp, rs, *lay.gate_up, epilogue=ops.EPI_GEGLU_PACKED, out_bf16=False, out_planes=True,
-                                  out_shift=SHIFT_FFN)
-        elif lay.gate_up is not None:
-            _, hp = ops.w8x3_geglu_packed(xp, SHIFT_NORMED, *lay.gate_up, out_bf16=False, out_planes=True,
-                                          out_shift=SHIFT_FFN)
-        else:
-            _, hp = ops.w8x3_geglu(xp, SHIFT_NORMED, *lay.gate, *lay.up, out_bf16=False, out_planes=True,
-                                   out_shift=SHIFT_FFN)
-        x, _ = ops.w8x3_linear(hp, SHIFT_FFN, *lay.down, epilogue=ops.EPI_RESIDUAL, residual=x, gate=gate_post,
-                               rows_per_gate=m)
-        return x
-
-    def _expert_pass(self, mods, fold, x, b, l, pos, caches, key_off, key_valid, wait=None):
-        """All expert layers of one denoise step on the suffix embedding ``x [B*L, W]``; ``wait(i)`` runs
-        before layer ``i``.  Below the two-plane threshold, and with the step's ``W shift`` constants at
-        hand (``fold``), only the first norm of the pass is a kernel: every later AdaRMS norm is folded
-        into the GEMM that writes its input (sums of squares, planes of ``x (1 + scale)``) and the GEMM
+    def _expert_pass(self, mods, fold, x, b, l, pos, caches, key_off, key_valid, wait=()):
+        """All expert layers of one denoise step on the suffix embedding ``x [B*L, W]`` (layers.py:268-308);
+        ``wait``: one recorded CUDA event per layer that the layer must come after.  Below the two-plane threshold, and with
+        the step's ``W shift`` constants at hand (``fold``), only the first norm of the pass is a kernel: every later AdaRMS
+        norm is folded into the GEMM that writes its input (sums of squares, planes of ``x (1 + scale)``) and the GEMM
         that reads its output (rstd and ``W shift`` in the epilogue)."""
-        spec = self.shape.expert
-        m, w = x.shape[0], spec.width
-        if fold is None or m >= TWO_PLANE_MIN_TOKENS:
-            for i, lay in enumerate(self.exp_layers):
-                if wait is not None:
-                    wait(i)
-                x = self._layer(spec, lay, x, b, l, pos, caches[i], key_off, key_valid, mods[i])
-            return x
-        carry = None  # (u_planes, ss_part) of the residual stream, written by the previous layer's down projection
-        last = len(self.exp_layers) - 1
-        for i, lay in enumerate(self.exp_layers):
-            if wait is not None:
-                wait(i)
-            mod_in, mod_post = mods[i]
-            cache = caches[i]
-            if carry is None:
-                xp = ops.rmsnorm(x, mod=mod_in, rows_per_group=m, out_shift=SHIFT_NORMED)[1]
-                q = ops.w8x3_qkv_rope(xp, SHIFT_NORMED, *lay.qkv_paired, pos, self.cos, self.sin, cache[0], cache[1],
-                                      heads=spec.num_heads, key_off=key_off)
-            else:
-                q = ops.w8x3_qkv_rope_adarms(carry[0], SHIFT_FOLD, carry[1], fold[i][0], *lay.qkv_paired, pos, self.cos,
-                                             self.sin, cache[0], cache[1], heads=spec.num_heads, key_off=key_off)
-            _, ap = ops.attention(q, cache[0], cache[1], key_valid, tokens=l, keys=key_off + l,
-                                  scale=spec.head_dim**-0.5, out_bf16=False, out_planes=True, out_shift=SHIFT_ATTN)
-            x, up, part = ops.w8x3_residual_next_adarms(ap, SHIFT_ATTN, *lay.o, x, mod_in[0, 2 * w :], mod_post[0, :w],
-                                                        out_shift=SHIFT_FOLD)
-            _, hp = ops.w8x3_geglu_packed_adarms(up, SHIFT_FOLD, part, fold[i][1], *lay.gate_up, out_bf16=False,
-                                                 out_planes=True, out_shift=SHIFT_FFN)
-            if i == last:
-                x, _ = ops.w8x3_linear(hp, SHIFT_FFN, *lay.down, epilogue=ops.EPI_RESIDUAL, residual=x,
-                                       gate=mod_post[:, 2 * w :], rows_per_gate=m)
-            else:
-                x, up, part = ops.w8x3_residual_next_adarms(hp, SHIFT_FFN, *lay.down, x, mod_post[0, 2 * w :],
-                                                            mods[i + 1][0][0, :w], out_shift=SHIFT_FOLD)
-                carry = (up, part)
-        return x
+        return self._expert.forward(x, b, l, pos, self.cos, self.sin, *caches, key_off, key_valid, mods, fold, 0,
+                                    len(self.exp_layers), [ev.cuda_event for ev in wait], [])
 
     # ------------------------------------------------------------------ prefix + denoise
-    def prefill(self, prefix_embs: torch.Tensor, pad: torch.Tensor, layer_done=None):
+    def prefill(self, prefix_embs: torch.Tensor, pad: torch.Tensor, layer_done=()):
         """VLM prefix pass filling the per-layer post-RoPE (K, V) caches (gemma.py:61-125,
-        use_cache); returns views ``[B, G, Lp, D]`` of the prefix part of every layer's cache."""
-        spec = self.shape.vlm
+        use_cache); returns views ``[B, G, Lp, D]`` of the prefix part of every layer's cache.
+        ``layer_done``: one CUDA event per layer, recorded after it."""
         b, l, w = prefix_embs.shape
-        caches = self._caches(b)
+        kc, vc = self._caches(b)
         pos = (torch.cumsum(pad, dim=1) - 1).clamp_min(0).to(torch.int32).reshape(-1)
         key_valid = pad.to(torch.uint8).contiguous()
-        x = prefix_embs.reshape(b * l, w)
-        for lay, cache in zip(self.vlm_layers, caches):
-            x = self._layer(spec, lay, x, b, l, pos, cache, 0, key_valid, None)
-            if layer_done is not None:
-                layer_done()
-        return [(kc[:, :, :l], vc[:, :, :l]) for kc, vc in caches]
+        self._vlm.forward(prefix_embs.reshape(b * l, w), b, l, pos, self.cos, self.sin, kc, vc, 0, key_valid, None, None, 0,
+                          len(self.vlm_layers), [], [ev.cuda_event for ev in layer_done])
+        return [(k[:, :, :l], v[:, :, :l]) for k, v in zip(kc, vc)]
 
     @torch.no_grad()
     def velocity_at(self, t: float, x_t: torch.Tensor, pad: torch.Tensor) -> torch.Tensor:
@@ -502,17 +425,13 @@ class PI05Model:
         with torch.cuda.stream(side):
             side.wait_event(fork)
             h = ops.action_tail(None, None, None, None, x_t, dt, *self.action_in)
-        done = []
-
-        def layer_done():
-            ev = torch.cuda.Event()
-            ev.record(main)
-            done.append(ev)
-
-        self.prefill(embs, pad, layer_done)
+        done = [torch.cuda.Event() for _ in self.vlm_layers]
+        for ev in done:
+            ev.record(main)  # creates the event; the prefix records it again after its layer
+        self.prefill(embs, pad, done)
         with torch.cuda.stream(side):
             x = self._expert_pass(self.mods[0], self.fold[0] if self.fold is not None else None, h, b, l, pos, caches,
-                                  lp, key_valid, wait=lambda i: side.wait_event(done[i]))
+                                  lp, key_valid, wait=done)
             h = ops.action_tail(x, self.final_mods[0], *self.action_out, x_t, dt, *self.action_in,
                                 rows_per_group=b * l, embed=s.steps > 1)
             join = torch.cuda.Event()
