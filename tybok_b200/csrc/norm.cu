@@ -42,7 +42,7 @@ struct NormParams {
   int* dbg;  // debugging aid: stage counters, NULL in production
 };
 
-// VEC = 8-element vectors per lane; FULL = every lane owns exactly VEC vectors (W == 256 * VEC),
+// Rows of at most 256 elements, one warp each.  VEC = 8-element vectors per lane; FULL = every lane owns exactly VEC vectors (W == 256 * VEC),
 // which removes the bounds predicates so that the loads can be hoisted and overlapped.
 template <int VEC, bool FULL>
 __global__ void __launch_bounds__(128) rmsnorm_kernel(const NormParams p) {
@@ -316,6 +316,135 @@ __global__ void __launch_bounds__(512) rmsnorm_row_kernel(const NormParams p) {
       uint8_t* dst = p.planes2 + static_cast<long long>(m) * p.W + c * 8;
       *reinterpret_cast<uint2*>(dst) = w1;
       *reinterpret_cast<uint2*>(dst + static_cast<long long>(p.M) * p.W) = w2;
+    }
+  }
+}
+
+// The LayerNorm forms (modulate and affine) with one CTA per row, eight elements per thread.  Bound by latency: a
+// 3072-wide row took the warp-per-row form about 20 us whatever the row count (twelve dependent trips for the two
+// vectors after two chains over the whole row; 27 CTAs for 106 rows), three times per DiT block.  Here every load of the
+// row is in flight at once and only the two sums run on one warp, in the order of the warp-per-row form (lane l adds
+// vectors l, l + 32, ... one element after the other), so results are the same bit for bit: 106 rows 20 -> 4 us,
+// 4146 rows 58 -> 32 us.
+__global__ void __launch_bounds__(512) layernorm_row_kernel(const NormParams p) {
+  __shared__ uint4 row_sh[512];
+  __shared__ float stat[2];
+  __shared__ float red_max[16];
+  if (p.pdl) pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int m = blockIdx.x, c = threadIdx.x, nvec = p.W / 8;
+  const bool live = c < nvec;
+  if (p.pdl) pdl_wait();
+  uint4 raw = make_uint4(0, 0, 0, 0), rs = raw, rh = raw;
+  if (live) {
+    const long long go = static_cast<long long>(m / p.rows_per_group) * p.ldmod;
+    raw = *reinterpret_cast<const uint4*>(p.x + m * p.ldx + c * 8);
+    rs = *reinterpret_cast<const uint4*>(p.ln_scale + go + c * 8);
+    rh = *reinterpret_cast<const uint4*>(p.ln_shift + go + c * 8);
+    row_sh[c] = raw;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    float sm = 0.f;
+#pragma unroll 4
+    for (int i = lane; i < nvec; i += 32) {
+      const uint4 r = row_sh[i];
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        sm += __bfloat162float(h[e].x);
+        sm += __bfloat162float(h[e].y);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
+    const float mean = sm / static_cast<float>(p.W);
+    float ss = 0.f;
+#pragma unroll 4
+    for (int i = lane; i < nvec; i += 32) {
+      const uint4 r = row_sh[i];
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&r);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float a = __bfloat162float(h[e].x) - mean, b = __bfloat162float(h[e].y) - mean;
+        ss = fmaf(a, a, ss);
+        ss = fmaf(b, b, ss);
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if (lane == 0) {
+      stat[0] = mean;
+      stat[1] = rsqrtf(ss / static_cast<float>(p.W) + p.eps);
+    }
+  }
+  __syncthreads();
+  const float mean = stat[0], rstd = stat[1];
+  const long long plane = static_cast<long long>(p.M) * p.W;
+  __nv_bfloat162 b[4];
+  float v[8];
+  float amax = 0.f;
+  if (live) {
+    const __nv_bfloat16* px = reinterpret_cast<const __nv_bfloat16*>(&raw);
+    const __nv_bfloat16* ps = reinterpret_cast<const __nv_bfloat16*>(&rs);
+    const __nv_bfloat16* ph = reinterpret_cast<const __nv_bfloat16*>(&rh);
+    float o[8];
+    if (p.ln_affine) {  // fp32 statistics and fp32 affine, one rounding (wan_base.py:141-148)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) o[e] = (__bfloat162float(px[e]) - mean) * rstd * __bfloat162float(ps[e]) + __bfloat162float(ph[e]);
+    } else {
+      // modulate(LN(x)) with every step rounded to bf16, as the reference's bf16 tensor ops
+      // do: n = bf16(LN), t = bf16(1 + scale), out = bf16(bf16(n * t) + shift).
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float nrm = bf16_round((__bfloat162float(px[e]) - mean) * rstd);
+        const float t = bf16_round(1.0f + __bfloat162float(ps[e]));
+        o[e] = bf16_round(nrm * t) + __bfloat162float(ph[e]);
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      b[e] = __floats2bfloat162_rn(o[2 * e], o[2 * e + 1]);
+      v[2 * e] = __bfloat162float(b[e].x);
+      v[2 * e + 1] = __bfloat162float(b[e].y);
+      amax = fmaxf(amax, fmaxf(fabsf(v[2 * e]), fabsf(v[2 * e + 1])));
+    }
+    if (p.y) *reinterpret_cast<uint4*>(p.y + m * p.ldy + c * 8) = *reinterpret_cast<const uint4*>(b);
+    if (p.planes) {
+      float lo[4], hi[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        lo[e] = v[e] * p.plane_scale;
+        hi[e] = v[4 + e] * p.plane_scale;
+      }
+      uint2 w1, w2, w3;
+      split3_quad(lo, w1.x, w2.x, w3.x);
+      split3_quad(hi, w1.y, w2.y, w3.y);
+      uint8_t* dst = p.planes + static_cast<long long>(m) * p.W + c * 8;
+      *reinterpret_cast<uint2*>(dst) = w1;
+      *reinterpret_cast<uint2*>(dst + plane) = w2;
+      *reinterpret_cast<uint2*>(dst + 2 * plane) = w3;
+    }
+  }
+  if (p.planes2) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    if (lane == 0) red_max[warp] = amax;
+    __syncthreads();
+    amax = 0.f;
+    for (int w = 0; w < nwarps; ++w) amax = fmaxf(amax, red_max[w]);
+    float up, down;
+    row_pow2(amax, up, down);
+    if (threadIdx.x == 0) p.row_scale[m] = down;
+    if (live) {
+      const float lo[4] = {v[0] * up, v[1] * up, v[2] * up, v[3] * up};
+      const float hi[4] = {v[4] * up, v[5] * up, v[6] * up, v[7] * up};
+      uint2 w1, w2;
+      split2_quad(lo, w1.x, w2.x);
+      split2_quad(hi, w1.y, w2.y);
+      uint8_t* dst = p.planes2 + static_cast<long long>(m) * p.W + c * 8;
+      *reinterpret_cast<uint2*>(dst) = w1;
+      *reinterpret_cast<uint2*>(dst + plane) = w2;
     }
   }
 }
@@ -670,21 +799,13 @@ static int launch_norm(const void* x, int64_t ldx, const float* weight, const fl
   cfg.attrs = attr;
   cfg.numAttrs = p.pdl;
   const int per_lane = (W / 8 + 31) / 32;
-  const bool full = W % 256 == 0 && W / 256 == per_lane && (per_lane & (per_lane - 1)) == 0;
   cudaError_t e;
-  if (!ln_scale && per_lane >= 2) {  // one CTA per row
+  if (per_lane >= 2) {  // more than 256 elements: one CTA per row
     cfg.gridDim = dim3(M);
     cfg.blockDim = dim3(per_lane * 32);
-    e = cudaLaunchKernelEx(&cfg, rmsnorm_row_kernel, p);
-  } else if (full && per_lane == 4) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<4, true>, p);
-  else if (full && per_lane == 8) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<8, true>, p);
-  else if (full && per_lane == 1) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<1, true>, p);
-  else if (full && per_lane == 2) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<2, true>, p);
-  else if (per_lane <= 1) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<1, false>, p);
-  else if (per_lane <= 2) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<2, false>, p);
-  else if (per_lane <= 4) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<4, false>, p);
-  else if (per_lane <= 8) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<8, false>, p);
-  else e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<NORM_MAX_VEC, false>, p);
+    e = ln_scale ? cudaLaunchKernelEx(&cfg, layernorm_row_kernel, p) : cudaLaunchKernelEx(&cfg, rmsnorm_row_kernel, p);
+  } else if (W == 256) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<1, true>, p);
+  else e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<1, false>, p);
   if (e != cudaSuccess) return host::fail_cuda("launch rmsnorm_kernel");
   host::count_launch();
   return TYBOK_OK;
