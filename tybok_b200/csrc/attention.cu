@@ -244,6 +244,7 @@ struct AttnParams {
   int dsplit;        // 1, or 2: two CTAs per (query tile, key block), each producing half of the output columns
   int nb_rows;       // key-loop form: the first nb_rows key blocks come from token-major rows [Lk][G*D], the others from
                      // the head-major caches (whose key 0 is then the first key of block nb_rows); 0 = all from the caches
+  int wide_out;      // key-loop form: out and out_planes are 32-byte aligned
   long long* trace;  // tuning aid: [CTA][16] SM-clock samples, NULL in production
   int* dbg;          // debugging aid: stage counters, NULL in production
 };
@@ -829,6 +830,21 @@ __device__ __forceinline__ float pf_exp2(float x) {
   return y;
 }
 
+// 32 bytes of registers (r[first] ..) to global memory: one 256-bit store, or two of 128 bits where the caller's tensor is
+// only 16-byte aligned.
+template <int N>
+__device__ __forceinline__ void st_global_32b(void* dst, const uint32_t (&r)[N], int first, int wide) {
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(r[first]), "r"(r[first + 1]),
+                 "r"(r[first + 2]), "r"(r[first + 3]), "r"(r[first + 4]), "r"(r[first + 5]), "r"(r[first + 6]), "r"(r[first + 7])
+                 : "memory");
+  } else {
+    uint4* d = static_cast<uint4*>(dst);
+    d[0] = make_uint4(r[first], r[first + 1], r[first + 2], r[first + 3]);
+    d[1] = make_uint4(r[first + 4], r[first + 5], r[first + 6], r[first + 7]);
+  }
+}
+
 struct __align__(8) PrefillBars {
   uint64_t q_full;
   uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2];
@@ -845,11 +861,7 @@ struct __align__(8) PrefillBars {
 };
 
 // HD = head dimension, 128 or 256.  Either way a CTA takes ALL 512 tensor-memory columns of its SM
-// and therefore has the SM's tensor memory to itself.  (At HD = 128 two CTAs of 256 columns each
-// would fit, and ran, but chains that alternate this kernel with the CTA-pair GEMM -- whose two CTAs
-// allocate 256 columns collectively on two SMs -- then stalled once in some 10^5 launches with one
-// GEMM pair waiting for tensor memory on an otherwise idle device.  Whole-SM allocations next to
-// the pair GEMM are the combination that has run the pi0.5 prefix 10^6 launches without a stall.)
+// and therefore has the SM's tensor memory to itself: its shared memory leaves no room for another CTA that allocates any.
 template <int HD>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -1127,71 +1139,49 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_EPILOGUE);
     }
     // ------------------------------------------------------------ output
-    // Normalised rows go through shared memory (Q, K and V are idle by now): bf16 rows of 512
-    // bytes and three plane rows of 256 bytes, each padded by 16 bytes against bank conflicts,
-    // then one warp per row, so that global memory sees whole rows.
+    // A thread holds 32 consecutive columns of its row: 64 bytes of bf16 and 32 bytes of every plane, which it stores as
+    // whole 32-byte sectors straight from its registers.  (Staging the rows in shared memory and sending one warp per
+    // row cost two barriers and about 8000 clocks at head_dim 256: 544 x 544 x 8 heads 16.7 -> 14.0 us.)
     if (tr && tid == 128) tr[13] = clock64();
     if (tid == 64) dbg_stage(p.dbg, KID, 3);
     tc_fence_before();
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    constexpr int OB = HD * 2 + 16, OP = HD + 16;  // padded row pitches
-    uint8_t* so = smem;
-    uint8_t* sp = smem + AT_BQ * OB;
-    const bool good = !bars.abort;
-    if (good && live) {  // warp-uniform: the tensor-memory loads below are warp-wide
+    asm volatile("bar.sync 1, 256;" ::: "memory");  // both halves' sums
+    if (!bars.abort && live) {  // warp-uniform: the tensor-memory loads below are warp-wide
       tc_fence_after();
       const float ls = bars.hsum[0][row] + bars.hsum[1][row];
       const float inv = ls > 0.f ? 1.0f / ls : 0.f;
+      const long long hd = static_cast<long long>(p.H) * HD;
+      const long long plane = static_cast<long long>(p.B) * p.L * hd;
+      const long long off = (static_cast<long long>(b) * p.L + qt * AT_BQ + row) * hd + static_cast<long long>(h) * HD;
+      const bool mine = row < nvalid;
 #pragma unroll 1
       for (int c = hf * OCH; c < hf * OCH + OCH; ++c) {
         uint32_t o[32];
         tmem_ld32(t_o + lane_addr + c * 32, o);
         tc_wait_ld();
+        uint32_t ob[16], w1[8], w2[8], w3[8];
 #pragma unroll
-        for (int e = 0; e < 32; e += 8) {
-          uint32_t ob[4], w1[2], w2[2], w3[2];
-#pragma unroll
-          for (int u = 0; u < 2; ++u) {
-            const __nv_bfloat162 o01 = __floats2bfloat162_rn(__uint_as_float(o[e + 4 * u]) * inv, __uint_as_float(o[e + 4 * u + 1]) * inv);
-            const __nv_bfloat162 o23 = __floats2bfloat162_rn(__uint_as_float(o[e + 4 * u + 2]) * inv, __uint_as_float(o[e + 4 * u + 3]) * inv);
-            ob[2 * u] = *reinterpret_cast<const uint32_t*>(&o01);
-            ob[2 * u + 1] = *reinterpret_cast<const uint32_t*>(&o23);
+        for (int e = 0; e < 8; ++e) {
+          const __nv_bfloat162 o01 = __floats2bfloat162_rn(__uint_as_float(o[4 * e]) * inv, __uint_as_float(o[4 * e + 1]) * inv);
+          const __nv_bfloat162 o23 = __floats2bfloat162_rn(__uint_as_float(o[4 * e + 2]) * inv, __uint_as_float(o[4 * e + 3]) * inv);
+          ob[2 * e] = *reinterpret_cast<const uint32_t*>(&o01);
+          ob[2 * e + 1] = *reinterpret_cast<const uint32_t*>(&o23);
+          if (p.out_planes) {
             const float xs[4] = {__bfloat162float(o01.x) * p.plane_scale, __bfloat162float(o01.y) * p.plane_scale,
                                  __bfloat162float(o23.x) * p.plane_scale, __bfloat162float(o23.y) * p.plane_scale};
-            split3_quad(xs, w1[u], w2[u], w3[u]);
+            split3_quad(xs, w1[e], w2[e], w3[e]);
           }
-          const int col = c * 32 + e;
-          *reinterpret_cast<uint4*>(so + row * OB + col * 2) = make_uint4(ob[0], ob[1], ob[2], ob[3]);
-          *reinterpret_cast<uint2*>(sp + row * OP + col) = make_uint2(w1[0], w1[1]);
-          *reinterpret_cast<uint2*>(sp + (AT_BQ + row) * OP + col) = make_uint2(w2[0], w2[1]);
-          *reinterpret_cast<uint2*>(sp + (2 * AT_BQ + row) * OP + col) = make_uint2(w3[0], w3[1]);
         }
-      }
-    }
-    if (tr && tid == 128) tr[15] = clock64();
-    asm volatile("bar.sync 1, 256;" ::: "memory");
-    if (good) {
-      // one warp per row: every lane moves HD / 32 elements of the bf16 row and of every plane
-      const long long hd = static_cast<long long>(p.H) * HD;
-      const long long plane = static_cast<long long>(p.B) * p.L * hd;
-#pragma unroll 2
-      for (int r = warp - 2; r < nvalid; r += 8) {
-        const long long off = (static_cast<long long>(b) * p.L + qt * AT_BQ + r) * hd + static_cast<long long>(h) * HD;
-        if (HD == 256) {
-          if (p.out) *reinterpret_cast<uint4*>(p.out + off + lane * 8) = *reinterpret_cast<const uint4*>(so + r * OB + lane * 16);
-          if (p.out_planes) {
-            uint8_t* dst = p.out_planes + off + lane * 8;
-            *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(sp + r * OP + lane * 8);
-            *reinterpret_cast<uint2*>(dst + plane) = *reinterpret_cast<const uint2*>(sp + (AT_BQ + r) * OP + lane * 8);
-            *reinterpret_cast<uint2*>(dst + 2 * plane) = *reinterpret_cast<const uint2*>(sp + (2 * AT_BQ + r) * OP + lane * 8);
+        if (mine) {
+          if (p.out) {
+            st_global_32b(p.out + off + c * 32, ob, 0, p.wide_out);
+            st_global_32b(p.out + off + c * 32 + 16, ob, 8, p.wide_out);
           }
-        } else {
-          if (p.out) *reinterpret_cast<uint2*>(p.out + off + lane * 4) = *reinterpret_cast<const uint2*>(so + r * OB + lane * 8);
           if (p.out_planes) {
-            uint8_t* dst = p.out_planes + off + lane * 4;
-            *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(sp + r * OP + lane * 4);
-            *reinterpret_cast<uint32_t*>(dst + plane) = *reinterpret_cast<const uint32_t*>(sp + (AT_BQ + r) * OP + lane * 4);
-            *reinterpret_cast<uint32_t*>(dst + 2 * plane) = *reinterpret_cast<const uint32_t*>(sp + (2 * AT_BQ + r) * OP + lane * 4);
+            uint8_t* dst = p.out_planes + off + c * 32;
+            st_global_32b(dst, w1, 0, p.wide_out);
+            st_global_32b(dst + plane, w2, 0, p.wide_out);
+            st_global_32b(dst + 2 * plane, w3, 0, p.wide_out);
           }
         }
       }
@@ -1377,6 +1367,7 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   p.out = static_cast<__nv_bfloat16*>(out);
   p.out_planes = static_cast<uint8_t*>(out_planes);
   p.plane_scale = ldexpf(1.0f, out_shift);
+  p.wide_out = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_planes)) & 31) == 0;
   p.status = status_word;
   p.pdl = host::pdl_enabled() ? 1 : 0;
   p.ws = static_cast<uint8_t*>(workspace);
@@ -1466,6 +1457,7 @@ int tybok_attention_rows(const void* q, const void* k_rows, const void* v_rows, 
   p.scale_log2e = scale * 1.4426950408889634f;
   p.key_valid = static_cast<const uint8_t*>(key_valid);
   p.out = static_cast<__nv_bfloat16*>(out); p.out_planes = static_cast<uint8_t*>(out_planes); p.plane_scale = ldexpf(1.0f, out_shift);
+  p.wide_out = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_planes)) & 31) == 0;
   p.status = status_word; p.pdl = host::pdl_enabled() ? 1 : 0; p.q_rows = AT_BQ; p.dsplit = 1;
   p.trace = host::trace_buffer(); p.dbg = host::counter_buffer();
   static bool attr_set[64] = {};
