@@ -1141,7 +1141,8 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     // ------------------------------------------------------------ output
     // A thread holds 32 consecutive columns of its row: 64 bytes of bf16 and 32 bytes of every plane, which it stores as
     // whole 32-byte sectors straight from its registers.  (Staging the rows in shared memory and sending one warp per
-    // row cost two barriers and about 8000 clocks at head_dim 256: 544 x 544 x 8 heads 16.7 -> 14.0 us.)
+    // row cost two more barriers: 4146 x 129 keys x 24 heads 51.8 -> 48.6 us.  What is left, 7500 clocks at head_dim 256,
+    // is the conversions of the plane split.)
     if (tr && tid == 128) tr[13] = clock64();
     if (tid == 64) dbg_stage(p.dbg, KID, 3);
     tc_fence_before();
@@ -1195,6 +1196,311 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     tmem_dealloc(tmem, T_COLS);
   }
   if (tid == 0) dbg_stage(p.dbg, KID, 4);
+}
+
+}  // namespace tb
+
+namespace tb {
+// ------------------------------------------------------------------------------ two-tile form
+// Long query sequences at head_dim 128: one CTA per (pair of query tiles = 256 rows, head, batch element).  The key-loop
+// form above spends 2400 clocks on a 128-row x 128-key block, of which the exponentials (16 per clock and SM) need
+// 1024: its eight warps share every block and meet at a barrier in each, so the chain of tensor-memory round trips is
+// exposed.  Here four warps own each tile with one thread per row, nothing is shared between rows, and the tiles take
+// turns: one's scores and products run under the other's exponentials.  Tensor memory: S / P and O of both tiles, 128
+// columns each.  Tensor order per block: PV_0(j), S_0(j+1), PV_1(j), S_1(j+1); a tile's S(j+1) follows its PV(j), which
+// reads the P that S overwrites, so a thread that sees S(j+1) also knows that PV(j) has landed.
+// Packed fp32 pairs (fma.f32x2, add.f32x2) halve the issue slots around the exponentials.
+struct __align__(8) TwoTileBars {
+  uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2];
+  uint64_t s_full[2], p_full[2];  // per tile
+  uint64_t done[2];               // per tile: its last product has landed
+  uint64_t mma_done;
+  uint32_t tmem_base;
+  volatile int abort;
+  uint32_t valid[PF_MAX_KEYS / 32];
+};
+constexpr int TT_SMEM = 2 * 32768 + 4 * 32768 + 1024;  // two Q tiles, two K and two V blocks
+
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f32x2_split(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+__global__ void __launch_bounds__(AT_THREADS, 1)
+attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
+                          const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ TwoTileBars bars;
+  constexpr int HD = 128, BK = 128, KV = 32768, CH = 16384;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sq = smem;
+  uint8_t* sk = smem + 2 * 32768;
+  uint8_t* sv = sk + 2 * KV;
+  const int qt = blockIdx.x, h = blockIdx.y, b = blockIdx.z, g = h / (p.H / p.G);
+  const int nkb = (p.Lk + BK - 1) / BK;
+  const int row_base = qt * 256;
+  const int ntile = p.L - row_base > 128 ? 2 : 1;  // the last pair of a sequence may hold one tile
+
+  if (tid == 0) {
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+    mbar_init(&bars.q_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bars.k_full[i], 1);
+      mbar_init(&bars.k_empty[i], 1);
+      mbar_init(&bars.v_full[i], 1);
+      mbar_init(&bars.v_empty[i], 1);
+      mbar_init(&bars.s_full[i], 1);
+      mbar_init(&bars.p_full[i], 4);
+      mbar_init(&bars.done[i], 1);
+    }
+    mbar_init(&bars.mma_done, 1);
+    bars.abort = 0;
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(&bars.tmem_base, 512);
+    tmem_relinquish();
+  }
+  if (warp >= 2) {  // validity bits of every key, 32 per word
+    if (p.key_valid && p.pdl) pdl_wait();
+    for (int w = warp - 2; w < (BK / 32) * nkb; w += 8) {
+      const int j = w * 32 + lane;
+      bool ok = j < p.Lk;
+      if (ok && p.key_valid) ok = p.key_valid[static_cast<long long>(b) * p.Lk + j] != 0;
+      const uint32_t bits = __ballot_sync(0xffffffffu, ok);
+      if (lane == 0) bars.valid[w] = bits;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = bars.tmem_base;  // S / P of tile t at 128 t, O of tile t at 256 + 128 t
+
+  if (warp == 0) {
+    if (lane == 0) {
+      if (p.pdl) pdl_launch_dependents();
+      if (p.pdl) pdl_wait();
+      mbar_arrive_expect_tx(&bars.q_full, ntile * 32768);
+      for (int t = 0; t < ntile; ++t)
+        for (int c = 0; c < 2; ++c)
+          tma_load_2d(sq + t * 32768 + c * CH, &tm_q, &bars.q_full, h * HD + c * 64, b * p.L + row_base + t * 128);
+      for (int j = 0; j < nkb; ++j) {
+        const int s = j & 1;
+        const uint32_t par = ((j >> 1) & 1) ^ 1;  // the ring slot's previous use
+        const int krow = (b * p.G + g) * p.Lcap + j * BK;
+        if (j >= 2 && !at_wait(&bars.k_empty[s], par, &bars.abort)) break;
+        mbar_arrive_expect_tx(&bars.k_full[s], KV);
+        for (int c = 0; c < 2; ++c) tma_load_2d(sk + s * KV + c * CH, &tm_k, &bars.k_full[s], c * 64, krow);
+        if (j >= 2 && !at_wait(&bars.v_empty[s], par, &bars.abort)) break;
+        mbar_arrive_expect_tx(&bars.v_full[s], KV);
+        for (int c = 0; c < 2; ++c) tma_load_2d(sv + s * KV + c * CH, &tm_v, &bars.v_full[s], c * 64, krow);
+      }
+    }
+  } else if (warp == 1) {
+    const bool leader = elect_one();
+    const uint64_t dk = smem_desc_sw128(0);
+    const uint32_t idesc_s = idesc_bf16_f32(128, BK), idesc_o = idesc_bf16_f32(128, HD) | (1u << 16);
+    auto issue_s = [&](int t, int j) {
+      const uint32_t q16 = (smem_u32(sq + t * 32768) & 0x3FFFFu) >> 4, k16 = (smem_u32(sk + (j & 1) * KV) & 0x3FFFFu) >> 4;
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {  // 16 of the head dimension per step
+        const uint32_t o = (ks >> 2) * (CH >> 4) + (ks & 3) * 2;
+        if (leader) umma_ss_bf16(tmem + t * 128, dk | (q16 + o), dk | (k16 + o), idesc_s, ks > 0 ? 1u : 0u);
+      }
+      if (leader) tc_commit(&bars.s_full[t]);
+    };
+    bool ok = __all_sync(0xffffffffu, at_wait(&bars.q_full, 0, &bars.abort) && at_wait(&bars.k_full[0], 0, &bars.abort));
+    if (ok) {
+      tc_fence_after();
+      for (int t = 0; t < ntile; ++t) issue_s(t, 0);
+      if (leader) tc_commit(&bars.k_empty[0]);
+      __syncwarp();
+    }
+#pragma unroll 1
+    for (int j = 0; j < nkb && ok; ++j) {
+      const int s = j & 1;
+      const uint32_t v_addr = smem_u32(sv + s * KV);
+      ok = __all_sync(0xffffffffu, at_wait(&bars.v_full[s], (j >> 1) & 1, &bars.abort));
+      if (ok && j + 1 < nkb) ok = __all_sync(0xffffffffu, at_wait(&bars.k_full[s ^ 1], ((j + 1) >> 1) & 1, &bars.abort));
+      for (int t = 0; t < ntile && ok; ++t) {
+        ok = __all_sync(0xffffffffu, at_wait(&bars.p_full[t], j & 1, &bars.abort));
+        if (!ok) break;
+        tc_fence_after();
+#pragma unroll
+        for (int ks = 0; ks < BK / 16; ++ks) {
+          const uint64_t bd = smem_desc_sw128_mn(v_addr + ks * 2048, CH);
+          if (leader) umma_ts_bf16(tmem + 256 + t * 128, tmem + t * 128 + ks * 8, bd, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+        }
+        if (j + 1 < nkb) issue_s(t, j + 1);
+        else if (leader) tc_commit(&bars.done[t]);
+      }
+      if (ok && leader) {
+        tc_commit(&bars.v_empty[s]);
+        if (j + 1 < nkb) tc_commit(&bars.k_empty[s ^ 1]);
+      }
+      __syncwarp();
+    }
+    // nothing of this CTA's tensor work may be in flight when it gives up its tensor memory
+    if (!ok && lane == 0) {
+      bars.abort = 1;
+      if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_MMA);
+    }
+    if (leader) tc_commit(&bars.mma_done);
+    __syncwarp();
+    mbar_wait(&bars.mma_done, 0);
+  } else {
+    const int t = (warp - 2) >> 2, q = warp & 3, row = q * 32 + lane;
+    const int nvalid = min(128, p.L - row_base - t * 128);
+    const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
+    const uint32_t t_s = tmem + t * 128 + lane_addr, t_o = tmem + 256 + t * 128 + lane_addr;
+    const bool live = q * 32 < nvalid;  // warp-uniform: this quadrant holds real query rows
+    bool ok = true;
+    float m_ref = -1e30f, l = 0.f;
+    if (t < ntile) {
+      const uint64_t c2 = f32x2(p.scale_log2e, p.scale_log2e);
+#pragma unroll 1
+      for (int j = 0; j < nkb; ++j) {
+        if (ok && !__all_sync(0xffffffffu, at_wait(&bars.s_full[t], j & 1, &bars.abort))) {
+          ok = false;
+          bars.abort = 1;
+        }
+        if (!ok) break;
+        if (live) {
+          tc_fence_after();
+          uint32_t v[4][32];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) tmem_ld32(t_s + w * 32, v[w]);
+          const uint32_t b0 = bars.valid[4 * j], b1 = bars.valid[4 * j + 1], b2 = bars.valid[4 * j + 2], b3 = bars.valid[4 * j + 3];
+          const uint32_t bits[4] = {b0, b1, b2, b3};
+          const bool all = (b0 & b1 & b2 & b3) == 0xffffffffu;
+          tc_wait_ld();
+          if (!all) {  // a masked score becomes so small that its exponential is zero
+#pragma unroll
+            for (int w = 0; w < 4; ++w)
+#pragma unroll
+              for (int e = 0; e < 32; ++e)
+                if (!((bits[w] >> e) & 1u)) v[w][e] = __float_as_uint(-1e30f);
+          }
+          float mx0 = -1e30f, mx1 = -1e30f, mx2 = -1e30f, mx3 = -1e30f;
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            mx0 = fmaxf(mx0, __uint_as_float(v[0][e]));
+            mx1 = fmaxf(mx1, __uint_as_float(v[1][e]));
+            mx2 = fmaxf(mx2, __uint_as_float(v[2][e]));
+            mx3 = fmaxf(mx3, __uint_as_float(v[3][e]));
+          }
+          const float m_blk = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2e;  // scale > 0
+          // the reference maximum only moves when a block exceeds it by more than 2^8 (or was all masked so far)
+          const bool grow = m_blk > m_ref + PF_RESCALE;
+          if (__any_sync(0xffffffffu, grow)) {
+            if (j > 0) {
+              const float f = grow ? pf_exp2(m_ref - m_blk) : 1.0f;
+#pragma unroll 1
+              for (int c = 0; c < 4; ++c) {
+                uint32_t o[32];
+                tmem_ld32(t_o + c * 32, o);
+                tc_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 32; ++e) o[e] = __float_as_uint(__uint_as_float(o[e]) * f);
+                tmem_st32(t_o + c * 32, o);
+              }
+              l *= f;
+            }
+            if (grow) m_ref = m_blk;
+          }
+          const float base = fmaxf(m_ref, -1e29f);  // an all-masked row so far: exponentials of -1e30 stay zero
+          const uint64_t nm = f32x2(-base, -base);
+          uint64_t sum0 = f32x2(0.f, 0.f), sum1 = sum0;
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            uint32_t pk[16];
+#pragma unroll
+            for (int e = 0; e < 32; e += 2) {
+              float x0, x1;
+              f32x2_split(f32x2_fma(f32x2(__uint_as_float(v[w][e]), __uint_as_float(v[w][e + 1])), c2, nm), x0, x1);
+              const float p0 = pf_exp2(x0), p1 = pf_exp2(x1);
+              if (w & 1) sum1 = f32x2_add(sum1, f32x2(p0, p1));
+              else sum0 = f32x2_add(sum0, f32x2(p0, p1));
+              const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
+              pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
+            }
+            tmem_st16(t_s + w * 16, pk);
+          }
+          float a0, a1;
+          f32x2_split(f32x2_add(sum0, sum1), a0, a1);
+          l += a0 + a1;
+          tc_wait_st();
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bars.p_full[t]);
+      }
+      if (ok && !__all_sync(0xffffffffu, at_wait(&bars.done[t], 0, &bars.abort))) ok = false;
+      if (!ok && lane == 0) {
+        bars.abort = 1;
+        if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_EPILOGUE);
+      }
+      if (ok && live) {
+        tc_fence_after();
+        const float inv = l > 0.f ? 1.0f / l : 0.f;
+        const long long hd = static_cast<long long>(p.H) * HD, plane = static_cast<long long>(p.B) * p.L * hd;
+        const long long off = (static_cast<long long>(b) * p.L + row_base + t * 128 + row) * hd + static_cast<long long>(h) * HD;
+        const bool mine = row < nvalid;
+#pragma unroll 1
+        for (int c = 0; c < 4; ++c) {
+          uint32_t o[32];
+          tmem_ld32(t_o + c * 32, o);
+          tc_wait_ld();
+          uint32_t ob[16], w1[8], w2[8], w3[8];
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const __nv_bfloat162 o01 = __floats2bfloat162_rn(__uint_as_float(o[4 * e]) * inv, __uint_as_float(o[4 * e + 1]) * inv);
+            const __nv_bfloat162 o23 = __floats2bfloat162_rn(__uint_as_float(o[4 * e + 2]) * inv, __uint_as_float(o[4 * e + 3]) * inv);
+            ob[2 * e] = *reinterpret_cast<const uint32_t*>(&o01);
+            ob[2 * e + 1] = *reinterpret_cast<const uint32_t*>(&o23);
+            if (p.out_planes) {
+              const float xs[4] = {__bfloat162float(o01.x) * p.plane_scale, __bfloat162float(o01.y) * p.plane_scale,
+                                   __bfloat162float(o23.x) * p.plane_scale, __bfloat162float(o23.y) * p.plane_scale};
+              split3_quad(xs, w1[e], w2[e], w3[e]);
+            }
+          }
+          if (mine) {
+            if (p.out) {
+              st_global_32b(p.out + off + c * 32, ob, 0, p.wide_out);
+              st_global_32b(p.out + off + c * 32 + 16, ob, 8, p.wide_out);
+            }
+            if (p.out_planes) {
+              uint8_t* dst = p.out_planes + off + c * 32;
+              st_global_32b(dst, w1, 0, p.wide_out);
+              st_global_32b(dst + plane, w2, 0, p.wide_out);
+              st_global_32b(dst + 2 * plane, w3, 0, p.wide_out);
+            }
+          }
+        }
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 512);
+  }
 }
 
 }  // namespace tb
@@ -1373,6 +1679,8 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   p.ws = static_cast<uint8_t*>(workspace);
   p.q_rows = q_rows;
   const int n_qt = (L + AT_BQ - 1) / AT_BQ;
+  // Two tiles per CTA wherever one each would need a second wave; within one wave the key-loop form has a tile per SM.
+  const bool two_tile = D == 128 && L > AT_BQ && static_cast<long long>(n_qt) * H * B > host::sm_count();
   p.dsplit = (nsplit > 1 && 2 * nsplit * H * n_qt * B <= host::sm_count()) ? 2 : 1;
   p.trace = host::trace_buffer();
   p.dbg = host::counter_buffer();
@@ -1384,15 +1692,16 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
     if (cudaFuncSetAttribute(attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) != cudaSuccess ||
+        cudaFuncSetAttribute(attention_two_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TT_SMEM) != cudaSuccess ||
         cudaFuncSetAttribute(attention_prefill_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem(256)) != cudaSuccess ||
         cudaFuncSetAttribute(attention_prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem(128)) != cudaSuccess)
       return host::fail_cuda("cudaFuncSetAttribute(attention_kernel)");
     attr_set[dev] = true;
   }
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = prefill ? dim3(n_qt, H, B) : dim3(nsplit, H * n_qt * p.dsplit, B);
+  cfg.gridDim = two_tile ? dim3((n_qt + 1) / 2, H, B) : prefill ? dim3(n_qt, H, B) : dim3(nsplit, H * n_qt * p.dsplit, B);
   cfg.blockDim = dim3(AT_THREADS);
-  cfg.dynamicSmemBytes = prefill ? pf_smem(D) : AT_SMEM;
+  cfg.dynamicSmemBytes = two_tile ? TT_SMEM : prefill ? pf_smem(D) : AT_SMEM;
   cfg.stream = static_cast<cudaStream_t>(stream);
   cudaLaunchAttribute attr[2];
   int na = 0;
@@ -1411,7 +1720,9 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   cfg.attrs = attr;
   cfg.numAttrs = na;
   cudaError_t e;
-  if (prefill)
+  if (two_tile)
+    e = cudaLaunchKernelEx(&cfg, attention_two_tile_kernel, tm_q, tm_k, tm_v, p);
+  else if (prefill)
     e = cudaLaunchKernelEx(&cfg, D == 128 ? attention_prefill_kernel<128> : attention_prefill_kernel<256>, tm_q, tm_k, tm_v, tm_k, tm_v, p);
   else
     e = cudaLaunchKernelEx(&cfg, push ? attention_kernel<true> : attention_kernel<false>, tm_q, tm_k, tm_v, p);
