@@ -1212,7 +1212,8 @@ namespace tb {
 // Packed fp32 pairs (fma.f32x2, add.f32x2) halve the issue slots around the exponentials.
 struct __align__(8) TwoTileBars {
   uint64_t q_full, k_full[2], k_empty[2], v_full[2], v_empty[2];
-  uint64_t s_full[2], p_full[2];  // per tile
+  uint64_t s_full[2];             // per tile
+  uint64_t p_full[2][2];          // per tile and half of the block's keys
   uint64_t done[2];               // per tile: its last product has landed
   uint64_t mma_done;
   uint32_t tmem_base;
@@ -1232,13 +1233,22 @@ __device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 __device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
   uint64_t r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
 
-__global__ void __launch_bounds__(AT_THREADS, 1)
+// Four control warps (two of them idle: register shares are per warpgroup) and four warps per tile.
+constexpr int TT_THREADS = 384;
+constexpr int TT_REGS_CONTROL = 56, TT_REGS_SOFTMAX = 224;  // launched with 168 each: 56 + 2 * 224 = 3 * 168
+
+__global__ void __launch_bounds__(TT_THREADS, 1)
 attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                           const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -1265,7 +1275,8 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       mbar_init(&bars.v_full[i], 1);
       mbar_init(&bars.v_empty[i], 1);
       mbar_init(&bars.s_full[i], 1);
-      mbar_init(&bars.p_full[i], 4);
+      mbar_init(&bars.p_full[i][0], 4);
+      mbar_init(&bars.p_full[i][1], 4);
       mbar_init(&bars.done[i], 1);
     }
     mbar_init(&bars.mma_done, 1);
@@ -1276,9 +1287,9 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     tmem_alloc(&bars.tmem_base, 512);
     tmem_relinquish();
   }
-  if (warp >= 2) {  // validity bits of every key, 32 per word
+  if (warp >= 4) {  // validity bits of every key, 32 per word
     if (p.key_valid && p.pdl) pdl_wait();
-    for (int w = warp - 2; w < (BK / 32) * nkb; w += 8) {
+    for (int w = warp - 4; w < (BK / 32) * nkb; w += 8) {
       const int j = w * 32 + lane;
       bool ok = j < p.Lk;
       if (ok && p.key_valid) ok = p.key_valid[static_cast<long long>(b) * p.Lk + j] != 0;
@@ -1291,6 +1302,8 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
   tc_fence_after();
   const uint32_t tmem = bars.tmem_base;  // S / P of tile t at 128 t, O of tile t at 256 + 128 t
 
+  if (warp < 4) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TT_REGS_CONTROL));
   if (warp == 0) {
     if (lane == 0) {
       if (p.pdl) pdl_launch_dependents();
@@ -1338,14 +1351,18 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       ok = __all_sync(0xffffffffu, at_wait(&bars.v_full[s], (j >> 1) & 1, &bars.abort));
       if (ok && j + 1 < nkb) ok = __all_sync(0xffffffffu, at_wait(&bars.k_full[s ^ 1], ((j + 1) >> 1) & 1, &bars.abort));
       for (int t = 0; t < ntile && ok; ++t) {
-        ok = __all_sync(0xffffffffu, at_wait(&bars.p_full[t], j & 1, &bars.abort));
-        if (!ok) break;
-        tc_fence_after();
+        for (int hf = 0; hf < 2 && ok; ++hf) {  // the first keys' product starts under the others' exponentials
+          ok = __all_sync(0xffffffffu, at_wait(&bars.p_full[t][hf], j & 1, &bars.abort));
+          if (!ok) break;
+          tc_fence_after();
 #pragma unroll
-        for (int ks = 0; ks < BK / 16; ++ks) {
-          const uint64_t bd = smem_desc_sw128_mn(v_addr + ks * 2048, CH);
-          if (leader) umma_ts_bf16(tmem + 256 + t * 128, tmem + t * 128 + ks * 8, bd, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+          for (int k4 = 0; k4 < 4; ++k4) {
+            const int ks = hf * 4 + k4;
+            const uint64_t bd = smem_desc_sw128_mn(v_addr + ks * 2048, CH);
+            if (leader) umma_ts_bf16(tmem + 256 + t * 128, tmem + t * 128 + ks * 8, bd, idesc_o, (j | ks) ? 1u : 0u);
+          }
         }
+        if (!ok) break;
         if (j + 1 < nkb) issue_s(t, j + 1);
         else if (leader) tc_commit(&bars.done[t]);
       }
@@ -1363,8 +1380,10 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     if (leader) tc_commit(&bars.mma_done);
     __syncwarp();
     mbar_wait(&bars.mma_done, 0);
+  }
   } else {
-    const int t = (warp - 2) >> 2, q = warp & 3, row = q * 32 + lane;
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TT_REGS_SOFTMAX));
+    const int t = (warp - 4) >> 2, q = warp & 3, row = q * 32 + lane;
     const int nvalid = min(128, p.L - row_base - t * 128);
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const uint32_t t_s = tmem + t * 128 + lane_addr, t_o = tmem + 256 + t * 128 + lane_addr;
@@ -1398,11 +1417,11 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           }
           float mx0 = -1e30f, mx1 = -1e30f, mx2 = -1e30f, mx3 = -1e30f;
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            mx0 = fmaxf(mx0, __uint_as_float(v[0][e]));
-            mx1 = fmaxf(mx1, __uint_as_float(v[1][e]));
-            mx2 = fmaxf(mx2, __uint_as_float(v[2][e]));
-            mx3 = fmaxf(mx3, __uint_as_float(v[3][e]));
+          for (int e = 0; e < 32; e += 2) {
+            mx0 = max3(mx0, __uint_as_float(v[0][e]), __uint_as_float(v[0][e + 1]));
+            mx1 = max3(mx1, __uint_as_float(v[1][e]), __uint_as_float(v[1][e + 1]));
+            mx2 = max3(mx2, __uint_as_float(v[2][e]), __uint_as_float(v[2][e + 1]));
+            mx3 = max3(mx3, __uint_as_float(v[3][e]), __uint_as_float(v[3][e + 1]));
           }
           const float m_blk = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * p.scale_log2e;  // scale > 0
           // the reference maximum only moves when a block exceeds it by more than 2^8 (or was all masked so far)
@@ -1440,6 +1459,12 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
               pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
             }
             tmem_st16(t_s + w * 16, pk);
+            if (w == 1) {
+              tc_wait_st();
+              tc_fence_before();
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bars.p_full[t][0]);
+            }
           }
           float a0, a1;
           f32x2_split(f32x2_add(sum0, sum1), a0, a1);
@@ -1448,7 +1473,10 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&bars.p_full[t]);
+        if (lane == 0) {
+          if (!live) mbar_arrive(&bars.p_full[t][0]);
+          mbar_arrive(&bars.p_full[t][1]);
+        }
       }
       if (ok && !__all_sync(0xffffffffu, at_wait(&bars.done[t], 0, &bars.abort))) ok = false;
       if (!ok && lane == 0) {
@@ -1700,7 +1728,7 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = two_tile ? dim3((n_qt + 1) / 2, H, B) : prefill ? dim3(n_qt, H, B) : dim3(nsplit, H * n_qt * p.dsplit, B);
-  cfg.blockDim = dim3(AT_THREADS);
+  cfg.blockDim = dim3(two_tile ? TT_THREADS : AT_THREADS);
   cfg.dynamicSmemBytes = two_tile ? TT_SMEM : prefill ? pf_smem(D) : AT_SMEM;
   cfg.stream = static_cast<cudaStream_t>(stream);
   cudaLaunchAttribute attr[2];
