@@ -91,3 +91,29 @@ def test_rotary_form_at_tile_edges(b, l, h, gr, d, key_off):
     for a, r in ((q0, q1), (c[0], c[2]), (c[1], c[3])):
         assert w8_ref.rel_l2(a.float().cpu(), r.float().cpu()) <= 2e-3
     assert not c[0][:, :, :key_off].any() and not c[0][:, :, key_off + l :].any()
+
+
+@pytest.mark.parametrize("m,n,k", [(333, 2048, 16384), (257, 2044, 16400), (512, 1796, 12304), (200, 3072, 14336)])
+def test_k_split_over_the_pairs_of_a_cluster(m, n, k):
+    """Long K with a tile count that fills neither kernel's plain plan: parts exchanged through shared memory, every
+    epilogue, two launches bit-equal."""
+    from tybok_b200 import ops
+
+    x, (w8, sc) = _x(m, k, m), _weights(n, k, n)
+    xp = ops.split3(x.cuda(), 4)
+    g = torch.Generator().manual_seed(7)
+    res = torch.empty(m, n).normal_(0, 1, generator=g).to(torch.bfloat16).cuda()
+    gate = torch.empty(2, n).normal_(0, 1, generator=g).to(torch.bfloat16).cuda()
+    bias = torch.empty(n).normal_(0, 1, generator=g).to(torch.bfloat16).cuda()
+    for kw in (dict(), dict(bias=bias, epilogue=ops.EPI_GELU, out_planes=True),
+               dict(bias=bias, epilogue=ops.EPI_RESIDUAL, residual=res, gate=gate, rows_per_gate=(m + 1) // 2)):
+        y, yp = ops.w8x3_linear(xp, 4, w8, sc, **kw)
+        again, _ = ops.w8x3_linear(xp, 4, w8, sc, **kw)
+        y1, yp1 = ops.w8x3_linear(xp, 4, w8, sc, token_tile=64, splits=1, **kw)
+        ops.check_status()
+        assert torch.equal(y, again)
+        assert w8_ref.rel_l2(y.float().cpu(), y1.float().cpu()) <= 2e-3
+        if kw.get("out_planes"):
+            f = lambda p: p.view(torch.float8_e5m2).float().sum(0)  # noqa: E731
+            assert w8_ref.rel_l2(f(yp).cpu(), f(yp1).cpu()) <= 2e-3
+    assert w8_ref.rel_l2(ops.w8x3_linear(xp, 4, w8, sc)[0].cpu(), w8_ref.w8_linear(x, w8.cpu(), sc.cpu())) <= 1e-2

@@ -838,8 +838,21 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   if (force_splits > MAX_SPLITS) return host::fail(TYBOK_ERR_ARG, "w8 gemm: at most 8 K splits (cluster size)");
   if (pl.n_tiles > 65535) return host::fail(TYBOK_ERR_ARG, "w8 gemm: grid too large");
   if (check_only) return TYBOK_OK;  // every argument check has passed; nothing was launched
-  if (force_bt <= 0 && force_splits <= 0 && !fold && gemm_pair_suits(M, N, nw, np)) {
+  const bool free_form = force_bt <= 0 && force_splits <= 0 && !fold;
+  // Within one wave of tiles: K over the pairs of a cluster where that is estimated to be clearly ahead of this plan
+  // (a K block costs the slower of its products and its operand fill at 50 bytes per clock; set-up and exchange on top).
+  // Those are the long K whose tile count leaves a third of the SMs idle but is too high for this kernel's own split:
+  // 333 x 2048 x 16384 48.9 -> 35.7 us, 400 tokens 49.1 -> 38.7, 200 x 3072 x 14336 43.6 -> 36.2; 544 x 2048 x 16384
+  // would stay at 51.
+  bool split = false;
+  if (free_form && M > 128 && !rope && (epi == EPI_NONE || epi == EPI_GELU || epi == EPI_RESIDUAL) && !gemm_pair_suits(M, N, nw, np)) {
+    const double here = pl.kb_per_split * std::max(2.0 * np * pl.bt, (16384.0 + np * 128.0 * pl.bt) / 50.0) + (pl.splits > 1 ? 3000.0 : 0.0);
+    const double there = gemm_pair_split_cost(M, N, K, np);
+    split = there > 0 && there + 6000.0 < 0.85 * here;
+  }
+  if (split || (free_form && gemm_pair_suits(M, N, nw, np))) {
     GemmCall c{};
+    c.split = split;
     c.planes = planes; c.np = np; c.row_scale = row_scale; c.w0 = w0; c.w1 = w1; c.s0 = s0; c.s1 = s1;
     c.bias = static_cast<const __nv_bfloat16*>(bias); c.y = static_cast<__nv_bfloat16*>(y); c.ldy = ldy;
     c.y_planes = static_cast<uint8_t*>(y_planes); c.M = M; c.N = N; c.K = K; c.n_out = n_out; c.epi = epi;

@@ -45,12 +45,15 @@ struct GemmCall {
   int rows_per_gate, gate_bf16;
   float out_scale, plane_scale;
   const RopeEpi* rope;
+  bool split;              // K over the pairs of a cluster (EPI_NONE, EPI_GELU, EPI_RESIDUAL)
   int* status;
   cudaStream_t stream;
 };
 
 // True when w8_gemm_pair.cu is the faster kernel for this shape (`nw` weight matrices of N rows).
 bool gemm_pair_suits(int M, int N, int nw, int np);
+// Estimated SM clocks of the split form (a cluster of pairs per tile) for one wave of clusters; negative: does not apply.
+double gemm_pair_split_cost(int M, int N, int K, int np);
 int launch_gemm_pair(const GemmCall& c);
 
 }  // namespace tb

@@ -47,6 +47,7 @@ struct PairParams {
   int np;
   int packed;            // gate / up and rotary forms: 1 = interleaved blocks of 64 rows, 0 = two matrices
   int kb;                // K blocks
+  int splits, kb_split;  // split form: pairs of a cluster that share a tile, K blocks of each
   int merge;             // 1: every plane has its own columns and the epilogue adds them (one accumulator, M <= 128)
   int nstages, stage_bytes;
   int ch_tiles, tok_tiles, group;  // tiles; token tiles per L2 group
@@ -140,7 +141,10 @@ __device__ __forceinline__ uint2 quad_transpose(uint32_t a, uint32_t b, int lane
 }
 
 // EPI: EPI_NONE, EPI_GELU, EPI_RESIDUAL, EPI_GEGLU (both layouts of gate and up, p.packed) or EPI_QKV_ROPE.
-template <int EPI>
+// SPLIT: long K and too few tiles for the device: a cluster of 2 * splits CTAs works on ONE tile, each pair on its part of
+// K.  Once all of them are through (their rings are idle then), every pair sends the token chunks it does not own
+// into the owners' shared memory, and a chunk's owner adds the parts in split order and finishes it.
+template <int EPI, bool SPLIT>
 __global__ void __launch_bounds__(P_THREADS, 1)
 w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                     const __grid_constant__ CUtensorMap tm_big, const __grid_constant__ CUtensorMap tm_small,
@@ -150,9 +154,12 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
   constexpr int NA = (EPI == EPI_GEGLU || EPI == EPI_QKV_ROPE) ? 2 : 1;  // accumulators (of <= 256 / NA tokens) per tile
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const uint32_t rank = cluster_ctarank();  // 0 issues the pair's products
-  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const uint32_t crank = cluster_ctarank(), rank = crank & 1u, lead = crank & ~1u;  // the even CTA issues the pair's products
+  const int split = SPLIT ? static_cast<int>(crank >> 1) : 0;
   const int tiles = p.ch_tiles * p.tok_tiles;
+  const int pair = SPLIT ? blockIdx.x / (2 * p.splits) : blockIdx.x >> 1, npairs = SPLIT ? tiles : gridDim.x >> 1;
+  const int kb0 = SPLIT ? split * p.kb_split : 0, nkb = SPLIT ? min(p.kb_split, p.kb - kb0) : p.kb;
+  const uint16_t both = static_cast<uint16_t>(3u << lead);
 
   if (tid == 0) {
     for (int i = 0; i < P_MAX_STAGES; ++i) {
@@ -184,7 +191,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     if (lane == 0) {
       if (p.pdl) pdl_launch_dependents();
       auto load_w = [&](int ch, int kb, uint8_t* st, uint32_t bar) {
-        const int k0 = kb * P_BK;
+        const int k0 = (kb0 + kb) * P_BK;
         if (NA == 1) {
           tma_load_2d_pair(st, &tm_w0, bar, k0, ch * 256 + static_cast<int>(rank) * 128);
         } else if (p.packed) {  // blocks of 64 + 64 rows: the first halves to one tile, the partners to the other
@@ -208,17 +215,17 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         const uint32_t bytes = 2u * (NA * P_WTILE + p.np * hrows * P_BK);
         if (!waited) {
           // Weights depend on nothing that runs before this kernel: fill the ring's weight tiles first.
-          const int pre = min(p.nstages, p.kb);
+          const int pre = min(p.nstages, nkb);
           for (int i = 0; i < pre; ++i) {
             if (rank == 0) mbar_arrive_expect_tx(&bars.full[i], bytes);
-            load_w(tl.ch, i, smem + i * p.stage_bytes, dsmem_addr(smem_u32(&bars.full[i]), 0));
+            load_w(tl.ch, i, smem + i * p.stage_bytes, dsmem_addr(smem_u32(&bars.full[i]), lead));
           }
           if (p.pdl) pdl_wait();
         }
-        for (int k = 0; k < p.kb; ++k) {
+        for (int k = 0; k < nkb; ++k) {
           const bool primed = !waited && k < p.nstages;
           uint8_t* st = smem + s * p.stage_bytes;
-          const uint32_t bar = dsmem_addr(smem_u32(&bars.full[s]), 0);
+          const uint32_t bar = dsmem_addr(smem_u32(&bars.full[s]), lead);
           if (!primed) {
             if (!pair_wait(&bars.empty[s], par, &bars, kWaitLimitCycles)) {
               pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_PRODUCER);
@@ -229,7 +236,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
             load_w(tl.ch, k, st, bar);
           }
           for (int pl = 0; pl < p.np; ++pl)
-            tma_load_3d_pair(st + NA * P_WTILE + pl * hrows * P_BK, tx, bar, k * P_BK,
+            tma_load_3d_pair(st + NA * P_WTILE + pl * hrows * P_BK, tx, bar, (kb0 + k) * P_BK,
                              tl.m0 + static_cast<int>(rank) * hrows, pl);
           ++n;
           if (++s == p.nstages) {
@@ -258,7 +265,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         const uint32_t idesc = p.np == 2 ? idesc_e4m3_e4m3_f32(256, tl.bt) : idesc_e4m3_e5m2_f32(256, tl.bt);
         ok = __all_sync(0xffffffffu, pair_wait(&bars.acc_empty[a], ((it >> 1) & 1) ^ 1, &bars, kWaitLimitCycles));
         tc_fence_after();
-        for (int k = 0; k < p.kb && ok; ++k) {
+        for (int k = 0; k < nkb && ok; ++k) {
           ok = __all_sync(0xffffffffu, pair_wait(&bars.full[s], par, &bars, kWaitLimitCycles));
           if (!ok) break;
           tc_fence_after();
@@ -276,19 +283,19 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
               }
             }
           }
-          if (leader) tc_commit_pair(&bars.empty[s], 3);
+          if (leader) tc_commit_pair(&bars.empty[s], both);
           __syncwarp();
           if (++s == p.nstages) {
             s = 0;
             par ^= 1;
           }
         }
-        if (ok && leader) tc_commit_pair(&bars.acc_full[a], 3);
+        if (ok && leader) tc_commit_pair(&bars.acc_full[a], both);
         __syncwarp();
       }
       if (!ok && lane == 0) pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
       // Both CTAs free their tensor memory at the end: first every product issued has to retire.
-      if (leader) tc_commit_pair(&bars.mma_done, 3);
+      if (leader) tc_commit_pair(&bars.mma_done, both);
       __syncwarp();
     }
     // The odd CTA's wait spans the whole launch: it only gives up once something else has failed.
@@ -306,7 +313,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const int g4 = (lane >> 2) * 4, j4 = lane & 3;   // after the transpose: first channel of four, token of four
     const long long plane = static_cast<long long>(p.M) * p.n_out;
-    const uint32_t acc_empty0 = dsmem_addr(smem_u32(&bars.acc_empty[0]), 0);
+    const uint32_t acc_empty0 = dsmem_addr(smem_u32(&bars.acc_empty[0]), lead);
     if (p.pdl) pdl_wait();
     bool ok = true;
     int it = 0;
@@ -354,37 +361,23 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         ok = false;
         if (lane == 0) pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_EPILOGUE);
       }
-      if (!ok) break;
+      if (!ok && !SPLIT) break;
       tc_fence_after();
       const int nchunk = tl.bt >> 5;
-      for (int c = half; c < nchunk; c += 2) {
-        const int mc = tl.m0 + c * 32;  // first token of this chunk
-        if (mc >= p.M) break;
-        uint32_t v[32];
-        uint32_t u[NA == 2 ? 32 : 1];
-        tmem_ld32(tmem + a * P_ACC_COLS + lane_addr + c * 32, v);
-        if constexpr (NA == 2) tmem_ld32(tmem + a * P_ACC_COLS + lane_addr + tl.bt + c * 32, u);
-        // 8 token rows per lane after the transpose: m = mc + 4 k + j4
-        uint2 rr[EPI == EPI_RESIDUAL ? 8 : 1];
-        if (EPI == EPI_RESIDUAL) {
+      // Accumulator values of chunk c (32 tokens from mc on; v, and u of the second accumulator) -> outputs.  The
+      // residual rows are requested first.
+      auto residual_rows = [&](int mc, uint2 (&rr)[EPI == EPI_RESIDUAL ? 8 : 1]) {
+        if (EPI == EPI_RESIDUAL) {  // 8 token rows per lane after the transpose: m = mc + 4 k + j4
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             const int m = mc + 4 * k + j4;
             if (m < p.M && quad_live) rr[EPI == EPI_RESIDUAL ? k : 0] = *reinterpret_cast<const uint2*>(p.res + m * p.ldres + n_first);
           }
         }
+      };
+      auto finish = [&](int mc, uint32_t (&v)[32], uint32_t (&u)[NA == 2 ? 32 : 1], uint2 (&rr)[EPI == EPI_RESIDUAL ? 8 : 1]) {
         float rs = 1.0f;
         if (p.row_scale) rs = p.row_scale[min(mc + lane, p.M - 1)];
-        tc_wait_ld();
-        if (NA == 1 && p.merge) {
-          for (int pl = 1; pl < p.np; ++pl) {
-            uint32_t v2[32];
-            tmem_ld32(tmem + a * P_ACC_COLS + lane_addr + pl * tl.bt + c * 32, v2);
-            tc_wait_ld();
-#pragma unroll
-            for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(v2[e]));
-          }
-        }
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           float o[4], w[4];
@@ -479,6 +472,65 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
             }
           }
         }
+      };
+      if constexpr (SPLIT) {
+        cluster_sync_all();  // every pair of the cluster has its part: all rings are idle
+        const int nown = (nchunk + p.splits - 1) / p.splits;
+        const uint32_t buf = smem_u32(smem);
+        for (int c = half; c < nchunk; c += 2) {
+          const int owner = c % p.splits;
+          if (owner == split || tl.m0 + c * 32 >= p.M) continue;
+          uint32_t v[32];
+          tmem_ld32(tmem + lane_addr + c * 32, v);
+          const uint32_t dst = dsmem_addr(buf + (((split * nown + c / p.splits) * 32) * 128 + row) * 4, owner * 2 + rank);
+          tc_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + e * 512), "f"(__uint_as_float(v[e])));
+        }
+        __syncwarp();
+        cluster_sync_all();  // every part has arrived
+        const float* part = reinterpret_cast<const float*>(smem);
+        for (int i = half; i < nown; i += 2) {
+          const int c = i * p.splits + split, mc = tl.m0 + c * 32;
+          if (c >= nchunk || mc >= p.M) break;
+          uint32_t v[32], t[32], u[NA == 2 ? 32 : 1];
+          uint2 rr[EPI == EPI_RESIDUAL ? 8 : 1];
+          residual_rows(mc, rr);
+          tmem_ld32(tmem + lane_addr + c * 32, t);
+          tc_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 32; ++e) v[e] = 0u;
+          for (int sp = 0; sp < p.splits; ++sp) {  // split order: bit-reproducible
+            const float* src = part + ((sp * nown + i) * 32) * 128 + row;
+#pragma unroll
+            for (int e = 0; e < 32; ++e)
+              v[e] = __float_as_uint(__uint_as_float(v[e]) + (sp == split ? __uint_as_float(t[e]) : src[e * 128]));
+          }
+          finish(mc, v, u, rr);
+        }
+      } else {
+        for (int c = half; c < nchunk; c += 2) {
+          const int mc = tl.m0 + c * 32;  // first token of this chunk
+          if (mc >= p.M) break;
+          uint32_t v[32];
+          uint32_t u[NA == 2 ? 32 : 1];
+          tmem_ld32(tmem + a * P_ACC_COLS + lane_addr + c * 32, v);
+          if constexpr (NA == 2) tmem_ld32(tmem + a * P_ACC_COLS + lane_addr + tl.bt + c * 32, u);
+          uint2 rr[EPI == EPI_RESIDUAL ? 8 : 1];
+          residual_rows(mc, rr);
+          tc_wait_ld();
+          if (NA == 1 && p.merge) {
+            for (int pl = 1; pl < p.np; ++pl) {
+              uint32_t v2[32];
+              tmem_ld32(tmem + a * P_ACC_COLS + lane_addr + pl * tl.bt + c * 32, v2);
+              tc_wait_ld();
+  #pragma unroll
+              for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(v2[e]));
+            }
+          }
+          finish(mc, v, u, rr);
+        }
       }
       tc_fence_before();
       __syncwarp();
@@ -486,6 +538,11 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     }
   }
 
+  if (SPLIT && warp < 2) {  // the two meeting points of the epilogue warps' exchange
+    __syncwarp();
+    cluster_sync_all();
+    cluster_sync_all();
+  }
   // The pair leaves together: both have read their accumulators, every remote arrival has been made.
   tc_fence_before();
   __syncwarp();
@@ -497,7 +554,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
 }
 
 struct PairPlan {
-  int ch_tiles, tok_tiles, n_big, bt_big, bt_small, nstages, stage_bytes, group, kb, merge;
+  int ch_tiles, tok_tiles, n_big, bt_big, bt_small, nstages, stage_bytes, group, kb, merge, splits, kb_split;
   double cost;  // SM clocks
 };
 
@@ -528,6 +585,8 @@ PairPlan plan_pair(int M, int rows, int K, int na, int np) {
       best.ch_tiles = ch; best.tok_tiles = tt; best.n_big = nb; best.bt_big = 32 * ub; best.bt_small = 32 * us; best.kb = kb;
     }
   }
+  best.splits = 1;
+  best.kb_split = best.kb;
   best.stage_bytes = na * P_WTILE + np * (best.bt_big / 2) * P_BK;
   best.nstages = std::min(P_MAX_STAGES, (P_SMEM - 1024) / best.stage_bytes);
   // L2 groups: as many token tiles as keep the group's planes within a quarter of L2
@@ -536,7 +595,66 @@ PairPlan plan_pair(int M, int rows, int K, int na, int np) {
   return best;
 }
 
+// Clusters of 2 * splits CTAs that the device holds at once.
+int resident_clusters(int splits) {
+  static int cached[5] = {};
+  if (cached[splits] == 0) {
+    auto* k = w8_gemm_pair_kernel<EPI_RESIDUAL, true>;
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM);
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(2 * splits);
+    cfg.blockDim = dim3(P_THREADS);
+    cfg.dynamicSmemBytes = P_SMEM;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2 * splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = host::sm_count() / (2 * splits + 2);
+    }
+    cached[splits] = n;
+  }
+  return cached[splits];
+}
+
+// Split form: one wave of clusters.  The exchange moves (splits - 1) / splits of a 128-channel fp32 tile through
+// distributed shared memory (about 18 bytes per clock and SM) between two cluster meetings.
+PairPlan plan_split(int M, int rows, int K, int np) {
+  PairPlan best{};
+  best.cost = -1.0;
+  const int units = (M + 31) / 32, ch = (rows + 255) / 256, kb = (K + P_BK - 1) / P_BK;
+  for (int sp = 2; sp <= 4; ++sp) {
+    const int cap = resident_clusters(sp), kbs = (kb + sp - 1) / sp;
+    if ((sp - 1) * kbs >= kb) continue;  // no empty split
+    for (int tt = (units + 7) / 8; tt <= units && static_cast<long long>(ch) * tt <= cap; ++tt) {
+      const int ub = (units + tt - 1) / tt;
+      const int stage = P_WTILE + np * 16 * ub * P_BK, ns = std::min(P_MAX_STAGES, (P_SMEM - 1024) / stage);
+      if (sp * ((ub + sp - 1) / sp) * 32 * 512 > ns * stage) continue;  // the parts land in the idle ring
+      const double mma = 64.0 * ub * np, fill = (16384.0 + np * 2048.0 * ub) / 36.0;  // one tile per pair: latency shows
+      const double cost = kbs * std::max(mma, fill) + 32.0 * ub * 512.0 * (sp - 1) / sp / 18.0 + 4000.0;
+      if (best.cost < 0 || cost < best.cost) {
+        best.cost = cost;
+        best.ch_tiles = ch; best.tok_tiles = tt; best.kb = kb; best.splits = sp; best.kb_split = kbs;
+        best.n_big = units % tt == 0 ? tt : units % tt;
+        best.bt_big = 32 * ub;
+        best.bt_small = units % tt == 0 ? 32 * ub : 32 * (ub - 1);
+        best.stage_bytes = stage;
+        best.nstages = ns;
+        best.group = tt;
+      }
+    }
+  }
+  return best;
+}
+
 }  // namespace
+
+double gemm_pair_split_cost(int M, int N, int K, int np) { return plan_split(M, N, K, np).cost; }
 
 // The pair form takes what the one-tile-per-CTA form (w8_gemm.cu) would run in more than one wave: more than one
 // 128-row x 80-token (three planes) or 128-token (two planes) tile per SM.  Within one wave that form is ahead, since
@@ -551,7 +669,7 @@ bool gemm_pair_suits(int M, int N, int nw, int np) {
 int launch_gemm_pair(const GemmCall& c) {
   const int na = (c.epi == EPI_QKV_ROPE || c.epi == EPI_GEGLU || c.epi == EPI_GEGLU_PACKED) ? 2 : 1;
   const bool packed = c.epi == EPI_GEGLU_PACKED || c.epi == EPI_QKV_ROPE;
-  const PairPlan pl = plan_pair(c.M, c.w1 ? 2 * c.N : c.N, c.K, na, c.np);
+  const PairPlan pl = c.split ? plan_split(c.M, c.N, c.K, c.np) : plan_pair(c.M, c.w1 ? 2 * c.N : c.N, c.K, na, c.np);
 
   CUtensorMap tm_w0, tm_w1, tm_big, tm_small;
   if (int rc = host::tensor_map_2d(&tm_w0, c.w0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, c.K, c.N, c.K, P_BK, packed ? 64 : 128)) return rc;
@@ -566,7 +684,7 @@ int launch_gemm_pair(const GemmCall& c) {
 
   PairParams p{};
   p.M = c.M; p.N = c.N; p.K = c.K; p.n_out = c.n_out; p.np = c.np; p.packed = packed ? 1 : 0;
-  p.kb = pl.kb; p.merge = pl.merge; p.nstages = pl.nstages; p.stage_bytes = pl.stage_bytes;
+  p.kb = pl.kb; p.splits = pl.splits; p.kb_split = pl.kb_split; p.merge = pl.merge; p.nstages = pl.nstages; p.stage_bytes = pl.stage_bytes;
   p.ch_tiles = pl.ch_tiles; p.tok_tiles = pl.tok_tiles; p.group = pl.group;
   p.n_big = pl.n_big; p.bt_big = pl.bt_big; p.bt_small = pl.bt_small;
   p.pdl = host::pdl_enabled() ? 1 : 0;
@@ -581,14 +699,16 @@ int launch_gemm_pair(const GemmCall& c) {
   static bool attr_set[64] = {};
   const int dev = host::current_device();
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    for (auto* k : {w8_gemm_pair_kernel<EPI_NONE>, w8_gemm_pair_kernel<EPI_GELU>, w8_gemm_pair_kernel<EPI_RESIDUAL>,
-                    w8_gemm_pair_kernel<EPI_GEGLU>, w8_gemm_pair_kernel<EPI_QKV_ROPE>})
+    for (auto* k : {w8_gemm_pair_kernel<EPI_NONE, false>, w8_gemm_pair_kernel<EPI_GELU, false>, w8_gemm_pair_kernel<EPI_RESIDUAL, false>,
+                    w8_gemm_pair_kernel<EPI_GEGLU, false>, w8_gemm_pair_kernel<EPI_QKV_ROPE, false>, w8_gemm_pair_kernel<EPI_NONE, true>,
+                    w8_gemm_pair_kernel<EPI_GELU, true>, w8_gemm_pair_kernel<EPI_RESIDUAL, true>})
       if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM) != cudaSuccess)
         return host::fail_cuda("cudaFuncSetAttribute(w8_gemm_pair_kernel)");
     attr_set[dev] = true;
   }
   cudaLaunchConfig_t cfg{};
-  const int pairs = std::min(pl.ch_tiles * pl.tok_tiles, std::max(1, host::sm_count() / 2));
+  const int tiles = pl.ch_tiles * pl.tok_tiles;
+  const int pairs = c.split ? tiles * pl.splits : std::min(tiles, std::max(1, host::sm_count() / 2));
   cfg.gridDim = dim3(2 * pairs);
   cfg.blockDim = dim3(P_THREADS);
   cfg.dynamicSmemBytes = P_SMEM;  // always the whole SM: no other user of tensor memory beside this CTA
@@ -601,19 +721,19 @@ int launch_gemm_pair(const GemmCall& c) {
     ++n_attr;
   }
   attr[n_attr].id = cudaLaunchAttributeClusterDimension;
-  attr[n_attr].val.clusterDim.x = 2;
+  attr[n_attr].val.clusterDim.x = 2 * pl.splits;
   attr[n_attr].val.clusterDim.y = 1;
   attr[n_attr].val.clusterDim.z = 1;
   ++n_attr;
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
-  auto* k = w8_gemm_pair_kernel<EPI_NONE>;
+  auto* k = c.split ? w8_gemm_pair_kernel<EPI_NONE, true> : w8_gemm_pair_kernel<EPI_NONE, false>;
   switch (c.epi) {
-    case EPI_GELU: k = w8_gemm_pair_kernel<EPI_GELU>; break;
-    case EPI_RESIDUAL: k = w8_gemm_pair_kernel<EPI_RESIDUAL>; break;
+    case EPI_GELU: k = c.split ? w8_gemm_pair_kernel<EPI_GELU, true> : w8_gemm_pair_kernel<EPI_GELU, false>; break;
+    case EPI_RESIDUAL: k = c.split ? w8_gemm_pair_kernel<EPI_RESIDUAL, true> : w8_gemm_pair_kernel<EPI_RESIDUAL, false>; break;
     case EPI_GEGLU:
-    case EPI_GEGLU_PACKED: k = w8_gemm_pair_kernel<EPI_GEGLU>; break;
-    case EPI_QKV_ROPE: k = w8_gemm_pair_kernel<EPI_QKV_ROPE>; break;
+    case EPI_GEGLU_PACKED: k = w8_gemm_pair_kernel<EPI_GEGLU, false>; break;
+    case EPI_QKV_ROPE: k = w8_gemm_pair_kernel<EPI_QKV_ROPE, false>; break;
     default: break;
   }
   if (cudaLaunchKernelEx(&cfg, k, tm_w0, tm_w1, tm_big, tm_small, p) != cudaSuccess) return host::fail_cuda("launch w8_gemm_pair_kernel");
