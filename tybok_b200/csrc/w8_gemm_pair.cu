@@ -566,9 +566,13 @@ PairPlan plan_pair(int M, int rows, int K, int na, int np) {
   // Up to 128 tokens the planes keep their own columns, as in the one-tile kernel: the sum over K and planes then has
   // the same order in both, so such a call's result does not depend on which of them the tile count selects.
   best.merge = (na == 1 && M <= 128) ? 1 : 0;
-  const int units = (M + 31) / 32, umax = best.merge ? 8 / np : 8 / na;
   const int pairs = std::max(1, host::sm_count() / 2);
   const int ch = (rows + 256 * na - 1) / (256 * na);
+  const int units = (M + 31) / 32;
+  // Those columns are a token tile's planes times its tokens: one accumulator takes 256 of them, and the whole of tensor
+  // memory (384 for three planes of 128 tokens) where no pair has a second tile.  One token tile reads the weights once
+  // (106 x 14336 x 3072: two tiles of 64 tokens 25.2 us, one of 128 20.7 us).
+  const int umax = best.merge ? (ch <= pairs ? 16 / np : 8 / np) : 8 / na;
   const int kb = (K + P_BK - 1) / P_BK;
   auto tile_cost = [&](int u) {
     const double mma = 64.0 * u * na * np, fill = (na * 16384.0 + np * 2048.0 * u) / 52.0;
