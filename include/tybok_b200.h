@@ -68,7 +68,7 @@ size_t tybok_w8a16_workspace_bytes(int M, int N, int K, int dual);
  *            (multiple of 16, <= 256) / the split-K factor (<= 8, one cluster per output tile)
  *   workspace  >= tybok_w8a16_workspace_bytes(...) bytes, 16-byte aligned
  *   status_word  optional device int; set non-zero if a bounded device wait ran out
- * Two launches: tybok_split3 into the workspace, then tybok_w8x3_linear.
+ * Two launches: tybok_split3 into the workspace, then tybok_w8x3_linear (one for few tokens, see below).
  * Replaces the reference's dequant-then-F.linear path
  * (tybok/policies/fastwam/models/policy.py:48-58,127-129) and its W8 GEMM body
  * (tybok/policies/fastwam/kernels/vdit_gemm_core.cu:68, epilogues EPI/RESID). */
@@ -76,6 +76,16 @@ int tybok_w8a16_linear(const void* x, const void* w8, const float* scale, const 
                        int K, int64_t ldx, int64_t ldy, int epilogue, const void* residual, int64_t ldres,
                        const void* gate, int64_t ldgate, int rows_per_gate, int gate_is_bf16, int token_tile,
                        int splits, void* workspace, size_t workspace_bytes, int* status_word, void* stream);
+
+/* The same in ONE launch and without a workspace, for up to 16 tokens on a matrix of at most one 128-row tile per SM (K a
+ * multiple of 8, x 8-byte aligned): the GEMM makes its activation planes itself.  Bit for bit the result of
+ * tybok_w8a16_linear, which takes this form by itself.  TYBOK_ERR_WORKSPACE, and nothing launched, for any other shape.
+ * tybok_w8a16_geglu_packed_direct: the gated FFN front half likewise, to the planes of its output. */
+int tybok_w8a16_linear_direct(const void* x, const void* w8, const float* scale, const void* bias, void* y, int M, int N, int K,
+                              int64_t ldx, int64_t ldy, int epilogue, const void* residual, int64_t ldres, const void* gate,
+                              int64_t ldgate, int rows_per_gate, int gate_is_bf16, int* status_word, void* stream);
+int tybok_w8a16_geglu_packed_direct(const void* x, int64_t ldx, const void* w8_packed, const float* scale_packed, void* h_planes,
+                                    int out_shift, int M, int I, int K, int* status_word, void* stream);
 
 /* Gated FFN front half: h[M,I] = bf16(bf16(gelu_tanh(g)) * u) with g = bf16(x.Wg^T*sg),
  * u = bf16(x.Wu^T*su); both weight matrices are e4m3 [I,K].  Replaces gate_proj / up_proj /

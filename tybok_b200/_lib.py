@@ -106,6 +106,14 @@ SIGNATURES = {
         [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_i64, c_i64, c_int, c_void_p, c_i64,
          c_void_p, c_i64, c_int, c_int, c_int, c_int, c_void_p, c_size_t, c_void_p, c_void_p],
     ),
+    "tybok_w8a16_linear_direct": (
+        c_int,
+        [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_i64, c_i64, c_int, c_void_p, c_i64, c_void_p, c_i64,
+         c_int, c_int, c_void_p, c_void_p],
+    ),
+    "tybok_w8a16_geglu_packed_direct": (
+        c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
+    ),
     "tybok_w8a16_linear_noalloc": (
         c_int,
         [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_i64, c_i64, c_int, c_void_p, c_i64,

@@ -90,8 +90,17 @@ static Tensor w8a16_linear(const Tensor& x, const Tensor& w8, const Tensor& scal
   std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
   shape.back() = n;
   Tensor y = at::empty(shape, x.options());
-  const Tensor planes = at::empty({3 * m * k}, x.options().dtype(at::kByte));
   void* st = stream_of(x);
+  if (m <= 16 && shift == TYBOK_DEFAULT_X_SHIFT && token_tile <= 0 && splits <= 0) {
+    const int rc = tybok_w8a16_linear_direct(ptr(x2), ptr(w8), f32(scale), ptr(bias), ptr(y), m, n, k, x2.stride(0), n, epilogue,
+                                             residual ? ptr(res) : nullptr, residual ? res.stride(0) : 0, ptr(gate), ldgate, rows_per_gate,
+                                             gate_bf16, status_ptr(x.get_device()), st);
+    if (rc != TYBOK_ERR_WORKSPACE) {
+      check(rc, "tybok_w8a16_linear");
+      return y;
+    }
+  }
+  const Tensor planes = at::empty({3 * m * k}, x.options().dtype(at::kByte));
   check(tybok_split3(ptr(x2), x2.stride(0), ptr(planes), m, k, shift, st), "tybok_split3");
   check(tybok_w8x3_linear(ptr(planes), shift, ptr(w8), f32(scale), ptr(bias), ptr(y), n, nullptr, 0, m, n, k, epilogue,
                           residual ? ptr(res) : nullptr, residual ? res.stride(0) : 0, ptr(gate), ldgate, rows_per_gate, gate_bf16,
@@ -147,14 +156,22 @@ class Mlp {
     a.allocate(x2);
     void* st = stream_of(x);
     int* status = status_ptr(x.get_device());
-    check(tybok_split3(ptr(x2), x2.stride(0), a.at(xp), m, k, SHIFT_NORMED, st), "tybok_split3");
-    if (packed_)
-      check(tybok_w8x3_geglu_packed(a.at(xp), SHIFT_NORMED, gu_.wp(), gu_.sp(), nullptr, i, a.at(hp), SHIFT_FFN, m, i, k, 0, 0, status, st),
-            "tybok_w8x3_geglu_packed");
-    else
-      check(tybok_w8x3_geglu(a.at(xp), SHIFT_NORMED, gu_.wp(), gu_.sp(), up_.wp(), up_.sp(), nullptr, i, a.at(hp), SHIFT_FFN, m, i, k, 0, 0,
-                             status, st),
-            "tybok_w8x3_geglu");
+    bool direct = false;  // few tokens: the gate/up GEMM makes its own planes
+    if (m <= 16 && packed_) {
+      const int rc = tybok_w8a16_geglu_packed_direct(ptr(x2), x2.stride(0), gu_.wp(), gu_.sp(), a.at(hp), SHIFT_FFN, m, i, k, status, st);
+      direct = rc != TYBOK_ERR_WORKSPACE;
+      if (direct) check(rc, "tybok_w8a16_geglu_packed");
+    }
+    if (!direct) {
+      check(tybok_split3(ptr(x2), x2.stride(0), a.at(xp), m, k, SHIFT_NORMED, st), "tybok_split3");
+      if (packed_)
+        check(tybok_w8x3_geglu_packed(a.at(xp), SHIFT_NORMED, gu_.wp(), gu_.sp(), nullptr, i, a.at(hp), SHIFT_FFN, m, i, k, 0, 0, status, st),
+              "tybok_w8x3_geglu_packed");
+      else
+        check(tybok_w8x3_geglu(a.at(xp), SHIFT_NORMED, gu_.wp(), gu_.sp(), up_.wp(), up_.sp(), nullptr, i, a.at(hp), SHIFT_FFN, m, i, k, 0, 0,
+                               status, st),
+              "tybok_w8x3_geglu");
+    }
     check(tybok_w8x3_linear(a.at(hp), SHIFT_FFN, down_.wp(), down_.sp(), nullptr, ptr(y), down_.n, nullptr, 0, m, down_.n, i, TYBOK_EPI_NONE,
                             nullptr, 0, nullptr, 0, 1, 0, 0, 0, status, st),
           "tybok_w8x3_linear");

@@ -80,6 +80,9 @@ struct GemmParams {
   int dn_tiles;
   float dn_inv_w, dn_eps;
   const float* bias_f32;  // consumer: [N] fp32 bias in weight-row order, or NULL
+  const __nv_bfloat16* xb;  // few tokens: bf16 activations [M][ldxb] that the idle epilogue warps turn into the planes of
+  long long ldxb;           // every stage themselves (no plane tensor, no launch that makes one), or NULL
+  float xb_mult;            // 2^x_shift
   int merge;     // 1: the planes are one UMMA of N = np*bt whose column groups the epilogue adds
   int epi;
   int pdl;
@@ -168,6 +171,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   const int x_bytes = p.np * p.bt * 128;              // np planes of bt rows x 128 bytes
   const int x_off = p.nw * W_TILE_BYTES;              // activation planes follow the weight tile(s)
   const int stage_bytes = x_off + x_bytes;
+  const int tx_bytes = p.xb ? x_off : stage_bytes;    // what the bulk copies bring
 
   const int t_tile = blockIdx.x, n_tile = blockIdx.y, split = blockIdx.z;
   const int kb0 = split * p.kb_per_split;
@@ -178,7 +182,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     if (p.nw == 2) tma_prefetch_desc(&tm_w1);
     tma_prefetch_desc(&tm_x);
     for (int i = 0; i < MAX_STAGES; ++i) {
-      mbar_init(&bars.full[i], 1);
+      mbar_init(&bars.full[i], p.xb ? 1 + EW : 1);
       mbar_init(&bars.empty[i], 1);
     }
     mbar_init(&bars.tmem_full, 1);
@@ -190,7 +194,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     const int pre = min(ns, nkb);
     for (int i = 0; i < pre; ++i) {
       uint8_t* st = smem + i * stage_bytes;
-      mbar_arrive_expect_tx(&bars.full[i], stage_bytes);
+      mbar_arrive_expect_tx(&bars.full[i], tx_bytes);
       const int k0 = (kb0 + i) * BK;
       tma_load_2d(st, &tm_w0, &bars.full[i], k0, n_tile * BN);
       if (p.nw == 2) tma_load_2d(st + W_TILE_BYTES, &tm_w1, &bars.full[i], k0, n_tile * BN);
@@ -235,8 +239,9 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       // are requested once the programmatic dependency has resolved.
       if (p.pdl) pdl_wait();
       dbg_stage(p.dbg, KID, 2);
-      for (int i = 0; i < pre; ++i)
-        tma_load_3d(smem + i * stage_bytes + x_off, &tm_x, &bars.full[i], (kb0 + i) * BK, t_tile * p.bt, 0);
+      if (!p.xb)
+        for (int i = 0; i < pre; ++i)
+          tma_load_3d(smem + i * stage_bytes + x_off, &tm_x, &bars.full[i], (kb0 + i) * BK, t_tile * p.bt, 0);
       issued = pre;
       for (int i = pre; i < nkb; ++i) {
         const int s = i % ns;
@@ -246,11 +251,11 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           break;
         }
         uint8_t* st = smem + s * stage_bytes;
-        mbar_arrive_expect_tx(&bars.full[s], stage_bytes);
+        mbar_arrive_expect_tx(&bars.full[s], tx_bytes);
         const int k0 = (kb0 + i) * BK;
         tma_load_2d(st, &tm_w0, &bars.full[s], k0, n_tile * BN);
         if (p.nw == 2) tma_load_2d(st + W_TILE_BYTES, &tm_w1, &bars.full[s], k0, n_tile * BN);
-        tma_load_3d(st + x_off, &tm_x, &bars.full[s], k0, t_tile * p.bt, 0);
+        if (!p.xb) tma_load_3d(st + x_off, &tm_x, &bars.full[s], k0, t_tile * p.bt, 0);
         issued = i + 1;
       }
       if (!ok || bars.abort) {
@@ -397,6 +402,43 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           }
         }
       }
+    }
+    if (EW == EPI_WARPS_WIDE && p.xb) {
+      // bt == 16 token rows: warp `ew` makes row ew of every plane of every stage, four values per lane, written where the
+      // bulk copy would have put them (128-byte swizzle).  Four stages of loads are in flight at a time.
+      const int row = ew;
+      const bool real = m_base + row < p.M;
+      const __nv_bfloat16* xr = p.xb + static_cast<long long>(m_base + row) * p.ldxb;
+      bool fine = true;
+      for (int i0 = 0; i0 < nkb && fine; i0 += 4) {
+        uint2 raw[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int kx = (kb0 + i0 + u) * BK + lane * 4;
+          raw[u] = i0 + u < nkb && real && kx < p.K ? *reinterpret_cast<const uint2*>(xr + kx) : make_uint2(0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u, s = i % ns;
+          if (i < nkb && fine) {
+            if (i >= ns) fine = __all_sync(0xffffffffu, wait_or_abort(&bars.empty[s], ((i / ns) & 1) ^ 1, &bars.abort));
+            if (fine) {
+              const float xs[4] = {__uint_as_float(raw[u].x << 16) * p.xb_mult, __uint_as_float(raw[u].x & 0xffff0000u) * p.xb_mult,
+                                   __uint_as_float(raw[u].y << 16) * p.xb_mult, __uint_as_float(raw[u].y & 0xffff0000u) * p.xb_mult};
+              uint32_t w1, w2, w3;
+              split3_quad(xs, w1, w2, w3);
+              uint8_t* dst = smem + s * stage_bytes + x_off + row * 128 + (((lane >> 2) ^ (row & 7)) << 4) + (lane & 3) * 4;
+              *reinterpret_cast<uint32_t*>(dst) = w1;
+              *reinterpret_cast<uint32_t*>(dst + 16 * 128) = w2;
+              *reinterpret_cast<uint32_t*>(dst + 32 * 128) = w3;
+              fence_proxy_async();  // the products read them through the async proxy
+              __syncwarp();
+              if (lane == 0) mbar_arrive(&bars.full[s]);
+            }
+          }
+        }
+      }
+      if (!fine && lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_CONVERT);
     }
     bool ok = __all_sync(0xffffffffu, wait_or_abort(&bars.tmem_full, 0, &bars.abort, p.epi_wait_limit));
     if (!ok && lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_EPILOGUE);
@@ -796,10 +838,11 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
                        const void* res, long long ldres, const void* gate, long long ldgate, int rows_per_gate,
                        int gate_bf16, int x_shift, int out_shift, int force_bt, int force_splits, int* status,
                        cudaStream_t stream, const RopeEpi* rope = nullptr, bool check_only = false,
-                       const float* row_scale = nullptr, const NormFold* fold = nullptr) {
+                       const float* row_scale = nullptr, const NormFold* fold = nullptr, const void* x_bf16 = nullptr,
+                       long long ldx = 0) {
   const int np = row_scale ? 2 : 3;  // two e4m3 planes with a per-token scale, or three e5m2 planes
   const int nw = w1 ? 2 : 1;
-  if (!planes || !w0 || !s0 || (!y && !y_planes && !rope)) return host::fail(TYBOK_ERR_ARG, "w8 gemm: null pointer argument");
+  if ((!planes && !x_bf16) || !w0 || !s0 || (!y && !y_planes && !rope)) return host::fail(TYBOK_ERR_ARG, "w8 gemm: null pointer argument");
   if (M <= 0 || N <= 0 || K <= 0) return host::fail(TYBOK_ERR_ARG, "w8 gemm: M, N, K must be positive");
   if (K % 16 != 0) return host::fail(TYBOK_ERR_ARG, "w8 gemm: K must be a multiple of 16 (TMA row pitch)");
   if (N % 4 != 0) return host::fail(TYBOK_ERR_ARG, "w8 gemm: N must be a multiple of 4 (vector epilogue)");
@@ -867,8 +910,10 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   tm_w1 = tm_w0;
   if (nw == 2)
     if (int rc = host::tensor_map_2d(&tm_w1, w1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, N, K, BK, BN)) return rc;
-  if (int rc = host::tensor_map_3d(&tm_x, planes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, M, np, K,
-                                   static_cast<uint64_t>(M) * K, BK, pl.bt, np))
+  if (x_bf16)
+    tm_x = tm_w0;  // not used
+  else if (int rc = host::tensor_map_3d(&tm_x, planes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, M, np, K,
+                                        static_cast<uint64_t>(M) * K, BK, pl.bt, np))
     return rc;
 
   GemmParams p{};
@@ -882,6 +927,7 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   p.y = static_cast<__nv_bfloat16*>(y); p.ldy = ldy; p.y_planes = static_cast<uint8_t*>(y_planes);
   p.res = static_cast<const __nv_bfloat16*>(res); p.ldres = ldres;
   p.gate = gate; p.ldgate = ldgate; p.rows_per_gate = rows_per_gate > 0 ? rows_per_gate : 1; p.gate_bf16 = gate_bf16;
+  p.xb = static_cast<const __nv_bfloat16*>(x_bf16); p.ldxb = ldx; p.xb_mult = ldexpf(1.0f, x_shift);
   p.status = status;
   p.trace = host::trace_buffer();
   p.dbg = host::counter_buffer();
@@ -930,6 +976,14 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
     return host::fail_cuda("launch w8_gemm_kernel");
   host::count_launch();
   return TYBOK_OK;
+}
+
+// Up to 16 tokens and at most one tile per SM: the GEMM makes its activation planes itself (GemmParams::xb).  One launch
+// instead of two (1 x 2560 x 2048 as one call: 8.9 -> 6.4 us, the launch and the allocation of the planes); beyond 16
+// tokens every CTA's share of the conversions, which all tiles repeat, outgrows the launch it saves.
+static bool takes_bf16(int M, int N, int nw, int K, const void* x, long long ldx) {
+  return M <= 16 && !gemm_pair_suits(M, N, nw, 3) && (static_cast<long long>(N) + BN - 1) / BN <= host::sm_count() && K % 8 == 0 &&
+         ldx % 4 == 0 && ldx >= K && !(reinterpret_cast<uintptr_t>(x) & 7);
 }
 
 static int launch_split3(const void* x, long long ldx, void* planes, int M, int K, int shift, cudaStream_t stream) {
@@ -1123,6 +1177,27 @@ int tybok_w8x3_qkv_rope_adarms(const void* u_planes, int u_shift, const float* s
                          nullptr, &f);
 }
 
+int tybok_w8a16_linear_direct(const void* x, const void* w8, const float* scale, const void* bias, void* y, int M, int N, int K,
+                              int64_t ldx, int64_t ldy, int epilogue, const void* residual, int64_t ldres, const void* gate,
+                              int64_t ldgate, int rows_per_gate, int gate_is_bf16, int* status_word, void* stream) {
+  if (!x || M <= 0 || K <= 0 || N <= 0 || !tb::takes_bf16(M, N, 1, K, x, ldx))
+    return tb::host::fail(TYBOK_ERR_WORKSPACE, "w8a16_linear_direct: not a call of up to 16 tokens on one tile per SM");
+  if (epilogue != TYBOK_EPI_NONE && epilogue != TYBOK_EPI_GELU && epilogue != TYBOK_EPI_RESIDUAL)
+    return tb::host::fail(TYBOK_ERR_ARG, "w8x3_linear: unknown epilogue");
+  return tb::launch_gemm(nullptr, w8, nullptr, scale, nullptr, bias, y, nullptr, M, N, K, ldy, epilogue, residual, ldres, gate, ldgate,
+                         rows_per_gate, gate_is_bf16, TYBOK_DEFAULT_X_SHIFT, 0, 0, 0, status_word, static_cast<cudaStream_t>(stream),
+                         nullptr, false, nullptr, nullptr, x, ldx);
+}
+
+int tybok_w8a16_geglu_packed_direct(const void* x, int64_t ldx, const void* w8_packed, const float* scale_packed, void* h_planes,
+                                    int out_shift, int M, int I, int K, int* status_word, void* stream) {
+  if (!x || M <= 0 || K <= 0 || I <= 0 || !tb::takes_bf16(M, 2 * I, 1, K, x, ldx))
+    return tb::host::fail(TYBOK_ERR_WORKSPACE, "w8a16_geglu_packed_direct: not a call of up to 16 tokens on one tile per SM");
+  return tb::launch_gemm(nullptr, w8_packed, nullptr, scale_packed, nullptr, nullptr, nullptr, h_planes, M, 2 * I, K, I, tb::EPI_GEGLU_PACKED,
+                         nullptr, 0, nullptr, 0, 1, 0, TYBOK_DEFAULT_X_SHIFT, out_shift, 0, 0, status_word, static_cast<cudaStream_t>(stream),
+                         nullptr, false, nullptr, nullptr, x, ldx);
+}
+
 int tybok_w8a16_linear(const void* x, const void* w8, const float* scale, const void* bias, void* y, int M, int N,
                        int K, int64_t ldx, int64_t ldy, int epilogue, const void* residual, int64_t ldres,
                        const void* gate, int64_t ldgate, int rows_per_gate, int gate_is_bf16, int token_tile,
@@ -1130,6 +1205,11 @@ int tybok_w8a16_linear(const void* x, const void* w8, const float* scale, const 
   if (!workspace || workspace_bytes < tybok_w8a16_workspace_bytes(M, N, K, 0))
     return tb::host::fail(TYBOK_ERR_WORKSPACE, "w8a16_linear: workspace must hold 3*M*K bytes of activation planes");
   const int shift = TYBOK_DEFAULT_X_SHIFT;
+  if (token_tile <= 0 && splits <= 0) {
+    const int rc = tybok_w8a16_linear_direct(x, w8, scale, bias, y, M, N, K, ldx, ldy, epilogue, residual, ldres, gate, ldgate, rows_per_gate,
+                                             gate_is_bf16, status_word, stream);
+    if (rc != TYBOK_ERR_WORKSPACE) return rc;
+  }
   // Refuse a bad GEMM argument before the split kernel has written anything.
   if (int rc = tb::check_linear_args(workspace, w8, scale, bias, y, ldy, M, N, K, epilogue, residual, ldres, gate, ldgate,
                                      rows_per_gate, gate_is_bf16, token_tile, splits))
