@@ -1,5 +1,6 @@
 """Attention with one key head, whose (token, head) pairs are the rows of the key-loop form: suffix batches around the
-size where it takes over from the cluster form, ragged row counts, masked keys, against a plain fp32 reference."""
+size where it takes over from the cluster form, ragged row counts, masked keys, and single suffixes of the cluster form, against
+a plain fp32 reference."""
 
 import pytest
 import torch
@@ -8,7 +9,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("b,l,keys,h,d", [(3, 50, 594, 8, 256), (4, 50, 594, 8, 256), (9, 50, 641, 8, 256), (32, 50, 994, 8, 256),
-                                          (40, 1, 130, 3, 256), (17, 128, 257, 5, 256), (2, 129, 129, 7, 256), (2, 33, 200, 8, 128)])
+                                          (40, 1, 130, 3, 256), (17, 128, 257, 5, 256), (2, 129, 129, 7, 256), (2, 33, 200, 8, 128),
+                                          # output columns split over two clusters per head, or not: around the clusters that fit
+                                          (1, 50, 896, 8, 256), (1, 50, 1018, 8, 256), (1, 56, 1018, 7, 256), (1, 7, 1024, 8, 256)])
 def test_one_key_head_matches_fp32(b, l, keys, h, d):
     from tybok_b200 import ops
 
