@@ -831,6 +831,12 @@ __device__ __forceinline__ float pf_exp2(float x) {
   return y;
 }
 
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+
 // 32 bytes of registers (r[first] ..) to global memory: one 256-bit store, or two of 128 bits where the caller's tensor is
 // only 16-byte aligned.
 template <int N>
@@ -1045,7 +1051,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     const int khf = SHORT ? q >> 1 : hf;
     const int srow = SHORT ? (q & 1) * 32 + lane : row;
     const bool slive = SHORT ? (q & 1) * 32 < nvalid : live;
-    // All walking warps take the blocks in step (one named barrier per block), whatever the waits
+    // The two warps of a row take the blocks in step (one named barrier per block), whatever the waits
     // return: after a failed wait `ok` stays false and the abort flag makes every later wait return.
     bool ok = true;
     float m_ref = -1e30f, l = 0.f;
@@ -1061,7 +1067,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       uint32_t bits[KW];
 #pragma unroll
       for (int w = 0; w < KW; ++w) bits[w] = bars.valid[(2 * j + khf) * KW + w];
-      float mx = -1e30f;
+      float mx = -1e30f, mx1 = -1e30f;
       if (ok && slive) {
         tc_fence_after();
 #pragma unroll
@@ -1069,9 +1075,12 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         tc_wait_ld();
 #pragma unroll
         for (int w = 0; w < KW; ++w) {
-          if (bits[w] == 0xffffffffu) {
+          if (bits[w] == 0xffffffffu) {  // two chains of three-way maxima: the warp has nothing else to do meanwhile
 #pragma unroll
-            for (int e = 0; e < 32; ++e) mx = fmaxf(mx, __uint_as_float(v[w][e]));
+            for (int e = 0; e < 32; e += 4) {
+              mx = max3(mx, __uint_as_float(v[w][e]), __uint_as_float(v[w][e + 1]));
+              mx1 = max3(mx1, __uint_as_float(v[w][e + 2]), __uint_as_float(v[w][e + 3]));
+            }
           } else if (bits[w] != 0u) {
 #pragma unroll
             for (int e = 0; e < 32; ++e)
@@ -1079,10 +1088,10 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
           }
         }
       }
-      bars.hmax[s][khf][srow] = mx;
+      bars.hmax[s][khf][srow] = fmaxf(mx, mx1);
       tc_fence_before();
-      if (SHORT) asm volatile("bar.sync 2, 128;" ::: "memory");
-      else asm volatile("bar.sync 1, 256;" ::: "memory");  // both halves of every row have read S_j
+      // Both halves of these 32 rows have read S_j: the two warps of the rows meet, nobody else.
+      asm volatile("bar.sync %0, 64;" ::"r"(2 + (SHORT ? q & 1 : q)) : "memory");
       if (ok && slive) {
         tc_fence_after();
         const float m_blk = fmaxf(bars.hmax[s][0][srow], bars.hmax[s][1][srow]) * p.scale_log2e;  // scale > 0
@@ -1263,11 +1272,6 @@ __device__ __forceinline__ void f32x2_split(uint64_t v, float& lo, float& hi) { 
 __device__ __forceinline__ uint64_t f32x2_fma(uint64_t a, uint64_t b, uint64_t c) {
   uint64_t r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
   return r;
 }
 __device__ __forceinline__ uint64_t f32x2_add(uint64_t a, uint64_t b) {
