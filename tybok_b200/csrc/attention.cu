@@ -881,7 +881,7 @@ struct __align__(8) PrefillBars {
 // and therefore has the SM's tensor memory to itself: its shared memory leaves no room for another CTA that allocates any.
 // SHORT (head_dim 128, up to 64 query rows): with one row per tensor-memory lane, 64 rows keep two of the four
 // sub-partitions of the SM busy, and their special-function units set the pace: 2 x 64 exponentials a lane and block at
-// 4 per clock are 1024 of the 2900 clocks of a block.  Here the Q tile holds the rows twice, so lanes 64..127 have the same
+// 4 per clock are 1024 of some 2300 clocks of a block.  Here the Q tile holds the rows twice, so lanes 64..127 have the same
 // scores (a product of 128 rows costs what one of 64 does); lanes 0..63 take the first 64 keys of every block, lanes
 // 64..127 the others, one warp per sub-partition.  The second half of P reaches its rows' lanes through shared memory, as
 // an operand of its own in the same sequence of products, so results are the same bit for bit.
