@@ -875,6 +875,7 @@ struct __align__(8) PrefillBars {
   uint32_t valid[PF_MAX_KEYS / 32];
   float hmax[2][2][AT_BQ];  // [block parity][half of the block's keys][row]: maximum of the valid scores
   float hsum[2][AT_BQ];     // [half][row]: sum of that half's probabilities over all blocks
+  float part[2][2][64];     // SHORT: [block parity][half][row]: sum of the half's first 32 keys
 };
 
 // HD = head dimension, 128 or 256.  Either way a CTA takes ALL 512 tensor-memory columns of its SM
@@ -883,9 +884,9 @@ struct __align__(8) PrefillBars {
 // sub-partitions of the SM busy, and their special-function units set the pace: 2 x 64 exponentials a lane and block at
 // 4 per clock are 1024 of some 2300 clocks of a block.  Here the Q tile holds the rows twice, so lanes 64..127 have the same
 // scores (a product of 128 rows costs what one of 64 does); lanes 0..63 take the first 64 keys of every block, lanes
-// 64..127 the others, one warp per sub-partition.  The second half of P reaches its rows' lanes through shared memory, as
+// 64..127 the others, two warps per sub-partition and 32 keys per thread.  The second half of P reaches its rows' lanes through shared memory, as
 // an operand of its own in the same sequence of products, so results are the same bit for bit.
-// 50 queries, 4146 keys, 24 heads: 52.0 -> 45.4 us.
+// 50 queries, 4146 keys, 24 heads: 52.0 -> 42.0 us (64 keys per thread on half of the warps: 43.8 us), 50 keys 6.9 -> 6.5 us.
 template <int HD, bool SHORT = false>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
@@ -901,7 +902,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   constexpr int PF_BK = pf_bk(HD);          // keys per block
   constexpr int PF_KCHUNK = pf_kchunk(HD);
   constexpr int PF_KV = NCH * PF_KCHUNK;    // one K or V block: PF_BK keys x HD
-  constexpr int KW = PF_BK / 64;            // 32-key words per thread and block (two threads per query row)
+  constexpr int KW = SHORT ? 1 : PF_BK / 64;  // 32-key words per thread and block (two threads per query row; SHORT: four)
   constexpr int Q_TILE = NCH * AT_CHUNK;    // 128 query rows x HD
   constexpr int T_COLS = 512;               // tensor memory: S / P at columns 0 and PF_BK, O from column 256
   constexpr int OCH = HD / 64;              // 32-column chunks of O per thread (its half of the row)
@@ -926,7 +927,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       mbar_init(&bars.v_full[i], 1);
       mbar_init(&bars.v_empty[i], 1);
       mbar_init(&bars.s_full[i], 1);
-      mbar_init(&bars.p_full[i], SHORT ? 4 : 8);
+      mbar_init(&bars.p_full[i], 8);
     }
     mbar_init(&bars.o_done, 1);
     mbar_init(&bars.all_done, 1);
@@ -1056,17 +1057,28 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     const int row = q * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const bool live = q * 32 < nvalid;  // warp-uniform: this quadrant holds real query rows
-    // The same three while the blocks go by (SHORT: by copy of the row, and one group of four warps only).
-    const bool walks = !SHORT || hf == 0;
+    // The same three while the blocks go by (SHORT: by copy of the row), and the thread's first 32-key word of a block.
     const int khf = SHORT ? q >> 1 : hf;
     const int srow = SHORT ? (q & 1) * 32 + lane : row;
     const bool slive = SHORT ? (q & 1) * 32 < nvalid : live;
-    // The two warps of a row take the blocks in step (one named barrier per block), whatever the waits
+    const int kw0 = SHORT ? 2 * khf + hf : khf * KW;
+    // SHORT: a half block's sum runs over 64 keys in order, and two threads have them.  The first leaves the sum of its 32
+    // behind; the second keeps its 16 pair sums and adds them to that one block later, after the warps have met again.
+    float tail[SHORT ? 16 : 1];
+    auto finish_sum = [&](int j, float& l) {
+      if constexpr (SHORT) {
+        float sum = bars.part[j & 1][khf][srow];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) sum += tail[e];
+        l += sum;
+      }
+    };
+    // The warps of a row take the blocks in step (one named barrier per block), whatever the waits
     // return: after a failed wait `ok` stays false and the abort flag makes every later wait return.
     bool ok = true;
     float m_ref = -1e30f, l = 0.f;
 #pragma unroll 1
-    for (int j = 0; j < nkb && walks; ++j) {
+    for (int j = 0; j < nkb; ++j) {
       const int s = j & 1;
       if (ok && !__all_sync(0xffffffffu, at_wait(&bars.s_full[s], (j >> 1) & 1, &bars.abort))) {
         ok = false;
@@ -1076,12 +1088,12 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       uint32_t v[KW][32];
       uint32_t bits[KW];
 #pragma unroll
-      for (int w = 0; w < KW; ++w) bits[w] = bars.valid[(2 * j + khf) * KW + w];
+      for (int w = 0; w < KW; ++w) bits[w] = bars.valid[j * (PF_BK / 32) + kw0 + w];
       float mx = -1e30f, mx1 = -1e30f;
       if (ok && slive) {
         tc_fence_after();
 #pragma unroll
-        for (int w = 0; w < KW; ++w) tmem_ld32(tmem + lane_addr + s * PF_BK + (khf * KW + w) * 32, v[w]);
+        for (int w = 0; w < KW; ++w) tmem_ld32(tmem + lane_addr + s * PF_BK + (kw0 + w) * 32, v[w]);
         tc_wait_ld();
 #pragma unroll
         for (int w = 0; w < KW; ++w) {
@@ -1098,20 +1110,22 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
           }
         }
       }
-      bars.hmax[s][khf][srow] = fmaxf(mx, mx1);
+      bars.hmax[s][khf][SHORT ? srow + 64 * hf : srow] = fmaxf(mx, mx1);
       tc_fence_before();
-      // Both halves of these 32 rows have read S_j: the two warps of the rows meet, nobody else.
-      asm volatile("bar.sync %0, 64;" ::"r"(2 + (SHORT ? q & 1 : q)) : "memory");
+      // All of S_j in these 32 rows has been read: the warps of the rows meet, nobody else.
+      asm volatile("bar.sync %0, %1;" ::"r"(2 + (SHORT ? q & 1 : q)), "n"(SHORT ? 128 : 64) : "memory");
       if (ok && slive) {
         tc_fence_after();
-        const float m_blk = fmaxf(bars.hmax[s][0][srow], bars.hmax[s][1][srow]) * p.scale_log2e;  // scale > 0
+        float m_blk = fmaxf(bars.hmax[s][0][srow], bars.hmax[s][1][srow]);
+        if (SHORT) m_blk = fmaxf(m_blk, fmaxf(bars.hmax[s][0][srow + 64], bars.hmax[s][1][srow + 64]));
+        m_blk *= p.scale_log2e;  // scale > 0
+        if (SHORT && hf && j > 0) finish_sum(j - 1, l);
         if (j == 0) {
           m_ref = m_blk;
         } else {
           const bool grow = m_blk > m_ref + PF_RESCALE;
           if (__any_sync(0xffffffffu, grow)) {
-            // Rescale this thread's half of the O row (SHORT: the row, by the thread in its lane) and
-            // its sum to the new reference maximum;
+            // Rescale this thread's half of the O row (SHORT: by the threads in its lane) and its sum to the new reference maximum;
             // rows of the warp that keep theirs multiply by one.  The previous P.V product must
             // have landed (it is at most one phase away, see PrefillBars::o_done).
             if (!__all_sync(0xffffffffu, at_wait(&bars.o_done, (j - 1) & 1, &bars.abort))) {
@@ -1121,7 +1135,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
               tc_fence_after();
               const float f = grow ? pf_exp2(m_ref - m_blk) : 1.0f;
 #pragma unroll 1
-              for (int c = SHORT ? 2 * OCH * khf : khf * OCH; c < (SHORT ? 2 * OCH : khf * OCH + OCH); ++c) {
+              for (int c = hf * OCH; c < (SHORT && khf ? 0 : hf * OCH + OCH); ++c) {
                 uint32_t o[32];
                 tmem_ld32(t_o + lane_addr + c * 32, o);
                 tc_wait_ld();
@@ -1138,6 +1152,10 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       }
       if (ok && slive) {
         float sum = 0.f;
+        auto add = [&](int e, float two) {
+          if (SHORT && hf) tail[SHORT ? e >> 1 : 0] = two;
+          else sum += two;
+        };
 #pragma unroll
         for (int w = 0; w < KW; ++w) {
           uint32_t pk[16];
@@ -1146,19 +1164,22 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             for (int e = 0; e < 32; e += 2) {
               const float p0 = pf_exp2(__uint_as_float(v[w][e]) * p.scale_log2e - m_ref);
               const float p1 = pf_exp2(__uint_as_float(v[w][e + 1]) * p.scale_log2e - m_ref);
-              sum += p0 + p1;
+              add(e, p0 + p1);
               const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
               pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
             }
           } else if (bits[w] == 0u) {
 #pragma unroll
-            for (int e = 0; e < 16; ++e) pk[e] = 0u;
+            for (int e = 0; e < 16; ++e) {
+              pk[e] = 0u;
+              add(2 * e, 0.f);
+            }
           } else {
 #pragma unroll
             for (int e = 0; e < 32; e += 2) {
               const float p0 = ((bits[w] >> e) & 1u) ? pf_exp2(__uint_as_float(v[w][e]) * p.scale_log2e - m_ref) : 0.f;
               const float p1 = ((bits[w] >> (e + 1)) & 1u) ? pf_exp2(__uint_as_float(v[w][e + 1]) * p.scale_log2e - m_ref) : 0.f;
-              sum += p0 + p1;
+              add(e, p0 + p1);
               const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
               pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
             }
@@ -1169,13 +1190,14 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             uint8_t* dst = spk + s * AT_CHUNK + srow * 128;  // free: S_j was issued after the products of block j - 2
 #pragma unroll
             for (int i = 0; i < 4; ++i)
-              *reinterpret_cast<uint4*>(dst + (((w * 4 + i) ^ (srow & 7)) << 4)) = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
+              *reinterpret_cast<uint4*>(dst + (((hf * 4 + i) ^ (srow & 7)) << 4)) = make_uint4(pk[4 * i], pk[4 * i + 1], pk[4 * i + 2], pk[4 * i + 3]);
           } else {
-            tmem_st16(tmem + lane_addr + s * PF_BK + (khf * KW + w) * 16, pk);
+            tmem_st16(tmem + lane_addr + s * PF_BK + (kw0 + w) * 16, pk);
           }
         }
         if (SHORT && khf) fence_proxy_async();  // read by the products
-        l += sum;
+        if (!SHORT) l += sum;
+        else if (!hf) bars.part[s][khf][srow] = sum;
         tc_wait_st();
       }
       tc_fence_before();
@@ -1183,7 +1205,15 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       if (ok && lane == 0) mbar_arrive(&bars.p_full[s]);
       if (tr && tid == 128 && j < 6) tr[2 + 2 * j] = clock64();
     }
-    if (walks) bars.hsum[khf][srow] = l;
+    if (SHORT) {
+      asm volatile("bar.sync %0, 128;" ::"r"(2 + (q & 1)) : "memory");
+      if (hf) {
+        if (ok && slive) finish_sum(nkb - 1, l);
+        bars.hsum[khf][srow] = l;
+      }
+    } else {
+      bars.hsum[khf][srow] = l;
+    }
     if (ok && !__all_sync(0xffffffffu, at_wait(&bars.all_done, 0, &bars.abort))) ok = false;
     if (!ok && lane == 0) {
       bars.abort = 1;
