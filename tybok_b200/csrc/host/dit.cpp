@@ -28,8 +28,6 @@ class DitBlock {
   Tensor forward(const Tensor& x, const Tensor& mods, const Tensor& cos, const Tensor& sin, const Tensor& k_cache, const Tensor& v_cache,
                  int key_off, const OptTensor& k_rows, const OptTensor& v_rows, const OptTensor& cross_k, const OptTensor& cross_v,
                  const OptTensor& ctx_valid) const {
-    require_cuda(x, "dit_block");
-    const c10::cuda::CUDAGuard guard(x.device());
     const Tensor x0 = rows_of(x);
     const int m = x0.size(0), a = heads_ * hd_, h = h_;
     if (!is_bf16(x0) || x0.size(1) != h) type_error("DiTBlock: x must be bf16 [S, H]");
@@ -37,8 +35,21 @@ class DitBlock {
     for (const Tensor* t : {&cos, &sin})
       if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() != static_cast<int64_t>(m) * (hd_ / 2))
         type_error("DiTBlock: cos/sin must be contiguous fp32 [S, D/2]");
-    check_cache(k_cache);
-    check_cache(v_cache);
+    // The kernels are told one key count and one capacity per pair of keys and values; both sides must have them.
+    const int lk = k_rows ? static_cast<int>(k_rows->size(0)) + m : key_off + m;
+    const int lc = ctx_valid ? static_cast<int>(ctx_valid->size(-1)) : cross_k ? static_cast<int>(cross_k->size(-2)) : 0;
+    check_pair(k_cache, v_cache, false);
+    if (k_rows.has_value() != v_rows.has_value()) value_error("DiTBlock: key rows come with value rows");
+    if (k_rows) check_pair(*k_rows, *v_rows, true);
+    if (cross_k.has_value() != cross_v.has_value()) value_error("DiTBlock: cross keys come with cross values");
+    if (cross_k) {
+      check_pair(*cross_k, *cross_v, cross_k->dim() == 2);
+      if (cross_k->size(-2) < lc) value_error("DiTBlock: the context mask is longer than the cross keys");
+    }
+    if (ctx_valid && (ctx_valid->scalar_type() != at::kByte || !ctx_valid->is_contiguous() || ctx_valid->numel() != lc))
+      type_error("attention: key_valid must be contiguous uint8 [B, Lk]");
+    require_cuda(x, "dit_block");
+    const c10::cuda::CUDAGuard guard(x.device());
     const int lcap = k_cache.size(-2);
     void* st = stream_of(x);
     int* status = status_ptr(x.get_device());
@@ -46,8 +57,6 @@ class DitBlock {
     const float scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(hd_)));
 
     // ---- workspace: normed planes | union of (qkv, q, attention planes) and the FFN's hidden planes | two residual rows
-    const int lk = k_rows ? static_cast<int>(k_rows->size(0)) + m : key_off + m;
-    const int lc = ctx_valid ? static_cast<int>(ctx_valid->size(-1)) : cross_k ? static_cast<int>(cross_k->size(-2)) : 0;
     size_t at_ws = 0;
     if (hd_ != 128) at_ws = std::max(tybok_attention_workspace_bytes(1, m, heads_, lk), lc ? tybok_attention_workspace_bytes(1, m, heads_, lc) : 0);
     Arena ar;
@@ -67,8 +76,6 @@ class DitBlock {
     gemm(two, ar.at(np), ar.at(rs), qkv_, ar.at(qkv), nullptr, m, TYBOK_EPI_NONE, status, st);
     int off = key_off;
     if (k_rows) {
-      check_rows(*k_rows, a);
-      check_rows(*v_rows, a);
       const int lv = k_rows->size(0);
       off = lv % 128;
       if (off)
@@ -100,17 +107,11 @@ class DitBlock {
       check(tybok_qknorm_rope_store(ar.at(qkv), a, 0, -1, -1, ptr(cnq_), nullptr, eps_, nullptr, nullptr, ar.at(q), nullptr, nullptr, 1, m,
                                     heads_, hd_, 0, 0, st),
             "tybok_qknorm_rope_store");
-      if (ctx_valid && (ctx_valid->scalar_type() != at::kByte || !ctx_valid->is_contiguous() || ctx_valid->numel() != lc))
-        type_error("attention: key_valid must be contiguous uint8 [B, Lk]");
       if (cross_k->dim() == 2) {
-        check_rows(*cross_k, a);
-        check_rows(*cross_v, a);
         check(tybok_attention_rows(ar.at(q), ptr(*cross_k), ptr(*cross_v), lc, nullptr, nullptr, 0, ptr(ctx_valid), nullptr, ar.at(ap),
                                    SHIFT_ATTN, m, heads_, hd_, lc, scale, status, st),
               "tybok_attention_rows");
       } else {
-        check_cache(*cross_k);
-        check_cache(*cross_v);
         check(tybok_attention(ar.at(q), ptr(*cross_k), ptr(*cross_v), ptr(ctx_valid), nullptr, ar.at(ap), SHIFT_ATTN, 1, m, heads_, heads_,
                               hd_, lc, cross_k->size(-2), scale, ar.at(ws), at_ws, status, st),
               "tybok_attention");
@@ -124,12 +125,16 @@ class DitBlock {
   }
 
  private:
-  void check_cache(const Tensor& t) const {
-    if (!is_bf16(t) || !t.is_contiguous() || t.dim() < 3 || t.size(-1) != hd_ || t.size(-3) != heads_)
-      type_error("DiTBlock: caches must be contiguous bf16 [1, heads, Lcap, D]");
-  }
-  static void check_rows(const Tensor& t, int a) {
-    if (!is_bf16(t) || !t.is_contiguous() || t.dim() != 2 || t.size(1) != a) type_error("DiTBlock: key / value rows must be contiguous bf16 [L, heads*D]");
+  // Keys and values of one shape: head-major [1, heads, Lcap, D] (a tail cache without the 1), or rows [L, heads*D].
+  void check_pair(const Tensor& k, const Tensor& v, bool rows) const {
+    for (const Tensor* t : {&k, &v}) {
+      if (rows && (!is_bf16(*t) || !t->is_contiguous() || t->dim() != 2 || t->size(1) != heads_ * hd_))
+        type_error("DiTBlock: key / value rows must be contiguous bf16 [L, heads*D]");
+      if (!rows && (!is_bf16(*t) || !t->is_contiguous() || t->dim() < 3 || t->size(-1) != hd_ || t->size(-3) != heads_ ||
+                    t->numel() != t->size(-2) * heads_ * hd_))
+        type_error("DiTBlock: caches must be contiguous bf16 [1, heads, Lcap, D]");
+    }
+    if (k.size(-2) != v.size(-2)) value_error("DiTBlock: keys and values differ in length");
   }
   void norm_modulate(const void* x, int64_t ld, const void* shift, const void* scale, int m, bool two, void* planes, void* rs, void* st) const {
     if (two)

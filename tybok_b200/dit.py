@@ -205,14 +205,16 @@ class DiTBlock:
         return y if self.ffn.world == 1 else self.ffn(y, mods[3], mods[4], mods[5])
 
 
-def _token_rows(t: torch.Tensor, width: int) -> torch.Tensor:
-    """``[1, L, width]`` (or ``[L, width]``) keys or values as contiguous bf16 rows ``[L, width]``; a view whenever the
-    caller's tensor already is that."""
+def _token_rows(t: torch.Tensor, rows: int, width: int) -> torch.Tensor:
+    """``[1, rows, width]`` (or ``[rows, width]``) keys or values as contiguous bf16 rows ``[rows, width]``; a view whenever
+    the caller's tensor already is that."""
+    if t.numel() != rows * width:
+        raise ValueError(f"keys / values of shape {tuple(t.shape)} are not {rows} rows of {width}")
     if t.dtype != torch.bfloat16 or not t.is_contiguous():
         t = t.to(torch.bfloat16).contiguous()
     if t.data_ptr() & 15:
         t = t.clone()
-    return t.view(-1, width)
+    return t.view(rows, width)
 
 
 def rotary_parts(freqs: torch.Tensor, device) -> tuple[torch.Tensor, torch.Tensor]:
@@ -309,6 +311,7 @@ class DiTDenoiser:
             if tail is None:  # zeroed once: whatever lies past a layer's own keys stays finite
                 cap = (127 + m + 127) // 128 * 128
                 tail = torch.zeros(2, blk.heads, cap, blk.hd, dtype=torch.bfloat16, device=self.device)
-            rows = lambda t, a=blk.attn_dim: _token_rows(t, a)  # noqa: E731
-            x = blk._forward(x, mods[i], cos, sin, tail[0], tail[1], 0, rows(vk), rows(vv), rows(cross_kv[i][0]), rows(cross_kv[i][1]), valid)
+            ck, cv = cross_kv[i]
+            rows = lambda k, v, a=blk.attn_dim: (_token_rows(k, k.shape[-2], a), _token_rows(v, k.shape[-2], a))  # noqa: E731
+            x = blk._forward(x, mods[i], cos, sin, tail[0], tail[1], 0, *rows(vk, vv), *rows(ck, cv), valid)
         return x[None]
