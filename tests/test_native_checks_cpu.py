@@ -69,3 +69,62 @@ def test_token_rows_of_another_count_are_refused():
     for bad in (_bf(2, LV, A), _bf(1, LV, 2 * A), _bf(1, LV - 1, A)):
         with pytest.raises(ValueError):
             _token_rows(bad, LV, A)
+
+
+def _meta(t):
+    """The tensor on another device than the rest of the call."""
+    return t.to("meta")
+
+
+def _gemma(w=256, inner=512, heads=2, g=1, hd=128, norms=True, layers=2):
+    from tybok_b200 import _lib
+
+    n = (torch.zeros(w), torch.zeros(w)) if norms else (None, None)
+    lay = lambda: (_w((heads + 2 * g) * hd, w, False), _w(w, heads * hd, False), _w(2 * inner, w, False), None,  # noqa: E731
+                   _w(w, inner, False), *n)
+    return _lib.native().GemmaStack(w, heads, g, hd, [lay() for _ in range(layers)])
+
+
+def _gemma_args(b=1, l=7, w=256, g=1, hd=128, layers=2, **over):
+    args = dict(x=_bf(b * l, w), b=b, l=l, pos=torch.zeros(b * l, dtype=torch.int32), cos=_bf(40, hd), sin=_bf(40, hd),
+                kc=[_bf(b, g, 20, hd) for _ in range(layers)], vc=[_bf(b, g, 20, hd) for _ in range(layers)], key_off=3,
+                key_valid=torch.ones(b, 3 + l, dtype=torch.uint8), mods=None, fold=None, first=0, count=layers, wait=[], record=[])
+    args.update(over)
+    return list(args.values())
+
+
+@pytest.mark.parametrize("name", ["x", "mods", "cos", "k_cache", "v_cache", "k_rows", "v_rows", "cross_k", "cross_v", "valid"])
+def test_dit_block_refuses_a_tensor_of_another_device(name):
+    good = dict(zip(("x", "mods", "cos", "sin", "k_cache", "v_cache", "key_off", "k_rows", "v_rows", "cross_k", "cross_v", "valid"),
+                    _block_args()))
+    with pytest.raises(ValueError, match="tensors on"):
+        _dit_block().forward(*_block_args(**{name: _meta(good[name])}))
+
+
+@pytest.mark.parametrize("over", [dict(pos=_meta(torch.zeros(7, dtype=torch.int32))), dict(key_valid=_meta(torch.ones(1, 10, dtype=torch.uint8))),
+                                  dict(kc=[_bf(1, 1, 20, 128), _meta(_bf(1, 1, 20, 128))]), dict(x=_meta(_bf(7, 256)))])
+def test_gemma_stack_refuses_a_tensor_of_another_device(over):
+    with pytest.raises(NotImplementedError):
+        _gemma().forward(*_gemma_args())
+    with pytest.raises(ValueError, match="tensors on"):
+        _gemma().forward(*_gemma_args(**over))
+
+
+def test_calls_and_weights_of_another_device_are_refused():
+    from tybok_b200 import _lib, ops
+
+    nat = _lib.native()
+    up, down = _w(FFN, H), _w(H, FFN)
+    mod = _bf(1, H)
+    calls = [
+        lambda: ops.w8a16_linear(_bf(3, H), *up[:2], _meta(up[2])),
+        lambda: ops.w8a16_linear(_bf(3, H), _meta(up[0]), up[1]),
+        lambda: ops.attention(_bf(4, 128), _bf(1, 1, 9, 128), _meta(_bf(1, 1, 9, 128)), tokens=4, keys=9, scale=1.0),
+        lambda: nat.Mlp(up, None, _w(H, FFN // 2)).forward(_meta(_bf(3, H))),
+        lambda: nat.FfnTail(up, down, 1e-6).forward(_bf(3, H), mod, mod, _meta(mod)),
+        lambda: nat.FfnTail(up, tuple(map(_meta, down)), 1e-6),
+        lambda: nat.FfnTail((up[0], _meta(up[1])), down, 1e-6),
+    ]
+    for call in calls:
+        with pytest.raises(ValueError, match="tensors on"):
+            call()

@@ -20,6 +20,7 @@ class DitBlock {
       down_ = w8_of(down, "dit");
     }
     h_ = qkv_.k;
+    same_device(qkv_.device(), "DiTBlock", {&o_.w, &cq_.w, &co_.w, ffn_ ? &up_.w : nullptr, ffn_ ? &down_.w : nullptr, &nq_, &nk_, &cnq_, &n3w_, &n3b_});
   }
 
   // x [S, H] bf16.  Keys and values: `k_cache` / `v_cache` [1, heads, Lcap, D] with this block's own appended at key_off;
@@ -48,6 +49,7 @@ class DitBlock {
     }
     if (ctx_valid && (ctx_valid->scalar_type() != at::kByte || !ctx_valid->is_contiguous() || ctx_valid->numel() != lc))
       type_error("attention: key_valid must be contiguous uint8 [B, Lk]");
+    same_device(qkv_.device(), "DiTBlock", {&x, &mods, &cos, &sin, &k_cache, &v_cache, opt(k_rows), opt(v_rows), opt(cross_k), opt(cross_v), opt(ctx_valid)});
     require_cuda(x, "dit_block");
     const c10::cuda::CUDAGuard guard(x.device());
     const int lcap = k_cache.size(-2);

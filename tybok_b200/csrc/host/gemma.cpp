@@ -27,6 +27,8 @@ class GemmaStack {
         l.norm_in = t[5].cast<Tensor>();
         l.norm_post = t[6].cast<Tensor>();
       }
+      const at::Device d = layers_.empty() ? l.qkv.device() : layers_[0].qkv.device();
+      same_device(d, "gemma_stack", {&l.qkv.w, &l.o.w, &l.gate_up.w, l.packed ? nullptr : &l.up.w, &l.down.w, opt(l.norm_in), opt(l.norm_post)});
       layers_.push_back(l);
     }
   }
@@ -39,8 +41,6 @@ class GemmaStack {
                  const std::vector<Tensor>& vc, int key_off, const Tensor& key_valid, const std::optional<std::vector<std::pair<Tensor, Tensor>>>& mods,
                  const std::optional<std::vector<std::pair<Tensor, Tensor>>>& fold, int first, int count, const std::vector<uint64_t>& wait,
                  const std::vector<uint64_t>& record) const {
-    require_cuda(x, "gemma_stack");
-    const c10::cuda::CUDAGuard guard(x.device());
     const int m = b * l, a = heads_ * hd_, keys = key_off + l;
     const Tensor x0 = rows_of(x);
     if (!is_bf16(x0) || x0.size(0) != m || x0.size(1) != w_) type_error("gemma_stack: x must be bf16 [B*L, W]");
@@ -62,6 +62,16 @@ class GemmaStack {
       for (int i = first; i < first + count; ++i)
         for (const Tensor* t : {&(*mods)[i].first, &(*mods)[i].second})
           if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() != 3 * w_) type_error("gemma_stack: modulations must be contiguous fp32 [1, 3W]");
+
+    const at::Device dev = layers_[0].qkv.device();
+    same_device(dev, "gemma_stack", {&x, &pos, &cos, &sin, &key_valid});
+    for (int i = first; i < first + count; ++i) {
+      same_device(dev, "gemma_stack", {&kc[i], &vc[i]});
+      if (mods) same_device(dev, "gemma_stack", {&(*mods)[i].first, &(*mods)[i].second});
+      if (fold) same_device(dev, "gemma_stack", {&(*fold)[i].first, &(*fold)[i].second});
+    }
+    require_cuda(x, "gemma_stack");
+    const c10::cuda::CUDAGuard guard(x.device());
 
     const int inner = layers_[0].down.k;
     const size_t at_ws = hd_ == 128 ? 0 : tybok_attention_workspace_bytes(b, l, heads_, keys);

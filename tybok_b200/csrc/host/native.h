@@ -7,6 +7,7 @@
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
 
+#include <initializer_list>
 #include <optional>
 #include <string>
 #include <vector>
@@ -43,6 +44,13 @@ inline void* ptr(const OptTensor& t) { return t ? t->data_ptr() : nullptr; }
 inline const float* f32(const Tensor& t) { return static_cast<const float*>(t.data_ptr()); }
 inline bool is_bf16(const Tensor& t) { return t.scalar_type() == at::kBFloat16; }
 
+// Kernels take plain addresses: a tensor of another device must not get as far as a launch.
+inline void same_device(at::Device d, const char* what, std::initializer_list<const Tensor*> tensors) {
+  for (const Tensor* t : tensors)
+    if (t && t->device() != d) value_error(std::string(what) + ": tensors on " + t->device().str() + " and " + d.str());
+}
+inline const Tensor* opt(const OptTensor& t) { return t ? &*t : nullptr; }
+
 // [rows, width] view of x with unit inner stride.
 Tensor rows_of(const Tensor& x);
 
@@ -54,6 +62,7 @@ struct W8 {
   const void* wp() const { return w.data_ptr(); }
   const float* sp() const { return f32(s); }
   const void* bp() const { return b ? b->data_ptr() : nullptr; }
+  at::Device device() const { return w.device(); }
 };
 W8 w8_of(const py::handle& t, const char* what);  // (weight, scale[, bias])
 

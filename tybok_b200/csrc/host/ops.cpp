@@ -57,6 +57,7 @@ W8 w8_of(const py::handle& t, const char* what) {
     r.b = u[2].cast<Tensor>();
     if (!is_bf16(*r.b) || r.b->numel() != r.w.size(0) || !r.b->is_contiguous()) type_error(std::string(what) + ": bias must be contiguous bf16 [N]");
   }
+  same_device(r.w.device(), what, {&r.s, opt(r.b)});
   r.n = static_cast<int>(r.w.size(0));
   r.k = static_cast<int>(r.w.size(1));
   return r;
@@ -65,7 +66,6 @@ W8 w8_of(const py::handle& t, const char* what) {
 // epilogue(x @ (w8 * scale).T + bias) for bf16 x: activation planes, then the GEMM.
 static Tensor w8a16_linear(const Tensor& x, const Tensor& w8, const Tensor& scale, const OptTensor& bias, int epilogue,
                            const OptTensor& residual, const OptTensor& gate, int rows_per_gate, int token_tile, int splits, int shift) {
-  require_cuda(x, "split3");
   if (!is_bf16(x)) type_error("split3: x must be bf16");
   check_w8(w8, "w8x3_linear");
   const int64_t n = w8.size(0), k = w8.size(1);
@@ -73,6 +73,8 @@ static Tensor w8a16_linear(const Tensor& x, const Tensor& w8, const Tensor& scal
   const Tensor x2 = rows_of(x);
   const int64_t m = x2.size(0);
   if (x2.size(1) != k) value_error("w8x3_linear: planes have K=" + std::to_string(x2.size(1)) + ", weight has K=" + std::to_string(k));
+  same_device(x.device(), "w8x3_linear", {&w8, &scale, opt(bias), opt(residual), opt(gate)});
+  require_cuda(x, "split3");
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor res;
   if (residual) {
@@ -111,7 +113,6 @@ static Tensor w8a16_linear(const Tensor& x, const Tensor& w8, const Tensor& scal
 
 static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& kc, const Tensor& vc, const OptTensor& valid, int tokens,
                                             int keys, double scale, bool out_bf16, bool out_planes, int out_shift) {
-  require_cuda(q, "attention");
   if (kc.dim() != 4) value_error("attention: caches must be [B, G, Lcap, D]");
   const int64_t b = kc.size(0), g = kc.size(1), lcap = kc.size(2), d = kc.size(3);
   if (!is_bf16(q) || q.dim() != 2 || !q.is_contiguous() || q.size(0) != b * tokens) type_error("attention: q must be contiguous bf16 [B*L, H*D]");
@@ -119,6 +120,8 @@ static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& kc, c
   if (valid && (valid->scalar_type() != at::kByte || valid->dim() != 2 || valid->size(0) != b || valid->size(1) != keys || !valid->is_contiguous()))
     type_error("attention: key_valid must be contiguous uint8 [B, Lk]");
   if (!out_bf16 && !out_planes) value_error("at least one of out_bf16 / out_planes must be set");
+  same_device(q.device(), "attention", {&kc, &vc, opt(valid)});
+  require_cuda(q, "attention");
   const c10::cuda::CUDAGuard guard(q.device());
   Tensor y = out_bf16 ? at::empty({b * tokens, h * d}, q.options()) : at::empty({0}, q.options());
   const auto bytes = q.options().dtype(at::kByte);
@@ -141,8 +144,11 @@ class Mlp {
     if (!packed_) up_ = w8_of(up, "mlp");
     inner_ = packed_ ? gu_.n / 2 : gu_.n;
     if (down_.k != inner_) value_error("mlp: down projection and intermediate width disagree");
+    same_device(gu_.device(), "mlp", {packed_ ? nullptr : &up_.w, &down_.w});
   }
   Tensor forward(const Tensor& x) const {
+    same_device(gu_.device(), "mlp", {&x});
+    require_cuda(x, "mlp");
     const c10::cuda::CUDAGuard guard(x.device());
     Tensor x2 = rows_of(x);
     if (!is_bf16(x2)) x2 = x2.to(at::kBFloat16);
@@ -188,8 +194,12 @@ class Mlp {
 // element: one chain for the whole batch.
 class FfnTail {
  public:
-  FfnTail(const py::tuple& up, const py::tuple& down, double eps) : up_(w8_of(up, "ffn_tail")), down_(w8_of(down, "ffn_tail")), eps_(eps) {}
+  FfnTail(const py::tuple& up, const py::tuple& down, double eps) : up_(w8_of(up, "ffn_tail")), down_(w8_of(down, "ffn_tail")), eps_(eps) {
+    same_device(up_.device(), "ffn_tail", {&down_.w});
+  }
   Tensor forward(const Tensor& x, const Tensor& shift, const Tensor& scale, const Tensor& gate) const {
+    same_device(up_.device(), "ffn_tail", {&x, &shift, &scale, &gate});
+    require_cuda(x, "ffn_tail");
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t h = x.size(-1), batch = x.dim() == 3 ? x.size(0) : 1;
     if (h != up_.k || down_.n != h) value_error("ffn_tail: input width differs from the weights'");
