@@ -128,3 +128,73 @@ def test_calls_and_weights_of_another_device_are_refused():
     for call in calls:
         with pytest.raises(ValueError, match="tensors on"):
             call()
+
+
+@pytest.mark.parametrize("over", [
+    dict(cos=torch.zeros(HD // 2, M)), dict(mods=_bf(5, H)), dict(x=_bf(M, H + 16)),
+])
+def test_dit_block_refuses_other_shapes(over):
+    with pytest.raises((TypeError, ValueError)):
+        _dit_block().forward(*_block_args(**over))
+
+
+@pytest.mark.parametrize("i,bad", [(3, _w(3 * A, H + 16)), (4, _w(H, A + 128)), (5, _w(A + 128, H)), (6, _w(H + 128, A)), (7, _w(FFN, H + 16)),
+                                   (8, _w(H, FFN + 16)), (9, _bf(A - 8)), (12, _bf(H + 8)), (13, torch.zeros(H))])
+def test_dit_block_refuses_weights_that_disagree(i, bad):
+    from tybok_b200 import _lib
+
+    args = [HEADS, HD, 1e-6, _w(3 * A, H), _w(H, A), _w(A, H), _w(H, A), _w(FFN, H), _w(H, FFN), _bf(A), _bf(A), _bf(A), _bf(H), _bf(H)]
+    _lib.native().DitBlock(*args)
+    args[i] = bad
+    with pytest.raises((TypeError, ValueError)):
+        _lib.native().DitBlock(*args)
+
+
+@pytest.mark.parametrize("i,bad", [(0, _w(512, 272, False)), (0, _w(640, 256, False)), (1, _w(256, 384, False)), (2, _w(1024, 272, False)),
+                                   (2, _w(1152, 256, False)), (4, _w(384, 512, False)), (4, _w(256, 640, False)), (5, torch.zeros(264))])
+def test_gemma_stack_refuses_weights_that_disagree(i, bad):
+    from tybok_b200 import _lib
+
+    lay = [_w(512, 256, False), _w(256, 256, False), _w(1024, 256, False), None, _w(256, 512, False), torch.zeros(256), torch.zeros(256)]
+    other = list(lay)
+    other[i] = bad
+    _lib.native().GemmaStack(256, 2, 1, 128, [tuple(lay), tuple(lay)])
+    with pytest.raises((TypeError, ValueError)):
+        _lib.native().GemmaStack(256, 2, 1, 128, [tuple(lay), tuple(other)])
+
+
+def test_gemma_stack_refuses_calls_that_disagree():
+    mod = lambda n=768: [(torch.zeros(1, n), torch.zeros(1, n))] * 2  # noqa: E731
+    fold = lambda q=512, gu=1024: [(torch.zeros(q), torch.zeros(gu))] * 2  # noqa: E731
+    with pytest.raises(NotImplementedError):
+        _gemma(norms=False).forward(*_gemma_args(mods=mod(), fold=fold()))
+    for over in (dict(fold=fold(q=504)), dict(fold=fold(gu=512)), dict(mods=mod(512)), dict(mods=None), dict(wait=[0]), dict(record=[0]),
+                 dict(sin=_bf(39, 128)), dict(kc=[_bf(1, 1, 20, 128), _bf(1, 1, 19, 128)]), dict(kc=[_bf(20, 128)] * 2)):
+        with pytest.raises((TypeError, ValueError)):
+            _gemma(norms=False).forward(*_gemma_args(**{**dict(mods=mod(), fold=fold()), **over}))
+
+
+def test_single_calls_refuse_disagreeing_operands():
+    from tybok_b200 import _lib, ops
+
+    nat = _lib.native()
+    w, s, b = _w(FFN, H)
+    kv = _bf(1, 1, 9, 128)
+    for good in (lambda: ops.w8a16_linear(_bf(3, H), w, s, b, epilogue=ops.EPI_RESIDUAL, residual=_bf(3, FFN), gate=_bf(2, FFN), rows_per_gate=2),
+                 lambda: ops.attention(_bf(4, 256), kv, kv, tokens=4, keys=9, scale=1.0)):
+        with pytest.raises(NotImplementedError):
+            good()
+    calls = [
+        lambda: ops.w8a16_linear(_bf(3, H), w, s, b.float()),
+        lambda: ops.w8a16_linear(_bf(3, H), w, s, _bf(FFN - 4)),
+        lambda: ops.w8a16_linear(_bf(3, H), w, s, epilogue=ops.EPI_RESIDUAL, residual=_bf(3, FFN), gate=_bf(1, FFN), rows_per_gate=2),
+        lambda: ops.attention(_bf(4, 256), kv, _bf(1, 1, 8, 128), tokens=4, keys=9, scale=1.0),
+        lambda: ops.attention(_bf(4, 256), kv, kv.float(), tokens=4, keys=9, scale=1.0),
+        lambda: ops.attention(_bf(4, 256), kv.transpose(2, 3).contiguous().transpose(2, 3), kv, tokens=4, keys=9, scale=1.0),
+        lambda: ops.attention(_bf(4, 192), kv, kv, tokens=4, keys=9, scale=1.0),
+        lambda: nat.Mlp(_w(FFN, H, False), _w(FFN, H + 16, False), _w(H, FFN, False)),
+        lambda: nat.FfnTail(_w(FFN, H), _w(H, FFN + 16), 1e-6),
+    ]
+    for call in calls:
+        with pytest.raises((TypeError, ValueError)):
+            call()

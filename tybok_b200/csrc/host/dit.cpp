@@ -20,6 +20,13 @@ class DitBlock {
       down_ = w8_of(down, "dit");
     }
     h_ = qkv_.k;
+    const int a = heads_ * hd_;
+    if (!qkv_.is(3 * a, h_) || !o_.is(h_, a) || !cq_.is(a, h_) || !co_.is(h_, a) || (ffn_ && (up_.k != h_ || !down_.is(h_, up_.n))))
+      value_error("DiTBlock: the weights' shapes disagree with heads, head_dim and one another");
+    for (const Tensor* t : {&nq_, &nk_, &cnq_})
+      if (!is_vector(*t, at::kBFloat16, a)) type_error("DiTBlock: qk-norm weights must be contiguous bf16 [H*D]");
+    for (const Tensor* t : {&n3w_, &n3b_})
+      if (!is_vector(*t, at::kBFloat16, h_)) type_error("DiTBlock: norm3 must be contiguous bf16 [H]");
     same_device(qkv_.device(), "DiTBlock", {&o_.w, &cq_.w, &co_.w, ffn_ ? &up_.w : nullptr, ffn_ ? &down_.w : nullptr, &nq_, &nk_, &cnq_, &n3w_, &n3b_});
   }
 
@@ -34,7 +41,7 @@ class DitBlock {
     if (!is_bf16(x0) || x0.size(1) != h) type_error("DiTBlock: x must be bf16 [S, H]");
     if (!is_bf16(mods) || !mods.is_contiguous() || mods.numel() != 6 * h) type_error("DiTBlock: mods must be contiguous bf16 [6, H]");
     for (const Tensor* t : {&cos, &sin})
-      if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() != static_cast<int64_t>(m) * (hd_ / 2))
+      if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->dim() != 2 || t->size(0) != m || t->size(1) != hd_ / 2)
         type_error("DiTBlock: cos/sin must be contiguous fp32 [S, D/2]");
     // The kernels are told one key count and one capacity per pair of keys and values; both sides must have them.
     const int lk = k_rows ? static_cast<int>(k_rows->size(0)) + m : key_off + m;

@@ -27,6 +27,13 @@ class GemmaStack {
         l.norm_in = t[5].cast<Tensor>();
         l.norm_post = t[6].cast<Tensor>();
       }
+      // every layer runs on one workspace, sized by the first one's widths
+      const int inner = l.down.k, a = heads_ * hd_;
+      if (!l.qkv.is((heads_ + 2 * kv_) * hd_, w_) || !l.o.is(w_, a) || !l.gate_up.is(l.packed ? 2 * inner : inner, w_) ||
+          (!l.packed && !l.up.is(inner, w_)) || l.down.n != w_ || (!layers_.empty() && inner != layers_[0].down.k))
+        value_error("gemma_stack: the weights' shapes disagree with the stack's widths");
+      if (l.norm_in && (!is_vector(*l.norm_in, at::kFloat, w_) || !is_vector(*l.norm_post, at::kFloat, w_)))
+        type_error("gemma_stack: norm weights must be contiguous fp32 [W]");
       const at::Device d = layers_.empty() ? l.qkv.device() : layers_[0].qkv.device();
       same_device(d, "gemma_stack", {&l.qkv.w, &l.o.w, &l.gate_up.w, l.packed ? nullptr : &l.up.w, &l.down.w, opt(l.norm_in), opt(l.norm_post)});
       layers_.push_back(l);
@@ -49,11 +56,14 @@ class GemmaStack {
       type_error("attention: key_valid must be contiguous uint8 [B, Lk]");
     for (const Tensor* t : {&cos, &sin})
       if (!is_bf16(*t) || !t->is_contiguous() || t->size(-1) != hd_) type_error("gemma_stack: cos/sin tables must be contiguous bf16 [max_pos, D]");
+    if (cos.sizes() != sin.sizes()) value_error("gemma_stack: cos and sin tables differ in shape");
     const int n = layers_.size();
     if (first < 0 || count <= 0 || first + count > n || static_cast<int>(kc.size()) < n || static_cast<int>(vc.size()) < n ||
         (mods && static_cast<int>(mods->size()) < n) || (fold && static_cast<int>(fold->size()) < n))
       value_error("gemma_stack: one cache pair and one set of modulations per layer");
-    const int lcap = kc[0].size(2);
+    if ((!wait.empty() && static_cast<int>(wait.size()) < first + count) || (!record.empty() && static_cast<int>(record.size()) < first + count))
+      value_error("gemma_stack: one event per layer");
+    const int lcap = kc[0].dim() == 4 ? kc[0].size(2) : -1;
     for (int i = first; i < first + count; ++i)
       for (const Tensor* t : {&kc[i], &vc[i]})
         if (!is_bf16(*t) || !t->is_contiguous() || t->dim() != 4 || t->size(0) != b || t->size(1) != kv_ || t->size(2) != lcap || t->size(3) != hd_)
@@ -63,6 +73,11 @@ class GemmaStack {
         for (const Tensor* t : {&(*mods)[i].first, &(*mods)[i].second})
           if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->numel() != 3 * w_) type_error("gemma_stack: modulations must be contiguous fp32 [1, 3W]");
 
+    for (int i = first; i < first + count; ++i) {
+      if (!mods && !layers_[i].norm_in) value_error("gemma_stack: a layer without norm weights needs its modulations");
+      if (fold && (!is_vector((*fold)[i].first, at::kFloat, layers_[i].qkv.n) || !is_vector((*fold)[i].second, at::kFloat, layers_[i].gate_up.n)))
+        type_error("gemma_stack: W shift rows must be contiguous fp32 [weight rows]");
+    }
     const at::Device dev = layers_[0].qkv.device();
     same_device(dev, "gemma_stack", {&x, &pos, &cos, &sin, &key_valid});
     for (int i = first; i < first + count; ++i) {

@@ -49,6 +49,7 @@ inline void same_device(at::Device d, const char* what, std::initializer_list<co
   for (const Tensor* t : tensors)
     if (t && t->device() != d) value_error(std::string(what) + ": tensors on " + t->device().str() + " and " + d.str());
 }
+inline bool is_vector(const Tensor& t, at::ScalarType type, int64_t n) { return t.scalar_type() == type && t.numel() == n && t.is_contiguous(); }
 inline const Tensor* opt(const OptTensor& t) { return t ? &*t : nullptr; }
 
 // [rows, width] view of x with unit inner stride.
@@ -63,6 +64,7 @@ struct W8 {
   const float* sp() const { return f32(s); }
   const void* bp() const { return b ? b->data_ptr() : nullptr; }
   at::Device device() const { return w.device(); }
+  bool is(int64_t rows, int64_t cols) const { return n == rows && k == cols; }
 };
 W8 w8_of(const py::handle& t, const char* what);  // (weight, scale[, bias])
 

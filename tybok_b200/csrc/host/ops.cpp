@@ -42,7 +42,7 @@ static void check_w8(const Tensor& w, const char* what) {
     type_error(std::string(what) + ": weight must be a contiguous e4m3 (or raw uint8) [N, K] tensor");
 }
 static void check_scale(const Tensor& s, int64_t rows, const char* what) {
-  if (s.scalar_type() != at::kFloat || s.numel() != rows || !s.is_contiguous())
+  if (!is_vector(s, at::kFloat, rows))
     type_error(std::string(what) + ": scale must be contiguous fp32 [" + std::to_string(rows) + "] (one per weight row)");
 }
 
@@ -55,7 +55,7 @@ W8 w8_of(const py::handle& t, const char* what) {
   check_scale(r.s, r.w.size(0), what);
   if (u.size() > 2 && !u[2].is_none()) {
     r.b = u[2].cast<Tensor>();
-    if (!is_bf16(*r.b) || r.b->numel() != r.w.size(0) || !r.b->is_contiguous()) type_error(std::string(what) + ": bias must be contiguous bf16 [N]");
+    if (!is_vector(*r.b, at::kBFloat16, r.w.size(0))) type_error(std::string(what) + ": bias must be contiguous bf16 [N]");
   }
   same_device(r.w.device(), what, {&r.s, opt(r.b)});
   r.n = static_cast<int>(r.w.size(0));
@@ -73,9 +73,7 @@ static Tensor w8a16_linear(const Tensor& x, const Tensor& w8, const Tensor& scal
   const Tensor x2 = rows_of(x);
   const int64_t m = x2.size(0);
   if (x2.size(1) != k) value_error("w8x3_linear: planes have K=" + std::to_string(x2.size(1)) + ", weight has K=" + std::to_string(k));
-  same_device(x.device(), "w8x3_linear", {&w8, &scale, opt(bias), opt(residual), opt(gate)});
-  require_cuda(x, "split3");
-  const c10::cuda::CUDAGuard guard(x.device());
+  if (bias && !is_vector(*bias, at::kBFloat16, n)) type_error("w8x3_linear: bias must be contiguous bf16 [N]");
   Tensor res;
   if (residual) {
     res = rows_of(*residual);
@@ -88,7 +86,12 @@ static Tensor w8a16_linear(const Tensor& x, const Tensor& w8, const Tensor& scal
       type_error("w8x3_linear: gate must be fp32 or bf16 [groups, N] with unit inner stride");
     gate_bf16 = is_bf16(*gate);
     ldgate = gate->dim() > 1 ? gate->stride(-2) : n;
+    if (epilogue == TYBOK_EPI_RESIDUAL && rows_per_gate > 0 && (gate->dim() > 1 ? gate->size(-2) : 1) * rows_per_gate < m)
+      value_error("w8x3_linear: fewer gate rows than groups of rows_per_gate tokens");
   }
+  same_device(x.device(), "w8x3_linear", {&w8, &scale, opt(bias), opt(residual), opt(gate)});
+  require_cuda(x, "split3");
+  const c10::cuda::CUDAGuard guard(x.device());
   std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
   shape.back() = n;
   Tensor y = at::empty(shape, x.options());
@@ -115,8 +118,11 @@ static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& kc, c
                                             int keys, double scale, bool out_bf16, bool out_planes, int out_shift) {
   if (kc.dim() != 4) value_error("attention: caches must be [B, G, Lcap, D]");
   const int64_t b = kc.size(0), g = kc.size(1), lcap = kc.size(2), d = kc.size(3);
+  if (!is_bf16(kc) || !is_bf16(vc) || !kc.is_contiguous() || !vc.is_contiguous()) type_error("attention: caches must be contiguous bf16");
+  if (vc.sizes() != kc.sizes()) value_error("attention: key and value caches differ in shape");
   if (!is_bf16(q) || q.dim() != 2 || !q.is_contiguous() || q.size(0) != b * tokens) type_error("attention: q must be contiguous bf16 [B*L, H*D]");
   const int64_t hd = q.size(1), h = hd / d;
+  if (hd != h * d) value_error("attention: the rows of q must hold whole heads");
   if (valid && (valid->scalar_type() != at::kByte || valid->dim() != 2 || valid->size(0) != b || valid->size(1) != keys || !valid->is_contiguous()))
     type_error("attention: key_valid must be contiguous uint8 [B, Lk]");
   if (!out_bf16 && !out_planes) value_error("at least one of out_bf16 / out_planes must be set");
@@ -144,6 +150,7 @@ class Mlp {
     if (!packed_) up_ = w8_of(up, "mlp");
     inner_ = packed_ ? gu_.n / 2 : gu_.n;
     if (down_.k != inner_) value_error("mlp: down projection and intermediate width disagree");
+    if (!packed_ && !up_.is(gu_.n, gu_.k)) value_error("mlp: gate and up weights differ in shape");
     same_device(gu_.device(), "mlp", {packed_ ? nullptr : &up_.w, &down_.w});
   }
   Tensor forward(const Tensor& x) const {
@@ -195,6 +202,7 @@ class Mlp {
 class FfnTail {
  public:
   FfnTail(const py::tuple& up, const py::tuple& down, double eps) : up_(w8_of(up, "ffn_tail")), down_(w8_of(down, "ffn_tail")), eps_(eps) {
+    if (!down_.is(up_.k, up_.n)) value_error("ffn_tail: the down weight is not the up weight's shape transposed");
     same_device(up_.device(), "ffn_tail", {&down_.w});
   }
   Tensor forward(const Tensor& x, const Tensor& shift, const Tensor& scale, const Tensor& gate) const {
@@ -202,7 +210,7 @@ class FfnTail {
     require_cuda(x, "ffn_tail");
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t h = x.size(-1), batch = x.dim() == 3 ? x.size(0) : 1;
-    if (h != up_.k || down_.n != h) value_error("ffn_tail: input width differs from the weights'");
+    if (h != up_.k) value_error("ffn_tail: input width differs from the weights'");
     Tensor x2 = rows_of(x);
     if (!is_bf16(x2)) x2 = x2.to(at::kBFloat16);
     const int m = x2.size(0), f = up_.n, per = batch ? m / batch : 1;
