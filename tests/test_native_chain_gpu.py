@@ -77,3 +77,43 @@ def test_batched_ffn_tail_equals_one_call_per_element(b, s, rows):
         one = [m if m.dim() == 1 else m[min(i, m.shape[0] - 1)] for m in mods]
         ref = fn(x[i], *one)
         assert float((y[i].float() - ref.float()).norm() / ref.float().norm()) <= 2e-3
+
+
+def _layouts(x):
+    """The rows of x [B, L, W] as a host framework may hand them over: with an odd stride, off a 16-byte boundary, both."""
+    b, l, w = x.shape
+    for wide, off in ((w + 1, 0), (w + 8, 3), (w + 5, 2)):
+        t = torch.zeros(b, l, wide, dtype=x.dtype, device=x.device)
+        t[:, :, off : off + w] = x
+        yield t[:, :, off : off + w]
+    yield torch.cat([x.flatten()[:1], x.flatten()])[1:].view(b, l, w)
+
+
+@pytest.mark.parametrize("m", [1, 5, 70])
+def test_hooks_take_rows_of_any_layout(m):
+    from tybok_b200 import ops
+    from tybok_b200.hooks import make_fused_ffn_tail, make_mlp_forward
+
+    w, f = 256, 640
+    g = torch.Generator(device="cuda").manual_seed(m)
+
+    class Lin:
+        def __init__(self, n, k):
+            self.weight, self.weight_scale = quantize_w8(_rnd(g, n, k, std=0.02))
+            self.bias = _rnd(g, n)
+
+    class Mod:
+        gate_proj, up_proj, down_proj = Lin(f, w), Lin(f, w), Lin(w, f)
+        ffn = [Lin(f, w), None, Lin(w, f)]
+
+    mlp, tail = make_mlp_forward(Mod), make_fused_ffn_tail(Mod)
+    x, table = _rnd(g, 2, m, w), _rnd(g, 5, 6, w, std=0.5)
+    mods = [table[:2, i : i + 1] for i in (3, 4, 5)]
+    want_mlp, want_tail = mlp(x), tail(x, *mods)
+    for y in _layouts(x):
+        assert torch.equal(mlp(y), want_mlp) and torch.equal(tail(y, *mods), want_tail)
+    same = x[:1, :1].expand(2, m, w)  # one row, repeated by a stride of zero
+    assert torch.equal(mlp(same), mlp(same.contiguous()))
+    assert torch.equal(tail(same, *mods), tail(same.contiguous(), *mods))
+    assert torch.equal(tail(x, *(table[:, i : i + 1] for i in (3, 4, 5))), want_tail)  # a table of more rows: the first ones
+    ops.check_status()

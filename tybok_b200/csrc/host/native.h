@@ -54,6 +54,9 @@ inline const Tensor* opt(const OptTensor& t) { return t ? &*t : nullptr; }
 
 // [rows, width] view of x with unit inner stride.
 Tensor rows_of(const Tensor& x);
+// The same in bf16 and as the kernels read rows in vectors: 16-byte aligned, row stride a multiple of 8 and at least the
+// width.  Anything else (a slice of wider rows, an expanded row, another type) is copied.
+Tensor vector_rows_of(const Tensor& x);
 
 // An e4m3 weight [n, k] with its fp32 scale [n] and optional bf16 bias [n].
 struct W8 {

@@ -37,6 +37,13 @@ Tensor rows_of(const Tensor& x) {
   return r.stride(-1) == 1 ? r : r.contiguous();
 }
 
+Tensor vector_rows_of(const Tensor& x) {
+  Tensor r = rows_of(x);
+  if (!is_bf16(r)) r = r.to(at::kBFloat16);
+  const bool fits = r.stride(0) % 8 == 0 && r.stride(0) >= r.size(1) && !(reinterpret_cast<uintptr_t>(r.data_ptr()) & 15);
+  return fits ? r : r.clone(at::MemoryFormat::Contiguous);
+}
+
 static void check_w8(const Tensor& w, const char* what) {
   if ((w.scalar_type() != at::kFloat8_e4m3fn && w.scalar_type() != at::kByte) || !w.is_contiguous() || w.dim() != 2)
     type_error(std::string(what) + ": weight must be a contiguous e4m3 (or raw uint8) [N, K] tensor");
@@ -157,8 +164,7 @@ class Mlp {
     same_device(gu_.device(), "mlp", {&x});
     require_cuda(x, "mlp");
     const c10::cuda::CUDAGuard guard(x.device());
-    Tensor x2 = rows_of(x);
-    if (!is_bf16(x2)) x2 = x2.to(at::kBFloat16);
+    const Tensor x2 = vector_rows_of(x);
     if (x2.size(1) != gu_.k) value_error("mlp: input width differs from the weights'");
     const int m = x2.size(0), k = gu_.k, i = inner_;
     std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
@@ -211,8 +217,7 @@ class FfnTail {
     const c10::cuda::CUDAGuard guard(x.device());
     const int64_t h = x.size(-1), batch = x.dim() == 3 ? x.size(0) : 1;
     if (h != up_.k) value_error("ffn_tail: input width differs from the weights'");
-    Tensor x2 = rows_of(x);
-    if (!is_bf16(x2)) x2 = x2.to(at::kBFloat16);
+    const Tensor x2 = vector_rows_of(x);
     const int m = x2.size(0), f = up_.n, per = batch ? m / batch : 1;
     Tensor sh = mod_rows(shift, batch, h), sc = mod_rows(scale, batch, h);
     const Tensor gt = mod_rows(gate, batch, h);
@@ -241,9 +246,11 @@ class FfnTail {
   }
 
  private:
-  // [1 or B, H] bf16 rows, 16-byte aligned, of a [B, 1, H], [1, 1, H] or [H] modulation (strided views are taken as they lie).
+  // [1 or B, H] bf16 rows, 16-byte aligned, of a [B, 1, H], [1, 1, H] or [H] modulation (strided views are taken as they lie;
+  // of a table of more rows, the first B).
   static Tensor mod_rows(const Tensor& t, int64_t batch, int64_t h) {
     Tensor r = t.reshape({-1, h});
+    if (r.size(0) > batch && batch > 0) r = r.narrow(0, 0, batch);
     if (r.size(0) != 1 && r.size(0) != batch) value_error("ffn_tail: modulation rows must be one, or one per batch element");
     if (!is_bf16(r)) r = r.to(at::kBFloat16);
     if (r.stride(1) != 1 || r.stride(0) % 8 != 0 || (reinterpret_cast<uintptr_t>(r.data_ptr()) & 15)) r = r.contiguous();
