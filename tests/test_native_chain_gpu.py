@@ -117,3 +117,16 @@ def test_hooks_take_rows_of_any_layout(m):
     assert torch.equal(tail(same, *mods), tail(same.contiguous(), *mods))
     assert torch.equal(tail(x, *(table[:, i : i + 1] for i in (3, 4, 5))), want_tail)  # a table of more rows: the first ones
     ops.check_status()
+
+
+def test_block_takes_modulation_rows_that_lie_apart():
+    from tybok_b200.dit import DiTBlock
+
+    s = DIT_TINY
+    g = torch.Generator(device="cuda").manual_seed(2)
+    blk = DiTBlock(quantize_dit_block(random_dit_block_params(s, seed=3, device="cuda")), s)
+    x, table = _rnd(g, 33, s.hidden), _rnd(g, 6, 2 * s.hidden, std=0.5)
+    cos, sin = torch.ones(33, s.head_dim // 2, device="cuda"), torch.zeros(33, s.head_dim // 2, device="cuda")
+    cache = lambda: [torch.zeros(1, s.heads, 33, s.head_dim, dtype=torch.bfloat16, device="cuda") for _ in range(2)]  # noqa: E731
+    mods = table[:, : s.hidden]
+    assert torch.equal(blk.forward(x, mods, cos, sin, cache()), blk.forward(x, mods.contiguous(), cos, sin, cache()))

@@ -37,6 +37,7 @@ def _block_args(**over):
     dict(cross_k=_bf(1, HEADS, C, HD), cross_v=_bf(1, HEADS, C, HD)),
     dict(k_rows=None, v_rows=None, k_cache=_bf(1, HEADS, M, HD), v_cache=_bf(1, HEADS, M, HD)),
     dict(cross_k=None, cross_v=None, valid=None),
+    dict(mods=_bf(6, 2 * H)[:, :H]),  # rows of a wider table
 ])
 def test_dit_block_takes_agreeing_sizes(over):
     with pytest.raises(NotImplementedError, match="no CPU implementation"):

@@ -39,7 +39,7 @@ class DitBlock {
     const Tensor x0 = rows_of(x);
     const int m = x0.size(0), a = heads_ * hd_, h = h_;
     if (!is_bf16(x0) || x0.size(1) != h) type_error("DiTBlock: x must be bf16 [S, H]");
-    if (!is_bf16(mods) || !mods.is_contiguous() || mods.numel() != 6 * h) type_error("DiTBlock: mods must be contiguous bf16 [6, H]");
+    if (!is_bf16(mods) || mods.size(0) != 6 || mods.numel() != 6 * h) type_error("DiTBlock: mods must be bf16 [6, H]");
     for (const Tensor* t : {&cos, &sin})
       if (t->scalar_type() != at::kFloat || !t->is_contiguous() || t->dim() != 2 || t->size(0) != m || t->size(1) != hd_ / 2)
         type_error("DiTBlock: cos/sin must be contiguous fp32 [S, D/2]");
@@ -77,7 +77,8 @@ class DitBlock {
     const size_t hp = qkv;
     ar.allocate(x0);
     Tensor y = at::empty({m, h}, x0.options());
-    const char* mod = static_cast<const char*>(mods.data_ptr());
+    const Tensor table = mods.contiguous();  // rows that lie apart are gathered
+    const char* mod = static_cast<const char*>(table.data_ptr());
     auto mrow = [&](int i) { return static_cast<const void*>(mod + size_t(2) * h * i); };
 
     // ---- modulated self-attention
