@@ -186,7 +186,7 @@ void bind_dit(py::module_& m) {
   py::class_<DitBlock>(m, "DitBlock")
       .def(py::init<int, int, double, const py::tuple&, const py::tuple&, const py::tuple&, const py::tuple&, const py::object&, const py::object&,
                     const Tensor&, const Tensor&, const Tensor&, const Tensor&, const Tensor&>())
-      .def("forward", &DitBlock::forward);
+      .def("forward", &DitBlock::forward, NoGil());
 }
 
 }  // namespace tbn

@@ -208,7 +208,7 @@ class GemmaStack {
 void bind_gemma(py::module_& m) {
   py::class_<GemmaStack>(m, "GemmaStack")
       .def(py::init<int, int, int, int, const py::list&>())
-      .def("forward", &GemmaStack::forward);
+      .def("forward", &GemmaStack::forward, NoGil());
 }
 
 }  // namespace tbn

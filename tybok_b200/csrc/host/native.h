@@ -28,6 +28,10 @@ constexpr int SHIFT_FOLD = 0;    // residual stream times (1 + scale), not norma
 // From this many token rows a GEMM fed by a norm takes two e4m3 planes with a per-row scale.
 constexpr int TWO_PLANE_MIN_TOKENS = 128;
 
+// Every call that launches runs without the interpreter lock: a launch waits while the device's queue is full, and other
+// threads' Python must go on meanwhile.  What touches Python objects in such a call takes the lock for itself.
+using NoGil = py::call_guard<py::gil_scoped_release>;
+
 [[noreturn]] void raise_status(int rc, const char* what);
 inline void check(int rc, const char* what) {
   if (rc != 0) raise_status(rc, what);

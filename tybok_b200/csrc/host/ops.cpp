@@ -15,6 +15,7 @@ void raise_status(int rc, const char* what) {
 
 void require_cuda(const Tensor& t, const char* what) {
   if (t.is_cuda()) return;
+  py::gil_scoped_acquire gil;
   PyErr_SetString(PyExc_NotImplementedError,
                   (std::string("tybok_b200::") + what + " runs on CUDA tensors only: there is no CPU implementation").c_str());
   throw py::error_already_set();
@@ -263,10 +264,12 @@ class FfnTail {
 
 void bind_ops(py::module_& m) {
   m.def("status_word", [](int device) { return status_tensor(device); });
-  m.def("w8a16_linear", &w8a16_linear);
-  m.def("attention", &attention);
-  py::class_<Mlp>(m, "Mlp").def(py::init<const py::tuple&, const py::object&, const py::tuple&>()).def("forward", &Mlp::forward);
-  py::class_<FfnTail>(m, "FfnTail").def(py::init<const py::tuple&, const py::tuple&, double>()).def("forward", &FfnTail::forward);
+  m.def("w8a16_linear", &w8a16_linear, NoGil());
+  m.def("attention", &attention, NoGil());
+  py::class_<Mlp>(m, "Mlp").def(py::init<const py::tuple&, const py::object&, const py::tuple&>()).def("forward", &Mlp::forward, NoGil());
+  py::class_<FfnTail>(m, "FfnTail")
+      .def(py::init<const py::tuple&, const py::tuple&, double>())
+      .def("forward", &FfnTail::forward, NoGil());
 }
 
 }  // namespace tbn
