@@ -1,0 +1,61 @@
+"""Every kernel with bounded waits comes back when one runs out: the epilogue's or softmax warps' limit is set to one SM
+clock, which no accumulator meets, the launch reports it in the status word, and the next launch gives the same bits as
+before.  What runs on the device is the kernels' own unwinding: copies and products in flight are seen to their end, tensor
+memory is freed, the CTAs leave."""
+
+import pytest
+import torch
+
+from oracle import w8_ref
+
+pytestmark = pytest.mark.gpu
+
+CONVERT, EPILOGUE = 103, 104  # TYBOK_DEV_TIMEOUT_*
+
+
+def _weights(n, k, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return w8_ref.quantize_w8(torch.empty(n, k, device="cuda").normal_(0, 0.02, generator=g))
+
+
+def _x(m, k, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.empty(m, k, device="cuda").normal_(0, 1, generator=g).to(torch.bfloat16)
+
+
+def _runs_out(launch, codes):
+    from tybok_b200 import ops
+
+    lib, dev = ops._lib.load(), torch.device("cuda")
+    good = launch()
+    ops.check_status()
+    lib.tybok_debug_set_epilogue_wait_limit(1)
+    try:
+        launch()
+        torch.cuda.synchronize()
+    finally:
+        lib.tybok_debug_set_epilogue_wait_limit(0)
+    assert int(ops.status_word(dev).item()) in codes
+    with pytest.raises(ops._lib.TybokError, match="bounded wait"):
+        ops.check_status()
+    again = launch()
+    ops.check_status()
+    assert torch.equal(again, good)
+
+
+@pytest.mark.parametrize("m,n,k,bt,splits", [(50, 1024, 4096, 0, 0), (50, 2560, 1024, 0, 0), (50, 8192, 1024, 0, 0), (300, 9600, 1024, 64, 1),
+                                             (64, 128, 256, 64, 1)])
+def test_one_tile_gemm(m, n, k, bt, splits):
+    """K over a cluster, one full-K wave, two CTAs per SM, and a producer that is through before anyone gives up."""
+    from tybok_b200 import ops
+
+    (w8, sc), xp = _weights(n, k), ops.split3(_x(m, k), 4)
+    _runs_out(lambda: ops.w8x3_linear(xp, 4, w8, sc, token_tile=bt, splits=splits)[0], (EPILOGUE,))
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 2560, 2048), (16, 18944, 16384)])
+def test_gemm_that_makes_its_planes(m, n, k):
+    from tybok_b200 import ops
+
+    (w8, sc), x = _weights(n, k), _x(m, k)
+    _runs_out(lambda: ops.w8a16_linear(x, w8, sc), (CONVERT, EPILOGUE))

@@ -64,6 +64,31 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// The same without the hardware's own wait inside.
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// Bounded wait that also ends once the CTA has given up.  A limit below the production one (a test's) is kept to the
+// clock: such a wait never suspends in hardware, where a short chain would complete before the limit is looked at.
+__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                              long long limit = kWaitLimitCycles) {
+  const bool test = limit < kWaitLimitCycles;
+  if (!test && mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!(test ? mbar_test_wait(bar, parity) : mbar_try_wait(bar, parity))) {
+    if (*abort_flag) return false;
+    if (clock64() - t0 > limit) return false;
+  }
+  return true;
+}
 // Bounded wait for the phase with the given parity to complete. Returns false on time-out.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
   if (mbar_try_wait(bar, parity)) return true;

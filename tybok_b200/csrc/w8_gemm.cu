@@ -113,23 +113,20 @@ struct __align__(8) Barriers {
   uint64_t tmem_full;
   uint64_t mma_done;  // every tensor-core instruction this CTA issued has retired
   uint32_t tmem_base;
+  volatile int issued;  // stages whose copies the producer has requested, once it is through; -1 before
   volatile int abort;
 };
-
-__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                              long long limit = kWaitLimitCycles) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {
-    if (*abort_flag) return false;
-    if (clock64() - t0 > limit) return false;
-  }
-  return true;
-}
 
 __device__ __forceinline__ void fail(Barriers* b, int* status, int code) {
   b->abort = 1;
   if (status) atomicCAS(status, 0, code);
+}
+// After a failed wait: the producer's stage count, once it has stopped (it sees the abort flag in its own waits).
+__device__ __noinline__ int stages_issued(const Barriers* b) {
+  const long long t0 = clock64();
+  while (b->issued < 0 && clock64() - t0 <= kWaitLimitCycles) {
+  }
+  return b->issued;
 }
 
 // Bounded for two CTAs per SM: multi-wave full-K launches run with a shallow ring so that one
@@ -188,6 +185,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     mbar_init(&bars.tmem_full, 1);
     mbar_init(&bars.mma_done, 1);
     bars.abort = 0;
+    bars.issued = -1;
     fence_barrier_init();
     // Weights depend on nothing that runs before this kernel: request the first stages now,
     // before the rest of the CTA has even finished its set-up.
@@ -229,8 +227,6 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
-      int issued = 0;
-      bool ok = true;
       // Dependents may start their own preamble (their weight prefetch) as soon as every CTA of
       // this grid is running; they still wait for this grid to complete before touching its output.
       if (p.pdl) pdl_launch_dependents();
@@ -242,12 +238,11 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       if (!p.xb)
         for (int i = 0; i < pre; ++i)
           tma_load_3d(smem + i * stage_bytes + x_off, &tm_x, &bars.full[i], (kb0 + i) * BK, t_tile * p.bt, 0);
-      issued = pre;
+      int issued = pre;
       for (int i = pre; i < nkb; ++i) {
         const int s = i % ns;
         if (!wait_or_abort(&bars.empty[s], ((i / ns) & 1) ^ 1, &bars.abort)) {
           fail(&bars, p.status, TYBOK_DEV_TIMEOUT_PRODUCER);
-          ok = false;
           break;
         }
         uint8_t* st = smem + s * stage_bytes;
@@ -258,11 +253,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         if (!p.xb) tma_load_3d(st + x_off, &tm_x, &bars.full[s], k0, t_tile * p.bt, 0);
         issued = i + 1;
       }
-      if (!ok || bars.abort) {
-        // Unwinding: do not leave the CTA while its own bulk copies may still land in its
-        // shared memory. Wait (bounded) for the newest copy of every stage.
-        for (int i = max(0, issued - ns); i < issued; ++i) mbar_wait(&bars.full[i % ns], (i / ns) & 1);
-      }
+      bars.issued = issued;
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
@@ -278,13 +269,14 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     const uint32_t plane16 = static_cast<uint32_t>(p.bt * 128) >> 4;  // plane pitch in 16-byte units
     const int acc_cols = p.merge ? p.np * p.bt : p.bt;
     bool ok = true;
+    int stop = 0;
     for (int i = 0; i < nkb; ++i) {
       const int s = i % ns;
       const long long c0 = tr ? clock64() : 0;
       const bool ready = wait_or_abort(&bars.full[s], (i / ns) & 1, &bars.abort);
       if (tr && leader) { const long long c1 = clock64(); tr[8] += c1 - c0; if (i == 0) tr[2] = c1; }
       if (!__all_sync(0xffffffffu, ready)) {
-        if (lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
+        stop = i;
         ok = false;
         break;
       }
@@ -316,6 +308,13 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       __syncwarp();
     }
     if (ok && leader) tc_commit(&bars.tmem_full);
+    if (!ok && lane == 0) {
+      fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
+      // The CTA must not leave while its own copies may still land in its shared memory, whoever gave up first.  The stages
+      // before this one have been waited for, the others are (each wait is bounded) now.
+#pragma unroll 1
+      for (int j = stop, n = stages_issued(&bars); j < n; ++j) mbar_wait(&bars.full[j % ns], (j / ns) & 1);
+    }
     if (tr && leader) tr[3] = clock64();
     // Whatever happened above, and whatever the other warps decide: this warp frees the tensor
     // memory at the end, so it first sees every instruction it issued retire.  On the normal path this completes together with
@@ -410,6 +409,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       const bool real = m_base + row < p.M;
       const __nv_bfloat16* xr = p.xb + static_cast<long long>(m_base + row) * p.ldxb;
       bool fine = true;
+      int made = 0;
       for (int i0 = 0; i0 < nkb && fine; i0 += 4) {
         uint2 raw[4];
 #pragma unroll
@@ -421,8 +421,9 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         for (int u = 0; u < 4; ++u) {
           const int i = i0 + u, s = i % ns;
           if (i < nkb && fine) {
-            if (i >= ns) fine = __all_sync(0xffffffffu, wait_or_abort(&bars.empty[s], ((i / ns) & 1) ^ 1, &bars.abort));
+            if (i >= ns) fine = __all_sync(0xffffffffu, wait_or_abort(&bars.empty[s], ((i / ns) & 1) ^ 1, &bars.abort, p.epi_wait_limit));
             if (fine) {
+              made = i + 1;
               const float xs[4] = {__uint_as_float(raw[u].x << 16) * p.xb_mult, __uint_as_float(raw[u].x & 0xffff0000u) * p.xb_mult,
                                    __uint_as_float(raw[u].y << 16) * p.xb_mult, __uint_as_float(raw[u].y & 0xffff0000u) * p.xb_mult};
               uint32_t w1, w2, w3;
@@ -438,7 +439,12 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           }
         }
       }
-      if (!fine && lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_CONVERT);
+      if (!fine && lane == 0) {
+        fail(&bars, p.status, TYBOK_DEV_TIMEOUT_CONVERT);
+        // this warp's rows of the stages on their way, or their barriers would not tell when the copies have landed
+#pragma unroll 1
+        for (int j = made, n = stages_issued(&bars); j < n; ++j) mbar_arrive(&bars.full[j % ns]);
+      }
     }
     bool ok = __all_sync(0xffffffffu, wait_or_abort(&bars.tmem_full, 0, &bars.abort, p.epi_wait_limit));
     if (!ok && lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_EPILOGUE);
