@@ -59,3 +59,33 @@ def test_gemm_that_makes_its_planes(m, n, k):
 
     (w8, sc), x = _weights(n, k), _x(m, k)
     _runs_out(lambda: ops.w8a16_linear(x, w8, sc), (CONVERT, EPILOGUE))
+
+
+@pytest.mark.parametrize("planes", [2, 3])
+@pytest.mark.parametrize("m,n,k", [(300, 19072, 256), (700, 9600, 4096), (60, 38400, 1024)])
+def test_pair_gemm(m, n, k, planes):
+    """Several tiles per pair, K within the ring and beyond it, token tiles of two sizes, planes in columns of their own."""
+    from tybok_b200 import ops
+
+    w8, sc = _weights(n, k)
+    if planes == 3:
+        xp = ops.split3(_x(m, k), 4)
+        _runs_out(lambda: ops.w8x3_linear(xp, 4, w8, sc)[0], (EPILOGUE,))
+    else:
+        xp, rs = ops.norm_planes2(_x(m, k), ops.NORM_RMS, torch.zeros(k, device="cuda"))
+        _runs_out(lambda: ops.w8x2_gemm(xp, rs, w8, sc)[0], (EPILOGUE,))
+
+
+def test_pair_gemm_of_two_accumulators():
+    from tybok_b200 import ops
+
+    (w8, sc), xp = _weights(16384, 1024), ops.split3(_x(500, 1024), 4)
+    _runs_out(lambda: ops.w8x3_geglu_packed(xp, 4, w8, sc)[0], (EPILOGUE,))
+
+
+@pytest.mark.parametrize("m,n,k", [(333, 2048, 16384), (257, 2044, 16400)])
+def test_pair_gemm_that_splits_k(m, n, k):
+    from tybok_b200 import ops
+
+    (w8, sc), xp = _weights(n, k), ops.split3(_x(m, k), 4)
+    _runs_out(lambda: ops.w8x3_linear(xp, 4, w8, sc)[0], (EPILOGUE,))

@@ -308,6 +308,12 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       __syncwarp();
     }
     if (ok && leader) tc_commit(&bars.tmem_full);
+    if (tr && leader) tr[3] = clock64();
+    // Whatever happened above, and whatever the other warps decide: this warp frees the tensor
+    // memory at the end, so it first sees every instruction it issued retire.  On the normal path this completes together with
+    // tmem_full; the warp has nothing else to do until the CTA meets.
+    if (leader) tc_commit(&bars.mma_done);
+    __syncwarp();
     if (!ok && lane == 0) {
       fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
       // The CTA must not leave while its own copies may still land in its shared memory, whoever gave up first.  The stages
@@ -315,12 +321,6 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
 #pragma unroll 1
       for (int j = stop, n = stages_issued(&bars); j < n; ++j) mbar_wait(&bars.full[j % ns], (j / ns) & 1);
     }
-    if (tr && leader) tr[3] = clock64();
-    // Whatever happened above, and whatever the other warps decide: this warp frees the tensor
-    // memory at the end, so it first sees every instruction it issued retire.  On the normal path this completes together with
-    // tmem_full; the warp has nothing else to do until the CTA meets.
-    if (leader) tc_commit(&bars.mma_done);
-    __syncwarp();
     if (!mbar_wait(&bars.mma_done, 0) && lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
   } else {
     // ------------------------------------------------------------ epilogue, phase A

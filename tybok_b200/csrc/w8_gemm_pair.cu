@@ -78,21 +78,17 @@ struct __align__(8) PairBars {
   uint64_t acc_empty[2];         // even CTA: the sixteen epilogue warps of the pair have read the accumulator
   uint64_t mma_done;             // every product this pair issued has retired
   uint32_t tmem_base;
+  volatile int issued;           // stages whose copies this CTA's producer has requested, once it is through; -1 before
   volatile int abort;
 };
 
-__device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity, PairBars* b, long long limit) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {
-    if (b->abort) return false;
-    if (clock64() - t0 > limit) return false;
-  }
-  return true;
-}
-__device__ __forceinline__ void pair_fail(PairBars* b, int* status, int code) {
-  b->abort = 1;
+// Gives up for the whole cluster, whose CTAs wait for one another's operands, products and parts.
+__device__ __noinline__ void pair_fail(PairBars* b, int* status, int code) {
   if (status) atomicCAS(status, 0, code);
+  uint32_t n;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
+  const uint32_t flag = smem_u32(const_cast<int*>(&b->abort));
+  for (uint32_t r = 0; r < n; ++r) asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], 1;" ::"r"(dsmem_addr(flag, r)) : "memory");
 }
 // One arrival on the barrier at shared::cluster address `addr` (this CTA's or its partner's).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
@@ -117,6 +113,33 @@ __device__ __forceinline__ Tile tile_at(const PairParams& p, int t) {
     o.bt = p.bt_small;
   }
   return o;
+}
+
+// Unwinding after a failed wait, in the even CTA, whose barriers count the copies of both: neither CTA may leave while its own
+// copies can still land in its shared memory.  Once both producers have stopped (the abort flag is the whole cluster's), a
+// stage that only one of them has requested is completed for the other, and the newest copies of every ring slot are
+// waited for.  Every wait is bounded.
+__device__ __forceinline__ void see_copies_land(const PairParams& p, PairBars* b, int pair, int npairs, int nkb, int na, uint32_t odd) {
+  const uint32_t theirs = dsmem_addr(smem_u32(const_cast<int*>(&b->issued)), odd);
+  const long long t0 = clock64();
+  int n0, n1;
+  do {
+    n0 = b->issued;
+    asm volatile("ld.relaxed.cluster.shared::cluster.s32 %0, [%1];" : "=r"(n1) : "r"(theirs) : "memory");
+  } while ((n0 < 0 || n1 < 0) && clock64() - t0 <= kWaitLimitCycles);
+  const int hi = max(n0, n1);
+  if (n0 >= 0 && n1 >= 0) {
+#pragma unroll 1
+    for (int i = min(n0, n1); i < hi; ++i) {
+      const Tile tl = tile_at(p, pair + i / nkb * npairs);
+      const uint32_t half = na * P_WTILE + p.np * (tl.bt >> 1) * P_BK;  // one CTA's bytes of the stage
+      uint64_t* bar = &b->full[i % p.nstages];
+      if (n1 > n0) mbar_arrive_expect_tx(bar, half);
+      else mbar_complete_tx(bar, half);
+    }
+  }
+#pragma unroll 1
+  for (int i = max(0, hi - p.nstages); i < hi; ++i) mbar_wait(&b->full[i % p.nstages], (i / p.nstages) & 1);
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
@@ -172,6 +195,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     }
     mbar_init(&bars.mma_done, 1);
     bars.abort = 0;
+    bars.issued = -1;
     fence_barrier_init();
     tma_prefetch_desc(&tm_w0);
     tma_prefetch_desc(&tm_big);
@@ -227,7 +251,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
           uint8_t* st = smem + s * p.stage_bytes;
           const uint32_t bar = dsmem_addr(smem_u32(&bars.full[s]), lead);
           if (!primed) {
-            if (!pair_wait(&bars.empty[s], par, &bars, kWaitLimitCycles)) {
+            if (!wait_or_abort(&bars.empty[s], par, &bars.abort)) {
               pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_PRODUCER);
               ok = false;
               break;
@@ -246,9 +270,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         }
         waited = true;
       }
-      // Unwinding: the even CTA sees the newest copies of every slot land before the pair leaves.
-      if (bars.abort && rank == 0)
-        for (int i = max(0, n - p.nstages); i < n; ++i) mbar_wait(&bars.full[i % p.nstages], (i / p.nstages) & 1);
+      bars.issued = n;
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer (even CTA)
@@ -263,10 +285,10 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         const int a = it & 1;
         const uint32_t plane16 = static_cast<uint32_t>(tl.bt * (P_BK / 2)) >> 4;
         const uint32_t idesc = p.np == 2 ? idesc_e4m3_e4m3_f32(256, tl.bt) : idesc_e4m3_e5m2_f32(256, tl.bt);
-        ok = __all_sync(0xffffffffu, pair_wait(&bars.acc_empty[a], ((it >> 1) & 1) ^ 1, &bars, kWaitLimitCycles));
+        ok = __all_sync(0xffffffffu, wait_or_abort(&bars.acc_empty[a], ((it >> 1) & 1) ^ 1, &bars.abort));
         tc_fence_after();
         for (int k = 0; k < nkb && ok; ++k) {
-          ok = __all_sync(0xffffffffu, pair_wait(&bars.full[s], par, &bars, kWaitLimitCycles));
+          ok = __all_sync(0xffffffffu, wait_or_abort(&bars.full[s], par, &bars.abort));
           if (!ok) break;
           tc_fence_after();
           const uint32_t st16 = (smem_u32(smem + s * p.stage_bytes) & 0x3FFFFu) >> 4;
@@ -293,9 +315,14 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         if (ok && leader) tc_commit_pair(&bars.acc_full[a], both);
         __syncwarp();
       }
-      if (!ok && lane == 0) pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
-      // Both CTAs free their tensor memory at the end: first every product issued has to retire.
+      // Both CTAs free their tensor memory at the end: first every product issued has to retire.  (The commit comes while the
+      // warp is still together: behind the branch below it reached one of the two CTAs only.)
       if (leader) tc_commit_pair(&bars.mma_done, both);
+      __syncwarp();
+      if (!ok && lane == 0) {
+        pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
+        see_copies_land(p, &bars, pair, npairs, nkb, NA, lead + 1);
+      }
       __syncwarp();
     }
     // The odd CTA's wait spans the whole launch: it only gives up once something else has failed.
@@ -357,7 +384,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
       const bool one_group = gate_group < 0 || (min(tl.m0 + tl.bt, p.M) - 1) / p.rows_per_gate == gate_group;
       const bool quad_live = NA == 1 || !p.packed ? n_first < p.N : live;
 
-      if (ok && !__all_sync(0xffffffffu, pair_wait(&bars.acc_full[a], (it >> 1) & 1, &bars, p.wait_limit))) {
+      if (ok && !__all_sync(0xffffffffu, wait_or_abort(&bars.acc_full[a], (it >> 1) & 1, &bars.abort, p.wait_limit))) {
         ok = false;
         if (lane == 0) pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_EPILOGUE);
       }
@@ -474,10 +501,11 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         }
       };
       if constexpr (SPLIT) {
-        cluster_sync_all();  // every pair of the cluster has its part: all rings are idle
+        cluster_sync_all();  // every pair of the cluster has its part (all rings are idle), or has given up
+        const bool whole = !bars.abort;  // the same in every CTA: nobody gives up after this point
         const int nown = (nchunk + p.splits - 1) / p.splits;
         const uint32_t buf = smem_u32(smem);
-        for (int c = half; c < nchunk; c += 2) {
+        for (int c = half; c < nchunk && whole; c += 2) {
           const int owner = c % p.splits;
           if (owner == split || tl.m0 + c * 32 >= p.M) continue;
           uint32_t v[32];
@@ -491,7 +519,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         __syncwarp();
         cluster_sync_all();  // every part has arrived
         const float* part = reinterpret_cast<const float*>(smem);
-        for (int i = half; i < nown; i += 2) {
+        for (int i = half; i < nown && whole; i += 2) {
           const int c = i * p.splits + split, mc = tl.m0 + c * 32;
           if (c >= nchunk || mc >= p.M) break;
           uint32_t v[32], t[32], u[NA == 2 ? 32 : 1];
