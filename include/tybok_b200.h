@@ -343,9 +343,9 @@ void tybok_debug_set_trace(void* device_buffer);
  * kernels).  Read from another stream, it tells where a stalled chain stands.  NULL (default) = off. */
 void tybok_debug_set_counters(void* device_buffer);
 
-/* Test aid: how many SM clocks the epilogue warps of the following launches of w8_gemm_kernel and
- * w8_gemm_pair_kernel wait (for their accumulator; for a ring slot, where they make the activation planes)
- * before they give up, record TYBOK_DEV_TIMEOUT_EPILOGUE / _CONVERT in the status word and skip
+/* Test aid: how many SM clocks the epilogue warps of the following GEMM launches wait (for their accumulator;
+ * for a ring slot, where they make the activation planes), and the softmax warps of the attention launches (for
+ * their scores), before they give up, record TYBOK_DEV_TIMEOUT_EPILOGUE / _CONVERT in the status word and skip
  * their stores (the producer, the MMA warp and the unwinding keep the production limit of about a
  * second).  0 (default) restores the production limit.  The error contract it lets a test
  * exercise is the reference's "error instead of exit" rule for its cooperative kernels

@@ -89,3 +89,15 @@ def test_pair_gemm_that_splits_k(m, n, k):
 
     (w8, sc), xp = _weights(n, k), ops.split3(_x(m, k), 4)
     _runs_out(lambda: ops.w8x3_linear(xp, 4, w8, sc)[0], (EPILOGUE,))
+
+
+# one key block in a CTA; rows pushed between the CTAs of a cluster, and staged in L2; the key loop at both head sizes, with
+# fewer blocks than its ring holds and more, its form of up to 64 rows, and the one of two tiles per CTA
+@pytest.mark.parametrize("b,l,keys,h,g,d", [(1, 50, 100, 8, 1, 256), (1, 50, 594, 8, 1, 256), (2, 50, 594, 8, 2, 256), (1, 300, 90, 2, 1, 256),
+                                            (1, 544, 544, 8, 1, 256), (1, 100, 200, 3, 3, 128), (1, 128, 1000, 24, 24, 128),
+                                            (1, 50, 4146, 24, 24, 128), (1, 1000, 200, 24, 24, 128), (1, 1030, 3000, 24, 24, 128)])
+def test_attention(b, l, keys, h, g, d):
+    from tybok_b200 import ops
+
+    q, k, v = _x(b * l, h * d), _x(b * g * keys, d, 1).view(b, g, keys, d), _x(b * g * keys, d, 2).view(b, g, keys, d)
+    _runs_out(lambda: ops.attention(q, k, v, tokens=l, keys=keys, scale=d**-0.5)[0], (EPILOGUE,))

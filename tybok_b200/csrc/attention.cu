@@ -247,6 +247,7 @@ struct AttnParams {
   int wide_out;      // key-loop form: out and out_planes are 32-byte aligned
   long long* trace;  // tuning aid: [CTA][16] SM-clock samples, NULL in production
   int* dbg;          // debugging aid: stage counters, NULL in production
+  long long wait_limit;  // SM clocks the softmax warps wait for their scores (kWaitLimitCycles in production)
 };
 
 struct __align__(16) AttnBars {
@@ -265,16 +266,6 @@ struct __align__(16) AttnBars {
   float hsum[2][AT_BQ];
   float wn[AT_MAX_SPLITS][AT_BQ];  // merge weights of the rows this CTA owns: exp2(m_s - m) / denominator
 };
-
-__device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (!mbar_try_wait(bar, parity)) {
-    if (*abort_flag) return false;
-    if (clock64() - t0 > kWaitLimitCycles) return false;
-  }
-  return true;
-}
 
 // 2^x by the special-function unit alone (results below 2^-126 flush to zero).
 __device__ __forceinline__ float pf_exp2(float x) {
@@ -299,6 +290,12 @@ __device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t smem_addr, uint3
   d |= static_cast<uint64_t>(1) << 46;
   d |= static_cast<uint64_t>(2) << 61;
   return d;
+}
+
+// Push form, a CTA that has given up: its peer gives up too, and counts as arrived the bytes that will not be sent.
+__device__ __forceinline__ void at_not_sent(AttnBars* b, uint64_t* bar, int peer, int bytes) {
+  st_dsmem(dsmem_addr(smem_u32(const_cast<int*>(&b->abort)), peer), 1u);
+  if (bytes > 0) mbar_complete_tx_peer(dsmem_addr(smem_u32(bar), peer), bytes);
 }
 
 // PUSH: short suffixes in the split-column form.  Every CTA sends the partial rows a peer will
@@ -406,7 +403,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
 #pragma unroll
       for (int ks = 0; ks < 16; ++ks) {  // D = 256 in steps of 16: chunk ks/4, 32 bytes per step
         if ((ks & 3) == 0 && ok) {
-          ok = __all_sync(0xffffffffu, at_wait(&bars.qk_full[ks >> 2], 0, &bars.abort));
+          ok = __all_sync(0xffffffffu, wait_or_abort(&bars.qk_full[ks >> 2], 0, &bars.abort));
           tc_fence_after();
         }
         const uint32_t off = (ks >> 2) * (AT_CHUNK >> 4) + (ks & 3) * 2;
@@ -416,7 +413,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     if (ok) {
       if (leader) tc_commit(&bars.s_full);
       __syncwarp();
-      ok = __all_sync(0xffffffffu, at_wait(&bars.v_full, 0, &bars.abort) && at_wait(&bars.p_full, 0, &bars.abort));
+      ok = __all_sync(0xffffffffu, wait_or_abort(&bars.v_full, 0, &bars.abort) && wait_or_abort(&bars.p_full, 0, &bars.abort));
     }
     if (ok) {
       tc_fence_after();
@@ -430,14 +427,18 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       if (leader) tc_commit(&bars.o_full);
       __syncwarp();
-    } else if (lane == 0) {
-      bars.abort = 1;
-      if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_MMA);
     }
     // This warp frees the tensor memory at the end, whatever the other warps decide: it first sees
     // every instruction it issued retire (on the normal path this completes together with o_full).
     if (leader) tc_commit(&bars.mma_done);
     __syncwarp();
+    if (!ok && lane == 0) {
+      bars.abort = 1;
+      if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_MMA);
+      // the CTA stays until its copies, which may not have been waited for, have landed in its shared memory
+      for (int c = 0; c < 4; ++c) mbar_wait(&bars.qk_full[c], 0);
+      mbar_wait(&bars.v_full, 0);
+    }
     mbar_wait(&bars.mma_done, 0);
   } else {
     // ------------------------------------------------------------ softmax, two threads per row
@@ -447,7 +448,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const bool live = q * 32 < nvalid;  // warp-uniform: this quadrant holds real query rows
     // Every named barrier below is reached by all eight warps whatever the waits returned.
-    bool ok = __all_sync(0xffffffffu, at_wait(&bars.s_full, 0, &bars.abort));
+    bool ok = __all_sync(0xffffffffu, wait_or_abort(&bars.s_full, 0, &bars.abort, p.wait_limit));
     if (tr && tid == 128) tr[2] = clock64();
     uint32_t v0[32], v1[32];
     // Issue-bound once the scores are there (64 per thread, two warps per sub-partition at best): the maximum runs as two
@@ -540,16 +541,17 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       fence_proxy_async();  // the statistics stores, for the bulk copy engine
       asm volatile("bar.sync 1, 256;" ::: "memory");
       cluster_wait_acquire();  // every peer's receive barriers are armed
-      if (ok && warp == 2 && lane < p.nsplit && lane != sp) {
+      if (warp == 2 && lane < p.nsplit && lane != sp) {
         const int rpr = (nvalid + p.nsplit - 1) / p.nsplit;
         const int rs = lane * rpr, ns = min(nvalid, rs + rpr) - rs;
-        if (ns > 0)
+        if (!ok) at_not_sent(&bars, &bars.recv_stat, lane, ns * 16);
+        else if (ns > 0)
           bulk_copy_to_peer(dsmem_addr(smem_u32(sv + AT_PUSH_RECV + AT_PUSH_STATS) + sp * rpr * 16, lane), &bars.stat[rs],
                             ns * 16, dsmem_addr(smem_u32(&bars.recv_stat), lane));
       }
     }
     // ---------------------------------------------------------- stage O (un-normalised), fp32
-    ok = ok && __all_sync(0xffffffffu, at_wait(&bars.o_full, 0, &bars.abort));
+    ok = ok && __all_sync(0xffffffffu, wait_or_abort(&bars.o_full, 0, &bars.abort));
     if (tr && tid == 128) tr[4] = clock64();
     if (ok && live) {
       tc_fence_after();
@@ -581,10 +583,12 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       // Send every peer the staged partial rows it merges: one bulk copy per peer, one lane each.
       fence_proxy_async();  // the staging stores, for the bulk copy engine
       asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (!bars.abort && warp == 2 && lane < p.nsplit && lane != sp) {
+      if (warp == 2 && lane < p.nsplit && lane != sp) {
         const int rpr = (nvalid + p.nsplit - 1) / p.nsplit;
         const int rs = lane * rpr, ns = min(nvalid, rs + rpr) - rs;
-        if (ns > 0) {
+        if (bars.abort) {
+          at_not_sent(&bars, &bars.recv, lane, ns * (AT_D / 2 * 4));
+        } else if (ns > 0) {
           const uint32_t recv = smem_u32(sv + AT_PUSH_RECV), bar = dsmem_addr(smem_u32(&bars.recv), lane);
           bulk_copy_to_peer(dsmem_addr(recv + sp * rpr * (AT_D / 2 * 4), lane), smem + rs * (AT_D / 2 * 4),
                             ns * (AT_D / 2 * 4), bar);
@@ -682,7 +686,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const float4* rstat = reinterpret_cast<const float4*>(sv + AT_PUSH_RECV + AT_PUSH_STATS);
     bool got = true;
     if (r0 + et < r1) {  // one thread per owned row: its weights, while the partial rows are in flight
-      got = at_wait(&bars.recv_stat, 0, &bars.abort);
+      got = wait_or_abort(&bars.recv_stat, 0, &bars.abort);
       float w[AT_MAX_SPLITS], l[AT_MAX_SPLITS];
 #pragma unroll
       for (int s = 0; s < AT_MAX_SPLITS; ++s) {
@@ -697,7 +701,11 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       merge_weights(et, w, l);
     }
     if (tr && tid == 64) tr[9] = clock64();
-    got = at_wait(&bars.recv, 0, &bars.abort) && got;
+    got = wait_or_abort(&bars.recv, 0, &bars.abort) && got;
+    if (!got) {  // what the peers have sent must land before they, or this CTA, may leave
+      mbar_wait(&bars.recv_stat, 0);
+      mbar_wait(&bars.recv, 0);
+    }
     cluster_arrive_release();  // this thread needs nothing more from the peers
     if (tr && tid == 64) tr[6] = clock64();
     if (!got) {
@@ -871,12 +879,27 @@ struct __align__(8) PrefillBars {
   uint64_t all_done;  // the last P.V product has landed
   uint64_t mma_done;  // unwinding: whatever was issued before a failed wait has retired
   uint32_t tmem_base;
+  volatile int nk, nv;  // K and V blocks that the producer has requested, once it is through; nk = -1 before
   volatile int abort;
   uint32_t valid[PF_MAX_KEYS / 32];
   float hmax[2][2][AT_BQ];  // [block parity][half of the block's keys][row]: maximum of the valid scores
   float hsum[2][AT_BQ];     // [half][row]: sum of that half's probabilities over all blocks
   float part[2][2][64];     // SHORT: [block parity][half][row]: sum of the half's first 32 keys
 };
+
+// Unwinding after a failed wait: the CTA stays until its copies have landed in its shared memory, the newest ones of every
+// ring slot.  The producer stops because it sees the abort flag in its own waits.
+template <class Bars>
+__device__ __forceinline__ void pf_see_copies_land(Bars* b) {
+  const long long t0 = clock64();
+  while (b->nk < 0 && clock64() - t0 <= kWaitLimitCycles) {
+  }
+  mbar_wait(&b->q_full, 0);
+#pragma unroll 1
+  for (int i = max(0, b->nk - 2); i < b->nk; ++i) mbar_wait(&b->k_full[i & 1], (i >> 1) & 1);
+#pragma unroll 1
+  for (int i = max(0, b->nv - 2); i < b->nv; ++i) mbar_wait(&b->v_full[i & 1], (i >> 1) & 1);
+}
 
 // HD = head dimension, 128 or 256.  Either way a CTA takes ALL 512 tensor-memory columns of its SM
 // and therefore has the SM's tensor memory to itself: its shared memory leaves no room for another CTA that allocates any.
@@ -933,6 +956,8 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     mbar_init(&bars.all_done, 1);
     mbar_init(&bars.mma_done, 1);
     bars.abort = 0;
+    bars.nk = -1;
+    bars.nv = 0;
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -969,6 +994,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         tma_load_2d(sq + c * AT_CHUNK, &tm_q, &bars.q_full, h * HD + c * 64, b * p.L + qt * AT_BQ);
         if (SHORT) tma_load_2d(sq + c * AT_CHUNK + AT_CHUNK / 2, &tm_q, &bars.q_full, h * HD + c * 64, b * p.L);
       }
+      int nk = 0, nv = 0;
       for (int j = 0; j < nkb; ++j) {
         const int s = j & 1;
         const uint32_t par = ((j >> 1) & 1) ^ 1;  // the ring slot's previous use
@@ -977,13 +1003,17 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         const CUtensorMap* mv = rows ? &tm_vr : &tm_v;
         const int kcol = rows ? g * HD : 0;
         const int krow = rows ? b * p.Lk + j * PF_BK : (b * p.G + g) * p.Lcap + (j - p.nb_rows) * PF_BK;
-        if (j >= 2 && !at_wait(&bars.k_empty[s], par, &bars.abort)) break;
+        if (j >= 2 && !wait_or_abort(&bars.k_empty[s], par, &bars.abort)) break;
         mbar_arrive_expect_tx(&bars.k_full[s], PF_KV);
         for (int c = 0; c < NCH; ++c) tma_load_2d(sk + s * PF_KV + c * PF_KCHUNK, mk, &bars.k_full[s], kcol + c * 64, krow);
-        if (j >= 2 && !at_wait(&bars.v_empty[s], par, &bars.abort)) break;
+        nk = j + 1;
+        if (j >= 2 && !wait_or_abort(&bars.v_empty[s], par, &bars.abort)) break;
         mbar_arrive_expect_tx(&bars.v_full[s], PF_KV);
         for (int c = 0; c < NCH; ++c) tma_load_2d(sv + s * PF_KV + c * PF_KCHUNK, mv, &bars.v_full[s], kcol + c * 64, krow);
+        nv = j + 1;
       }
+      bars.nv = nv;
+      bars.nk = nk;
     }
   } else if (warp == 1) {
     const bool leader = elect_one();
@@ -991,10 +1021,10 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     const uint32_t idesc_s = idesc_bf16_f32(AT_BQ, PF_BK);
     const uint32_t idesc_o = idesc_bf16_f32(AT_BQ, HD) | (1u << 16);
     const uint32_t q16 = (smem_u32(sq) & 0x3FFFFu) >> 4;
-    bool ok = __all_sync(0xffffffffu, at_wait(&bars.q_full, 0, &bars.abort));
+    bool ok = __all_sync(0xffffffffu, wait_or_abort(&bars.q_full, 0, &bars.abort));
     auto issue_s = [&](int j) {  // S_j = Q K_j^T into columns PF_BK * (j & 1); frees the K slot when done
       const int s = j & 1;
-      ok = ok && __all_sync(0xffffffffu, at_wait(&bars.k_full[s], (j >> 1) & 1, &bars.abort));
+      ok = ok && __all_sync(0xffffffffu, wait_or_abort(&bars.k_full[s], (j >> 1) & 1, &bars.abort));
       if (!ok) return;
       tc_fence_after();
       const uint32_t k16 = (smem_u32(sk + s * PF_KV) & 0x3FFFFu) >> 4;
@@ -1015,7 +1045,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     for (int j = 0; j < nkb && ok; ++j) {
       const int s = j & 1;
       const uint32_t par = (j >> 1) & 1;
-      ok = __all_sync(0xffffffffu, at_wait(&bars.p_full[s], par, &bars.abort) && at_wait(&bars.v_full[s], par, &bars.abort));
+      ok = __all_sync(0xffffffffu, wait_or_abort(&bars.p_full[s], par, &bars.abort) && wait_or_abort(&bars.v_full[s], par, &bars.abort));
       if (!ok) break;
       tc_fence_after();
       const uint32_t v_addr = smem_u32(sv + s * PF_KV);
@@ -1038,14 +1068,16 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       if (j + 2 < nkb) issue_s(j + 2);  // over P_j, which the product just issued reads first
     }
     // nothing of this CTA's tensor work may be in flight when it gives up its tensor memory
-    ok = ok && __all_sync(0xffffffffu, at_wait(&bars.all_done, 0, &bars.abort));
+    ok = ok && __all_sync(0xffffffffu, wait_or_abort(&bars.all_done, 0, &bars.abort));
     if (!ok) {
+      // a failed wait left the loop early: see what was issued before it retire, and what was requested land
+      if (leader) tc_commit(&bars.mma_done);
+      __syncwarp();
       if (lane == 0) {
         bars.abort = 1;
         if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_MMA);
+        pf_see_copies_land(&bars);
       }
-      // a failed wait left the loop early: see what was issued before it retire
-      if (leader) tc_commit(&bars.mma_done);
       __syncwarp();
       mbar_wait(&bars.mma_done, 0);
     }
@@ -1080,7 +1112,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 #pragma unroll 1
     for (int j = 0; j < nkb; ++j) {
       const int s = j & 1;
-      if (ok && !__all_sync(0xffffffffu, at_wait(&bars.s_full[s], (j >> 1) & 1, &bars.abort))) {
+      if (ok && !__all_sync(0xffffffffu, wait_or_abort(&bars.s_full[s], (j >> 1) & 1, &bars.abort, p.wait_limit))) {
         ok = false;
         bars.abort = 1;
       }
@@ -1128,7 +1160,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
             // Rescale this thread's half of the O row (SHORT: by the threads in its lane) and its sum to the new reference maximum;
             // rows of the warp that keep theirs multiply by one.  The previous P.V product must
             // have landed (it is at most one phase away, see PrefillBars::o_done).
-            if (!__all_sync(0xffffffffu, at_wait(&bars.o_done, (j - 1) & 1, &bars.abort))) {
+            if (!__all_sync(0xffffffffu, wait_or_abort(&bars.o_done, (j - 1) & 1, &bars.abort))) {
               ok = false;
               bars.abort = 1;
             } else {
@@ -1214,7 +1246,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     } else {
       bars.hsum[khf][srow] = l;
     }
-    if (ok && !__all_sync(0xffffffffu, at_wait(&bars.all_done, 0, &bars.abort))) ok = false;
+    if (ok && !__all_sync(0xffffffffu, wait_or_abort(&bars.all_done, 0, &bars.abort))) ok = false;
     if (!ok && lane == 0) {
       bars.abort = 1;
       if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_EPILOGUE);
@@ -1298,6 +1330,7 @@ struct __align__(8) TwoTileBars {
   uint64_t done[2];               // per tile: its last product has landed
   uint64_t mma_done;
   uint32_t tmem_base;
+  volatile int nk, nv;            // as in PrefillBars
   volatile int abort;
   uint32_t valid[PF_MAX_KEYS / 32];
 };
@@ -1357,6 +1390,8 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     }
     mbar_init(&bars.mma_done, 1);
     bars.abort = 0;
+    bars.nk = -1;
+    bars.nv = 0;
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -1388,17 +1423,22 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       for (int t = 0; t < ntile; ++t)
         for (int c = 0; c < 2; ++c)
           tma_load_2d(sq + t * 32768 + c * CH, &tm_q, &bars.q_full, h * HD + c * 64, b * p.L + row_base + t * 128);
+      int nk = 0, nv = 0;
       for (int j = 0; j < nkb; ++j) {
         const int s = j & 1;
         const uint32_t par = ((j >> 1) & 1) ^ 1;  // the ring slot's previous use
         const int krow = (b * p.G + g) * p.Lcap + j * BK;
-        if (j >= 2 && !at_wait(&bars.k_empty[s], par, &bars.abort)) break;
+        if (j >= 2 && !wait_or_abort(&bars.k_empty[s], par, &bars.abort)) break;
         mbar_arrive_expect_tx(&bars.k_full[s], KV);
         for (int c = 0; c < 2; ++c) tma_load_2d(sk + s * KV + c * CH, &tm_k, &bars.k_full[s], c * 64, krow);
-        if (j >= 2 && !at_wait(&bars.v_empty[s], par, &bars.abort)) break;
+        nk = j + 1;
+        if (j >= 2 && !wait_or_abort(&bars.v_empty[s], par, &bars.abort)) break;
         mbar_arrive_expect_tx(&bars.v_full[s], KV);
         for (int c = 0; c < 2; ++c) tma_load_2d(sv + s * KV + c * CH, &tm_v, &bars.v_full[s], c * 64, krow);
+        nv = j + 1;
       }
+      bars.nv = nv;
+      bars.nk = nk;
     }
   } else if (warp == 1) {
     const bool leader = elect_one();
@@ -1413,7 +1453,7 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       }
       if (leader) tc_commit(&bars.s_full[t]);
     };
-    bool ok = __all_sync(0xffffffffu, at_wait(&bars.q_full, 0, &bars.abort) && at_wait(&bars.k_full[0], 0, &bars.abort));
+    bool ok = __all_sync(0xffffffffu, wait_or_abort(&bars.q_full, 0, &bars.abort) && wait_or_abort(&bars.k_full[0], 0, &bars.abort));
     if (ok) {
       tc_fence_after();
       for (int t = 0; t < ntile; ++t) issue_s(t, 0);
@@ -1424,11 +1464,11 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     for (int j = 0; j < nkb && ok; ++j) {
       const int s = j & 1;
       const uint32_t v_addr = smem_u32(sv + s * KV);
-      ok = __all_sync(0xffffffffu, at_wait(&bars.v_full[s], (j >> 1) & 1, &bars.abort));
-      if (ok && j + 1 < nkb) ok = __all_sync(0xffffffffu, at_wait(&bars.k_full[s ^ 1], ((j + 1) >> 1) & 1, &bars.abort));
+      ok = __all_sync(0xffffffffu, wait_or_abort(&bars.v_full[s], (j >> 1) & 1, &bars.abort));
+      if (ok && j + 1 < nkb) ok = __all_sync(0xffffffffu, wait_or_abort(&bars.k_full[s ^ 1], ((j + 1) >> 1) & 1, &bars.abort));
       for (int t = 0; t < ntile && ok; ++t) {
         for (int hf = 0; hf < 2 && ok; ++hf) {  // the first keys' product starts under the others' exponentials
-          ok = __all_sync(0xffffffffu, at_wait(&bars.p_full[t][hf], j & 1, &bars.abort));
+          ok = __all_sync(0xffffffffu, wait_or_abort(&bars.p_full[t][hf], j & 1, &bars.abort));
           if (!ok) break;
           tc_fence_after();
 #pragma unroll
@@ -1449,11 +1489,13 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       __syncwarp();
     }
     // nothing of this CTA's tensor work may be in flight when it gives up its tensor memory
+    if (leader) tc_commit(&bars.mma_done);
+    __syncwarp();
     if (!ok && lane == 0) {
       bars.abort = 1;
       if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_MMA);
+      pf_see_copies_land(&bars);
     }
-    if (leader) tc_commit(&bars.mma_done);
     __syncwarp();
     mbar_wait(&bars.mma_done, 0);
   }
@@ -1470,7 +1512,7 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
       const uint64_t c2 = f32x2(p.scale_log2e, p.scale_log2e);
 #pragma unroll 1
       for (int j = 0; j < nkb; ++j) {
-        if (ok && !__all_sync(0xffffffffu, at_wait(&bars.s_full[t], j & 1, &bars.abort))) {
+        if (ok && !__all_sync(0xffffffffu, wait_or_abort(&bars.s_full[t], j & 1, &bars.abort, p.wait_limit))) {
           ok = false;
           bars.abort = 1;
         }
@@ -1554,7 +1596,7 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           mbar_arrive(&bars.p_full[t][1]);
         }
       }
-      if (ok && !__all_sync(0xffffffffu, at_wait(&bars.done[t], 0, &bars.abort))) ok = false;
+      if (ok && !__all_sync(0xffffffffu, wait_or_abort(&bars.done[t], 0, &bars.abort))) ok = false;
       if (!ok && lane == 0) {
         bars.abort = 1;
         if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_EPILOGUE);
@@ -1791,6 +1833,7 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   p.dsplit = (!prefill && nsplit > 1 && 2 * nsplit * H * n_qt * B <= host::sm_count() && 2 * H * n_qt * B <= at_resident_clusters(nsplit)) ? 2 : 1;
   p.trace = host::trace_buffer();
   p.dbg = host::counter_buffer();
+  p.wait_limit = host::epilogue_wait_limit() > 0 ? host::epilogue_wait_limit() : kWaitLimitCycles;
   const int rows_per_rank = (std::min(L, AT_BQ) + nsplit - 1) / nsplit;
   const bool push = p.dsplit == 2 && n_qt == 1 && nsplit * rows_per_rank <= AT_PUSH_MAX_ROWS;
 
@@ -1882,6 +1925,7 @@ int tybok_attention_rows(const void* q, const void* k_rows, const void* v_rows, 
   p.wide_out = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_planes)) & 31) == 0;
   p.status = status_word; p.pdl = host::pdl_enabled() ? 1 : 0; p.q_rows = AT_BQ; p.dsplit = 1;
   p.trace = host::trace_buffer(); p.dbg = host::counter_buffer();
+  p.wait_limit = host::epilogue_wait_limit() > 0 ? host::epilogue_wait_limit() : kWaitLimitCycles;
   static bool attr_set[64] = {};
   const int dev = host::current_device();
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {

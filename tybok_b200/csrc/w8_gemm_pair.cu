@@ -88,7 +88,7 @@ __device__ __noinline__ void pair_fail(PairBars* b, int* status, int code) {
   uint32_t n;
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(n));
   const uint32_t flag = smem_u32(const_cast<int*>(&b->abort));
-  for (uint32_t r = 0; r < n; ++r) asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], 1;" ::"r"(dsmem_addr(flag, r)) : "memory");
+  for (uint32_t r = 0; r < n; ++r) st_dsmem(dsmem_addr(flag, r), 1u);
 }
 // One arrival on the barrier at shared::cluster address `addr` (this CTA's or its partner's).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t addr) {
