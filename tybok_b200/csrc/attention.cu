@@ -1654,9 +1654,9 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 namespace tb {
 // Clusters of `nsplit` attention CTAs (one CTA per SM) that the device holds at once.
 static int at_resident_clusters(int nsplit) {
-  static int cached[AT_MAX_SPLITS + 1] = {};
+  static host::DeviceCache cache[AT_MAX_SPLITS + 1];
   if (nsplit > AT_MAX_SPLITS) return 1;
-  if (cached[nsplit] == 0) {
+  return host::per_device(cache[nsplit], [nsplit] {
     cudaFuncSetAttribute(attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(nsplit);
@@ -1674,9 +1674,19 @@ static int at_resident_clusters(int nsplit) {
       cudaGetLastError();
       n = host::sm_count() / (nsplit + 1);
     }
-    cached[nsplit] = n;
-  }
-  return cached[nsplit];
+    return n;
+  });
+}
+
+static int at_set_attributes() {
+  static host::DeviceCache cache;
+  const bool done = host::per_device(cache, [] {
+    const auto set = [](auto* kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; };
+    return static_cast<int>(set(attention_kernel<false>, AT_SMEM) && set(attention_kernel<true>, AT_SMEM) && set(attention_two_tile_kernel, TT_SMEM) &&
+                            set(attention_prefill_kernel<256>, pf_smem(256)) && set(attention_prefill_kernel<128, true>, PF_SMEM_SHORT) &&
+                            set(attention_prefill_kernel<128>, pf_smem(128)));
+  });
+  return done ? TYBOK_OK : host::fail_cuda("cudaFuncSetAttribute(attention kernels)");
 }
 }  // namespace tb
 
@@ -1837,18 +1847,7 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   const int rows_per_rank = (std::min(L, AT_BQ) + nsplit - 1) / nsplit;
   const bool push = p.dsplit == 2 && n_qt == 1 && nsplit * rows_per_rank <= AT_PUSH_MAX_ROWS;
 
-  static bool attr_set[64] = {};
-  const int dev = host::current_device();
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_two_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, TT_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_prefill_kernel<256>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem(256)) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_prefill_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM_SHORT) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem(128)) != cudaSuccess)
-      return host::fail_cuda("cudaFuncSetAttribute(attention_kernel)");
-    attr_set[dev] = true;
-  }
+  if (int rc = at_set_attributes()) return rc;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = two_tile ? dim3((n_qt + 1) / 2, H, B) : prefill ? dim3(n_qt, H, B) : dim3(nsplit, H * n_qt * p.dsplit, B);
   cfg.blockDim = dim3(two_tile ? TT_THREADS : AT_THREADS);
@@ -1926,14 +1925,7 @@ int tybok_attention_rows(const void* q, const void* k_rows, const void* v_rows, 
   p.status = status_word; p.pdl = host::pdl_enabled() ? 1 : 0; p.q_rows = AT_BQ; p.dsplit = 1;
   p.trace = host::trace_buffer(); p.dbg = host::counter_buffer();
   p.wait_limit = host::epilogue_wait_limit() > 0 ? host::epilogue_wait_limit() : kWaitLimitCycles;
-  static bool attr_set[64] = {};
-  const int dev = host::current_device();
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(attention_prefill_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_smem(128)) != cudaSuccess ||
-        cudaFuncSetAttribute(attention_prefill_kernel<128, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, PF_SMEM_SHORT) != cudaSuccess)
-      return host::fail_cuda("cudaFuncSetAttribute(attention_prefill_kernel)");
-    attr_set[dev] = true;
-  }
+  if (int rc = at_set_attributes()) return rc;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((L + AT_BQ - 1) / AT_BQ, H, 1);
   cfg.blockDim = dim3(AT_THREADS);

@@ -35,37 +35,23 @@ int current_device() {
   return dev;
 }
 
-struct DevInfo {
-  bool known = false;
-  int major = 0;
-  int sms = 0;
-};
-static DevInfo g_dev[64];
-
-static const DevInfo* dev_info() {
+static int attribute(cudaDeviceAttr what) {  // of the current device; 0 when there is none
   const int dev = current_device();
-  if (dev < 0 || dev >= 64) return nullptr;
-  DevInfo& d = g_dev[dev];
-  if (!d.known) {
-    int major = 0, sms = 0;
-    if (cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev) != cudaSuccess) return nullptr;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return nullptr;
-    d.major = major;
-    d.sms = sms;
-    d.known = true;
-  }
-  return &d;
+  int v = 0;
+  return dev >= 0 && cudaDeviceGetAttribute(&v, what, dev) == cudaSuccess ? v : 0;
 }
 
 int sm_count() {
-  const DevInfo* d = dev_info();
-  return d ? d->sms : 148;  // planning without a device (workspace sizing): assume a B200
+  static DeviceCache cache;
+  const int sms = per_device(cache, [] { return attribute(cudaDevAttrMultiProcessorCount); });
+  return sms > 0 ? sms : 148;  // planning without a device (workspace sizing): assume a B200
 }
 
 int require_sm100() {
-  const DevInfo* d = dev_info();
-  if (!d) return fail_cuda("query device");
-  if (d->major != 10) return fail(TYBOK_ERR_ARCH, "tybok_b200 kernels need an sm_100 (B200) device");
+  static DeviceCache cache;
+  const int major = per_device(cache, [] { return attribute(cudaDevAttrComputeCapabilityMajor); });
+  if (major == 0) return fail_cuda("query device");
+  if (major != 10) return fail(TYBOK_ERR_ARCH, "tybok_b200 kernels need an sm_100 (B200) device");
   return TYBOK_OK;
 }
 
@@ -80,13 +66,15 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
+  static std::atomic<EncodeTiledFn> found{nullptr};
+  EncodeTiledFn fn = found.load(std::memory_order_acquire);
   if (!fn) {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
         q == cudaDriverEntryPointSuccess)
       fn = reinterpret_cast<EncodeTiledFn>(p);
+    found.store(fn, std::memory_order_release);
   }
   return fn;
 }

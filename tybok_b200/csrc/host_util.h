@@ -4,6 +4,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 
 namespace tb {
@@ -18,6 +19,23 @@ int current_device();
 int sm_count();
 // TYBOK_OK when the current device is compute capability 10.x, TYBOK_ERR_ARCH otherwise.
 int require_sm100();
+
+// An answer that belongs to a device (an occupancy, "attributes set"), looked up on its first use there and kept in
+// `cache`; 0 stands for "not known yet" and is asked for again.  Threads that come first together look it up each and
+// store the same.
+constexpr int MAX_DEVICES = 64;
+using DeviceCache = std::atomic<int>[MAX_DEVICES];
+template <class Query>
+int per_device(DeviceCache& cache, Query query) {
+  const int dev = current_device();
+  if (dev < 0 || dev >= MAX_DEVICES) return query();
+  int v = cache[dev].load(std::memory_order_acquire);
+  if (v == 0) {
+    v = query();
+    cache[dev].store(v, std::memory_order_release);
+  }
+  return v;
+}
 
 bool pdl_enabled();
 void count_launch();

@@ -729,9 +729,9 @@ static int round_up(int a, int b) { return (a + b - 1) / b * b; }
 // inside one GPC, so this is less than SMs / splits: 15 clusters of 8 on a B200).  A launch with
 // more clusters than that runs its last ones as a second wave.
 static int max_active_clusters(int splits) {
-  static int cached[MAX_SPLITS + 1] = {};
+  static host::DeviceCache cache[MAX_SPLITS + 1];
   if (splits <= 1) return 1 << 30;
-  if (cached[splits] == 0) {
+  return host::per_device(cache[splits], [splits] {
     cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(1, 1, splits);
@@ -749,9 +749,8 @@ static int max_active_clusters(int splits) {
       cudaGetLastError();
       n = host::sm_count() / (2 * splits);  // conservative guess
     }
-    cached[splits] = std::max(1, n);
-  }
-  return cached[splits];
+    return std::max(1, n);
+  });
 }
 
 static bool make_plan(int M, int N, int K, int nw, int force_bt, int force_splits, Plan& pl, int np = 3) {
@@ -946,14 +945,13 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
     p.dn_eps = fold->eps; p.bias_f32 = fold->bias_rows;
   }
 
-  static bool attr_set[64] = {};
-  const int dev = host::current_device();
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) != cudaSuccess ||
-        cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) != cudaSuccess)
-      return host::fail_cuda("cudaFuncSetAttribute(w8_gemm_kernel)");
-    attr_set[dev] = true;
-  }
+  static host::DeviceCache attr_set;
+  if (!host::per_device(attr_set, [] {
+        return static_cast<int>(
+            cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) == cudaSuccess &&
+            cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) == cudaSuccess);
+      }))
+    return host::fail_cuda("cudaFuncSetAttribute(w8_gemm_kernel)");
 
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(pl.t_tiles, pl.n_tiles, pl.splits);

@@ -629,8 +629,8 @@ PairPlan plan_pair(int M, int rows, int K, int na, int np) {
 
 // Clusters of 2 * splits CTAs that the device holds at once.
 int resident_clusters(int splits) {
-  static int cached[5] = {};
-  if (cached[splits] == 0) {
+  static host::DeviceCache cache[5];
+  return host::per_device(cache[splits], [splits] {
     auto* k = w8_gemm_pair_kernel<EPI_RESIDUAL, true>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM);
     cudaLaunchConfig_t cfg{};
@@ -649,9 +649,8 @@ int resident_clusters(int splits) {
       cudaGetLastError();
       n = host::sm_count() / (2 * splits + 2);
     }
-    cached[splits] = n;
-  }
-  return cached[splits];
+    return n;
+  });
 }
 
 // Split form: one wave of clusters.  The exchange moves (splits - 1) / splits of a 128-channel fp32 tile through
@@ -728,16 +727,15 @@ int launch_gemm_pair(const GemmCall& c) {
   p.wait_limit = host::epilogue_wait_limit() > 0 ? host::epilogue_wait_limit() : kWaitLimitCycles;
   if (c.rope) p.rope = *c.rope;
 
-  static bool attr_set[64] = {};
-  const int dev = host::current_device();
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    for (auto* k : {w8_gemm_pair_kernel<EPI_NONE, false>, w8_gemm_pair_kernel<EPI_GELU, false>, w8_gemm_pair_kernel<EPI_RESIDUAL, false>,
-                    w8_gemm_pair_kernel<EPI_GEGLU, false>, w8_gemm_pair_kernel<EPI_QKV_ROPE, false>, w8_gemm_pair_kernel<EPI_NONE, true>,
-                    w8_gemm_pair_kernel<EPI_GELU, true>, w8_gemm_pair_kernel<EPI_RESIDUAL, true>})
-      if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM) != cudaSuccess)
-        return host::fail_cuda("cudaFuncSetAttribute(w8_gemm_pair_kernel)");
-    attr_set[dev] = true;
-  }
+  static host::DeviceCache attr_set;
+  if (!host::per_device(attr_set, [] {
+        for (auto* k : {w8_gemm_pair_kernel<EPI_NONE, false>, w8_gemm_pair_kernel<EPI_GELU, false>, w8_gemm_pair_kernel<EPI_RESIDUAL, false>,
+                        w8_gemm_pair_kernel<EPI_GEGLU, false>, w8_gemm_pair_kernel<EPI_QKV_ROPE, false>, w8_gemm_pair_kernel<EPI_NONE, true>,
+                        w8_gemm_pair_kernel<EPI_GELU, true>, w8_gemm_pair_kernel<EPI_RESIDUAL, true>})
+          if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM) != cudaSuccess) return 0;
+        return 1;
+      }))
+    return host::fail_cuda("cudaFuncSetAttribute(w8_gemm_pair_kernel)");
   cudaLaunchConfig_t cfg{};
   const int tiles = pl.ch_tiles * pl.tok_tiles;
   const int pairs = c.split ? tiles * pl.splits : std::min(tiles, std::max(1, host::sm_count() / 2));
