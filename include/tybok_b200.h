@@ -263,8 +263,8 @@ int tybok_w8x3_qkv_rope(const void* x_planes, int x_shift, const void* w8_paired
  *   q          [B*L, H*D] bf16 (already rotated);  k_cache / v_cache  [B, G, Lcap, D] bf16, finite
  *   key_valid  NULL or uint8 [B, Lk]: 0 masks a key for every query of that batch element
  *   out        bf16 [B*L, H*D] and/or out_planes [3][B*L][H*D] planes of out * 2^out_shift
- *   workspace  >= tybok_attention_workspace_bytes(B, L, H, Lk) bytes, 16-byte aligned (0 bytes, and
- *              NULL allowed, when Lk <= 128 or L > 128): where the key blocks of a query tile are
+ *   workspace  >= tybok_attention_workspace_needed(B, L, H, G, D, Lk) bytes, 16-byte aligned (0 bytes, and
+ *              NULL allowed, wherever no form that exchanges is taken): where the key blocks of a query tile are
  *              spread over a cluster and the partial outputs do not fit the exchange through
  *              shared memory, they pass through it (L2) and merge in block order.  L > 128, and every
  *              head_dim 128 call, runs one CTA per query tile and head over all keys and exchanges nothing.
@@ -273,6 +273,8 @@ int tybok_w8x3_qkv_rope(const void* x_planes, int x_shift, const void* w8_paired
 int tybok_attention(const void* q, const void* k_cache, const void* v_cache, const void* key_valid, void* out,
                     void* out_planes, int out_shift, int B, int L, int H, int G, int D, int Lk, int Lcap, float scale,
                     void* workspace, size_t workspace_bytes, int* status_word, void* stream);
+/* What tybok_attention of these sizes takes on the current device, and an upper bound over G, D and devices. */
+size_t tybok_attention_workspace_needed(int B, int L, int H, int G, int D, int Lk);
 size_t tybok_attention_workspace_bytes(int B, int L, int H, int Lk);
 
 /* Attention of one sequence at head_dim 128 whose first n_rows keys / values lie token-major, as a host framework keeps

@@ -130,3 +130,26 @@ def test_block_takes_modulation_rows_that_lie_apart():
     cache = lambda: [torch.zeros(1, s.heads, 33, s.head_dim, dtype=torch.bfloat16, device="cuda") for _ in range(2)]  # noqa: E731
     mods = table[:, : s.hidden]
     assert torch.equal(blk.forward(x, mods, cos, sin, cache()), blk.forward(x, mods.contiguous(), cos, sin, cache()))
+
+
+def test_stack_reserves_what_its_forms_take():
+    """Peak of one expert-width layer beside its inputs at batch 32: no exchange workspace where the key loop runs (338 MB), no
+    planes of the folded form where the norms are kernels."""
+    from tybok_b200 import _lib, ops
+
+    b, w, inner, a, l, keys = 32, 1024, 4096, 2048, 50, 594
+    lin = lambda n, k: quantize_w8(torch.full((n, k), 0.01, dtype=torch.bfloat16, device="cuda"))  # noqa: E731
+    stack = _lib.native().GemmaStack(w, 8, 1, 256, [(lin(2560, w), lin(w, 2048), lin(2 * inner, w), None, lin(w, inner), None, None)])
+    mk = lambda *s: torch.zeros(*s, dtype=torch.bfloat16, device="cuda")  # noqa: E731
+    mods = [(torch.zeros(1, 3 * w, device="cuda"), torch.zeros(1, 3 * w, device="cuda"))]
+    args = (mk(b * l, w), b, l, torch.zeros(b * l, dtype=torch.int32, device="cuda"), mk(700, 256), mk(700, 256), [mk(b, 1, keys, 256)],
+            [mk(b, 1, keys, 256)], keys - l, torch.ones(b, keys, dtype=torch.uint8, device="cuda"), mods, None, 0, 1, [], [])
+    stack.forward(*args)
+    torch.cuda.synchronize()
+    base = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    stack.forward(*args)
+    ops.check_status()
+    # two planes and a scale of the norm, q, three planes of the attention and of the hidden rows, three bf16 streams, the result
+    rows = b * l * (2 * w + 4 + 2 * a + 3 * a + 3 * inner + 3 * 2 * w + 2 * w)
+    assert torch.cuda.max_memory_allocated() - base <= rows + (1 << 20)

@@ -199,3 +199,20 @@ def test_single_calls_refuse_disagreeing_operands():
     for call in calls:
         with pytest.raises((TypeError, ValueError)):
             call()
+
+
+def test_attention_workspace_of_the_form_that_is_taken():
+    """Many clusters over one key head, several query tiles and head_dim 128 exchange nothing; what is needed is never more
+    than the bound that knows neither heads nor head size."""
+    from tybok_b200 import _lib
+
+    lib = _lib.load()
+    need = lib.tybok_attention_workspace_needed
+    one = need(1, 50, 8, 1, 256, 594)
+    assert one == lib.tybok_attention_workspace_bytes(1, 50, 8, 594) == 2 * 5 * 8 * (128 * 256 * 4 + 128 * 8)
+    assert need(32, 50, 8, 1, 256, 594) == 0 < lib.tybok_attention_workspace_bytes(32, 50, 8, 594)
+    assert need(32, 50, 8, 2, 256, 594) == 32 * one
+    assert need(1, 50, 8, 1, 256, 128) == need(1, 129, 8, 8, 256, 594) == need(1, 50, 24, 24, 128, 4146) == 0
+    for b in range(1, 40):
+        for keys in (100, 129, 594, 1024):
+            assert need(b, 50, 8, 1, 256, keys) <= lib.tybok_attention_workspace_bytes(b, 50, 8, keys)

@@ -44,6 +44,7 @@ SIGNATURES = {
                                  c_int, c_int, c_int, c_int, c_int, c_int, c_void_p]),
     "tybok_attention": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
                                 c_int, c_int, c_int, c_int, ctypes.c_float, c_void_p, c_size_t, c_void_p, c_void_p]),
+    "tybok_attention_workspace_needed": (c_size_t, [c_int, c_int, c_int, c_int, c_int, c_int]),
     "tybok_attention_workspace_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "tybok_attention_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                      c_int, c_int, c_int, c_int, c_int, ctypes.c_float, c_void_p, c_void_p]),

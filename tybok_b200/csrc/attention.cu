@@ -1678,6 +1678,27 @@ static int at_resident_clusters(int nsplit) {
   });
 }
 
+// Which form a call takes: the key loop for several query tiles or head_dim 128, and for one key head of many clusters.
+// One key head: its query heads are rows of the same product, because row (token, head) of q and of the output lies
+// at (token * H + head) * D.  The key-loop form then runs on L * H rows in full 128-row tiles and reads every key
+// block once, instead of one tile of L rows per head (50 queries, 594 keys, batch 32: 101 -> 18.5 us; 544 x 544,
+// batch 8: 48 -> 34 us).  The cluster form of short suffixes stays ahead while its clusters run in few enough waves:
+// a wave takes about 9 us, the key loop 7.5 us and 2 us per 128 keys (594 keys: batch 3 is 9.5 against 17.6 us,
+// batch 4 18.1 against 17.8; 994 keys: batch 3 17.9 against 23.5, batch 4 26.4 against 23.7).
+static bool at_key_loop(int B, int L, int H, int G, int D, int Lk) {
+  if ((L > AT_BQ || D == 128) && Lk <= PF_MAX_KEYS) return true;
+  const int nsplit = (Lk + AT_BK - 1) / AT_BK;
+  if (G != 1 || H <= 1 || nsplit <= 1 || nsplit > AT_MAX_SPLITS) return false;
+  const int clusters = H * B, resident = at_resident_clusters(nsplit);
+  return 9.0 * ((clusters + resident - 1) / resident) >= 7.5 + 2.0 * nsplit;
+}
+
+static size_t at_workspace(bool key_loop, int B, int L, int H, int Lk) {
+  if (key_loop || Lk <= AT_BK) return 0;  // the key loop exchanges nothing, a single key block merges inside its CTA
+  const size_t nsplit = (static_cast<size_t>(Lk) + AT_BK - 1) / AT_BK, n_qt = (static_cast<size_t>(L) + AT_BQ - 1) / AT_BQ;
+  return 2 * nsplit * n_qt * H * B * AT_WS_PER_CTA;  // room for the split-column form of small grids
+}
+
 static int at_set_attributes() {
   static host::DeviceCache cache;
   const bool done = host::per_device(cache, [] {
@@ -1766,12 +1787,16 @@ int tybok_qknorm_rope_store(const void* src, int64_t ld, int q_off, int k_off, i
   return TYBOK_OK;
 }
 
+size_t tybok_attention_workspace_needed(int B, int L, int H, int G, int D, int Lk) {
+  using namespace tb;
+  if (B <= 0 || L <= 0 || H <= 0 || G <= 0 || Lk <= 0) return 0;
+  return at_workspace(at_key_loop(B, L, H, G, D, Lk), B, L, H, Lk);
+}
+
 size_t tybok_attention_workspace_bytes(int B, int L, int H, int Lk) {
   using namespace tb;
-  if (B <= 0 || L <= 0 || H <= 0 || Lk <= AT_BK) return 0;  // a single key block merges inside its CTA
-  if (L > AT_BQ && Lk <= PF_MAX_KEYS) return 0;             // the key-loop form exchanges nothing
-  const size_t nsplit = (static_cast<size_t>(Lk) + AT_BK - 1) / AT_BK, n_qt = (static_cast<size_t>(L) + AT_BQ - 1) / AT_BQ;
-  return 2 * nsplit * n_qt * H * B * AT_WS_PER_CTA;  // room for the split-column form of small grids
+  if (B <= 0 || L <= 0 || H <= 0) return 0;
+  return at_workspace(L > AT_BQ && Lk <= PF_MAX_KEYS, B, L, H, Lk);
 }
 
 int tybok_attention(const void* q, const void* k_cache, const void* v_cache, const void* key_valid, void* out,
@@ -1783,8 +1808,7 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   if (B <= 0 || L <= 0 || H <= 0 || G <= 0 || H % G != 0 || Lk <= 0 || Lk > Lcap)
     return host::fail(TYBOK_ERR_ARG, "attention: bad shape (H % G == 0, 0 < Lk <= Lcap)");
   const int nsplit = (Lk + AT_BK - 1) / AT_BK;
-  // several query tiles, or head_dim 128: the key-loop form
-  bool prefill = (L > AT_BQ || D == 128) && Lk <= PF_MAX_KEYS;
+  const bool prefill = at_key_loop(B, L, H, G, D, Lk);
   if (D == 128 && !prefill) return host::fail(TYBOK_ERR_ARG, "attention: at most 8192 keys at head_dim 128");
   if (!prefill && nsplit > AT_MAX_SPLITS)
     return host::fail(TYBOK_ERR_ARG, "attention: at most 1024 keys (8 blocks of 128 per cluster) for up to 128 queries, "
@@ -1793,19 +1817,9 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
        reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_planes)) & 15)
     return host::fail(TYBOK_ERR_ARG, "attention: tensors must be 16-byte aligned");
   if (out_shift < -60 || out_shift > 60) return host::fail(TYBOK_ERR_ARG, "attention: exponent shift out of range");
-  // One key head: its query heads are rows of the same product, because row (token, head) of q and of the output lies
-  // at (token * H + head) * D.  The key-loop form then runs on L * H rows in full 128-row tiles and reads every key
-  // block once, instead of one tile of L rows per head (50 queries, 594 keys, batch 32: 101 -> 18.5 us; 544 x 544,
-  // batch 8: 48 -> 34 us).  The cluster form of short suffixes stays ahead while its clusters run in few enough waves:
-  // a wave takes about 9 us, the key loop 7.5 us and 2 us per 128 keys (594 keys: batch 3 is 9.5 against 17.6 us,
-  // batch 4 18.1 against 17.8; 994 keys: batch 3 17.9 against 23.5, batch 4 26.4 against 23.7).
-  if (!prefill && G == 1 && H > 1 && nsplit > 1) {
-    const int clusters = H * B, resident = at_resident_clusters(nsplit);
-    prefill = 9.0 * ((clusters + resident - 1) / resident) >= 7.5 + 2.0 * nsplit;
-  }
-  const size_t need = prefill ? 0 : tybok_attention_workspace_bytes(B, L, H, Lk);
+  const size_t need = at_workspace(prefill, B, L, H, Lk);
   if (need && (!workspace || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 15)))
-    return host::fail(TYBOK_ERR_WORKSPACE, "attention: workspace must hold tybok_attention_workspace_bytes(), 16-byte aligned");
+    return host::fail(TYBOK_ERR_WORKSPACE, "attention: workspace must hold tybok_attention_workspace_needed(), 16-byte aligned");
   if (int rc = host::require_sm100()) return rc;
 
   if (prefill && G == 1) {

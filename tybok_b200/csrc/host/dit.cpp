@@ -66,8 +66,8 @@ class DitBlock {
     const float scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(hd_)));
 
     // ---- workspace: normed planes | union of (qkv, q, attention planes) and the FFN's hidden planes | two residual rows
-    size_t at_ws = 0;
-    if (hd_ != 128) at_ws = std::max(tybok_attention_workspace_bytes(1, m, heads_, lk), lc ? tybok_attention_workspace_bytes(1, m, heads_, lc) : 0);
+    size_t at_ws = k_rows ? 0 : tybok_attention_workspace_needed(1, m, heads_, heads_, hd_, lk);
+    if (cross_k && cross_k->dim() != 2) at_ws = std::max(at_ws, tybok_attention_workspace_needed(1, m, heads_, heads_, hd_, lc));
     Arena ar;
     const size_t np = ar.add(size_t(two ? 2 : 3) * m * h), rs = ar.add(size_t(4) * m);
     const size_t x1 = ar.add(size_t(2) * m * h), x2 = ar.add(size_t(2) * m * h), ws = ar.add(at_ws);

@@ -89,13 +89,19 @@ class GemmaStack {
     const c10::cuda::CUDAGuard guard(x.device());
 
     const int inner = layers_[0].down.k;
-    const size_t at_ws = hd_ == 128 ? 0 : tybok_attention_workspace_bytes(b, l, heads_, keys);
+    bool packed = true, any_packed = false;
+    for (int i = first; i < first + count; ++i) {
+      packed = packed && layers_[i].packed;
+      any_packed = any_packed || layers_[i].packed;
+    }
+    const bool folds = mods && fold && m < TWO_PLANE_MIN_TOKENS && any_packed;
+    const size_t at_ws = tybok_attention_workspace_needed(b, l, heads_, kv_, hd_, keys);
+    const size_t u = folds ? size_t(3) * m * w_ : 0, part = folds ? size_t(4) * m * (w_ / 128 + 1) : 0;
     Arena ar;
-    const size_t np = ar.add(size_t(3) * m * w_), rs = ar.add(size_t(4) * m), q = ar.add(size_t(2) * m * a), ap = ar.add(size_t(3) * m * a);
-    const size_t hp = ar.add(size_t(3) * m * inner), x1 = ar.add(size_t(2) * m * w_), ws = ar.add(at_ws);
-    const size_t xa = ar.add(size_t(2) * m * w_), xb = ar.add(size_t(2) * m * w_);
-    const size_t up0 = ar.add(size_t(3) * m * w_), up1 = ar.add(size_t(3) * m * w_);
-    const size_t part0 = ar.add(size_t(4) * m * (w_ / 128 + 1)), part1 = ar.add(size_t(4) * m * (w_ / 128 + 1));
+    const size_t np = ar.add(size_t(packed && m >= TWO_PLANE_MIN_TOKENS ? 2 : 3) * m * w_), rs = ar.add(size_t(4) * m);
+    const size_t q = ar.add(size_t(2) * m * a), ap = ar.add(size_t(3) * m * a), hp = ar.add(size_t(3) * m * inner);
+    const size_t x1 = ar.add(size_t(2) * m * w_), xa = ar.add(size_t(2) * m * w_), xb = ar.add(size_t(2) * m * w_), ws = ar.add(at_ws);
+    const size_t up0 = ar.add(u), up1 = ar.add(u), part0 = ar.add(part), part1 = ar.add(part);
     ar.allocate(x0);
     Tensor y = at::empty({m, w_}, x0.options());
     void* st = stream_of(x);

@@ -140,8 +140,7 @@ static std::tuple<Tensor, Tensor> attention(const Tensor& q, const Tensor& kc, c
   Tensor y = out_bf16 ? at::empty({b * tokens, h * d}, q.options()) : at::empty({0}, q.options());
   const auto bytes = q.options().dtype(at::kByte);
   Tensor yp = out_planes ? at::empty({3, b * tokens, h * d}, bytes) : at::empty({0}, bytes);
-  // head_dim 128 always takes the key-loop kernel, which exchanges nothing
-  const size_t need = d == 128 ? 0 : tybok_attention_workspace_bytes(b, tokens, h, keys);
+  const size_t need = tybok_attention_workspace_needed(b, tokens, h, g, d, keys);
   Tensor ws;
   if (need) ws = at::empty({static_cast<int64_t>(need)}, bytes);
   check(tybok_attention(ptr(q), ptr(kc), ptr(vc), ptr(valid), out_bf16 ? ptr(y) : nullptr, out_planes ? ptr(yp) : nullptr, out_shift, b,
