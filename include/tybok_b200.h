@@ -63,7 +63,8 @@ size_t tybok_w8a16_workspace_bytes(int M, int N, int K, int dual);
  *   y        bf16, row stride ldy (ldy % 4 == 0, pointer 8-byte aligned)
  *   epilogue TYBOK_EPI_*; residual bf16 [M,N] stride ldres (EPI_RESIDUAL only)
  *   gate     NULL, or per-row-group gate [ceil(M/rows_per_gate), N] with row stride ldgate:
- *            fp32 when gate_is_bf16 == 0 (rounded to bf16 before use), bf16 otherwise
+ *            fp32 when gate_is_bf16 == 0 (rounded to bf16 before use), bf16 otherwise; 16-byte (bf16: 8-byte) aligned
+ *            rows, ldgate % 4 == 0, wherever the one-tile kernel runs
  *   token_tile, splits  0 = choose automatically; otherwise force the token tile
  *            (multiple of 16, <= 256) / the split-K factor (<= 8, one cluster per output tile)
  *   workspace  >= tybok_w8a16_workspace_bytes(...) bytes, 16-byte aligned

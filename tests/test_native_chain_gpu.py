@@ -153,3 +153,24 @@ def test_stack_reserves_what_its_forms_take():
     # two planes and a scale of the norm, q, three planes of the attention and of the hidden rows, three bf16 streams, the result
     rows = b * l * (2 * w + 4 + 2 * a + 3 * a + 3 * inner + 3 * 2 * w + 2 * w)
     assert torch.cuda.max_memory_allocated() - base <= rows + (1 << 20)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("m,n", [(20, 256), (300, 9600)])  # one tile per CTA, which reads gates in vectors; CTA pairs, which do not
+def test_gate_off_its_alignment(m, n, dtype):
+    from tybok_b200 import _lib, ops
+
+    g = torch.Generator(device="cuda").manual_seed(m)
+    w8, sc = quantize_w8(_rnd(g, n, 256, std=0.02))
+    x, res, gate = _rnd(g, m, 256), _rnd(g, m, n), _rnd(g, 2, n).to(dtype)
+    run = lambda gt: ops.w8a16_linear(x, w8, sc, epilogue=ops.EPI_RESIDUAL, residual=res, gate=gt, rows_per_gate=(m + 1) // 2)  # noqa: E731
+    want = run(gate)
+    for off, wide in ((1, n + 4), (4, n + 3)):
+        t = torch.zeros(2 * wide + 8, dtype=dtype, device="cuda")[off : off + 2 * wide].view(2, wide)[:, :n]
+        t.copy_(gate)
+        if m == 20:
+            with pytest.raises(_lib.TybokError, match="gate must be"):
+                run(t)
+        else:
+            assert torch.equal(run(t), want)
+    ops.check_status()

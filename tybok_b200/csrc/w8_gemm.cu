@@ -910,6 +910,10 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
     return launch_gemm_pair(c);
   }
 
+  // this kernel reads four gate values at a time (the pair kernel reads one)
+  if (epi == EPI_RESIDUAL && gate && ((reinterpret_cast<uintptr_t>(gate) & (gate_bf16 ? 7 : 15)) || ldgate % 4 != 0))
+    return host::fail(TYBOK_ERR_ARG, "w8 gemm: gate must be 16-byte aligned (bf16: 8), ldgate % 4 == 0");
+
   CUtensorMap tm_w0, tm_w1, tm_x;
   if (int rc = host::tensor_map_2d(&tm_w0, w0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, K, N, K, BK, BN)) return rc;
   tm_w1 = tm_w0;
