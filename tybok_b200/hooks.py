@@ -50,14 +50,13 @@ def make_mlp_forward(mlp, device: str | torch.device = "cuda"):
     ``GemmaMLP`` (tybok/policies/pi05/models/layers.py:87-95): bf16 -> planes, one gate/up GEMM
     whose epilogue writes the planes of the intermediate, the down projection."""
     gate, up, down = _w8(mlp.gate_proj, device), _w8(mlp.up_proj, device), _w8(mlp.down_proj, device)
-    if gate[0].shape[0] % 64 == 0:
-        chain = _lib.native().Mlp(ops.pack_gate_up(*gate, *up), None, down)
-    else:
-        chain = _lib.native().Mlp(gate, up, down)
+    weights = (ops.pack_gate_up(*gate, *up), None, down) if gate[0].shape[0] % 64 == 0 else (gate, up, down)
+    chain = _lib.native().Mlp(*weights)
+    tensors = [t for w in weights for t in (w or (None, None))]
 
     def forward(x: torch.Tensor) -> torch.Tensor:
         _need_cuda(x)
-        return chain.forward(x)
+        return chain.forward(x) if ops.native_takes(x) else torch.ops.tybok_b200.mlp(x, *tensors)
 
     return forward
 
@@ -70,10 +69,13 @@ def make_fused_ffn_tail(blk, device: str | torch.device = "cuda"):
     ``[B, 6, H]`` table are fine); the whole batch is one launch chain."""
     up = (*_w8(blk.ffn[0], device), _bias(blk.ffn[0], device))
     down = (*_w8(blk.ffn[2], device), _bias(blk.ffn[2], device))
-    chain = _lib.native().FfnTail(up, down, float(getattr(blk, "eps", 1e-6)))
+    eps = float(getattr(blk, "eps", 1e-6))
+    chain = _lib.native().FfnTail(up, down, eps)
 
     def tail(x: torch.Tensor, shift_mlp: torch.Tensor, scale_mlp: torch.Tensor, gate_mlp: torch.Tensor) -> torch.Tensor:
         _need_cuda(x)
+        if not ops.native_takes(x, shift_mlp, scale_mlp, gate_mlp):
+            return torch.ops.tybok_b200.ffn_tail(x, shift_mlp, scale_mlp, gate_mlp, *up, *down, eps)
         return chain.forward(x, shift_mlp, scale_mlp, gate_mlp)
 
     return tail

@@ -76,6 +76,13 @@ _L.define("w8x3_qkv_rope_adarms(Tensor u_planes, int shift, Tensor ss_part, floa
           "Tensor scale_paired, Tensor pos, Tensor cos, Tensor sin, Tensor(a!) k_cache, Tensor(b!) v_cache, int heads, "
           "int key_off, int token_tile, int splits) -> Tensor")
 
+_L.define("w8a16_linear(Tensor x, Tensor w8, Tensor scale, Tensor? bias, int epilogue, Tensor? residual, Tensor? gate, "
+          "int rows_per_gate, int token_tile, int splits, int shift) -> Tensor")
+_L.define("mlp(Tensor x, Tensor gate_up, Tensor gate_up_scale, Tensor? up, Tensor? up_scale, Tensor down, Tensor down_scale) "
+          "-> Tensor")
+_L.define("ffn_tail(Tensor x, Tensor shift, Tensor scale, Tensor gate, Tensor up, Tensor up_scale, Tensor? up_bias, Tensor down, "
+          "Tensor down_scale, Tensor? down_bias, float eps) -> Tensor")
+
 NORM_RMS, NORM_ADARMS, NORM_LN_MODULATE, NORM_LN_AFFINE = 0, 1, 2, 3
 EPI_GEGLU_PACKED = 4
 
@@ -238,6 +245,27 @@ def _rope_store_cuda(qkv, pos, cos, sin, k_cache, v_cache, heads, key_off):
                               int(key_off), _stream(qkv))
     _lib.check(rc, "tybok_rope_store")
     return q
+
+
+def native_takes(*tensors: torch.Tensor | None) -> bool:
+    """Whether a call on these may go to the native extension as it stands.  Inside a function transform (``vmap``, ``jvp``) or a
+    dispatch mode, and for tensor subclasses, it goes through the registered op of the same name, so that whoever
+    intercepts torch ops still sees one; that op ends in the same native call."""
+    if torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack():
+        return False
+    return all(t is None or type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in tensors)
+
+
+def _w8a16_linear_cuda(*args):
+    return _lib.native().w8a16_linear(*args)
+
+
+def _mlp_cuda(x, gate_up, gate_up_scale, up, up_scale, down, down_scale):
+    return _lib.native().Mlp((gate_up, gate_up_scale), None if up is None else (up, up_scale), (down, down_scale)).forward(x)
+
+
+def _ffn_tail_cuda(x, shift, scale, gate, up, up_scale, up_bias, down, down_scale, down_bias, eps):
+    return _lib.native().FfnTail((up, up_scale, up_bias), (down, down_scale, down_bias), eps).forward(x, shift, scale, gate)
 
 
 def _attention_cuda(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift):
@@ -442,6 +470,9 @@ _L.impl("layernorm_affine", _layernorm_affine_cuda, "CUDA")
 _L.impl("qknorm_rope_store", _qknorm_rope_store_cuda, "CUDA")
 _L.impl("add_layernorm", _add_layernorm_any, "CUDA")
 _L.impl("split3", _split3_cuda, "CUDA")
+_L.impl("w8a16_linear", _w8a16_linear_cuda, "CUDA")
+_L.impl("mlp", _mlp_cuda, "CUDA")
+_L.impl("ffn_tail", _ffn_tail_cuda, "CUDA")
 _L.impl("w8x3_linear", _w8x3_linear_cuda, "CUDA")
 _L.impl("w8x3_geglu", _w8x3_geglu_cuda, "CUDA")
 
@@ -511,7 +542,8 @@ def w8x3_geglu_packed(planes, shift, w8_packed, scale_packed, *, out_bf16=True, 
 def w8a16_linear(x, w8, scale, bias=None, *, epilogue=EPI_NONE, residual=None, gate=None, rows_per_gate=1,
                  token_tile=0, splits=0, shift=DEFAULT_SHIFT) -> torch.Tensor:
     """``epilogue(x @ (w8*scale).T + bias)`` for bf16 ``x``: ``split3`` then ``w8x3_linear``, as one native call."""
-    return _lib.native().w8a16_linear(x, w8, scale, bias, epilogue, residual, gate, rows_per_gate, token_tile, splits, shift)
+    call = _lib.native().w8a16_linear if native_takes(x, w8, scale, bias, residual, gate) else torch.ops.tybok_b200.w8a16_linear
+    return call(x, w8, scale, bias, epilogue, residual, gate, rows_per_gate, token_tile, splits, shift)
 
 
 def w8a16_geglu(x, w8_gate, scale_gate, w8_up, scale_up, *, token_tile=0, splits=0, shift=DEFAULT_SHIFT):
@@ -538,7 +570,8 @@ def attention(q, k_cache, v_cache, key_valid=None, *, tokens, keys, scale, out_b
               out_shift=DEFAULT_SHIFT):
     """GQA attention over the first ``keys`` cache rows; returns ``(out_bf16, out_planes)``; see
     ``tybok_attention``."""
-    return _lib.native().attention(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
+    call = _lib.native().attention if native_takes(q, k_cache, v_cache, key_valid) else torch.ops.tybok_b200.attention
+    return call(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
 
 
 def layernorm_modulate(x, shift, scale, *, eps=1e-6, out_bf16=False, out_planes=True, out_shift=DEFAULT_SHIFT):
