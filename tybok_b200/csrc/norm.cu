@@ -1,7 +1,8 @@
-// RMS normalisation that feeds a W8 GEMM: one warp per token row, fp32 statistics, output as
-// the three e5m2 activation planes (and/or bf16).
+// The norms that feed a W8 GEMM: one CTA per token row (one warp for rows of at most 256 elements), fp32 statistics, output
+// as activation planes (three e5m2, or two e4m3 with a row scale) and/or bf16; further down the SigLIP tower's residual
+// add + LayerNorm.
 //
-// Two forms, both from tybok/policies/pi05/models/layers.py:34-84:
+// The RMS forms, both from tybok/policies/pi05/models/layers.py:34-84:
 //   plain Gemma norm   y = bf16( x * rsqrt(mean(x^2) + eps) * (1 + weight) )
 //   AdaRMS norm        y = bf16( x * rsqrt(mean(x^2) + eps) * (1 + scale) + shift )
 // where scale/shift are the first two thirds of a precomputed dense(cond) row
@@ -18,7 +19,7 @@
 
 namespace tb {
 
-constexpr int NORM_MAX_VEC = 16;  // 16 vectors of 8 elements per lane: W <= 4096
+constexpr int NORM_MAX_W = 4096;
 
 struct NormParams {
   const __nv_bfloat16* x;
@@ -42,175 +43,131 @@ struct NormParams {
   int* dbg;  // debugging aid: stage counters, NULL in production
 };
 
-// Rows of at most 256 elements, one warp each.  VEC = 8-element vectors per lane; FULL = every lane owns exactly VEC vectors (W == 256 * VEC),
-// which removes the bounds predicates so that the loads can be hoisted and overlapped.
-template <int VEC, bool FULL>
-__global__ void __launch_bounds__(128) rmsnorm_kernel(const NormParams p) {
+// Rows of at most 256 elements: one warp each, eight elements per lane.
+__global__ void __launch_bounds__(128) norm_small_kernel(const NormParams p) {
   // Let the next kernel in the stream start its preamble (weight prefetch) right away; it still
   // waits for this grid to finish before it reads what is written here.
   if (p.pdl) pdl_launch_dependents();
   if (threadIdx.x == 0) dbg_stage(p.dbg, 8, 0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m = blockIdx.x * 4 + warp;
-  const int nvec = p.W / 8;  // 8-element vectors per row
+  const int lane = threadIdx.x & 31, m = blockIdx.x * 4 + (threadIdx.x >> 5), c = lane * 8;
+  const bool live = c < p.W;
   // Scale / shift are constants of the step: fetch them before waiting for the previous kernel.
   const float* mod = (p.mod && m < p.M) ? p.mod + static_cast<long long>(m / p.rows_per_group) * p.ldmod : nullptr;
-  constexpr bool PRE = VEC <= 8;  // wider rows would not fit the constants in registers
-  float4 csc[PRE ? VEC : 1][2], csh[PRE ? VEC : 1][2];
-  if (PRE && !p.ln_scale && m < p.M) {
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      const int c = lane + 32 * i;
-      if (FULL || c < nvec) {
-        const float* a = mod ? mod + c * 8 : p.weight + c * 8;
-        csc[PRE ? i : 0][0] = *reinterpret_cast<const float4*>(a);
-        csc[PRE ? i : 0][1] = *reinterpret_cast<const float4*>(a + 4);
-        if (mod) {
-          csh[PRE ? i : 0][0] = *reinterpret_cast<const float4*>(a + p.W);
-          csh[PRE ? i : 0][1] = *reinterpret_cast<const float4*>(a + p.W + 4);
-        }
-      }
+  float4 q0 = make_float4(0.f, 0.f, 0.f, 0.f), q1 = q0, h0 = q0, h1 = q0;
+  if (!p.ln_scale && m < p.M && live) {
+    const float* a = mod ? mod + c : p.weight + c;
+    q0 = *reinterpret_cast<const float4*>(a);
+    q1 = *reinterpret_cast<const float4*>(a + 4);
+    if (mod) {
+      h0 = *reinterpret_cast<const float4*>(a + p.W);
+      h1 = *reinterpret_cast<const float4*>(a + p.W + 4);
     }
   }
   if (p.pdl) pdl_wait();
   if (threadIdx.x == 0) dbg_stage(p.dbg, 8, 2);
-  if (m < p.M) {
-    const __nv_bfloat16* row = p.x + m * p.ldx;
-    float v[VEC][8];
-    float ss = 0.f;
+  if (m >= p.M) return;
+  float v[8] = {};
+  float ss = 0.f;
+  if (live) {
+    const uint4 raw = *reinterpret_cast<const uint4*>(p.x + m * p.ldx + c);
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
 #pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      const int c = lane + 32 * i;
-      if (FULL || c < nvec) {
-        const uint4 raw = *reinterpret_cast<const uint4*>(row + c * 8);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&raw);
+    for (int e = 0; e < 4; ++e) {
+      v[2 * e] = __bfloat162float(h[e].x);
+      v[2 * e + 1] = __bfloat162float(h[e].y);
+      ss += v[2 * e] * v[2 * e] + v[2 * e + 1] * v[2 * e + 1];
+    }
+  }
+  if (p.ln_scale) {  // LayerNorm: centre first, then the variance of the centred values
+    float sm = 0.f;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          v[i][2 * e] = __bfloat162float(h[e].x);
-          v[i][2 * e + 1] = __bfloat162float(h[e].y);
-          ss += v[i][2 * e] * v[i][2 * e] + v[i][2 * e + 1] * v[i][2 * e + 1];
-        }
+    for (int e = 0; e < 8; ++e) sm += v[e];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
+    const float mean = sm / static_cast<float>(p.W);
+    ss = 0.f;
+    if (live) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        v[e] -= mean;
+        ss += v[e] * v[e];
       }
     }
-    float mean = 0.f;
-    if (p.ln_scale) {  // LayerNorm: centre first, then the variance of the centred values
-      float sm = 0.f;
+  }
 #pragma unroll
-      for (int i = 0; i < VEC; ++i)
-        if (FULL || lane + 32 * i < nvec) {
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  const float rstd = rsqrtf(ss / static_cast<float>(p.W) + p.eps);
+  const long long plane = static_cast<long long>(p.M) * p.W;
+  float amax = 0.f;
+  if (live) {
+    float o[8];
+    if (p.ln_scale) {
+      // modulate(LN(x)) with every step rounded to bf16, as the reference's bf16 tensor ops
+      // do: n = bf16(LN), t = bf16(1 + scale), out = bf16(bf16(n * t) + shift).
+      const long long go = static_cast<long long>(m / p.rows_per_group) * p.ldmod;
+      const uint4 rs = *reinterpret_cast<const uint4*>(p.ln_scale + go + c);
+      const uint4 rh = *reinterpret_cast<const uint4*>(p.ln_shift + go + c);
+      const __nv_bfloat16* ps = reinterpret_cast<const __nv_bfloat16*>(&rs);
+      const __nv_bfloat16* ph = reinterpret_cast<const __nv_bfloat16*>(&rh);
+      if (p.ln_affine) {  // fp32 statistics and fp32 affine, one rounding (wan_base.py:141-148)
 #pragma unroll
-          for (int e = 0; e < 8; ++e) sm += v[i][e];
-        }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sm += __shfl_xor_sync(0xffffffffu, sm, o);
-      mean = sm / static_cast<float>(p.W);
-      ss = 0.f;
-#pragma unroll
-      for (int i = 0; i < VEC; ++i)
-        if (FULL || lane + 32 * i < nvec) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            v[i][e] -= mean;
-            ss += v[i][e] * v[i][e];
-          }
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-    const float rstd = rsqrtf(ss / static_cast<float>(p.W) + p.eps);
-    const long long plane = static_cast<long long>(p.M) * p.W;
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < VEC; ++i) {
-      const int c = lane + 32 * i;
-      if (FULL || c < nvec) {
-        float o[8];
-        if (p.ln_scale) {
-          // modulate(LN(x)) with every step rounded to bf16, as the reference's bf16 tensor ops
-          // do: n = bf16(LN), t = bf16(1 + scale), out = bf16(bf16(n * t) + shift).
-          const long long go = static_cast<long long>(m / p.rows_per_group) * p.ldmod;
-          const uint4 rs = *reinterpret_cast<const uint4*>(p.ln_scale + go + c * 8);
-          const uint4 rh = *reinterpret_cast<const uint4*>(p.ln_shift + go + c * 8);
-          const __nv_bfloat16* ps = reinterpret_cast<const __nv_bfloat16*>(&rs);
-          const __nv_bfloat16* ph = reinterpret_cast<const __nv_bfloat16*>(&rh);
-          if (p.ln_affine) {  // fp32 statistics and fp32 affine, one rounding (wan_base.py:141-148)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = v[i][e] * rstd * __bfloat162float(ps[e]) + __bfloat162float(ph[e]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-              const float nrm = bf16_round(v[i][e] * rstd);
-              const float t = bf16_round(1.0f + __bfloat162float(ps[e]));
-              o[e] = bf16_round(nrm * t) + __bfloat162float(ph[e]);
-            }
-          }
-        } else {
-        // x * rstd is formed in fp32 (the bf16 x promotes), as in the reference's _norm
-        float4 q0, q1, h0 = make_float4(0.f, 0.f, 0.f, 0.f), h1 = h0;
-        if (PRE) {
-          q0 = csc[PRE ? i : 0][0]; q1 = csc[PRE ? i : 0][1];
-          if (mod) { h0 = csh[PRE ? i : 0][0]; h1 = csh[PRE ? i : 0][1]; }
-        } else {
-          const float* a = mod ? mod + c * 8 : p.weight + c * 8;
-          q0 = *reinterpret_cast<const float4*>(a); q1 = *reinterpret_cast<const float4*>(a + 4);
-          if (mod) { h0 = *reinterpret_cast<const float4*>(a + p.W); h1 = *reinterpret_cast<const float4*>(a + p.W + 4); }
-        }
-        const float sc[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        const float sh[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+        for (int e = 0; e < 8; ++e) o[e] = v[e] * rstd * __bfloat162float(ps[e]) + __bfloat162float(ph[e]);
+      } else {
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          float t = v[i][e] * rstd * (1.0f + sc[e]);
-          if (mod) t = v[i][e] * rstd * (1.0f + sc[e]) + sh[e];
-          o[e] = t;
+          const float nrm = bf16_round(v[e] * rstd);
+          const float t = bf16_round(1.0f + __bfloat162float(ps[e]));
+          o[e] = bf16_round(nrm * t) + __bfloat162float(ph[e]);
         }
-        }
-        __nv_bfloat162 b[4];
+      }
+    } else {
+      // x * rstd is formed in fp32 (the bf16 x promotes), as in the reference's _norm
+      const float sc[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+      const float sh[8] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) b[e] = __floats2bfloat162_rn(o[2 * e], o[2 * e + 1]);
-        if (p.y) *reinterpret_cast<uint4*>(p.y + m * p.ldy + c * 8) = *reinterpret_cast<const uint4*>(b);
-        if (p.planes) {
-          const float lo[4] = {__bfloat162float(b[0].x) * p.plane_scale, __bfloat162float(b[0].y) * p.plane_scale,
-                               __bfloat162float(b[1].x) * p.plane_scale, __bfloat162float(b[1].y) * p.plane_scale};
-          const float hi[4] = {__bfloat162float(b[2].x) * p.plane_scale, __bfloat162float(b[2].y) * p.plane_scale,
-                               __bfloat162float(b[3].x) * p.plane_scale, __bfloat162float(b[3].y) * p.plane_scale};
-          uint2 w1, w2, w3;
-          split3_quad(lo, w1.x, w2.x, w3.x);
-          split3_quad(hi, w1.y, w2.y, w3.y);
-          uint8_t* dst = p.planes + static_cast<long long>(m) * p.W + c * 8;
-          *reinterpret_cast<uint2*>(dst) = w1;
-          *reinterpret_cast<uint2*>(dst + plane) = w2;
-          *reinterpret_cast<uint2*>(dst + 2 * plane) = w3;
-        }
-        if (p.planes2) {  // keep the rounded row (over v, which is dead now) until its maximum is known
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            v[i][2 * e] = __bfloat162float(b[e].x);
-            v[i][2 * e + 1] = __bfloat162float(b[e].y);
-            amax = fmaxf(amax, fmaxf(fabsf(v[i][2 * e]), fabsf(v[i][2 * e + 1])));
-          }
-        }
+      for (int e = 0; e < 8; ++e) {
+        float t = v[e] * rstd * (1.0f + sc[e]);
+        if (mod) t = v[e] * rstd * (1.0f + sc[e]) + sh[e];
+        o[e] = t;
       }
     }
-    if (p.planes2) {
+    __nv_bfloat162 b[4];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-      float up, down;
-      row_pow2(amax, up, down);
-      if (lane == 0) p.row_scale[m] = down;
+    for (int e = 0; e < 4; ++e) b[e] = __floats2bfloat162_rn(o[2 * e], o[2 * e + 1]);
+    if (p.y) *reinterpret_cast<uint4*>(p.y + m * p.ldy + c) = *reinterpret_cast<const uint4*>(b);
 #pragma unroll
-      for (int i = 0; i < VEC; ++i) {
-        const int c = lane + 32 * i;
-        if (FULL || c < nvec) {
-          const float lo[4] = {v[i][0] * up, v[i][1] * up, v[i][2] * up, v[i][3] * up};
-          const float hi[4] = {v[i][4] * up, v[i][5] * up, v[i][6] * up, v[i][7] * up};
-          uint2 w1, w2;
-          split2_quad(lo, w1.x, w2.x);
-          split2_quad(hi, w1.y, w2.y);
-          uint8_t* dst = p.planes2 + static_cast<long long>(m) * p.W + c * 8;
-          *reinterpret_cast<uint2*>(dst) = w1;
-          *reinterpret_cast<uint2*>(dst + plane) = w2;
-        }
-      }
+    for (int e = 0; e < 4; ++e) {  // the rounded values
+      v[2 * e] = __bfloat162float(b[e].x);
+      v[2 * e + 1] = __bfloat162float(b[e].y);
+      amax = fmaxf(amax, fmaxf(fabsf(v[2 * e]), fabsf(v[2 * e + 1])));
+    }
+    if (p.planes) {
+      const float lo[4] = {v[0] * p.plane_scale, v[1] * p.plane_scale, v[2] * p.plane_scale, v[3] * p.plane_scale};
+      const float hi[4] = {v[4] * p.plane_scale, v[5] * p.plane_scale, v[6] * p.plane_scale, v[7] * p.plane_scale};
+      uint2 w1, w2, w3;
+      split3_quad(lo, w1.x, w2.x, w3.x);
+      split3_quad(hi, w1.y, w2.y, w3.y);
+      uint8_t* dst = p.planes + static_cast<long long>(m) * p.W + c;
+      *reinterpret_cast<uint2*>(dst) = w1;
+      *reinterpret_cast<uint2*>(dst + plane) = w2;
+      *reinterpret_cast<uint2*>(dst + 2 * plane) = w3;
+    }
+  }
+  if (p.planes2) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    float up, down;
+    row_pow2(amax, up, down);
+    if (lane == 0) p.row_scale[m] = down;
+    if (live) {
+      const float lo[4] = {v[0] * up, v[1] * up, v[2] * up, v[3] * up};
+      const float hi[4] = {v[4] * up, v[5] * up, v[6] * up, v[7] * up};
+      uint2 w1, w2;
+      split2_quad(lo, w1.x, w2.x);
+      split2_quad(hi, w1.y, w2.y);
+      uint8_t* dst = p.planes2 + static_cast<long long>(m) * p.W + c;
+      *reinterpret_cast<uint2*>(dst) = w1;
+      *reinterpret_cast<uint2*>(dst + plane) = w2;
     }
   }
 }
@@ -785,7 +742,7 @@ static int launch_norm(const void* x, int64_t ldx, const float* weight, const fl
   if (!x || (!y && !y_planes && !y_planes2) || (!weight && !mod && !ln_scale)) return host::fail(TYBOK_ERR_ARG, "rmsnorm: null pointer argument");
   if ((y_planes2 != nullptr) != (row_scale != nullptr) || (reinterpret_cast<uintptr_t>(y_planes2) & 7))
     return host::fail(TYBOK_ERR_ARG, "norm: two-plane output needs both planes (8-byte aligned) and row_scale");
-  if (M <= 0 || W <= 0 || W % 8 != 0 || W > NORM_MAX_VEC * 256)
+  if (M <= 0 || W <= 0 || W % 8 != 0 || W > NORM_MAX_W)
     return host::fail(TYBOK_ERR_ARG, "rmsnorm: W must be a multiple of 8 and <= 4096");
   if (ldx % 8 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) || (y && ((reinterpret_cast<uintptr_t>(y) & 15) || ldy % 8 != 0)) ||
       (y_planes && (reinterpret_cast<uintptr_t>(y_planes) & 7)) ||
@@ -804,23 +761,18 @@ static int launch_norm(const void* x, int64_t ldx, const float* weight, const fl
   p.y = static_cast<__nv_bfloat16*>(y); p.ldy = ldy; p.pdl = host::pdl_enabled() ? 1 : 0;
   p.dbg = host::counter_buffer();
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((M + 3) / 4);
-  cfg.blockDim = dim3(128);
+  const int warps = (W / 8 + 31) / 32;  // of eight elements per lane
+  const bool small = warps == 1;
+  cfg.gridDim = dim3(small ? (M + 3) / 4 : M);
+  cfg.blockDim = dim3(32 * (small ? 4 : ln_scale ? warps : (warps + RMS_V - 1) / RMS_V));
   cfg.stream = static_cast<cudaStream_t>(stream);
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.pdl;
-  const int per_lane = (W / 8 + 31) / 32;
-  cudaError_t e;
-  if (per_lane >= 2) {  // more than 256 elements: one CTA per row
-    cfg.gridDim = dim3(M);
-    cfg.blockDim = dim3((ln_scale ? per_lane : (per_lane + RMS_V - 1) / RMS_V) * 32);
-    e = ln_scale ? cudaLaunchKernelEx(&cfg, layernorm_row_kernel, p) : cudaLaunchKernelEx(&cfg, rmsnorm_row_kernel, p);
-  } else if (W == 256) e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<1, true>, p);
-  else e = cudaLaunchKernelEx(&cfg, rmsnorm_kernel<1, false>, p);
-  if (e != cudaSuccess) return host::fail_cuda("launch rmsnorm_kernel");
+  if (cudaLaunchKernelEx(&cfg, small ? norm_small_kernel : ln_scale ? layernorm_row_kernel : rmsnorm_row_kernel, p) != cudaSuccess)
+    return host::fail_cuda("launch of a norm kernel");
   host::count_launch();
   return TYBOK_OK;
 }

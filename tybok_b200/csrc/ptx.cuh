@@ -120,26 +120,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* m, uin
       "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(crd0), "r"(crd1)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_2d_hint(void* dst, const CUtensorMap* m, uint64_t* bar, int crd0, int crd1,
-                                                 uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], "
-      "[%2], %5;" ::"r"(smem_u32(dst)),
-      "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(crd0), "r"(crd1), "l"(policy)
-      : "memory");
-}
-__device__ __forceinline__ uint64_t policy_evict_first() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ uint64_t policy_evict_last() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-
-
 // 3-D tiled load (crd0 innermost).
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* m, uint64_t* bar, int crd0, int crd1,
                                             int crd2) {
@@ -192,16 +172,6 @@ __device__ __forceinline__ uint32_t dsmem_addr(uint32_t local, uint32_t rank) {
 __device__ __forceinline__ void st_dsmem(uint32_t addr, uint32_t v) {
   asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
-__device__ __forceinline__ float4 ld_dsmem_f4(uint32_t addr) {
-  float4 v;
-  // volatile (ordered after the cluster barrier, itself a volatile asm) but without a memory
-  // clobber, so that ordinary loads/stores around it can still be scheduled freely.
-  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "r"(addr));
-  return v;
-}
-
 // Instruction descriptor for kind::f8f6f4 with A = e4m3, B = e5m2 (both K-major), fp32
 // accumulation: [4,6) D format 1 = f32, [7,10) A format 0 = e4m3, [10,13) B format 1 = e5m2,
 // [17,23) N >> 3, [24,29) M >> 4.
@@ -368,13 +338,7 @@ __device__ __forceinline__ void umma_ss_bf16(uint32_t d_tmem, uint64_t a_desc, u
       : "memory");
 }
 
-// 32 lanes x 8 consecutive 32-bit columns: thread i of the warp reads lane (base + i).
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(taddr)
-               : "memory");
-}
+// 32 lanes x 16 consecutive 32-bit columns: thread i of the warp reads lane (base + i).
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
@@ -405,31 +369,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
 }
 
 // ---------------------------------------------------------------- numerics
-// Expand two e4m3 bytes, already placed in the HIGH byte of each 16-bit half of `p`, into two
-// exact bf16 values. (b & 0x7f) << 4 puts the 4 exponent and 3 mantissa bits into the bf16
-// exponent/mantissa fields, which reads as value * 2^-120 (e4m3 subnormals map onto bf16
-// subnormals, zero onto zero); one bf16x2 multiply by 2^120 restores the value exactly.
-// The two e4m3 NaN encodings (0x7f, 0xff) come out as +-480: weights never hold them.
-__device__ __forceinline__ uint32_t e4m3x2_hi_to_bf16x2(uint32_t p) {
-  uint32_t o = ((p >> 4) & 0x07F007F0u) | (p & 0x80008000u);
-  __nv_bfloat162 v = *reinterpret_cast<__nv_bfloat162*>(&o);
-  const uint32_t kbits = 0x7B807B80u;  // {2^120, 2^120} in bf16
-  __nv_bfloat162 k = *reinterpret_cast<const __nv_bfloat162*>(&kbits);
-  v = __hmul2(v, k);
-  return *reinterpret_cast<uint32_t*>(&v);
-}
-// 4 e4m3 bytes (k, k+1, k+2, k+3 from the low byte up) -> {bf16x2(k,k+1), bf16x2(k+2,k+3)}.
-__device__ __forceinline__ void e4m3x4_to_bf16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
-  lo = e4m3x2_hi_to_bf16x2(__byte_perm(w, 0u, 0x1404));
-  hi = e4m3x2_hi_to_bf16x2(__byte_perm(w, 0u, 0x3424));
-}
-
-__device__ __forceinline__ float gelu_tanh_f(float x) {
-  // 0.5 x (1 + tanh(sqrt(2/pi) (x + 0.044715 x^3))), the form torch's approximate="tanh" uses.
-  const float k0 = 0.7978845608028654f, k1 = 0.044715f;
-  float inner = k0 * (x + k1 * x * x * x);
-  return 0.5f * x * (1.0f + tanhf(inner));
-}
 __device__ __forceinline__ float bf16_round(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
 // Rotate-half RoPE element in bf16 arithmetic with the rounding points of the reference's torch
