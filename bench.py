@@ -264,7 +264,7 @@ def _gemm_roofline(shape, batch: int, dev, peaks, peaks_kind, sweep: bool) -> di
     ``achieved`` aggregates the action-expert launches (M = 50*batch, HBM-bound, 720 of the 792
     launches of a chunk); the prefix launches (M = 544*batch, tensor-bound) are reported beside."""
     from tybok_b200 import ops
-    from tybok_b200.pi05 import TWO_PLANE_MIN_TOKENS
+    from tybok_b200._lib import native
 
     s = shape
 
@@ -287,7 +287,7 @@ def _gemm_roofline(shape, batch: int, dev, peaks, peaks_kind, sweep: bool) -> di
             xp = ops.split3(x, 4)
             res = torch.randn(m, n, device=dev).to(torch.bfloat16)
             # the GEMMs fed by a norm take two e4m3 planes from the model's two-plane threshold on
-            two = m >= TWO_PLANE_MIN_TOKENS and name in ("qkv", "geglu")
+            two = m >= native().TWO_PLANE_MIN_TOKENS and name in ("qkv", "geglu")
             if two:
                 x2, rs = ops.norm_planes2(x, ops.NORM_RMS, torch.zeros(k, device=dev))
 

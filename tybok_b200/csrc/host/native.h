@@ -25,7 +25,8 @@ constexpr int SHIFT_NORMED = 4;  // normalised activations, O(1)
 constexpr int SHIFT_ATTN = 6;    // attention outputs: convex combinations of value rows
 constexpr int SHIFT_FFN = 4;     // FFN intermediates
 constexpr int SHIFT_FOLD = 0;    // residual stream times (1 + scale), not normalised
-// From this many token rows a GEMM fed by a norm takes two e4m3 planes with a per-row scale.
+// From this many token rows a GEMM fed by a norm takes two e4m3 planes with a per-row scale (a third less tensor work, token
+// tiles to 128); below it the GEMMs are bound by launch latency and keep the three-plane form.
 constexpr int TWO_PLANE_MIN_TOKENS = 128;
 
 // Every call that launches runs without the interpreter lock: a launch waits while the device's queue is full, and other

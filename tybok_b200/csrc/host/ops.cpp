@@ -262,6 +262,7 @@ class FfnTail {
 };
 
 void bind_ops(py::module_& m) {
+  m.attr("TWO_PLANE_MIN_TOKENS") = TWO_PLANE_MIN_TOKENS;
   m.def("status_word", [](int device) { return status_tensor(device); });
   m.def("w8a16_linear", &w8a16_linear, NoGil());
   m.def("attention", &attention, NoGil());

@@ -29,14 +29,12 @@ from .weights import quantize_w8
 SHIFT_IN = 4
 SHIFT_HIDDEN = 4
 SHIFT_ATTN = 6  # attention outputs are convex combinations of value rows
-#: From this many token rows the GEMMs fed by a norm take two e4m3 planes with a per-row scale.
-TWO_PLANE_MIN_TOKENS = 128
 
 
 def _ln_planes(x, shift, scale, eps):
     """modulate(LayerNorm(x)) as GEMM input: ``(planes, row_scale)`` (two-plane form) or
     ``(planes, None)`` (three planes at SHIFT_IN)."""
-    if x.shape[0] >= TWO_PLANE_MIN_TOKENS:
+    if x.shape[0] >= _lib.native().TWO_PLANE_MIN_TOKENS:
         return ops.norm_planes2(x, ops.NORM_LN_MODULATE, shift, scale, eps=eps)
     return ops.layernorm_modulate(x, shift, scale, eps=eps, out_shift=SHIFT_IN)[1], None
 
@@ -93,22 +91,21 @@ class DiTFFN:
         self.up, self.down = up, down
         self.world, self.group, self.eps = world, group, eps
 
-    def partial(self, x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
-        """This rank's un-biased contribution ``[M, H]`` bf16 to ``down(gelu(up(...)))``."""
+    def _down(self, x, shift, scale, *bias, **epilogue):
+        """The down projection of ``gelu(up(modulate(LayerNorm(x))))`` on this rank's shard."""
         xp, rs = _ln_planes(x, shift, scale, self.eps)
         _, hp = _gemm(xp, rs, *self.up, epilogue=ops.EPI_GELU, out_bf16=False, out_planes=True, out_shift=SHIFT_HIDDEN)
-        y, _ = ops.w8x3_linear(hp, SHIFT_HIDDEN, self.down[0], self.down[1])
-        return y
+        return ops.w8x3_linear(hp, SHIFT_HIDDEN, *self.down[:2], *bias, **epilogue)[0]
+
+    def partial(self, x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor) -> torch.Tensor:
+        """This rank's un-biased contribution ``[M, H]`` bf16 to ``down(gelu(up(...)))``."""
+        return self._down(x, shift, scale)
 
     def __call__(self, x: torch.Tensor, shift: torch.Tensor, scale: torch.Tensor, gate: torch.Tensor) -> torch.Tensor:
         """``x [M, H]`` bf16; ``shift``/``scale``/``gate`` bf16 ``[H]``."""
-        m = x.shape[0]
         if self.world == 1:
-            xp, rs = _ln_planes(x, shift, scale, self.eps)
-            _, hp = _gemm(xp, rs, *self.up, epilogue=ops.EPI_GELU, out_bf16=False, out_planes=True, out_shift=SHIFT_HIDDEN)
-            y, _ = ops.w8x3_linear(hp, SHIFT_HIDDEN, *self.down, epilogue=ops.EPI_RESIDUAL, residual=x,
-                                   gate=gate.reshape(1, -1), rows_per_gate=m)
-            return y
+            return self._down(x, shift, scale, self.down[2], epilogue=ops.EPI_RESIDUAL, residual=x, gate=gate.reshape(1, -1),
+                              rows_per_gate=x.shape[0])
         import torch.distributed as dist
 
         part = self.partial(x, shift, scale)

@@ -27,11 +27,6 @@ from . import _lib, ops
 from .shapes import GemmaSpec, PI05Shape
 from .weights import EXPERT, PROJECTOR, VISION, VLM, quantize_w8
 
-#: From this many token rows a GEMM fed by a norm takes its activations as two e4m3 planes with a
-#: per-row power-of-two scale (a third less tensor work, token tiles to 128); below it the GEMMs are
-#: bound by launch latency and keep the three-plane form.  (The rule itself is in csrc/host/native.h.)
-TWO_PLANE_MIN_TOKENS = 128
-
 
 class _Layer:
     """Packed weights of one Gemma decoder layer."""
