@@ -84,12 +84,21 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
-// Bounded wait that also ends once the CTA has given up.  A limit below the production one (a test's) is kept to the
-// clock: such a wait never suspends in hardware, where a short chain would complete before the limit is looked at.
-__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                              long long limit = kWaitLimitCycles) {
+// Bounded wait that also ends once the CTA has given up.
+__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (!mbar_try_wait(bar, parity)) {
+    if (*abort_flag) return false;
+    if (clock64() - t0 > kWaitLimitCycles) return false;
+  }
+  return true;
+}
+// The same with a limit of the launch's own.  One below the production limit (a test's) is kept to the clock: such a wait
+// never suspends in hardware, where a short chain would complete before the limit is looked at.
+__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag, long long limit) {
+  if (mbar_test_wait(bar, parity)) return true;
   const bool test = limit < kWaitLimitCycles;
-  if (!test && mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   while (!(test ? mbar_test_wait(bar, parity) : mbar_try_wait(bar, parity))) {
     if (*abort_flag) return false;

@@ -129,10 +129,13 @@ __device__ __noinline__ int stages_issued(const Barriers* b) {
   return b->issued;
 }
 
-// Bounded for two CTAs per SM: multi-wave full-K launches run with a shallow ring so that one
-// tile's epilogue overlaps the other's main loop (register budget 64K / 640 threads).
-// EW: epilogue warps.  A split-K CTA has the SM to itself and a long serial epilogue per thread
-// (accumulator groups to push, rows to finish): sixteen warps halve both.
+// Every copy from stage `from` on that the producer has requested lands (each wait is bounded).  Out of line, like the count
+// above: in the kernel's own code it cost a launch 0.5-1 % by the layout of what surrounds it.
+__device__ __noinline__ void see_copies_land(Barriers* b, int from, int ns) {
+#pragma unroll 1
+  for (int j = from, n = stages_issued(b); j < n; ++j) mbar_wait(&b->full[j % ns], (j / ns) & 1);
+}
+
 // rsqrt(mean(x^2) + eps) of token row m from the producer's per-channel-tile partial sums (fixed order).
 // The partial sums were written by other SMs a moment ago (an L2 round trip each), so eight loads are
 // in flight at a time.
@@ -149,6 +152,10 @@ __device__ __forceinline__ float deferred_rstd(const GemmParams& p, int m) {
   return rsqrtf(t * p.dn_inv_w + p.dn_eps);
 }
 
+// Bounded for two CTAs per SM: multi-wave full-K launches run with a shallow ring so that one
+// tile's epilogue overlaps the other's main loop (register budget 64K / 640 threads).
+// EW: epilogue warps.  A split-K CTA has the SM to itself and a long serial epilogue per thread
+// (accumulator groups to push, rows to finish): sixteen warps halve both.
 template <int EW>
 __global__ void __launch_bounds__(32 * (2 + EW), EW == EPI_WARPS ? 2 : 1)
 w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
@@ -318,8 +325,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
       // The CTA must not leave while its own copies may still land in its shared memory, whoever gave up first.  The stages
       // before this one have been waited for, the others are (each wait is bounded) now.
-#pragma unroll 1
-      for (int j = stop, n = stages_issued(&bars); j < n; ++j) mbar_wait(&bars.full[j % ns], (j / ns) & 1);
+      see_copies_land(&bars, stop, ns);
     }
     if (!mbar_wait(&bars.mma_done, 0) && lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
   } else {
