@@ -931,7 +931,7 @@ def run_dit(args, rank: int, world: int) -> None:
             "e2e": {"value": round(e2e_ms, 3), "unit": "ms", "h2d_bytes_per_step": sum(v.numel() * 2 for v in pinned.values()),
                     "d2h_bytes_per_step": host_out.numel() * 2},
             "parity": parity,
-            "roofline": {"bound": "tensor", "kernel": "whole pass (w8_gemm_kernel pairs + attention_prefill_kernel<128>)",
+            "roofline": {"bound": "tensor", "kernel": "whole pass (w8_gemm_pair_kernel + attention_two_tile_kernel)",
                          "achieved": round(tf, 1), "peak": peak, "unit": "TFLOP/s", "frac": round(tf / peak, 4),
                          "traffic": None, "peak_source": peaks_kind + " (sustained bf16 x ranks; only the FFN is sharded)",
                          "flops_per_pass": flops},
