@@ -3,6 +3,8 @@
 #pragma once
 
 #include <ATen/ATen.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -32,6 +34,18 @@ constexpr int TWO_PLANE_MIN_TOKENS = 128;
 // Every call that launches runs without the interpreter lock: a launch waits while the device's queue is full, and other
 // threads' Python must go on meanwhile.  What touches Python objects in such a call takes the lock for itself.
 using NoGil = py::call_guard<py::gil_scoped_release>;
+
+// Whether a call on these may run as it stands.  Inside a function transform or a dispatch mode, and for tensors that intercept
+// torch ops, it has to go through the dispatcher: the Python side then calls the registered op, which ends in the
+// unchecked form of the same call.  (Asked here: in Python the question cost a call 1 us.)
+inline bool plain(std::initializer_list<const Tensor*> tensors) {
+  using K = c10::DispatchKey;
+  if (c10::impl::dispatch_mode_enabled() || c10::impl::tls_is_dispatch_key_included(K::FuncTorchDynamicLayerFrontMode)) return false;
+  constexpr c10::DispatchKeySet intercepts{K::Python, K::FuncTorchBatched, K::FuncTorchGradWrapper, K::Functionalize};
+  for (const Tensor* t : tensors)
+    if (t && t->key_set().has_any(intercepts)) return false;
+  return true;
+}
 
 [[noreturn]] void raise_status(int rc, const char* what);
 inline void check(int rc, const char* what) {

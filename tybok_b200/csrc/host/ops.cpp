@@ -264,12 +264,39 @@ class FfnTail {
 void bind_ops(py::module_& m) {
   m.attr("TWO_PLANE_MIN_TOKENS") = TWO_PLANE_MIN_TOKENS;
   m.def("status_word", [](int device) { return status_tensor(device); });
-  m.def("w8a16_linear", &w8a16_linear, NoGil());
-  m.def("attention", &attention, NoGil());
-  py::class_<Mlp>(m, "Mlp").def(py::init<const py::tuple&, const py::object&, const py::tuple&>()).def("forward", &Mlp::forward, NoGil());
+  // `…_op` / `run`: what the registered ops end in.  The others return None where the call is the dispatcher's.
+  m.def("w8a16_linear_op", &w8a16_linear, NoGil());
+  m.def("attention_op", &attention, NoGil());
+  m.def(
+      "w8a16_linear",
+      [](const Tensor& x, const Tensor& w8, const Tensor& scale, const OptTensor& bias, int epilogue, const OptTensor& residual,
+         const OptTensor& gate, int rows_per_gate, int token_tile, int splits, int shift) -> OptTensor {
+        if (!plain({&x, &w8, &scale, opt(bias), opt(residual), opt(gate)})) return std::nullopt;
+        return w8a16_linear(x, w8, scale, bias, epilogue, residual, gate, rows_per_gate, token_tile, splits, shift);
+      },
+      NoGil());
+  m.def(
+      "attention",
+      [](const Tensor& q, const Tensor& kc, const Tensor& vc, const OptTensor& valid, int tokens, int keys, double scale, bool out_bf16,
+         bool out_planes, int out_shift) -> std::optional<std::tuple<Tensor, Tensor>> {
+        if (!plain({&q, &kc, &vc, opt(valid)})) return std::nullopt;
+        return attention(q, kc, vc, valid, tokens, keys, scale, out_bf16, out_planes, out_shift);
+      },
+      NoGil());
+  py::class_<Mlp>(m, "Mlp")
+      .def(py::init<const py::tuple&, const py::object&, const py::tuple&>())
+      .def("run", &Mlp::forward, NoGil())
+      .def(
+          "forward", [](const Mlp& c, const Tensor& x) -> OptTensor { return plain({&x}) ? OptTensor(c.forward(x)) : std::nullopt; }, NoGil());
   py::class_<FfnTail>(m, "FfnTail")
       .def(py::init<const py::tuple&, const py::tuple&, double>())
-      .def("forward", &FfnTail::forward, NoGil());
+      .def("run", &FfnTail::forward, NoGil())
+      .def(
+          "forward",
+          [](const FfnTail& c, const Tensor& x, const Tensor& shift, const Tensor& scale, const Tensor& gate) -> OptTensor {
+            return plain({&x, &shift, &scale, &gate}) ? OptTensor(c.forward(x, shift, scale, gate)) : std::nullopt;
+          },
+          NoGil());
 }
 
 }  // namespace tbn

@@ -56,7 +56,8 @@ def make_mlp_forward(mlp, device: str | torch.device = "cuda"):
 
     def forward(x: torch.Tensor) -> torch.Tensor:
         _need_cuda(x)
-        return chain.forward(x) if ops.native_takes(x) else torch.ops.tybok_b200.mlp(x, *tensors)
+        y = chain.forward(x) if type(x) is torch.Tensor else None  # None: the dispatcher's call
+        return torch.ops.tybok_b200.mlp(x, *tensors) if y is None else y
 
     return forward
 
@@ -74,8 +75,7 @@ def make_fused_ffn_tail(blk, device: str | torch.device = "cuda"):
 
     def tail(x: torch.Tensor, shift_mlp: torch.Tensor, scale_mlp: torch.Tensor, gate_mlp: torch.Tensor) -> torch.Tensor:
         _need_cuda(x)
-        if not ops.native_takes(x, shift_mlp, scale_mlp, gate_mlp):
-            return torch.ops.tybok_b200.ffn_tail(x, shift_mlp, scale_mlp, gate_mlp, *up, *down, eps)
-        return chain.forward(x, shift_mlp, scale_mlp, gate_mlp)
+        y = chain.forward(x, shift_mlp, scale_mlp, gate_mlp) if type(x) is torch.Tensor else None
+        return torch.ops.tybok_b200.ffn_tail(x, shift_mlp, scale_mlp, gate_mlp, *up, *down, eps) if y is None else y
 
     return tail

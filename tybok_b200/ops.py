@@ -247,29 +247,20 @@ def _rope_store_cuda(qkv, pos, cos, sin, k_cache, v_cache, heads, key_off):
     return q
 
 
-def native_takes(*tensors: torch.Tensor | None) -> bool:
-    """Whether a call on these may go to the native extension as it stands.  Inside a function transform (``vmap``, ``jvp``) or a
-    dispatch mode, and for tensor subclasses, it goes through the registered op of the same name, so that whoever
-    intercepts torch ops still sees one; that op ends in the same native call."""
-    if torch._C._functorch.peek_interpreter_stack() is not None or torch._C._len_torch_dispatch_stack():
-        return False
-    return all(t is None or type(t) is torch.Tensor or type(t) is torch.nn.Parameter for t in tensors)
-
-
 def _w8a16_linear_cuda(*args):
-    return _lib.native().w8a16_linear(*args)
+    return _lib.native().w8a16_linear_op(*args)
 
 
 def _mlp_cuda(x, gate_up, gate_up_scale, up, up_scale, down, down_scale):
-    return _lib.native().Mlp((gate_up, gate_up_scale), None if up is None else (up, up_scale), (down, down_scale)).forward(x)
+    return _lib.native().Mlp((gate_up, gate_up_scale), None if up is None else (up, up_scale), (down, down_scale)).run(x)
 
 
 def _ffn_tail_cuda(x, shift, scale, gate, up, up_scale, up_bias, down, down_scale, down_bias, eps):
-    return _lib.native().FfnTail((up, up_scale, up_bias), (down, down_scale, down_bias), eps).forward(x, shift, scale, gate)
+    return _lib.native().FfnTail((up, up_scale, up_bias), (down, down_scale, down_bias), eps).run(x, shift, scale, gate)
 
 
 def _attention_cuda(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift):
-    return _lib.native().attention(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
+    return _lib.native().attention_op(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
 
 
 def _layernorm_modulate_cuda(x, shift, scale, eps, out_bf16, out_planes, out_shift):
@@ -542,8 +533,10 @@ def w8x3_geglu_packed(planes, shift, w8_packed, scale_packed, *, out_bf16=True, 
 def w8a16_linear(x, w8, scale, bias=None, *, epilogue=EPI_NONE, residual=None, gate=None, rows_per_gate=1,
                  token_tile=0, splits=0, shift=DEFAULT_SHIFT) -> torch.Tensor:
     """``epilogue(x @ (w8*scale).T + bias)`` for bf16 ``x``: ``split3`` then ``w8x3_linear``, as one native call."""
-    call = _lib.native().w8a16_linear if native_takes(x, w8, scale, bias, residual, gate) else torch.ops.tybok_b200.w8a16_linear
-    return call(x, w8, scale, bias, epilogue, residual, gate, rows_per_gate, token_tile, splits, shift)
+    args = (x, w8, scale, bias, epilogue, residual, gate, rows_per_gate, token_tile, splits, shift)
+    # None: inside a transform or a dispatch mode the call is the dispatcher's, as it is for tensor subclasses
+    y = _lib.native().w8a16_linear(*args) if type(x) is torch.Tensor else None
+    return torch.ops.tybok_b200.w8a16_linear(*args) if y is None else y
 
 
 def w8a16_geglu(x, w8_gate, scale_gate, w8_up, scale_up, *, token_tile=0, splits=0, shift=DEFAULT_SHIFT):
@@ -570,8 +563,9 @@ def attention(q, k_cache, v_cache, key_valid=None, *, tokens, keys, scale, out_b
               out_shift=DEFAULT_SHIFT):
     """GQA attention over the first ``keys`` cache rows; returns ``(out_bf16, out_planes)``; see
     ``tybok_attention``."""
-    call = _lib.native().attention if native_takes(q, k_cache, v_cache, key_valid) else torch.ops.tybok_b200.attention
-    return call(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
+    args = (q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
+    y = _lib.native().attention(*args) if type(q) is torch.Tensor else None  # as w8a16_linear
+    return torch.ops.tybok_b200.attention(*args) if y is None else y
 
 
 def layernorm_modulate(x, shift, scale, *, eps=1e-6, out_bf16=False, out_planes=True, out_shift=DEFAULT_SHIFT):
