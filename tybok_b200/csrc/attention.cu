@@ -1655,7 +1655,6 @@ namespace tb {
 // Clusters of `nsplit` attention CTAs (one CTA per SM) that the device holds at once.
 static int at_resident_clusters(int nsplit) {
   static host::DeviceCache cache[AT_MAX_SPLITS + 1];
-  if (nsplit > AT_MAX_SPLITS) return 1;
   return host::per_device(cache[nsplit], [nsplit] {
     cudaFuncSetAttribute(attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM);
     cudaLaunchConfig_t cfg{};
@@ -1685,12 +1684,16 @@ static int at_resident_clusters(int nsplit) {
 // batch 8: 48 -> 34 us).  The cluster form of short suffixes stays ahead while its clusters run in few enough waves:
 // a wave takes about 9 us, the key loop 7.5 us and 2 us per 128 keys (594 keys: batch 3 is 9.5 against 17.6 us,
 // batch 4 18.1 against 17.8; 994 keys: batch 3 17.9 against 23.5, batch 4 26.4 against 23.7).
-static bool at_key_loop(int B, int L, int H, int G, int D, int Lk) {
-  if ((L > AT_BQ || D == 128) && Lk <= PF_MAX_KEYS) return true;
+struct AtForm {
+  bool key_loop;
+  int resident;  // cluster form: clusters that the device holds at once (0: not asked)
+};
+static AtForm at_form(int B, int L, int H, int G, int D, int Lk) {
   const int nsplit = (Lk + AT_BK - 1) / AT_BK;
-  if (G != 1 || H <= 1 || nsplit <= 1 || nsplit > AT_MAX_SPLITS) return false;
+  if ((L > AT_BQ || D == 128) && Lk <= PF_MAX_KEYS) return {true, 0};
+  if (nsplit <= 1 || nsplit > AT_MAX_SPLITS) return {false, 0};
   const int clusters = H * B, resident = at_resident_clusters(nsplit);
-  return 9.0 * ((clusters + resident - 1) / resident) >= 7.5 + 2.0 * nsplit;
+  return {G == 1 && H > 1 && 9.0 * ((clusters + resident - 1) / resident) >= 7.5 + 2.0 * nsplit, resident};
 }
 
 static size_t at_workspace(bool key_loop, int B, int L, int H, int Lk) {
@@ -1790,7 +1793,7 @@ int tybok_qknorm_rope_store(const void* src, int64_t ld, int q_off, int k_off, i
 size_t tybok_attention_workspace_needed(int B, int L, int H, int G, int D, int Lk) {
   using namespace tb;
   if (B <= 0 || L <= 0 || H <= 0 || G <= 0 || Lk <= 0) return 0;
-  return at_workspace(at_key_loop(B, L, H, G, D, Lk), B, L, H, Lk);
+  return at_workspace(at_form(B, L, H, G, D, Lk).key_loop, B, L, H, Lk);
 }
 
 size_t tybok_attention_workspace_bytes(int B, int L, int H, int Lk) {
@@ -1808,7 +1811,8 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   if (B <= 0 || L <= 0 || H <= 0 || G <= 0 || H % G != 0 || Lk <= 0 || Lk > Lcap)
     return host::fail(TYBOK_ERR_ARG, "attention: bad shape (H % G == 0, 0 < Lk <= Lcap)");
   const int nsplit = (Lk + AT_BK - 1) / AT_BK;
-  const bool prefill = at_key_loop(B, L, H, G, D, Lk);
+  const AtForm form = at_form(B, L, H, G, D, Lk);
+  const bool prefill = form.key_loop;
   if (D == 128 && !prefill) return host::fail(TYBOK_ERR_ARG, "attention: at most 8192 keys at head_dim 128");
   if (!prefill && nsplit > AT_MAX_SPLITS)
     return host::fail(TYBOK_ERR_ARG, "attention: at most 1024 keys (8 blocks of 128 per cluster) for up to 128 queries, "
@@ -1854,7 +1858,7 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   // Small grids split the output columns over two clusters, but only while all of them run at once: a cluster lives inside
   // one GPC, so 16 of eight CTAs are two waves on a B200 (50 queries, 1018 keys, 8 heads: 13.1 us with the columns split,
   // 8.9 us without).
-  p.dsplit = (!prefill && nsplit > 1 && 2 * nsplit * H * n_qt * B <= host::sm_count() && 2 * H * n_qt * B <= at_resident_clusters(nsplit)) ? 2 : 1;
+  p.dsplit = (!prefill && nsplit > 1 && 2 * nsplit * H * n_qt * B <= host::sm_count() && 2 * H * n_qt * B <= form.resident) ? 2 : 1;
   p.trace = host::trace_buffer();
   p.dbg = host::counter_buffer();
   p.wait_limit = host::epilogue_wait_limit() > 0 ? host::epilogue_wait_limit() : kWaitLimitCycles;

@@ -86,6 +86,8 @@ _L.define("ffn_tail(Tensor x, Tensor shift, Tensor scale, Tensor gate, Tensor up
 NORM_RMS, NORM_ADARMS, NORM_LN_MODULATE, NORM_LN_AFFINE = 0, 1, 2, 3
 EPI_GEGLU_PACKED = 4
 
+_Tensor = torch.Tensor
+
 def _dev_index(device: torch.device) -> int:
     return device.index if device.index is not None else torch.cuda.current_device()
 
@@ -533,10 +535,11 @@ def w8x3_geglu_packed(planes, shift, w8_packed, scale_packed, *, out_bf16=True, 
 def w8a16_linear(x, w8, scale, bias=None, *, epilogue=EPI_NONE, residual=None, gate=None, rows_per_gate=1,
                  token_tile=0, splits=0, shift=DEFAULT_SHIFT) -> torch.Tensor:
     """``epilogue(x @ (w8*scale).T + bias)`` for bf16 ``x``: ``split3`` then ``w8x3_linear``, as one native call."""
-    args = (x, w8, scale, bias, epilogue, residual, gate, rows_per_gate, token_tile, splits, shift)
-    # None: inside a transform or a dispatch mode the call is the dispatcher's, as it is for tensor subclasses
-    y = _lib.native().w8a16_linear(*args) if type(x) is torch.Tensor else None
-    return torch.ops.tybok_b200.w8a16_linear(*args) if y is None else y
+    if type(x) is _Tensor:  # a subclass is the dispatcher's; so, inside a transform or a dispatch mode, is what comes back None
+        y = _lib.native().w8a16_linear(x, w8, scale, bias, epilogue, residual, gate, rows_per_gate, token_tile, splits, shift)
+        if y is not None:
+            return y
+    return torch.ops.tybok_b200.w8a16_linear(x, w8, scale, bias, epilogue, residual, gate, rows_per_gate, token_tile, splits, shift)
 
 
 def w8a16_geglu(x, w8_gate, scale_gate, w8_up, scale_up, *, token_tile=0, splits=0, shift=DEFAULT_SHIFT):
@@ -563,9 +566,11 @@ def attention(q, k_cache, v_cache, key_valid=None, *, tokens, keys, scale, out_b
               out_shift=DEFAULT_SHIFT):
     """GQA attention over the first ``keys`` cache rows; returns ``(out_bf16, out_planes)``; see
     ``tybok_attention``."""
-    args = (q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
-    y = _lib.native().attention(*args) if type(q) is torch.Tensor else None  # as w8a16_linear
-    return torch.ops.tybok_b200.attention(*args) if y is None else y
+    if type(q) is _Tensor:  # as w8a16_linear
+        y = _lib.native().attention(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
+        if y is not None:
+            return y
+    return torch.ops.tybok_b200.attention(q, k_cache, v_cache, key_valid, tokens, keys, scale, out_bf16, out_planes, out_shift)
 
 
 def layernorm_modulate(x, shift, scale, *, eps=1e-6, out_bf16=False, out_planes=True, out_shift=DEFAULT_SHIFT):
