@@ -245,6 +245,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       if (!p.xb)
         for (int i = 0; i < pre; ++i)
           tma_load_3d(smem + i * stage_bytes + x_off, &tm_x, &bars.full[i], (kb0 + i) * BK, t_tile * p.bt, 0);
+      if (EW == EPI_WARPS_WIDE && p.splits > 1) cluster_arrive_relaxed();
       int issued = pre;
       for (int i = pre; i < nkb; ++i) {
         const int s = i % ns;
@@ -261,6 +262,8 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         issued = i + 1;
       }
       bars.issued = issued;
+    } else if (EW == EPI_WARPS_WIDE && p.splits > 1) {
+      cluster_arrive_relaxed();
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
@@ -275,6 +278,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     const uint64_t desc_const = smem_desc_sw128(0);
     const uint32_t plane16 = static_cast<uint32_t>(p.bt * 128) >> 4;  // plane pitch in 16-byte units
     const int acc_cols = p.merge ? p.np * p.bt : p.bt;
+    if (EW == EPI_WARPS_WIDE && p.splits > 1) cluster_arrive_relaxed();
     bool ok = true;
     int stop = 0;
     for (int i = 0; i < nkb; ++i) {
@@ -387,6 +391,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           }
         }
       }
+      if (EW == EPI_WARPS_WIDE && p.splits > 1) cluster_arrive_relaxed();
       // These warps are idle until the accumulator is complete, so they wait for the previous
       // kernel now, under the main loop, not between the accumulator and the stores.
       if (p.pdl) pdl_wait();
@@ -452,6 +457,11 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         for (int j = made, n = stages_issued(&bars); j < n; ++j) mbar_arrive(&bars.full[j % ns]);
       }
     }
+    // Split-K writes into the peers' shared memory, so they must have started.  They have, thousands of clocks ago, but only
+    // this phase of the cluster barrier says so.  Each warp arrives where it waits for something else anyway, and the
+    // accumulator is not complete yet here.  (50-token MLP 14.59 -> 14.64 us; 1 x 2560 x 2048, whose epilogue warps are
+    // busy until here, 6.39 -> 6.52 us; arrivals at the kernel's start cost twice that.)
+    if (EW == EPI_WARPS_WIDE && p.splits > 1) cluster_wait_acquire();
     bool ok = __all_sync(0xffffffffu, wait_or_abort(&bars.tmem_full, 0, &bars.abort, p.epi_wait_limit));
     if (!ok && lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_EPILOGUE);
     if (tr && ew == 0 && lane == 0) tr[4] = clock64();
@@ -519,6 +529,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   if (tr && tid == 64) tr[5] = clock64();
   tc_fence_before();
   if (p.splits > 1) {
+    if (warp < 2) cluster_wait_acquire();  // the phase that says every peer runs
     __syncwarp();
     cluster_sync_all();
   } else {
