@@ -51,12 +51,8 @@ def _calls():
     }
 
 
-@pytest.mark.parametrize("name", ["linear", "attention", "mlp", "ffn_tail", "dit_block", "gemma_stack"])
-def test_other_threads_run_while_a_call_waits_for_the_launch_queue(name):
-    call = _calls()[name]
-    for _ in range(3):
-        call()
-    torch.cuda.synchronize()
+def _longest_stall(call):
+    """Seconds that a ticking thread stood still while ``call`` ran into a launch queue filled behind a sleeping device."""
     stop, longest = threading.Event(), [0.0]
 
     def ticker():
@@ -78,7 +74,17 @@ def test_other_threads_run_while_a_call_waits_for_the_launch_queue(name):
         stop.set()
         thread.join()
     torch.cuda.synchronize()
-    assert longest[0] < 0.1
+    return longest[0]
+
+
+@pytest.mark.parametrize("name", ["linear", "attention", "mlp", "ffn_tail", "dit_block", "gemma_stack"])
+def test_other_threads_run_while_a_call_waits_for_the_launch_queue(name):
+    call = _calls()[name]
+    for _ in range(3):
+        call()
+    torch.cuda.synchronize()
+    # a call that holds the lock stalls the others every time; a busy host may do so once
+    assert min(_longest_stall(call) for _ in range(3)) < 0.1
 
 
 def test_errors_of_calls_without_the_lock():
