@@ -8,10 +8,12 @@
 //     plane count.  Operand fill per CTA and 128-wide K block: 16 KB of weights + np x 16 KB of planes for
 //     np x 512 clocks of tensor work = 48 (np = 2) or 43 (np = 3) bytes per clock, under the ~50-60 that
 //     an SM draws from L2; the 128 x 80-token tiles used before needed 70 and were bound by it.
-//   * two accumulators of 256 columns take turns: eight epilogue warps empty one while the next tile's
-//     products fill the other.  Before, each tile's epilogue ran on a second resident CTA, which halved the
+//   * two accumulators of 256 columns take turns: sixteen epilogue warps, 16 tokens at a time, empty one while the next
+//     tile's products fill the other.  (Eight warps with 32 tokens each did not keep up where a tile's K is short and its epilogue
+//     long: four warps per scheduler instead of two hide the latencies of its chains, results are rounded to bf16 in
+//     pairs, and half the registers do.  DiT denoiser at 106 tokens 16.48 -> 16.15 ms, same bits.)  Before, each tile's epilogue ran on a second resident CTA, which halved the
 //     ring (two 46 KB stages in flight per CTA).  Now the ring has 4 (np = 2) or 3 stages of 48 / 64 KB.
-//   * an epilogue thread holds one channel (its tensor-memory lane) of 32 tokens, so scale, bias and gate
+//   * an epilogue thread holds one channel (its tensor-memory lane) of 16 tokens, so scale, bias and gate
 //     are per-thread scalars; results turn into four channels per thread by a 4 x 4 transpose across
 //     four lanes (two shuffles per 16 values), without a trip through shared memory.
 //   * one CTA per SM that takes all 512 tensor-memory columns: nothing else that allocates tensor memory
@@ -37,7 +39,8 @@ namespace {
 constexpr int P_BK = 128;             // K per stage
 constexpr int P_WTILE = 128 * P_BK;   // weight bytes of one 128-row tile and stage
 constexpr int P_MAX_STAGES = 8;
-constexpr int P_EPI_WARPS = 8;
+constexpr int P_EPI_WARPS = 16;
+constexpr int P_CHUNK = 16;           // tokens that an epilogue warp finishes at a time
 constexpr int P_THREADS = 32 * (2 + P_EPI_WARPS);
 constexpr int P_SMEM = 226 * 1024;
 constexpr int P_ACC_COLS = 256;       // tensor-memory columns of one accumulator (two per CTA)
@@ -75,7 +78,7 @@ struct __align__(8) PairBars {
   uint64_t full[P_MAX_STAGES];   // even CTA: both CTAs' operand bytes of a stage have landed
   uint64_t empty[P_MAX_STAGES];  // each CTA: the pair's products have read the stage
   uint64_t acc_full[2];          // each CTA: accumulator complete
-  uint64_t acc_empty[2];         // even CTA: the sixteen epilogue warps of the pair have read the accumulator
+  uint64_t acc_empty[2];         // even CTA: the epilogue warps of both CTAs have read the accumulator
   uint64_t mma_done;             // every product this pair issued has retired
   uint32_t tmem_base;
   volatile int issued;           // stages whose copies this CTA's producer has requested, once it is through; -1 before
@@ -335,7 +338,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     if (!done && lane == 0) pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
   } else {
     // ------------------------------------------------------------ epilogue
-    const int q = warp & 3, half = (warp - 2) >> 2;  // tensor-memory lane quadrant; which of its two warps
+    const int q = warp & 3, part = (warp - 2) >> 2;  // tensor-memory lane quadrant; which of its four warps
     const int row = q * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     const int g4 = (lane >> 2) * 4, j4 = lane & 3;   // after the transpose: first channel of four, token of four
@@ -390,27 +393,28 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
       }
       if (!ok && !SPLIT) break;
       tc_fence_after();
-      const int nchunk = tl.bt >> 5;
-      // Accumulator values of chunk c (32 tokens from mc on; v, and u of the second accumulator) -> outputs.  The
+      const int nchunk = (tl.bt + P_CHUNK - 1) / P_CHUNK, m_end = min(p.M, tl.m0 + tl.bt);
+      // Accumulator values of chunk c (16 tokens from mc on; v, and u of the second accumulator) -> outputs.  The
       // residual rows are requested first.
-      auto residual_rows = [&](int mc, uint2 (&rr)[EPI == EPI_RESIDUAL ? 8 : 1]) {
-        if (EPI == EPI_RESIDUAL) {  // 8 token rows per lane after the transpose: m = mc + 4 k + j4
+      auto residual_rows = [&](int mc, uint2 (&rr)[EPI == EPI_RESIDUAL ? 4 : 1]) {
+        if (EPI == EPI_RESIDUAL) {  // 4 token rows per lane after the transpose: m = mc + 4 k + j4
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
+          for (int k = 0; k < 4; ++k) {
             const int m = mc + 4 * k + j4;
-            if (m < p.M && quad_live) rr[EPI == EPI_RESIDUAL ? k : 0] = *reinterpret_cast<const uint2*>(p.res + m * p.ldres + n_first);
+            if (m < m_end && quad_live) rr[EPI == EPI_RESIDUAL ? k : 0] = *reinterpret_cast<const uint2*>(p.res + m * p.ldres + n_first);
           }
         }
       };
-      auto finish = [&](int mc, uint32_t (&v)[32], uint32_t (&u)[NA == 2 ? 32 : 1], uint2 (&rr)[EPI == EPI_RESIDUAL ? 8 : 1]) {
+      auto finish = [&](int mc, uint32_t (&v)[16], uint32_t (&u)[NA == 2 ? 16 : 1], uint2 (&rr)[EPI == EPI_RESIDUAL ? 4 : 1]) {
         float rs = 1.0f;
-        if (p.row_scale) rs = p.row_scale[min(mc + lane, p.M - 1)];
+        if (p.row_scale) rs = p.row_scale[min(mc + (lane & 15), p.M - 1)];
+        uint32_t pk[8], pw[EPI == EPI_QKV_ROPE ? 8 : 1];  // bf16 results of two tokens each (and of the rotary partners)
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          float o[4], w[4];
+          float o[2], w[2];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int i = 4 * k + e;
+          for (int e = 0; e < 2; ++e) {
+            const int i = 2 * k + e;
             float x = __uint_as_float(v[i]);
             float r = 1.0f;
             if (p.row_scale) {
@@ -419,30 +423,44 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
             }
             o[e] = x * sc0;
             if constexpr (NA == 2) w[e] = __uint_as_float(u[i]) * r * sc1;
-            // Rounding points of the reference's bf16 modules: linear output, GELU output, product, gated value, sum.
-            if (NA == 1) {
-              o[e] += bi;
-              if (EPI == EPI_GELU) {
-                o[e] = gelu_tanh_fast(bf16_round(o[e]));
-              } else if (EPI == EPI_RESIDUAL && p.gate) {
-                float gv = gt;
-                if (!one_group) {
-                  const int m = min(mc + i, p.M - 1);
-                  const long long gi = static_cast<long long>(m / p.rows_per_gate) * p.ldgate + rows[0];
-                  gv = !live ? 0.f : p.gate_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.gate)[gi])
-                                                 : bf16_round(static_cast<const float*>(p.gate)[gi]);
-                }
-                o[e] = bf16_round(o[e]) * gv;
-              }
-            } else if (EPI == EPI_GEGLU) {
-              o[e] = bf16_round(gelu_tanh_fast(bf16_round(o[e]))) * bf16_round(w[e]);
-            }
+            if (NA == 1) o[e] += bi;
           }
-          uint2 t0 = quad_transpose(pack_bf16(o[0], o[1]), pack_bf16(o[2], o[3]), lane);
+          // Rounding points of the reference's bf16 modules: linear output, GELU output, product, gated value, sum.
+          if (EPI == EPI_GELU || EPI == EPI_GEGLU || (EPI == EPI_RESIDUAL && p.gate)) {
+            const uint32_t lin = pack_bf16(o[0], o[1]);
+            o[0] = bf16_lo(lin);
+            o[1] = bf16_hi(lin);
+          }
+          if (EPI == EPI_GELU) {
+            o[0] = gelu_tanh_fast(o[0]);
+            o[1] = gelu_tanh_fast(o[1]);
+          } else if (EPI == EPI_RESIDUAL && p.gate) {
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              float gv = gt;
+              if (!one_group) {
+                const int m = min(mc + 2 * k + e, p.M - 1);
+                const long long gi = static_cast<long long>(m / p.rows_per_gate) * p.ldgate + rows[0];
+                gv = !live ? 0.f : p.gate_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(p.gate)[gi])
+                                               : bf16_round(static_cast<const float*>(p.gate)[gi]);
+              }
+              o[e] *= gv;
+            }
+          } else if (EPI == EPI_GEGLU) {
+            const uint32_t g = pack_bf16(gelu_tanh_fast(o[0]), gelu_tanh_fast(o[1])), uw = pack_bf16(w[0], w[1]);
+            o[0] = bf16_lo(g) * bf16_lo(uw);
+            o[1] = bf16_hi(g) * bf16_hi(uw);
+          }
+          pk[k] = pack_bf16(o[0], o[1]);
+          if constexpr (EPI == EPI_QKV_ROPE) pw[k] = pack_bf16(w[0], w[1]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          uint2 t0 = quad_transpose(pk[2 * k], pk[2 * k + 1], lane);
           const int m = mc + 4 * k + j4;
           if constexpr (EPI == EPI_QKV_ROPE) {
-            const uint2 t1 = quad_transpose(pack_bf16(w[0], w[1]), pack_bf16(w[2], w[3]), lane);
-            if (m < p.M && quad_live) {
+            const uint2 t1 = quad_transpose(pw[2 * k], pw[2 * k + 1], lane);
+            if (m < m_end && quad_live) {
               const RopeEpi& rp = p.rope;
               const int tps = rp.D >> 7, slot = blk / tps, hd2 = rp.D >> 1;
               const int d = (blk - slot * tps) * 64 + (q & 1) * 32 + g4;
@@ -479,7 +497,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
               *reinterpret_cast<uint2*>(dst + hd2 + d) = hi;
             }
           } else {
-            if (m < p.M && quad_live) {
+            if (m < m_end && quad_live) {
               if (EPI == EPI_RESIDUAL) {
                 const uint2 r2 = rr[EPI == EPI_RESIDUAL ? k : 0];
                 t0 = make_uint2(pack_bf16(bf16_lo(t0.x) + bf16_lo(r2.x), bf16_hi(t0.x) + bf16_hi(r2.x)),
@@ -505,56 +523,56 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         const bool whole = !bars.abort;  // the same in every CTA: nobody gives up after this point
         const int nown = (nchunk + p.splits - 1) / p.splits;
         const uint32_t buf = smem_u32(smem);
-        for (int c = half; c < nchunk && whole; c += 2) {
+        for (int c = part; c < nchunk && whole; c += 4) {
           const int owner = c % p.splits;
-          if (owner == split || tl.m0 + c * 32 >= p.M) continue;
-          uint32_t v[32];
-          tmem_ld32(tmem + lane_addr + c * 32, v);
-          const uint32_t dst = dsmem_addr(buf + (((split * nown + c / p.splits) * 32) * 128 + row) * 4, owner * 2 + rank);
+          if (owner == split || tl.m0 + c * P_CHUNK >= m_end) continue;
+          uint32_t v[16];
+          tmem_ld16(tmem + lane_addr + c * P_CHUNK, v);
+          const uint32_t dst = dsmem_addr(buf + (((split * nown + c / p.splits) * P_CHUNK) * 128 + row) * 4, owner * 2 + rank);
           tc_wait_ld();
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
+          for (int e = 0; e < 16; ++e)
             asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + e * 512), "f"(__uint_as_float(v[e])));
         }
         __syncwarp();
         cluster_sync_all();  // every part has arrived
-        const float* part = reinterpret_cast<const float*>(smem);
-        for (int i = half; i < nown && whole; i += 2) {
-          const int c = i * p.splits + split, mc = tl.m0 + c * 32;
-          if (c >= nchunk || mc >= p.M) break;
-          uint32_t v[32], t[32], u[NA == 2 ? 32 : 1];
-          uint2 rr[EPI == EPI_RESIDUAL ? 8 : 1];
+        const float* parts = reinterpret_cast<const float*>(smem);
+        for (int i = part; i < nown && whole; i += 4) {
+          const int c = i * p.splits + split, mc = tl.m0 + c * P_CHUNK;
+          if (c >= nchunk || mc >= m_end) break;
+          uint32_t v[16], t[16], u[NA == 2 ? 16 : 1];
+          uint2 rr[EPI == EPI_RESIDUAL ? 4 : 1];
           residual_rows(mc, rr);
-          tmem_ld32(tmem + lane_addr + c * 32, t);
+          tmem_ld16(tmem + lane_addr + c * P_CHUNK, t);
           tc_wait_ld();
 #pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] = 0u;
+          for (int e = 0; e < 16; ++e) v[e] = 0u;
           for (int sp = 0; sp < p.splits; ++sp) {  // split order: bit-reproducible
-            const float* src = part + ((sp * nown + i) * 32) * 128 + row;
+            const float* src = parts + ((sp * nown + i) * P_CHUNK) * 128 + row;
 #pragma unroll
-            for (int e = 0; e < 32; ++e)
+            for (int e = 0; e < 16; ++e)
               v[e] = __float_as_uint(__uint_as_float(v[e]) + (sp == split ? __uint_as_float(t[e]) : src[e * 128]));
           }
           finish(mc, v, u, rr);
         }
       } else {
-        for (int c = half; c < nchunk; c += 2) {
-          const int mc = tl.m0 + c * 32;  // first token of this chunk
-          if (mc >= p.M) break;
-          uint32_t v[32];
-          uint32_t u[NA == 2 ? 32 : 1];
-          tmem_ld32(tmem + a * P_ACC_COLS + lane_addr + c * 32, v);
-          if constexpr (NA == 2) tmem_ld32(tmem + a * P_ACC_COLS + lane_addr + tl.bt + c * 32, u);
-          uint2 rr[EPI == EPI_RESIDUAL ? 8 : 1];
+        for (int c = part; c < nchunk; c += 4) {
+          const int mc = tl.m0 + c * P_CHUNK;  // first token of this chunk
+          if (mc >= m_end) break;
+          uint32_t v[16];
+          uint32_t u[NA == 2 ? 16 : 1];
+          tmem_ld16(tmem + a * P_ACC_COLS + lane_addr + c * P_CHUNK, v);
+          if constexpr (NA == 2) tmem_ld16(tmem + a * P_ACC_COLS + lane_addr + tl.bt + c * P_CHUNK, u);
+          uint2 rr[EPI == EPI_RESIDUAL ? 4 : 1];
           residual_rows(mc, rr);
           tc_wait_ld();
           if (NA == 1 && p.merge) {
             for (int pl = 1; pl < p.np; ++pl) {
-              uint32_t v2[32];
-              tmem_ld32(tmem + a * P_ACC_COLS + lane_addr + pl * tl.bt + c * 32, v2);
+              uint32_t v2[16];
+              tmem_ld16(tmem + a * P_ACC_COLS + lane_addr + pl * tl.bt + c * P_CHUNK, v2);
               tc_wait_ld();
-  #pragma unroll
-              for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(v2[e]));
+#pragma unroll
+              for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(v2[e]));
             }
           }
           finish(mc, v, u, rr);
@@ -665,7 +683,7 @@ PairPlan plan_split(int M, int rows, int K, int np) {
     for (int tt = (units + 7) / 8; tt <= units && static_cast<long long>(ch) * tt <= cap; ++tt) {
       const int ub = (units + tt - 1) / tt;
       const int stage = P_WTILE + np * 16 * ub * P_BK, ns = std::min(P_MAX_STAGES, (P_SMEM - 1024) / stage);
-      if (sp * ((ub + sp - 1) / sp) * 32 * 512 > ns * stage) continue;  // the parts land in the idle ring
+      if (sp * ((2 * ub + sp - 1) / sp) * P_CHUNK * 512 > ns * stage) continue;  // the parts land in the idle ring
       const double mma = 64.0 * ub * np, fill = (16384.0 + np * 2048.0 * ub) / 36.0;  // one tile per pair: latency shows
       const double cost = kbs * std::max(mma, fill) + 32.0 * ub * 512.0 * (sp - 1) / sp / 18.0 + 4000.0;
       if (best.cost < 0 || cost < best.cost) {
