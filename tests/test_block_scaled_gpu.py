@@ -165,7 +165,7 @@ def test_layernorm_into_the_form(m, w, groups):
 def test_which_products_take_the_form():
     _, lib, _ = _lib()
     assert lib.tybok_w8mx_suits(4146, 14336, 3072) and lib.tybok_w8mx_suits(333, 2048, 16384)
-    for m, n, k in [(128, 16384, 2048), (50, 8192, 1024), (800, 2560, 1024), (4146, 14336, 3080), (4146, 14336, 0)]:
+    for m, n, k in [(160, 16384, 2048), (50, 8192, 1024), (800, 2560, 1024), (4146, 14336, 3080), (4146, 14336, 0)]:
         assert not lib.tybok_w8mx_suits(m, n, k)
 
 
