@@ -48,6 +48,21 @@ class GemmaStack {
                  const std::vector<Tensor>& vc, int key_off, const Tensor& key_valid, const std::optional<std::vector<std::pair<Tensor, Tensor>>>& mods,
                  const std::optional<std::vector<std::pair<Tensor, Tensor>>>& fold, int first, int count, const std::vector<uint64_t>& wait,
                  const std::vector<uint64_t>& record) const {
+    return run(x, b, l, pos, cos, sin, kc, vc, key_off, key_valid, mods, fold, first, count, wait, record, false);
+  }
+  // The same for the caches alone: a prefix whose output nobody reads ends with its last layer's keys and values.  That layer's
+  // attention, output projection and FFN are nearly an eighteenth of the pass (chunk 10.06 -> 9.94 ms at batch 1, 101.3 -> 97.6 ms
+  // at batch 32).
+  void fill_caches(const Tensor& x, int b, int l, const Tensor& pos, const Tensor& cos, const Tensor& sin, const std::vector<Tensor>& kc,
+                   const std::vector<Tensor>& vc, const Tensor& key_valid, const std::vector<uint64_t>& record) const {
+    run(x, b, l, pos, cos, sin, kc, vc, 0, key_valid, std::nullopt, std::nullopt, 0, static_cast<int>(layers_.size()), {}, record, true);
+  }
+
+ private:
+  Tensor run(const Tensor& x, int b, int l, const Tensor& pos, const Tensor& cos, const Tensor& sin, const std::vector<Tensor>& kc,
+             const std::vector<Tensor>& vc, int key_off, const Tensor& key_valid, const std::optional<std::vector<std::pair<Tensor, Tensor>>>& mods,
+             const std::optional<std::vector<std::pair<Tensor, Tensor>>>& fold, int first, int count, const std::vector<uint64_t>& wait,
+             const std::vector<uint64_t>& record, bool caches_only) const {
     const int m = b * l, a = heads_ * hd_, keys = key_off + l;
     const Tensor x0 = rows_of(x);
     if (!is_bf16(x0) || x0.size(0) != m || x0.size(1) != w_) type_error("gemma_stack: x must be bf16 [B*L, W]");
@@ -105,7 +120,7 @@ class GemmaStack {
     const size_t x1 = ar.add(size_t(2) * m * w_), xa = ar.add(size_t(2) * m * w_), xb = ar.add(size_t(2) * m * w_), ws = ar.add(at_ws);
     const size_t up0 = ar.add(u), up1 = ar.add(u), part0 = ar.add(part), part1 = ar.add(part);
     ar.allocate(x0);
-    Tensor y = at::empty({m, w_}, x0.options());
+    Tensor y = at::empty({caches_only ? 0 : m, w_}, x0.options());
     void* st = stream_of(x);
     int* status = status_ptr(x.get_device());
     const float eps = 1e-6f, scale = static_cast<float>(1.0 / std::sqrt(static_cast<double>(hd_)));
@@ -140,6 +155,10 @@ class GemmaStack {
           check(tybok_w8x3_qkv_rope(ar.at(np), SHIFT_NORMED, lay.qkv.wp(), lay.qkv.sp(), static_cast<const int*>(ptr(pos)), ptr(cos), ptr(sin),
                                     ar.at(q), k, v, b, l, heads_, kv_, hd_, lcap, key_off, w_, 0, 0, status, st),
                 "tybok_w8x3_qkv_rope");
+      }
+      if (caches_only && last) {
+        record_event(record, i, st);
+        break;
       }
       check(tybok_attention(ar.at(q), k, v, ptr(key_valid), nullptr, ar.at(ap), SHIFT_ATTN, b, l, heads_, kv_, hd_, keys, lcap, scale, ar.at(ws),
                             at_ws, status, st),
@@ -199,7 +218,6 @@ class GemmaStack {
     return y;
   }
 
- private:
   static void record_event(const std::vector<uint64_t>& events, int i, void* st) {
     if (!events.empty() && cudaEventRecord(reinterpret_cast<cudaEvent_t>(events[i]), static_cast<cudaStream_t>(st)) != cudaSuccess)
       value_error("gemma_stack: cudaEventRecord failed");
@@ -232,7 +250,8 @@ class GemmaStack {
 void bind_gemma(py::module_& m) {
   py::class_<GemmaStack>(m, "GemmaStack")
       .def(py::init<int, int, int, int, const py::list&>())
-      .def("forward", &GemmaStack::forward, NoGil());
+      .def("forward", &GemmaStack::forward, NoGil())
+      .def("fill_caches", &GemmaStack::fill_caches, NoGil());
 }
 
 }  // namespace tbn

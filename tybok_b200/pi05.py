@@ -331,8 +331,8 @@ class PI05Model:
         kc, vc = self._caches(b)
         pos = (torch.cumsum(pad, dim=1) - 1).clamp_min(0).to(torch.int32).reshape(-1)
         key_valid = pad.to(torch.uint8).contiguous()
-        self._vlm.forward(prefix_embs.reshape(b * l, w), b, l, pos, self.cos, self.sin, kc, vc, 0, key_valid, None, None, 0,
-                          len(self.vlm_layers), [], [ev.cuda_event for ev in layer_done])
+        self._vlm.fill_caches(prefix_embs.reshape(b * l, w), b, l, pos, self.cos, self.sin, kc, vc, key_valid,
+                              [ev.cuda_event for ev in layer_done])
         return [(k[:, :, :l], v[:, :, :l]) for k, v in zip(kc, vc)]
 
     @torch.no_grad()
