@@ -59,13 +59,15 @@ constexpr int MAX_SPLITS = 8;             // portable cluster size
 struct GemmParams {
   int M, N, K;
   int n_out;     // width of the output rows: N, or N / 2 for EPI_GEGLU_PACKED
-  int bt;        // token tile (UMMA N), multiple of 16, <= 256 (<= 128 when nw == 2)
+  int bt;        // token tile, <= 256 (<= 128 when nw == 2)
   int nw;        // weight matrices per CTA: 1, or 2 for the gated form
   int splits;    // split-K factor == cluster size along z
   int kb_total;  // ceil(K / BK)
   int kb_per_split;
   int nstages;
   int tmem_cols;
+  int mma_n;        // UMMA N: np * bt rounded up to 16 where the planes are one UMMA, else bt
+  int stage_bytes;
   int stage_off;  // byte offset of the epilogue staging tile: 0 (over the idle ring) without split-K,
                   // behind the ring with split-K, because peers write into it while this CTA still streams
   int np;        // activation planes: 3 (e5m2, fixed exponent shift) or 2 (e4m3, per-token scale row_scale[m])
@@ -139,43 +141,58 @@ __device__ __noinline__ void see_copies_land(Barriers* b, int from, int ns) {
 // rsqrt(mean(x^2) + eps) of token row m from the producer's per-channel-tile partial sums (fixed order).
 // The partial sums were written by other SMs a moment ago (an L2 round trip each), so eight loads are
 // in flight at a time.
-__device__ __forceinline__ float deferred_rstd(const GemmParams& p, int m) {
+__device__ __forceinline__ float deferred_rstd(const float* part, int tiles, int M, float inv_w, float eps, int m) {
   float t = 0.f;
-  for (int i0 = 0; i0 < p.dn_tiles; i0 += 8) {
+#pragma unroll 1
+  for (int i0 = 0; i0 < tiles; i0 += 8) {
     float v[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-      v[i] = i0 + i < p.dn_tiles ? __ldcg(p.dn_part + static_cast<long long>(i0 + i) * p.M + m) : 0.f;
+    for (int i = 0; i < 8; ++i) v[i] = i0 + i < tiles ? __ldcg(part + static_cast<long long>(i0 + i) * M + m) : 0.f;
 #pragma unroll
     for (int i = 0; i < 8; ++i) t += v[i];
   }
-  return rsqrtf(t * p.dn_inv_w + p.dn_eps);
+  return rsqrtf(t * inv_w + eps);
+}
+// The same out of line, for the rows that a thread finishes after its first.
+__device__ __noinline__ float deferred_rstd_again(const float* part, int tiles, int M, float inv_w, float eps, int m) {
+  return deferred_rstd(part, tiles, M, inv_w, eps, m);
 }
 
 // Bounded for two CTAs per SM: multi-wave full-K launches run with a shallow ring so that one
 // tile's epilogue overlaps the other's main loop (register budget 64K / 640 threads).
 // EW: epilogue warps.  A split-K CTA has the SM to itself and a long serial epilogue per thread
 // (accumulator groups to push, rows to finish): sixteen warps halve both.
-template <int EW>
+// FORM, EPI: what an image is compiled for.  A CTA runs this code once, so a launch waits for its instructions (over 2000 of a
+// launch's 10000 clk), and chains of small launches alternate between images that should all stay in the instruction cache.
+// So the forms that such chains consist of (one weight matrix, three planes in columns of their own; and the one that makes its
+// planes) have images of a third to a half of the size, without the others' code and the tuning aids, which run in the image that
+// takes every form.  One image per epilogue is no better than one for none, GELU and residual together: 50-token MLP 12.7
+// against 12.9 us, but DiT block chains 3.84 against 3.71 ms.  With the row pairs and tiles below, batch-1 chunk 9.90 -> 9.22 ms,
+// 50-token MLP 14.6 -> 12.9 us, DiT runner 4.00 -> 3.72 ms, denoiser at 106 tokens 16.2 -> 14.6 ms, 1 x 2560 x 2048 6.5 -> 5.4 us.
+enum : int { FORM_ANY = 0, FORM_PLANES3 = 1, FORM_BF16 = 2, EPI_ANY = -1, EPI_LINEAR = -2 };  // (LINEAR: none, GELU or residual)
+template <int EW, int FORM, int EPI>
 __global__ void __launch_bounds__(32 * (2 + EW), EW == EPI_WARPS ? 2 : 1)
 w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                const __grid_constant__ CUtensorMap tm_x, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ Barriers bars;
 
-  const long long t_start = clock64();
+  constexpr bool ANY = FORM == FORM_ANY;
+  auto is = [&](int e) { return EPI == EPI_ANY ? p.epi == e : EPI == EPI_LINEAR ? e <= EPI_RESIDUAL && p.epi == e : e == EPI; };
+  const int np = ANY ? p.np : 3, nw = ANY ? p.nw : 1;
+  const bool merge = ANY ? p.merge : true, xb = ANY ? p.xb != nullptr : FORM == FORM_BF16;
+  const long long t_start = ANY ? clock64() : 0;
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
   const int lane = tid & 31;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int KID = EW == EPI_WARPS ? 0 : 1;
-  if (tid == 0) dbg_stage(p.dbg, KID, 0);
+  if (ANY && tid == 0) dbg_stage(p.dbg, KID, 0);
 
   const int ns = p.nstages;
-  const int x_bytes = p.np * p.bt * 128;              // np planes of bt rows x 128 bytes
-  const int x_off = p.nw * W_TILE_BYTES;              // activation planes follow the weight tile(s)
-  const int stage_bytes = x_off + x_bytes;
-  const int tx_bytes = p.xb ? x_off : stage_bytes;    // what the bulk copies bring
+  const int x_off = nw * W_TILE_BYTES;                // activation planes (np of bt rows x 128 bytes) follow the weight tile(s)
+  const int stage_bytes = p.stage_bytes;
+  const int tx_bytes = x_off + (xb ? 0 : np * p.bt * 128);  // what the bulk copies bring
 
   const int t_tile = blockIdx.x, n_tile = blockIdx.y, split = blockIdx.z;
   const int kb0 = split * p.kb_per_split;
@@ -183,10 +200,11 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
 
   if (warp == 0 && lane == 0) {
     tma_prefetch_desc(&tm_w0);
-    if (p.nw == 2) tma_prefetch_desc(&tm_w1);
+    if (nw == 2) tma_prefetch_desc(&tm_w1);
     tma_prefetch_desc(&tm_x);
+#pragma unroll 1
     for (int i = 0; i < MAX_STAGES; ++i) {
-      mbar_init(&bars.full[i], p.xb ? 1 + EW : 1);
+      mbar_init(&bars.full[i], xb ? 1 + EW : 1);
       mbar_init(&bars.empty[i], 1);
     }
     mbar_init(&bars.tmem_full, 1);
@@ -197,12 +215,13 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     // Weights depend on nothing that runs before this kernel: request the first stages now,
     // before the rest of the CTA has even finished its set-up.
     const int pre = min(ns, nkb);
+#pragma unroll 1
     for (int i = 0; i < pre; ++i) {
       uint8_t* st = smem + i * stage_bytes;
       mbar_arrive_expect_tx(&bars.full[i], tx_bytes);
       const int k0 = (kb0 + i) * BK;
       tma_load_2d(st, &tm_w0, &bars.full[i], k0, n_tile * BN);
-      if (p.nw == 2) tma_load_2d(st + W_TILE_BYTES, &tm_w1, &bars.full[i], k0, n_tile * BN);
+      if (nw == 2) tma_load_2d(st + W_TILE_BYTES, &tm_w1, &bars.full[i], k0, n_tile * BN);
     }
   }
   if (warp == 1) {
@@ -212,7 +231,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (tid == 0) dbg_stage(p.dbg, KID, 1);
+  if (ANY && tid == 0) dbg_stage(p.dbg, KID, 1);
   const uint32_t tmem = bars.tmem_base;
   // Per-thread epilogue constants (4 consecutive channels), fetched while the main loop runs.
   float s0[4] = {0, 0, 0, 0}, s1[4] = {0, 0, 0, 0}, b0[4] = {0, 0, 0, 0};
@@ -222,13 +241,15 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   uint2 res_pf[4] = {};  // residual of this thread's first four token rows, fetched early
   float4 gate_pf = make_float4(0.f, 0.f, 0.f, 0.f);  // gate values of the first token row's group (fp32 form)
   int gate_pf_group = -1;
-  // Split-K ownership: the tile's real token rows are divided evenly over the cluster ranks.
+  // Split-K ownership: pairs of the tile's token rows go round the cluster ranks.  Row rl of a rank is token_of(rl).  (Blocks
+  // of rows, a warp's 16 tokens straddling up to three owners, took an epilogue thread over 200 instructions to send.)
   const int m_base = t_tile * p.bt;
   const int nvalid = min(p.bt, p.M - m_base);
-  const int rpr = (nvalid + p.splits - 1) / p.splits;
+  const int rpr = 2 * (((nvalid + 1) / 2 + p.splits - 1) / p.splits);
   const int rank = p.splits > 1 ? static_cast<int>(cluster_ctarank()) : 0;
-  const int own_rows = max(0, min(nvalid, rank * rpr + rpr) - rank * rpr);
-  long long* tr = p.trace ? p.trace + 16ll * ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) : nullptr;
+  auto token_of = [&](int rl) { return 2 * ((rl >> 1) * p.splits + rank) + (rl & 1); };
+  const float* const row_scale = ANY ? p.row_scale : nullptr;
+  long long* tr = ANY && p.trace ? p.trace + 16ll * ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) : nullptr;
   if (tr && tid == 0) { tr[0] = t_start; tr[1] = clock64(); }
 
   if (warp == 0) {
@@ -241,8 +262,9 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       // The weight tiles of the first stages were requested during set-up; the activation planes
       // are requested once the programmatic dependency has resolved.
       if (p.pdl) pdl_wait();
-      dbg_stage(p.dbg, KID, 2);
-      if (!p.xb)
+      if (ANY) dbg_stage(p.dbg, KID, 2);
+      if (!xb)
+#pragma unroll 1
         for (int i = 0; i < pre; ++i)
           tma_load_3d(smem + i * stage_bytes + x_off, &tm_x, &bars.full[i], (kb0 + i) * BK, t_tile * p.bt, 0);
       if (EW == EPI_WARPS_WIDE && p.splits > 1) cluster_arrive_relaxed();
@@ -257,8 +279,8 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         mbar_arrive_expect_tx(&bars.full[s], tx_bytes);
         const int k0 = (kb0 + i) * BK;
         tma_load_2d(st, &tm_w0, &bars.full[s], k0, n_tile * BN);
-        if (p.nw == 2) tma_load_2d(st + W_TILE_BYTES, &tm_w1, &bars.full[s], k0, n_tile * BN);
-        if (!p.xb) tma_load_3d(st + x_off, &tm_x, &bars.full[s], k0, t_tile * p.bt, 0);
+        if (nw == 2) tma_load_2d(st + W_TILE_BYTES, &tm_w1, &bars.full[s], k0, n_tile * BN);
+        if (!xb) tma_load_3d(st + x_off, &tm_x, &bars.full[s], k0, t_tile * p.bt, 0);
         issued = i + 1;
       }
       bars.issued = issued;
@@ -273,11 +295,11 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     // with N = 3*bt multiplies a K slice by all of them (one column group per plane) -- 4
     // instead of 12 instructions per weight tile and K block.  Larger tiles issue one UMMA per
     // plane into the same accumulator.
-    const int mma_n = p.merge ? p.np * p.bt : p.bt;
-    const uint32_t idesc = p.np == 2 ? idesc_e4m3_e4m3_f32(BN, mma_n) : idesc_e4m3_e5m2_f32(BN, mma_n);
+    const int mma_n = p.mma_n;  // merged: np * bt rounded up to 16 (what the rows past the planes hold goes to columns nobody reads)
+    const uint32_t idesc = np == 2 ? idesc_e4m3_e4m3_f32(BN, mma_n) : idesc_e4m3_e5m2_f32(BN, mma_n);
     const uint64_t desc_const = smem_desc_sw128(0);
     const uint32_t plane16 = static_cast<uint32_t>(p.bt * 128) >> 4;  // plane pitch in 16-byte units
-    const int acc_cols = p.merge ? p.np * p.bt : p.bt;
+    const int acc_cols = mma_n;
     if (EW == EPI_WARPS_WIDE && p.splits > 1) cluster_arrive_relaxed();
     bool ok = true;
     int stop = 0;
@@ -294,10 +316,10 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       tc_fence_after();
       const uint32_t st16 = (smem_u32(smem + s * stage_bytes) & 0x3FFFFu) >> 4;
       const uint32_t x16 = st16 + (x_off >> 4);
-      for (int w = 0; w < p.nw; ++w) {
+      for (int w = 0; w < nw; ++w) {
         const uint32_t w16 = st16 + w * (W_TILE_BYTES >> 4);
         const uint32_t d_addr = tmem + w * acc_cols;
-        if (p.merge) {
+        if (merge) {
 #pragma unroll
           for (int j = 0; j < 4; ++j) {  // K = 32 per instruction: 32 bytes = 2 sixteen-byte units
             const uint64_t a_desc = desc_const | (w16 + j * 2);
@@ -305,7 +327,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
             if (leader) umma_ss_f8(d_addr, a_desc, b_desc, idesc, (i > 0 || j > 0) ? 1u : 0u);
           }
         } else {
-          for (int pl = 0; pl < p.np; ++pl) {
+          for (int pl = 0; pl < np; ++pl) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const uint64_t a_desc = desc_const | (w16 + j * 2);
@@ -342,14 +364,14 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     const int row = q * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(q * 32) << 16;
     {
-      const bool packed = p.epi == EPI_GEGLU_PACKED || p.epi == EPI_QKV_ROPE;  // paired half tiles
+      const bool packed = is(EPI_GEGLU_PACKED) || is(EPI_QKV_ROPE);  // paired half tiles
       const int v4p = (tid - 64) & 31;
       const int col0 = packed ? (v4p & 15) * 4 : v4p * 4;
-      const int n = p.epi == EPI_GEGLU_PACKED ? n_tile * (BN / 2) + col0 : n_tile * BN + col0;  // first output channel
+      const int n = is(EPI_GEGLU_PACKED) ? n_tile * (BN / 2) + col0 : n_tile * BN + col0;  // first output channel
       if (n < p.n_out) {  // weights-side data: independent of the previous kernel in the stream
         const float4 t = *reinterpret_cast<const float4*>(p.scale0 + n_tile * BN + col0);
         s0[0] = t.x * p.out_scale; s0[1] = t.y * p.out_scale; s0[2] = t.z * p.out_scale; s0[3] = t.w * p.out_scale;
-        if (p.nw == 2 || packed) {
+        if (nw == 2 || packed) {
           const float4 u = packed ? *reinterpret_cast<const float4*>(p.scale0 + n_tile * BN + BN / 2 + col0)
                                   : *reinterpret_cast<const float4*>(p.scale1 + n);
           s1[0] = u.x * p.out_scale; s1[1] = u.y * p.out_scale; s1[2] = u.z * p.out_scale; s1[3] = u.w * p.out_scale;
@@ -370,20 +392,20 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           const float4 t0 = *reinterpret_cast<const float4*>(p.nn_scale + n);
           nsc[0] = 1.0f + t0.x; nsc[1] = 1.0f + t0.y; nsc[2] = 1.0f + t0.z; nsc[3] = 1.0f + t0.w;
         }
-        if (p.epi == EPI_RESIDUAL && p.gate && !p.gate_bf16) {
+        if (is(EPI_RESIDUAL) && p.gate && !p.gate_bf16) {
           // fp32 gates are per-step constants (precomputed modulations), touched once per chunk
           // and therefore cold in L2: fetch them now, not between the accumulator and the stores.
-          gate_pf_group = (m_base + rank * rpr) / p.rows_per_gate;
+          gate_pf_group = (m_base + 2 * rank) / p.rows_per_gate;
           gate_pf = *reinterpret_cast<const float4*>(static_cast<const float*>(p.gate) +
                                                      static_cast<long long>(gate_pf_group) * p.ldgate + n);
         }
-        if (p.epi == EPI_QKV_ROPE) {
+        if (is(EPI_QKV_ROPE)) {
           // Positions and tables are constants: fetch the cos/sin of this thread's first row now.
           const RopeEpi& r = p.rope;
           const int tps = r.D >> 7;
           const int rl = ((tid - 64) >> 5) * 2 + (v4p >> 4);
-          if (rl < own_rows && n_tile / tps < r.H + r.G) {
-            const long long tb = static_cast<long long>(r.pos[m_base + rank * rpr + rl]) * r.D + (n_tile % tps) * 64 + col0;
+          if (token_of(rl) < nvalid && n_tile / tps < r.H + r.G) {
+            const long long tb = static_cast<long long>(r.pos[m_base + token_of(rl)]) * r.D + (n_tile % tps) * 64 + col0;
             res_pf[0] = *reinterpret_cast<const uint2*>(r.cos + tb);
             res_pf[1] = *reinterpret_cast<const uint2*>(r.cos + tb + (r.D >> 1));
             res_pf[2] = *reinterpret_cast<const uint2*>(r.sin + tb);
@@ -398,22 +420,21 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       if (n < p.n_out) {
         if (p.dn_part) {  // written by the previous GEMM: this thread's first row, under the main loop
           const int rl = packed ? ((tid - 64) >> 5) * 2 + (v4p >> 4) : (tid - 64) >> 5;
-          if (rl < own_rows) rs_pf = deferred_rstd(p, m_base + rank * rpr + rl);
+          if (token_of(rl) < nvalid) rs_pf = deferred_rstd(p.dn_part, p.dn_tiles, p.M, p.dn_inv_w, p.dn_eps, m_base + token_of(rl));
         }
-        if (p.epi == EPI_RESIDUAL) {
+        if (is(EPI_RESIDUAL)) {
           // The residual was written by an earlier kernel: fetch the rows this thread will finish
           // first, long before the accumulator is ready.
 #pragma unroll
           for (int u = 0; u < 4; ++u) {
             const int rl = ((tid - 64) >> 5) + EW * u;
-            if (rl < own_rows)
-              res_pf[u] = *reinterpret_cast<const uint2*>(
-                  p.res + static_cast<long long>(m_base + rank * rpr + rl) * p.ldres + n);
+            if (token_of(rl) < nvalid)
+              res_pf[u] = *reinterpret_cast<const uint2*>(p.res + static_cast<long long>(m_base + token_of(rl)) * p.ldres + n);
           }
         }
       }
     }
-    if (EW == EPI_WARPS_WIDE && p.xb) {
+    if (EW == EPI_WARPS_WIDE && (ANY || FORM == FORM_BF16) && xb) {
       // bt == 16 token rows: warp `ew` makes row ew of every plane of every stage, four values per lane, written where the
       // bulk copy would have put them (128-byte swizzle).  Four stages of loads are in flight at a time.
       const int row = ew;
@@ -473,19 +494,19 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       // own shared memory.
       const uint32_t stage_addr = smem_u32(smem + p.stage_off);
       const int ngroups = (nvalid + 15) / 16;
-      const int acc_cols = p.merge ? p.np * p.bt : p.bt;
-      for (int w = 0; w < p.nw; ++w) {
+      const int acc_cols = p.mma_n;
+      for (int w = 0; w < nw; ++w) {
         for (int g = half; g < ngroups; g += EW / 4) {
           uint32_t v[16];
           const uint32_t col = tmem + lane_addr + w * acc_cols + g * 16;
           tmem_ld16(col, v);
-          if (p.merge && p.np == 2) {  // add the per-plane column groups in plane order
+          if (merge && np == 2) {  // add the per-plane column groups in plane order
             uint32_t v2[16];
             tmem_ld16(col + p.bt, v2);
             tc_wait_ld();
 #pragma unroll
             for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(v2[e]));
-          } else if (p.merge) {
+          } else if (merge) {
             uint32_t v2[16], v3[16];
             tmem_ld16(col + p.bt, v2);
             tmem_ld16(col + 2 * p.bt, v3);
@@ -503,20 +524,20 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
             for (int e = 0; e < 16; ++e)
               if (g * 16 + e < nvalid) dst[e * BN] = __uint_as_float(v[e]);
           } else {
-            // Up to three owners per group of 16 tokens; an owner's window is linear, so one
-            // address translation per owner and 512-byte steps inside it.
+            // Two rows per owner in turn: one address translation and two stores.
             const int t0 = g * 16;
-            int owner = t0 / rpr, rl = t0 - owner * rpr;
-            const uint32_t slot = stage_addr + (((split * p.nw + w) * rpr) * BN + row) * 4;
-            uint32_t base = dsmem_addr(slot, owner);
+            int lr = (g * 8) / p.splits, owner = g * 8 - lr * p.splits;
+            const uint32_t slot = stage_addr + (((split * nw + w) * rpr) * BN + row) * 4;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              if (t0 + e < nvalid)
-                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(base + rl * (BN * 4)), "f"(__uint_as_float(v[e])));
-              if (++rl == rpr) {
-                rl = 0;
-                ++owner;
-                if (owner < p.splits) base = dsmem_addr(slot, owner);
+            for (int e = 0; e < 16; e += 2) {
+              if (t0 + e < nvalid) {
+                const uint32_t dst = dsmem_addr(slot + lr * (2 * BN * 4), owner);
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(__uint_as_float(v[e])));
+                if (t0 + e + 1 < nvalid) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + BN * 4), "f"(__uint_as_float(v[e + 1])));
+              }
+              if (++owner == p.splits) {
+                owner = 0;
+                ++lr;
               }
             }
           }
@@ -537,7 +558,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   }
 
   if (tr && tid == 64) tr[6] = clock64();
-  if (tid == 0) dbg_stage(p.dbg, KID, 3);
+  if (ANY && tid == 0) dbg_stage(p.dbg, KID, 3);
   if (warp >= 2 && !bars.abort) {
     // ---------------------------------------------------------- epilogue, phase B
     // 4 consecutive channels per thread, 8 token rows per pass; with split-K, rank r owns token
@@ -548,9 +569,9 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     const int rgrp = et >> 5;
     // Packed gated form: 16 lanes cover the 64 output channels of a row, so a warp takes two
     // rows per pass; otherwise 32 lanes cover the 128 channels of one row.
-    const bool packed = p.epi == EPI_GEGLU_PACKED || p.epi == EPI_QKV_ROPE;
+    const bool packed = is(EPI_GEGLU_PACKED) || is(EPI_QKV_ROPE);
     const int col0 = packed ? (v4 & 15) * 4 : v4 * 4;
-    const int n = p.epi == EPI_GEGLU_PACKED ? n_tile * (BN / 2) + col0 : n_tile * BN + col0;
+    const int n = is(EPI_GEGLU_PACKED) ? n_tile * (BN / 2) + col0 : n_tile * BN + col0;
     const bool n_ok = n < p.n_out;  // n_out % 4 == 0, so all four channels are valid together
     const int row0 = packed ? rgrp * 2 + (v4 >> 4) : rgrp;
     const int rstep = packed ? 2 * EW : EW;
@@ -558,23 +579,23 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     const long long plane = static_cast<long long>(p.M) * p.n_out;
     if (tr && tid == 64) tr[10] = clock64();
 #pragma unroll 1
-    for (int rl = row0; rl < own_rows && n_ok; rl += rstep) {
-      const int m = m_base + rank * rpr + rl;
+    for (int rl = row0; token_of(rl) < nvalid && n_ok; rl += rstep) {
+      const int m = m_base + token_of(rl);
       float4 a0 = make_float4(0.f, 0.f, 0.f, 0.f), a1 = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 1
       for (int sp = 0; sp < p.splits; ++sp) {  // split order: bit-reproducible
-        const float* r0p = stage + ((sp * p.nw) * rpr + rl) * BN;
+        const float* r0p = stage + ((sp * nw) * rpr + rl) * BN;
         const float4 f = *reinterpret_cast<const float4*>(r0p + col0);
         a0.x += f.x; a0.y += f.y; a0.z += f.z; a0.w += f.w;
-        if (p.nw == 2 || packed) {
+        if (nw == 2 || packed) {
           const float4 g = packed ? *reinterpret_cast<const float4*>(r0p + BN / 2 + col0)
-                                  : *reinterpret_cast<const float4*>(stage + ((sp * p.nw + 1) * rpr + rl) * BN + col0);
+                                  : *reinterpret_cast<const float4*>(stage + ((sp * nw + 1) * rpr + rl) * BN + col0);
           a1.x += g.x; a1.y += g.y; a1.z += g.z; a1.w += g.w;
         }
       }
-      if (p.row_scale || p.dn_part) {
+      if (row_scale || p.dn_part) {
         // two-plane form: undo the token's power-of-two pre-scale (exact); deferred norm: the row's rstd
-        const float rs = p.row_scale ? p.row_scale[m] : (rl == row0 ? rs_pf : deferred_rstd(p, m));
+        const float rs = row_scale ? row_scale[m] : (rl == row0 ? rs_pf : deferred_rstd_again(p.dn_part, p.dn_tiles, p.M, p.dn_inv_w, p.dn_eps, m));
         a0.x *= rs; a0.y *= rs; a0.z *= rs; a0.w *= rs;
         a1.x *= rs; a1.y *= rs; a1.z *= rs; a1.w *= rs;
       }
@@ -583,15 +604,15 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       // GELU output, product, gated value, residual sum.
       float o[4] = {bf16_round(a0.x * s0[0] + b0[0]), bf16_round(a0.y * s0[1] + b0[1]),
                     bf16_round(a0.z * s0[2] + b0[2]), bf16_round(a0.w * s0[3] + b0[3])};
-      if (p.epi == EPI_GELU) {
+      if (is(EPI_GELU)) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[e] = gelu_tanh_fast(o[e]);
-      } else if (p.epi == EPI_GEGLU || p.epi == EPI_GEGLU_PACKED) {
+      } else if (is(EPI_GEGLU) || is(EPI_GEGLU_PACKED)) {
         const float u[4] = {bf16_round(a1.x * s1[0] + b1[0]), bf16_round(a1.y * s1[1] + b1[1]),
                             bf16_round(a1.z * s1[2] + b1[2]), bf16_round(a1.w * s1[3] + b1[3])};
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[e] = bf16_round(gelu_tanh_fast(o[e])) * u[e];
-      } else if (p.epi == EPI_QKV_ROPE) {
+      } else if (is(EPI_QKV_ROPE)) {
         // o = dimensions d..d+3 of one head slot, u = their partners d + D/2; rotate q and k
         // slots (bf16 rounding points of rope.py:67-75), pass v through, store both halves.
         const RopeEpi& r = p.rope;
@@ -636,7 +657,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         st.x = *reinterpret_cast<const uint32_t*>(&h01); st.y = *reinterpret_cast<const uint32_t*>(&h23);
         *reinterpret_cast<uint2*>(dst + half + d) = st;
         continue;
-      } else if (p.epi == EPI_RESIDUAL) {
+      } else if (is(EPI_RESIDUAL)) {
         if (p.gate) {
           const long long gi = static_cast<long long>(m / p.rows_per_gate) * p.ldgate + n;
           float gv[4];
@@ -704,7 +725,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     tc_fence_after();
     tmem_dealloc(tmem, p.tmem_cols);
   }
-  if (tid == 0) dbg_stage(p.dbg, KID, 4);
+  if (ANY && tid == 0) dbg_stage(p.dbg, KID, 4);
 }
 
 // ------------------------------------------------------------------------------------ split kernel
@@ -776,7 +797,7 @@ __global__ void __launch_bounds__(256) split_mx_kernel(const __nv_bfloat16* __re
 
 // ------------------------------------------------------------------------------------ host
 struct Plan {
-  int bt, t_tiles, n_tiles, splits, kb_total, kb_per_split, nstages, smem_bytes, tmem_cols, merge, stage_off;
+  int bt, t_tiles, n_tiles, splits, kb_total, kb_per_split, nstages, smem_bytes, tmem_cols, merge, mma_n, stage_bytes, stage_off;
 };
 
 static int round_up(int a, int b) { return (a + b - 1) / b * b; }
@@ -788,7 +809,7 @@ static int max_active_clusters(int splits) {
   static host::DeviceCache cache[MAX_SPLITS + 1];
   if (splits <= 1) return 1 << 30;
   return host::per_device(cache[splits], [splits] {
-    cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX);
+    cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS_WIDE, FORM_ANY, EPI_ANY>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(1, 1, splits);
     cfg.blockDim = dim3(THREADS_WIDE);
@@ -801,7 +822,7 @@ static int max_active_clusters(int splits) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, w8_gemm_kernel<EPI_WARPS_WIDE>, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, w8_gemm_kernel<EPI_WARPS_WIDE, FORM_ANY, EPI_ANY>, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = host::sm_count() / (2 * splits);  // conservative guess
     }
@@ -855,12 +876,18 @@ static bool make_plan(int M, int N, int K, int nw, int force_bt, int force_split
     while (splits > 1 && tiles > max_active_clusters(splits)) --splits;
   }
   splits = std::max(1, std::min(std::min(splits, MAX_SPLITS), pl.kb_total));
-  const int stage_bytes = nw * W_TILE_BYTES + np * bt * 128;
+  // Merged planes are one run of rows in shared memory: the tile need not be a multiple of 16 tokens, only the UMMA's N, and
+  // the tokens spread evenly over the tiles (50 tokens: 150 rows to fetch per K block instead of 192).
+  pl.merge = (np * bt <= 256 && nw * np * bt <= 512) ? 1 : 0;
+  if (pl.merge && force_bt <= 0) pl.bt = bt = (M + pl.t_tiles - 1) / pl.t_tiles;
+  pl.mma_n = pl.merge ? round_up(np * bt, 16) : bt;
+  pl.stage_bytes = nw * W_TILE_BYTES + (pl.merge ? pl.mma_n : np * bt) * 128;
+  const int stage_bytes = pl.stage_bytes;
   for (;; --splits) {  // fewer splits if the split-K staging tile does not fit beside the ring
     pl.kb_per_split = (pl.kb_total + splits - 1) / splits;
     pl.splits = (pl.kb_total + pl.kb_per_split - 1) / pl.kb_per_split;  // no empty split
     // Staging tile of the epilogue: [splits][nw][rows per rank][128] fp32.
-    const int rpr = (bt + pl.splits - 1) / pl.splits;
+    const int rpr = 2 * (((bt + 1) / 2 + pl.splits - 1) / pl.splits);
     const int staging = round_up(pl.splits * nw * rpr * BN * 4, 1024);
     const int extra = pl.splits > 1 ? staging : 0;
     pl.nstages = std::min(MAX_STAGES, (DYN_SMEM_MAX - 1024 - extra) / stage_bytes);  // 1 KB of alignment slack
@@ -877,9 +904,8 @@ static bool make_plan(int M, int N, int K, int nw, int force_bt, int force_split
     if (pl.nstages >= 2 && pl.nstages <= MAX_STAGES && pl.smem_bytes <= DYN_SMEM_MAX) break;
     if (splits == 1) return false;
   }
-  pl.merge = (np * bt <= 256 && nw * np * bt <= 512) ? 1 : 0;
-  pl.tmem_cols = 32;
-  while (pl.tmem_cols < nw * bt * (pl.merge ? np : 1)) pl.tmem_cols *= 2;
+  pl.tmem_cols = 32;  // the epilogue reads columns in groups of 16 from every plane's first one on
+  while (pl.tmem_cols < (nw - 1) * pl.mma_n + (pl.merge ? std::max(pl.mma_n, (np - 1) * bt + round_up(bt, 16)) : bt)) pl.tmem_cols *= 2;
   return true;
 }
 
@@ -899,6 +925,15 @@ struct NormFold {
   float eps = 0.f;
   const float* bias_rows = nullptr;
 };
+
+using GemmKernel = void(const CUtensorMap, const CUtensorMap, const CUtensorMap, const GemmParams);
+static GemmKernel* lean_kernel(int epi) {
+  switch (epi) {
+    case EPI_GEGLU_PACKED: return w8_gemm_kernel<EPI_WARPS_WIDE, FORM_PLANES3, EPI_GEGLU_PACKED>;
+    case EPI_QKV_ROPE: return w8_gemm_kernel<EPI_WARPS_WIDE, FORM_PLANES3, EPI_QKV_ROPE>;
+    default: return w8_gemm_kernel<EPI_WARPS_WIDE, FORM_PLANES3, EPI_LINEAR>;
+  }
+}
 
 static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, const float* s0, const float* s1,
                        const void* bias, void* y, void* y_planes, int M, int N, int K, long long ldy, int epi,
@@ -943,7 +978,7 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   if (int rc = host::require_sm100()) return rc;
 
   Plan pl;
-  if (!make_plan(M, N, K, nw, force_bt, force_splits, pl, np))
+  if (!make_plan(M, N, K, nw, x_bf16 ? 16 : force_bt, force_splits, pl, np))  // (the planes that it makes itself are 16 rows each)
     return host::fail(TYBOK_ERR_ARG, "w8 gemm: unsupported token tile (multiple of 16, <= 256, <= 128 when gated)");
   if (force_splits > MAX_SPLITS) return host::fail(TYBOK_ERR_ARG, "w8 gemm: at most 8 K splits (cluster size)");
   if (pl.n_tiles > 65535) return host::fail(TYBOK_ERR_ARG, "w8 gemm: grid too large");
@@ -988,7 +1023,7 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   GemmParams p{};
   p.M = M; p.N = N; p.K = K; p.n_out = n_out;
   p.bt = pl.bt; p.nw = nw; p.splits = pl.splits; p.kb_total = pl.kb_total; p.kb_per_split = pl.kb_per_split;
-  p.nstages = pl.nstages; p.tmem_cols = pl.tmem_cols; p.merge = pl.merge; p.stage_off = pl.stage_off; p.epi = epi; p.pdl = host::pdl_enabled() ? 1 : 0;
+  p.nstages = pl.nstages; p.tmem_cols = pl.tmem_cols; p.merge = pl.merge; p.mma_n = pl.mma_n; p.stage_bytes = pl.stage_bytes; p.stage_off = pl.stage_off; p.epi = epi; p.pdl = host::pdl_enabled() ? 1 : 0;
   p.np = np; p.row_scale = row_scale;
   p.out_scale = row_scale ? 1.0f : ldexpf(1.0f, -x_shift);
   p.plane_scale = ldexpf(1.0f, out_shift);
@@ -1011,9 +1046,11 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
 
   static host::DeviceCache attr_set;
   if (!host::per_device(attr_set, [] {
-        return static_cast<int>(
-            cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) == cudaSuccess &&
-            cudaFuncSetAttribute(w8_gemm_kernel<EPI_WARPS_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) == cudaSuccess);
+        for (GemmKernel* k : {w8_gemm_kernel<EPI_WARPS, FORM_ANY, EPI_ANY>, w8_gemm_kernel<EPI_WARPS_WIDE, FORM_ANY, EPI_ANY>,
+                              w8_gemm_kernel<EPI_WARPS_WIDE, FORM_BF16, EPI_LINEAR>,
+                              w8_gemm_kernel<EPI_WARPS_WIDE, FORM_BF16, EPI_GEGLU_PACKED>, lean_kernel(EPI_NONE), lean_kernel(EPI_GEGLU_PACKED), lean_kernel(EPI_QKV_ROPE)})
+          if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) != cudaSuccess) return 0;
+        return 1;
       }))
     return host::fail_cuda("cudaFuncSetAttribute(w8_gemm_kernel)");
 
@@ -1040,7 +1077,13 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  if (cudaLaunchKernelEx(&cfg, wide ? w8_gemm_kernel<EPI_WARPS_WIDE> : w8_gemm_kernel<EPI_WARPS>, tm_w0, tm_w1, tm_x, p) != cudaSuccess)
+  const bool plain = nw == 1 && np == 3 && pl.merge && !p.trace && !p.dbg;
+  GemmKernel* k = !wide ? w8_gemm_kernel<EPI_WARPS, FORM_ANY, EPI_ANY>
+                  : !plain ? w8_gemm_kernel<EPI_WARPS_WIDE, FORM_ANY, EPI_ANY>
+                  : !x_bf16 ? lean_kernel(epi)
+                  : epi == EPI_GEGLU_PACKED ? w8_gemm_kernel<EPI_WARPS_WIDE, FORM_BF16, EPI_GEGLU_PACKED>
+                                            : w8_gemm_kernel<EPI_WARPS_WIDE, FORM_BF16, EPI_LINEAR>;
+  if (cudaLaunchKernelEx(&cfg, k, tm_w0, tm_w1, tm_x, p) != cudaSuccess)
     return host::fail_cuda("launch w8_gemm_kernel");
   host::count_launch();
   return TYBOK_OK;
