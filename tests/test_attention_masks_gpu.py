@@ -1,0 +1,46 @@
+"""Rows that meet masked keys only, for a block or for all of them, in every attention form and at scales on both sides of the usual
+one; and the images with the tuning aids against those without: the same bits."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# suffix over key blocks (rows pushed, and staged in L2), one block, the key loop at both head sizes, up to 64 rows, two tiles
+FORMS = [(1, 50, 594, 8, 1, 256), (2, 50, 594, 8, 2, 256), (1, 50, 100, 8, 1, 256), (1, 300, 300, 8, 1, 256), (1, 106, 400, 3, 3, 128),
+         (1, 50, 700, 24, 24, 128), (1, 1030, 400, 24, 24, 128)]
+
+
+@pytest.mark.parametrize("b,l,keys,h,g,d", FORMS)
+@pytest.mark.parametrize("scale", [0.002, 0.0625, 1.5])
+@pytest.mark.parametrize("first,last", [(128, 0), (200, 60), (0, 0), (10**9, 0)])
+def test_masked_blocks(b, l, keys, h, g, d, scale, first, last):
+    from tybok_b200 import ops
+
+    gen = torch.Generator(device="cuda").manual_seed(l + keys)
+    rnd = lambda *s: torch.empty(*s, device="cuda").normal_(0, 1, generator=gen).to(torch.bfloat16)  # noqa: E731
+    q, k, v = rnd(b * l, h * d), rnd(b, g, keys, d), rnd(b, g, keys, d)
+    valid = torch.ones(b, keys, dtype=torch.uint8, device="cuda")
+    valid[:, : min(first, keys)] = 0
+    if last:
+        valid[:, keys - last :] = 0
+    call = lambda: ops.attention(q, k, v, valid, tokens=l, keys=keys, scale=scale, out_planes=True)  # noqa: E731
+    y, yp = call()
+    ops.check_status()
+    s = torch.einsum("bthd,bhnd->bhtn", q.view(b, l, h, d).double(), k.double().repeat_interleave(h // g, 1)) * scale
+    s = s.masked_fill(valid[:, None, None] == 0, float("-inf"))
+    p = torch.softmax(s, -1).nan_to_num(0.0)  # no key at all: zero, as the kernels have it
+    ref = torch.einsum("bhtn,bhnd->bthd", p, v.double().repeat_interleave(h // g, 1)).reshape(b * l, h * d)
+    # probabilities and output are rounded to bf16: 2^-8 of the values' weighted mean magnitude, and of the result
+    room = torch.einsum("bhtn,bhnd->bthd", p, v.double().abs().repeat_interleave(h // g, 1)).reshape(b * l, h * d)
+    assert bool(((y.double() - ref).abs() <= 2.0**-8 * (room + ref.abs()) + 1e-6).all())
+    lib = ops._lib.load()
+    trace = torch.zeros(16 * 8192, dtype=torch.int64, device="cuda")
+    lib.tybok_debug_set_trace(trace.data_ptr())
+    try:
+        y1, yp1 = call()
+        torch.cuda.synchronize()
+    finally:
+        lib.tybok_debug_set_trace(None)
+    assert torch.equal(y, y1) and torch.equal(yp, yp1)

@@ -267,6 +267,9 @@ struct __align__(16) AttnBars {
   float wn[AT_MAX_SPLITS][AT_BQ];  // merge weights of the rows this CTA owns: exp2(m_s - m) / denominator
 };
 
+// Score of a masked key: so small that its exponential is zero beside any other (and beside half of itself, which stands in for
+// the reference maximum of a row that has seen masked keys only).
+constexpr float PF_MASKED = -1e30f;
 // 2^x by the special-function unit alone (results below 2^-126 flush to zero).
 __device__ __forceinline__ float pf_exp2(float x) {
   float y;
@@ -302,13 +305,16 @@ __device__ __forceinline__ void at_not_sent(AttnBars* b, uint64_t* bar, int peer
 // merge straight into that peer's shared memory (the idle half of its V tile) with bulk copies
 // credited to the peer's barrier, so the merge starts when the rows land: no trip through L2,
 // no cluster-wide meeting point before it.
-template <bool PUSH>
+// AIDS: the image with the tuning aids in it.  A launch waits for its instructions, so the others go without them, mask scores once
+// instead of having three forms of the softmax, and keep serial loops rolled (49 -> 38 KB here, 45 -> 34 KB for the key loops:
+// DiT denoiser at 106 tokens 14.53 -> 14.17 ms, batch-1 chunk 9.27 -> 9.24 ms).
+template <bool PUSH, bool AIDS>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                  const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ AttnBars bars;
-  const long long t_start = clock64();
+  const long long t_start = AIDS ? clock64() : 0;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sq = smem;
@@ -330,6 +336,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
+#pragma unroll 1
     for (int c = 0; c < 4; ++c) mbar_init(&bars.qk_full[c], 1);
     mbar_init(&bars.v_full, 1);
     mbar_init(&bars.s_full, 1);
@@ -375,7 +382,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   const uint32_t t_s = tmem, t_p = tmem + 128, t_o = tmem + 256;
   const int nvalid = min(AT_BQ, p.L - qt * AT_BQ);  // real query rows of this tile
   uint8_t* my_ws = p.ws + static_cast<long long>((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * AT_WS_PER_CTA;
-  long long* tr = p.trace ? p.trace + 16ll * ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) : nullptr;
+  long long* tr = AIDS && p.trace ? p.trace + 16ll * ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) : nullptr;
   if (tr && tid == 0) { tr[0] = t_start; tr[1] = clock64(); }
 
   if (warp == 0) {
@@ -384,6 +391,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (p.pdl) pdl_wait();
       const int qrow = b * p.L + qt * AT_BQ;
       const int krow = (b * p.G + g) * p.Lcap + key0;
+#pragma unroll 1
       for (int c = 0; c < 4; ++c) {
         mbar_arrive_expect_tx(&bars.qk_full[c], AT_CHUNK + p.q_rows * 128);
         tma_load_2d(sq + c * AT_CHUNK, &tm_q, &bars.qk_full[c], h * AT_D + c * 64, qrow);
@@ -391,6 +399,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       }
       const int nvc = dv / 64;  // 64-column chunks of V this CTA multiplies
       mbar_arrive_expect_tx(&bars.v_full, nvc * AT_CHUNK);
+#pragma unroll 1
       for (int c = 0; c < nvc; ++c) tma_load_2d(sv + c * AT_CHUNK, &tm_v, &bars.v_full, dh * dv + c * 64, krow);
     }
   } else if (warp == 1) {
@@ -400,7 +409,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     {
       const uint32_t idesc_s = idesc_bf16_f32(AT_BQ, AT_BK);
       const uint32_t q16 = (smem_u32(sq) & 0x3FFFFu) >> 4, k16 = (smem_u32(sk) & 0x3FFFFu) >> 4;
-#pragma unroll
+#pragma unroll 4
       for (int ks = 0; ks < 16; ++ks) {  // D = 256 in steps of 16: chunk ks/4, 32 bytes per step
         if ((ks & 3) == 0 && ok) {
           ok = __all_sync(0xffffffffu, wait_or_abort(&bars.qk_full[ks >> 2], 0, &bars.abort));
@@ -420,7 +429,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       // O[128 x 256] = P[128 x 128 keys] . V[keys x 256]: B operand N = D (MN-major), K = keys.
       const uint32_t idesc_o = idesc_bf16_f32(AT_BQ, dv) | (1u << 16);
       const uint32_t v_addr = smem_u32(sv);
-#pragma unroll
+#pragma unroll 2
       for (int ks = 0; ks < 8; ++ks) {  // 16 keys per step: 16 rows x 128 bytes inside every chunk
         const uint64_t bd = smem_desc_sw128_mn(v_addr + ks * 2048, AT_CHUNK);
         if (leader) umma_ts_bf16(t_o, t_p + ks * 8, bd, idesc_o, ks > 0 ? 1u : 0u);
@@ -436,6 +445,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       bars.abort = 1;
       if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_MMA);
       // the CTA stays until its copies, which may not have been waited for, have landed in its shared memory
+#pragma unroll 1
       for (int c = 0; c < 4; ++c) mbar_wait(&bars.qk_full[c], 0);
       mbar_wait(&bars.v_full, 0);
     }
@@ -461,28 +471,17 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       tmem_ld32(t_s + lane_addr + (hf * 2 + 1) * 32, v1);
       tc_wait_ld();
       const uint32_t b0 = bars.valid[hf * 2], b1 = bars.valid[hf * 2 + 1];
-      // per 32-key chunk: all valid -> no per-element selects; none valid -> nothing to do
-      if (b0 == 0xffffffffu) {
+      if ((b0 & b1) != 0xffffffffu) {  // a masked score becomes so small that its exponential is zero
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          mx = max3(mx, __uint_as_float(v0[e]), __uint_as_float(v0[e + 1]));
-          mx1 = max3(mx1, __uint_as_float(v0[e + 2]), __uint_as_float(v0[e + 3]));
+        for (int e = 0; e < 32; ++e) {
+          if (!((b0 >> e) & 1u)) v0[e] = __float_as_uint(PF_MASKED);
+          if (!((b1 >> e) & 1u)) v1[e] = __float_as_uint(PF_MASKED);
         }
-      } else if (b0 != 0u) {
-#pragma unroll
-        for (int e = 0; e < 32; ++e)
-          if ((b0 >> e) & 1u) mx = fmaxf(mx, __uint_as_float(v0[e]));
       }
-      if (b1 == 0xffffffffu) {
 #pragma unroll
-        for (int e = 0; e < 32; e += 4) {
-          mx = max3(mx, __uint_as_float(v1[e]), __uint_as_float(v1[e + 1]));
-          mx1 = max3(mx1, __uint_as_float(v1[e + 2]), __uint_as_float(v1[e + 3]));
-        }
-      } else if (b1 != 0u) {
-#pragma unroll
-        for (int e = 0; e < 32; ++e)
-          if ((b1 >> e) & 1u) mx = fmaxf(mx, __uint_as_float(v1[e]));
+      for (int e = 0; e < 32; e += 2) {
+        mx = max3(mx, __uint_as_float(v0[e]), __uint_as_float(v0[e + 1]));
+        mx1 = max3(mx1, __uint_as_float(v1[e]), __uint_as_float(v1[e + 1]));
       }
     }
     bars.hmax[hf][row] = fmaxf(mx, mx1);
@@ -490,32 +489,17 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const float m2 = fmaxf(bars.hmax[0][row], bars.hmax[1][row]) * p.scale_log2e;  // scale > 0
     float sum = 0.f;
     if (ok && live) {
+      const float base = fmaxf(m2, 0.5f * PF_MASKED * p.scale_log2e);  // a row whose keys are all masked: its exponentials stay zero
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
-        const uint32_t bits = bars.valid[hf * 2 + c];
         uint32_t pk[16];
-        if (bits == 0xffffffffu) {
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const float s0 = __uint_as_float(c == 0 ? v0[e] : v1[e]), s1 = __uint_as_float(c == 0 ? v0[e + 1] : v1[e + 1]);
-            const float p0 = pf_exp2(s0 * p.scale_log2e - m2), p1 = pf_exp2(s1 * p.scale_log2e - m2);
-            sum += p0 + p1;
-            const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
-            pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
-          }
-        } else if (bits == 0u) {
-#pragma unroll
-          for (int e = 0; e < 16; ++e) pk[e] = 0u;
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const float s0 = __uint_as_float(c == 0 ? v0[e] : v1[e]), s1 = __uint_as_float(c == 0 ? v0[e + 1] : v1[e + 1]);
-            const float p0 = ((bits >> e) & 1u) ? pf_exp2(s0 * p.scale_log2e - m2) : 0.f;
-            const float p1 = ((bits >> (e + 1)) & 1u) ? pf_exp2(s1 * p.scale_log2e - m2) : 0.f;
-            sum += p0 + p1;
-            const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
-            pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
-          }
+        for (int e = 0; e < 32; e += 2) {
+          const float s0 = __uint_as_float(c == 0 ? v0[e] : v1[e]), s1 = __uint_as_float(c == 0 ? v0[e + 1] : v1[e + 1]);
+          const float p0 = pf_exp2(s0 * p.scale_log2e - base), p1 = pf_exp2(s1 * p.scale_log2e - base);
+          sum += p0 + p1;
+          const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
+          pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
         }
         tmem_st16(t_p + lane_addr + (hf * 2 + c) * 16, pk);
       }
@@ -667,7 +651,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     float denom = 0.f;
 #pragma unroll
     for (int s = 0; s < AT_MAX_SPLITS; ++s) {
-      w[s] = s < p.nsplit ? exp2f(w_in[s] - mx) : 0.f;  // 0 for a block without valid keys
+      w[s] = s < p.nsplit ? pf_exp2(w_in[s] - mx) : 0.f;  // 0 for a block without valid keys
       denom += w[s] * l[s];
     }
     const float inv = denom > 0.f ? 1.0f / denom : 0.f;
@@ -715,6 +699,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     asm volatile("bar.sync 1, 256;" ::: "memory");
     if (tr && tid == 64) tr[7] = clock64();
     if (!bars.abort) {
+#pragma unroll 1
       for (int r = r0 + rsub; r < r1; r += rstep) {
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
         const int sw = c4 ^ (r & 7);
@@ -787,7 +772,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       float denom = 0.f;
 #pragma unroll
       for (int s = 0; s < AT_MAX_SPLITS; ++s) {
-        w[s] = s < p.nsplit ? exp2f(w[s] - mx) : 0.f;  // 0 for a block without valid keys
+        w[s] = s < p.nsplit ? pf_exp2(w[s] - mx) : 0.f;  // 0 for a block without valid keys
         denom += w[s] * l[s];
       }
       const float inv = denom > 0.f ? 1.0f / denom : 0.f;
@@ -910,7 +895,7 @@ __device__ __forceinline__ void pf_see_copies_land(Bars* b) {
 // 64..127 the others, two warps per sub-partition and 32 keys per thread.  The second half of P reaches its rows' lanes through shared memory, as
 // an operand of its own in the same sequence of products, so results are the same bit for bit.
 // 50 queries, 4146 keys, 24 heads: 52.0 -> 42.0 us (64 keys per thread on half of the warps: 43.8 us), 50 keys 6.9 -> 6.5 us.
-template <int HD, bool SHORT = false>
+template <int HD, bool SHORT, bool AIDS>
 __global__ void __launch_bounds__(AT_THREADS, 1)
 attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                          const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_kr,
@@ -920,7 +905,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   constexpr int KID = HD == 256 ? 5 : 6;
-  if (tid == 0) dbg_stage(p.dbg, KID, 0);
+  if (AIDS && tid == 0) dbg_stage(p.dbg, KID, 0);
   constexpr int NCH = HD / 64;              // 64-column chunks of a Q, K or V row
   constexpr int PF_BK = pf_bk(HD);          // keys per block
   constexpr int PF_KCHUNK = pf_kchunk(HD);
@@ -966,6 +951,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   }
   if (warp >= 2 && warp < 6) {  // validity bits of every key, 32 per word
     if (p.key_valid && p.pdl) pdl_wait();
+#pragma unroll 1
     for (int w = warp - 2; w < (PF_BK / 32) * nkb; w += 4) {
       const int j = w * 32 + lane;
       bool ok = j < p.Lk;
@@ -979,22 +965,24 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
   tc_fence_after();
   const uint32_t tmem = bars.tmem_base;
   const uint32_t t_o = tmem + 256;  // S_j (and P_j over it) at columns PF_BK * (j & 1)
-  if (tid == 0) dbg_stage(p.dbg, KID, 1);
-  long long* tr = p.trace ? p.trace + 16ll * ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) : nullptr;
-  const long long t_start = clock64();
+  if (AIDS && tid == 0) dbg_stage(p.dbg, KID, 1);
+  long long* tr = AIDS && p.trace ? p.trace + 16ll * ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) : nullptr;
+  const long long t_start = AIDS ? clock64() : 0;
   if (tr && tid == 0) tr[0] = t_start;
 
   if (warp == 0) {
     if (lane == 0) {
       if (p.pdl) pdl_launch_dependents();
       if (p.pdl) pdl_wait();
-      dbg_stage(p.dbg, KID, 2);
+      if (AIDS) dbg_stage(p.dbg, KID, 2);
       mbar_arrive_expect_tx(&bars.q_full, Q_TILE);
+#pragma unroll 1
       for (int c = 0; c < NCH; ++c) {
         tma_load_2d(sq + c * AT_CHUNK, &tm_q, &bars.q_full, h * HD + c * 64, b * p.L + qt * AT_BQ);
         if (SHORT) tma_load_2d(sq + c * AT_CHUNK + AT_CHUNK / 2, &tm_q, &bars.q_full, h * HD + c * 64, b * p.L);
       }
       int nk = 0, nv = 0;
+#pragma unroll 1
       for (int j = 0; j < nkb; ++j) {
         const int s = j & 1;
         const uint32_t par = ((j >> 1) & 1) ^ 1;  // the ring slot's previous use
@@ -1005,10 +993,12 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         const int krow = rows ? b * p.Lk + j * PF_BK : (b * p.G + g) * p.Lcap + (j - p.nb_rows) * PF_BK;
         if (j >= 2 && !wait_or_abort(&bars.k_empty[s], par, &bars.abort)) break;
         mbar_arrive_expect_tx(&bars.k_full[s], PF_KV);
+#pragma unroll 1
         for (int c = 0; c < NCH; ++c) tma_load_2d(sk + s * PF_KV + c * PF_KCHUNK, mk, &bars.k_full[s], kcol + c * 64, krow);
         nk = j + 1;
         if (j >= 2 && !wait_or_abort(&bars.v_empty[s], par, &bars.abort)) break;
         mbar_arrive_expect_tx(&bars.v_full[s], PF_KV);
+#pragma unroll 1
         for (int c = 0; c < NCH; ++c) tma_load_2d(sv + s * PF_KV + c * PF_KCHUNK, mv, &bars.v_full[s], kcol + c * 64, krow);
         nv = j + 1;
       }
@@ -1039,32 +1029,32 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
       }
       __syncwarp();
     };
-    if (ok) issue_s(0);
-    if (ok && nkb > 1) issue_s(1);
 #pragma unroll 1
-    for (int j = 0; j < nkb && ok; ++j) {
-      const int s = j & 1;
-      const uint32_t par = (j >> 1) & 1;
-      ok = __all_sync(0xffffffffu, wait_or_abort(&bars.p_full[s], par, &bars.abort) && wait_or_abort(&bars.v_full[s], par, &bars.abort));
-      if (!ok) break;
-      tc_fence_after();
-      const uint32_t v_addr = smem_u32(sv + s * PF_KV);
+    for (int j = -2; j < nkb && ok; ++j) {  // (the code that issues scores once)
+      if (j >= 0) {
+        const int s = j & 1;
+        const uint32_t par = (j >> 1) & 1;
+        ok = __all_sync(0xffffffffu, wait_or_abort(&bars.p_full[s], par, &bars.abort) && wait_or_abort(&bars.v_full[s], par, &bars.abort));
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t v_addr = smem_u32(sv + s * PF_KV);
 #pragma unroll
-      for (int ks = 0; ks < PF_BK / 16; ++ks) {  // 16 keys per step: 16 rows x 128 bytes inside every chunk
-        const uint64_t bd = smem_desc_sw128_mn(v_addr + ks * 2048, PF_KCHUNK);
-        if (SHORT && ks >= PF_BK / 32) {
-          const uint32_t p16 = (smem_u32(spk + s * AT_CHUNK) & 0x3FFFFu) >> 4;
-          if (leader) umma_ss_bf16(t_o, dk | (p16 + (ks & 3) * 2), bd, idesc_o, 1u);
-        } else {
-          if (leader) umma_ts_bf16(t_o, tmem + s * PF_BK + ks * 8, bd, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+        for (int ks = 0; ks < PF_BK / 16; ++ks) {  // 16 keys per step: 16 rows x 128 bytes inside every chunk
+          const uint64_t bd = smem_desc_sw128_mn(v_addr + ks * 2048, PF_KCHUNK);
+          if (SHORT && ks >= PF_BK / 32) {
+            const uint32_t p16 = (smem_u32(spk + s * AT_CHUNK) & 0x3FFFFu) >> 4;
+            if (leader) umma_ss_bf16(t_o, dk | (p16 + (ks & 3) * 2), bd, idesc_o, 1u);
+          } else {
+            if (leader) umma_ts_bf16(t_o, tmem + s * PF_BK + ks * 8, bd, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
+          }
         }
+        if (leader) {
+          tc_commit(&bars.v_empty[s]);
+          tc_commit(&bars.o_done);
+          if (j == nkb - 1) tc_commit(&bars.all_done);
+        }
+        __syncwarp();
       }
-      if (leader) {
-        tc_commit(&bars.v_empty[s]);
-        tc_commit(&bars.o_done);
-        if (j == nkb - 1) tc_commit(&bars.all_done);
-      }
-      __syncwarp();
       if (j + 2 < nkb) issue_s(j + 2);  // over P_j, which the product just issued reads first
     }
     // nothing of this CTA's tensor work may be in flight when it gives up its tensor memory
@@ -1129,16 +1119,15 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         tc_wait_ld();
 #pragma unroll
         for (int w = 0; w < KW; ++w) {
-          if (bits[w] == 0xffffffffu) {  // two chains of three-way maxima: the warp has nothing else to do meanwhile
-#pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-              mx = max3(mx, __uint_as_float(v[w][e]), __uint_as_float(v[w][e + 1]));
-              mx1 = max3(mx1, __uint_as_float(v[w][e + 2]), __uint_as_float(v[w][e + 3]));
-            }
-          } else if (bits[w] != 0u) {
+          if (bits[w] != 0xffffffffu) {
 #pragma unroll
             for (int e = 0; e < 32; ++e)
-              if ((bits[w] >> e) & 1u) mx = fmaxf(mx, __uint_as_float(v[w][e]));
+              if (!((bits[w] >> e) & 1u)) v[w][e] = __float_as_uint(PF_MASKED);
+          }
+#pragma unroll
+          for (int e = 0; e < 32; e += 4) {  // two chains of three-way maxima: the warp has nothing else to do meanwhile
+            mx = max3(mx, __uint_as_float(v[w][e]), __uint_as_float(v[w][e + 1]));
+            mx1 = max3(mx1, __uint_as_float(v[w][e + 2]), __uint_as_float(v[w][e + 3]));
           }
         }
       }
@@ -1183,6 +1172,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         }
       }
       if (ok && slive) {
+        const float base = fmaxf(m_ref, 0.5f * PF_MASKED * p.scale_log2e);
         float sum = 0.f;
         auto add = [&](int e, float two) {
           if (SHORT && hf) tail[SHORT ? e >> 1 : 0] = two;
@@ -1191,30 +1181,13 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
 #pragma unroll
         for (int w = 0; w < KW; ++w) {
           uint32_t pk[16];
-          if (bits[w] == 0xffffffffu) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 2) {
-              const float p0 = pf_exp2(__uint_as_float(v[w][e]) * p.scale_log2e - m_ref);
-              const float p1 = pf_exp2(__uint_as_float(v[w][e + 1]) * p.scale_log2e - m_ref);
-              add(e, p0 + p1);
-              const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
-              pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
-            }
-          } else if (bits[w] == 0u) {
-#pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              pk[e] = 0u;
-              add(2 * e, 0.f);
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 32; e += 2) {
-              const float p0 = ((bits[w] >> e) & 1u) ? pf_exp2(__uint_as_float(v[w][e]) * p.scale_log2e - m_ref) : 0.f;
-              const float p1 = ((bits[w] >> (e + 1)) & 1u) ? pf_exp2(__uint_as_float(v[w][e + 1]) * p.scale_log2e - m_ref) : 0.f;
-              add(e, p0 + p1);
-              const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
-              pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
-            }
+          for (int e = 0; e < 32; e += 2) {
+            const float p0 = pf_exp2(__uint_as_float(v[w][e]) * p.scale_log2e - base);
+            const float p1 = pf_exp2(__uint_as_float(v[w][e + 1]) * p.scale_log2e - base);
+            add(e, p0 + p1);
+            const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
+            pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
           }
           // P_j as bf16 pairs over the start of S_j: 16 columns per 32 keys (every thread of the row
           // has read its scores before the named barrier above)
@@ -1257,7 +1230,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     // row cost two more barriers: 4146 x 129 keys x 24 heads 51.8 -> 48.6 us.  What is left, 7500 clocks at head_dim 256,
     // is the conversions of the plane split.)
     if (tr && tid == 128) tr[13] = clock64();
-    if (tid == 64) dbg_stage(p.dbg, KID, 3);
+    if (AIDS && tid == 64) dbg_stage(p.dbg, KID, 3);
     tc_fence_before();
     asm volatile("bar.sync 1, 256;" ::: "memory");  // both halves' sums
     if (!bars.abort && live) {  // warp-uniform: the tensor-memory loads below are warp-wide
@@ -1308,7 +1281,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     tc_fence_after();
     tmem_dealloc(tmem, T_COLS);
   }
-  if (tid == 0) dbg_stage(p.dbg, KID, 4);
+  if (AIDS && tid == 0) dbg_stage(p.dbg, KID, 4);
 }
 
 }  // namespace tb
@@ -1531,7 +1504,7 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             for (int w = 0; w < 4; ++w)
 #pragma unroll
               for (int e = 0; e < 32; ++e)
-                if (!((bits[w] >> e) & 1u)) v[w][e] = __float_as_uint(-1e30f);
+                if (!((bits[w] >> e) & 1u)) v[w][e] = __float_as_uint(PF_MASKED);
           }
           float mx0 = -1e30f, mx1 = -1e30f, mx2 = -1e30f, mx3 = -1e30f;
 #pragma unroll
@@ -1560,7 +1533,7 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             }
             if (grow) m_ref = m_blk;
           }
-          const float base = fmaxf(m_ref, -1e29f);  // an all-masked row so far: exponentials of -1e30 stay zero
+          const float base = fmaxf(m_ref, 0.5f * PF_MASKED * p.scale_log2e);  // (a row that has seen masked keys only)
           const uint64_t nm = f32x2(-base, -base);
           uint64_t sum0 = f32x2(0.f, 0.f), sum1 = sum0;
 #pragma unroll
@@ -1652,11 +1625,22 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 }  // namespace tb
 
 namespace tb {
+using AtKernel = void(const CUtensorMap, const CUtensorMap, const CUtensorMap, const AttnParams);
+static AtKernel* at_kernel(bool push, bool aids) {
+  return push ? (aids ? attention_kernel<true, true> : attention_kernel<true, false>)
+              : (aids ? attention_kernel<false, true> : attention_kernel<false, false>);
+}
+using PfKernel = void(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const AttnParams);
+static PfKernel* pf_kernel(int D, bool short_form, bool aids) {
+  if (short_form) return aids ? attention_prefill_kernel<128, true, true> : attention_prefill_kernel<128, true, false>;
+  if (D == 128) return aids ? attention_prefill_kernel<128, false, true> : attention_prefill_kernel<128, false, false>;
+  return aids ? attention_prefill_kernel<256, false, true> : attention_prefill_kernel<256, false, false>;
+}
 // Clusters of `nsplit` attention CTAs (one CTA per SM) that the device holds at once.
 static int at_resident_clusters(int nsplit) {
   static host::DeviceCache cache[AT_MAX_SPLITS + 1];
   return host::per_device(cache[nsplit], [nsplit] {
-    cudaFuncSetAttribute(attention_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM);
+    cudaFuncSetAttribute(attention_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(nsplit);
     cfg.blockDim = dim3(AT_THREADS);
@@ -1669,7 +1653,7 @@ static int at_resident_clusters(int nsplit) {
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, attention_kernel<false>, &cfg) != cudaSuccess || n <= 0) {
+    if (cudaOccupancyMaxActiveClusters(&n, attention_kernel<false, false>, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = host::sm_count() / (nsplit + 1);
     }
@@ -1706,9 +1690,13 @@ static int at_set_attributes() {
   static host::DeviceCache cache;
   const bool done = host::per_device(cache, [] {
     const auto set = [](auto* kernel, int bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; };
-    return static_cast<int>(set(attention_kernel<false>, AT_SMEM) && set(attention_kernel<true>, AT_SMEM) && set(attention_two_tile_kernel, TT_SMEM) &&
-                            set(attention_prefill_kernel<256>, pf_smem(256)) && set(attention_prefill_kernel<128, true>, PF_SMEM_SHORT) &&
-                            set(attention_prefill_kernel<128>, pf_smem(128)));
+    bool ok = set(attention_two_tile_kernel, TT_SMEM);
+    for (int aids = 0; aids < 2; ++aids) {
+      ok = ok && set(at_kernel(false, aids), AT_SMEM) && set(at_kernel(true, aids), AT_SMEM);
+      ok = ok && set(pf_kernel(256, false, aids), pf_smem(256)) && set(pf_kernel(128, true, aids), PF_SMEM_SHORT) &&
+           set(pf_kernel(128, false, aids), pf_smem(128));
+    }
+    return static_cast<int>(ok);
   });
   return done ? TYBOK_OK : host::fail_cuda("cudaFuncSetAttribute(attention kernels)");
 }
@@ -1892,10 +1880,10 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
   if (two_tile)
     e = cudaLaunchKernelEx(&cfg, attention_two_tile_kernel, tm_q, tm_k, tm_v, p);
   else if (prefill)
-    e = cudaLaunchKernelEx(&cfg, short_form ? attention_prefill_kernel<128, true> : D == 128 ? attention_prefill_kernel<128> : attention_prefill_kernel<256>,
+    e = cudaLaunchKernelEx(&cfg, pf_kernel(D, short_form, p.trace || p.dbg),
                            tm_q, tm_k, tm_v, tm_k, tm_v, p);
   else
-    e = cudaLaunchKernelEx(&cfg, push ? attention_kernel<true> : attention_kernel<false>, tm_q, tm_k, tm_v, p);
+    e = cudaLaunchKernelEx(&cfg, at_kernel(push, p.trace != nullptr), tm_q, tm_k, tm_v, p);
   if (e != cudaSuccess)
     return host::fail_cuda("launch attention_kernel");
   host::count_launch();
@@ -1954,7 +1942,7 @@ int tybok_attention_rows(const void* q, const void* k_rows, const void* v_rows, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = p.pdl;
-  if (cudaLaunchKernelEx(&cfg, short_form ? attention_prefill_kernel<128, true> : attention_prefill_kernel<128>, tm_q, tm_k, tm_v, tm_kr, tm_vr, p) !=
+  if (cudaLaunchKernelEx(&cfg, pf_kernel(128, short_form, p.trace || p.dbg), tm_q, tm_k, tm_v, tm_kr, tm_vr, p) !=
       cudaSuccess)
     return host::fail_cuda("launch attention_prefill_kernel");
   host::count_launch();
