@@ -564,6 +564,8 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       if (p.status) atomicCAS(p.status, 0, TYBOK_DEV_TIMEOUT_EPILOGUE);
     }
     if (PUSH) {
+      tc_fence_before();
+      asm volatile("bar.arrive 2, 288;" ::: "memory");  // to the MMA warp: nobody reads tensor memory any more
       // Send every peer the staged partial rows it merges: one bulk copy per peer, one lane each.
       fence_proxy_async();  // the staging stores, for the bulk copy engine
       asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -605,6 +607,11 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   if (tr && tid == 64) tr[5] = clock64();
   tc_fence_before();
   if (PUSH) {
+    if (warp == 1) {
+      asm volatile("bar.sync 2, 288;" ::: "memory");
+      tc_fence_after();
+      tmem_dealloc(tmem, 512);
+    }
     if (warp < 2) {  // the two service warps only keep the cluster barrier's books
       cluster_wait_acquire();
       cluster_arrive_release();
@@ -808,7 +815,10 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
   // Pull form: nothing after the meeting point touches a peer's shared memory, CTAs leave on
   // their own.  Push form: a CTA stays until every peer holds the rows it was sent, which is
   // when the copies have finished reading this CTA's shared memory.
-  if (PUSH) cluster_wait_acquire();
+  if (PUSH) {
+    cluster_wait_acquire();
+    return;  // the tensor memory was given back beside the exchange
+  }
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();

@@ -559,6 +559,12 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
 
   if (tr && tid == 64) tr[6] = clock64();
   if (ANY && tid == 0) dbg_stage(p.dbg, KID, 3);
+  // After the meeting point nobody touches another CTA's shared memory, nor tensor memory: it is given back here, beside the last
+  // stage, and the warps leave on their own.
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, p.tmem_cols);
+  }
   if (warp >= 2 && !bars.abort) {
     // ---------------------------------------------------------- epilogue, phase B
     // 4 consecutive channels per thread, 8 token rows per pass; with split-K, rank r owns token
@@ -677,8 +683,12 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           for (int e = 0; e < 4; ++e) o[e] = bf16_round(o[e] * gv[e]);
         }
         const int u = (rl - rgrp) / EW;
-        const uint2 rr = u < 4 ? res_pf[u < 4 ? u : 0]
-                               : *reinterpret_cast<const uint2*>(p.res + static_cast<long long>(m) * p.ldres + n);
+        uint2 rr;  // (an index would put the array into local memory, which the meeting point's acquire throws out of L1)
+        if (u == 0) rr = res_pf[0];
+        else if (u == 1) rr = res_pf[1];
+        else if (u == 2) rr = res_pf[2];
+        else if (u == 3) rr = res_pf[3];
+        else rr = *reinterpret_cast<const uint2*>(p.res + static_cast<long long>(m) * p.ldres + n);
         const __nv_bfloat162 r01 = *reinterpret_cast<const __nv_bfloat162*>(&rr.x);
         const __nv_bfloat162 r23 = *reinterpret_cast<const __nv_bfloat162*>(&rr.y);
         o[0] += __bfloat162float(r01.x); o[1] += __bfloat162float(r01.y);
@@ -719,12 +729,6 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   }
 
   if (tr && tid == 64) tr[7] = clock64();
-  // After the meeting point nobody touches another CTA's shared memory: CTAs leave on their own.
-  __syncthreads();
-  if (warp == 1) {
-    tc_fence_after();
-    tmem_dealloc(tmem, p.tmem_cols);
-  }
   if (ANY && tid == 0) dbg_stage(p.dbg, KID, 4);
 }
 
