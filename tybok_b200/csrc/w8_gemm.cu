@@ -153,7 +153,31 @@ __device__ __forceinline__ float deferred_rstd(const float* part, int tiles, int
   }
   return rsqrtf(t * inv_w + eps);
 }
-// The same out of line, for the rows that a thread finishes after its first.
+// Gate values of four channels of token m (rounded to bf16), and where the q / k / v tile of head slot `slot` stores token m.
+__device__ __forceinline__ float4 gate_of(const void* gate, int bf16, long long ldgate, int rows_per_gate, int m, int n) {
+  const long long gi = static_cast<long long>(m / rows_per_gate) * ldgate + n;
+  if (bf16) {
+    const uint2 g = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(gate) + gi);
+    return make_float4(__uint_as_float(g.x << 16), __uint_as_float(g.x & 0xffff0000u), __uint_as_float(g.y << 16),
+                       __uint_as_float(g.y & 0xffff0000u));
+  }
+  const float4 g = *reinterpret_cast<const float4*>(static_cast<const float*>(gate) + gi);
+  return make_float4(bf16_round(g.x), bf16_round(g.y), bf16_round(g.z), bf16_round(g.w));
+}
+__device__ __forceinline__ __nv_bfloat16* rope_row(__nv_bfloat16* q, __nv_bfloat16* kc, __nv_bfloat16* vc, int H, int G, int D, int L, int Lcap,
+                                                   int key_off, int slot, int m) {
+  if (slot < H) return q + (static_cast<long long>(m) * H + slot) * D;
+  const int g = (slot - H) % G, b = m / L, t = m - b * L;
+  return (slot < H + G ? kc : vc) + ((static_cast<long long>(b) * G + g) * Lcap + key_off + t) * D;
+}
+// The same three out of line, for the rows that a thread finishes after its first.
+__device__ __noinline__ float4 gate_of_again(const void* gate, int bf16, long long ldgate, int rows_per_gate, int m, int n) {
+  return gate_of(gate, bf16, ldgate, rows_per_gate, m, n);
+}
+__device__ __noinline__ __nv_bfloat16* rope_row_again(__nv_bfloat16* q, __nv_bfloat16* kc, __nv_bfloat16* vc, int H, int G, int D, int L, int Lcap,
+                                                      int key_off, int slot, int m) {
+  return rope_row(q, kc, vc, H, G, D, L, Lcap, key_off, slot, m);
+}
 __device__ __noinline__ float deferred_rstd_again(const float* part, int tiles, int M, float inv_w, float eps, int m) {
   return deferred_rstd(part, tiles, M, inv_w, eps, m);
 }
@@ -239,8 +263,12 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   float nsc[4] = {0, 0, 0, 0};  // 1 + scale of the next norm for this thread's channels (producer form)
   float rs_pf = 1.0f;           // deferred norm: rstd of this thread's first token row
   uint2 res_pf[4] = {};  // residual of this thread's first four token rows, fetched early
-  float4 gate_pf = make_float4(0.f, 0.f, 0.f, 0.f);  // gate values of the first token row's group (fp32 form)
-  int gate_pf_group = -1;
+  // What the last stage needs beside the sums is worked out for a thread's first row (mostly its only one) while the products
+  // run: gate values, and where the rotary form stores.  (Divisions and a load on the way from the meeting point to the stores;
+  // with the owners' addresses below, 50-token MLP 12.58 -> 12.42 us, DiT runner 3.67 -> 3.64 ms.)
+  float4 gate_pf = make_float4(1.f, 1.f, 1.f, 1.f);
+  int rope_slot = 0, rope_d = 0;
+  __nv_bfloat16* rope_dst = nullptr;
   // Split-K ownership: pairs of the tile's token rows go round the cluster ranks.  Row rl of a rank is token_of(rl).  (Blocks
   // of rows, a warp's 16 tokens straddling up to three owners, took an epilogue thread over 200 instructions to send.)
   const int m_base = t_tile * p.bt;
@@ -395,17 +423,18 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         if (is(EPI_RESIDUAL) && p.gate && !p.gate_bf16) {
           // fp32 gates are per-step constants (precomputed modulations), touched once per chunk
           // and therefore cold in L2: fetch them now, not between the accumulator and the stores.
-          gate_pf_group = (m_base + 2 * rank) / p.rows_per_gate;
-          gate_pf = *reinterpret_cast<const float4*>(static_cast<const float*>(p.gate) +
-                                                     static_cast<long long>(gate_pf_group) * p.ldgate + n);
+          gate_pf = gate_of(p.gate, 0, p.ldgate, p.rows_per_gate, min(m_base + token_of((tid - 64) >> 5), p.M - 1), n);
         }
         if (is(EPI_QKV_ROPE)) {
           // Positions and tables are constants: fetch the cos/sin of this thread's first row now.
           const RopeEpi& r = p.rope;
-          const int tps = r.D >> 7;
+          const int tps = r.D >> 7;  // 128-row tiles per head slot
+          rope_slot = n_tile / tps;
+          rope_d = (n_tile - rope_slot * tps) * 64 + col0;
           const int rl = ((tid - 64) >> 5) * 2 + (v4p >> 4);
-          if (token_of(rl) < nvalid && n_tile / tps < r.H + r.G) {
-            const long long tb = static_cast<long long>(r.pos[m_base + token_of(rl)]) * r.D + (n_tile % tps) * 64 + col0;
+          rope_dst = rope_row(r.q, r.kcache, r.vcache, r.H, r.G, r.D, r.L, r.Lcap, r.key_off, rope_slot, m_base + token_of(rl));
+          if (token_of(rl) < nvalid && rope_slot < r.H + r.G) {
+            const long long tb = static_cast<long long>(r.pos[m_base + token_of(rl)]) * r.D + rope_d;
             res_pf[0] = *reinterpret_cast<const uint2*>(r.cos + tb);
             res_pf[1] = *reinterpret_cast<const uint2*>(r.cos + tb + (r.D >> 1));
             res_pf[2] = *reinterpret_cast<const uint2*>(r.sin + tb);
@@ -422,6 +451,8 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
           const int rl = packed ? ((tid - 64) >> 5) * 2 + (v4p >> 4) : (tid - 64) >> 5;
           if (token_of(rl) < nvalid) rs_pf = deferred_rstd(p.dn_part, p.dn_tiles, p.M, p.dn_inv_w, p.dn_eps, m_base + token_of(rl));
         }
+        if (is(EPI_RESIDUAL) && p.gate && p.gate_bf16)  // an input like the rows, maybe the previous kernel's
+          gate_pf = gate_of(p.gate, 1, p.ldgate, p.rows_per_gate, min(m_base + token_of((tid - 64) >> 5), p.M - 1), n);
         if (is(EPI_RESIDUAL)) {
           // The residual was written by an earlier kernel: fetch the rows this thread will finish
           // first, long before the accumulator is ready.
@@ -482,6 +513,23 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     // this phase of the cluster barrier says so.  Each warp arrives where it waits for something else anyway, and the
     // accumulator is not complete yet here.  (50-token MLP 14.59 -> 14.64 us; 1 x 2560 x 2048, whose epilogue warps are
     // busy until here, 6.39 -> 6.52 us; arrivals at the kernel's start cost twice that.)
+    // Where this warp's first 16 rows go: pairs of them to the owners in turn (0: past the tile's end).
+    const uint32_t stage_addr = smem_u32(smem + p.stage_off);
+    uint32_t peer[8];
+    auto peers = [&](int g) {
+      int lr = (g * 8) / p.splits, owner = g * 8 - lr * p.splits;
+      const uint32_t slot = stage_addr + ((split * nw * rpr) * BN + row) * 4;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        peer[e] = g * 16 + 2 * e < nvalid ? dsmem_addr(slot + lr * (2 * BN * 4), owner) : 0u;
+        if (++owner == p.splits) {
+          owner = 0;
+          ++lr;
+        }
+      }
+    };
+    constexpr bool AHEAD = FORM != FORM_BF16;  // (warps that make planes have no time to spare here)
+    if (AHEAD && p.splits > 1 && half * 16 < nvalid) peers(half);
     if (EW == EPI_WARPS_WIDE && p.splits > 1) cluster_wait_acquire();
     bool ok = __all_sync(0xffffffffu, wait_or_abort(&bars.tmem_full, 0, &bars.abort, p.epi_wait_limit));
     if (!ok && lane == 0) fail(&bars, p.status, TYBOK_DEV_TIMEOUT_EPILOGUE);
@@ -492,7 +540,6 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
       // (slot [split][w][row within owner][128 channels], through distributed shared memory when
       // the owner is another rank), so that after the meeting point each owner only reads its
       // own shared memory.
-      const uint32_t stage_addr = smem_u32(smem + p.stage_off);
       const int ngroups = (nvalid + 15) / 16;
       const int acc_cols = p.mma_n;
       for (int w = 0; w < nw; ++w) {
@@ -524,21 +571,13 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
             for (int e = 0; e < 16; ++e)
               if (g * 16 + e < nvalid) dst[e * BN] = __uint_as_float(v[e]);
           } else {
-            // Two rows per owner in turn: one address translation and two stores.
-            const int t0 = g * 16;
-            int lr = (g * 8) / p.splits, owner = g * 8 - lr * p.splits;
-            const uint32_t slot = stage_addr + (((split * nw + w) * rpr) * BN + row) * 4;
+            if (!AHEAD || g != half) peers(g);
 #pragma unroll
-            for (int e = 0; e < 16; e += 2) {
-              if (t0 + e < nvalid) {
-                const uint32_t dst = dsmem_addr(slot + lr * (2 * BN * 4), owner);
-                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(__uint_as_float(v[e])));
-                if (t0 + e + 1 < nvalid) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + BN * 4), "f"(__uint_as_float(v[e + 1])));
-              }
-              if (++owner == p.splits) {
-                owner = 0;
-                ++lr;
-              }
+            for (int e = 0; e < 8; ++e) {
+              const uint32_t dst = peer[e] + w * rpr * (BN * 4);
+              if (peer[e]) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst), "f"(__uint_as_float(v[2 * e])));
+              if (g * 16 + 2 * e + 1 < nvalid)
+                asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + BN * 4), "f"(__uint_as_float(v[2 * e + 1])));
             }
           }
         }
@@ -624,11 +663,8 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         const RopeEpi& r = p.rope;
         float u[4] = {bf16_round(a1.x * s1[0] + b1[0]), bf16_round(a1.y * s1[1] + b1[1]),
                       bf16_round(a1.z * s1[2] + b1[2]), bf16_round(a1.w * s1[3] + b1[3])};
-        const int tps = r.D >> 7;  // 128-row tiles per head slot
-        const int slot = n_tile / tps;
-        const int d = (n_tile - slot * tps) * 64 + col0;
-        const int half = r.D >> 1;
-        if (slot < r.H + r.G) {
+        const int d = rope_d, half = r.D >> 1;
+        if (rope_slot < r.H + r.G) {
           uint2 c0 = res_pf[0], c1 = res_pf[1], n0 = res_pf[2], n1 = res_pf[3];
           if (rl != row0) {
             const long long tb = static_cast<long long>(r.pos[m]) * r.D + d;
@@ -646,15 +682,8 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
             u[e] = rope1(hi, lo, __bfloat162float(pc1[e]), __bfloat162float(pn1[e]));
           }
         }
-        __nv_bfloat16* dst;
-        if (slot < r.H) {
-          dst = r.q + (static_cast<long long>(m) * r.H + slot) * r.D;
-        } else {
-          const int g = (slot - r.H) % r.G;
-          const int b = m / r.L, t = m - b * r.L;
-          dst = (slot < r.H + r.G ? r.kcache : r.vcache) +
-                ((static_cast<long long>(b) * r.G + g) * r.Lcap + r.key_off + t) * r.D;
-        }
+        __nv_bfloat16* dst = rl == row0 ? rope_dst
+                                       : rope_row_again(r.q, r.kcache, r.vcache, r.H, r.G, r.D, r.L, r.Lcap, r.key_off, rope_slot, m);
         const __nv_bfloat162 l01 = __floats2bfloat162_rn(o[0], o[1]), l23 = __floats2bfloat162_rn(o[2], o[3]);
         const __nv_bfloat162 h01 = __floats2bfloat162_rn(u[0], u[1]), h23 = __floats2bfloat162_rn(u[2], u[3]);
         uint2 st;
@@ -665,20 +694,8 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
         continue;
       } else if (is(EPI_RESIDUAL)) {
         if (p.gate) {
-          const long long gi = static_cast<long long>(m / p.rows_per_gate) * p.ldgate + n;
-          float gv[4];
-          if (p.gate_bf16) {
-            const uint2 gr = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(p.gate) + gi);
-            const __nv_bfloat162 g01 = *reinterpret_cast<const __nv_bfloat162*>(&gr.x);
-            const __nv_bfloat162 g23 = *reinterpret_cast<const __nv_bfloat162*>(&gr.y);
-            gv[0] = __bfloat162float(g01.x); gv[1] = __bfloat162float(g01.y);
-            gv[2] = __bfloat162float(g23.x); gv[3] = __bfloat162float(g23.y);
-          } else {
-            const float4 gr = m / p.rows_per_gate == gate_pf_group
-                                  ? gate_pf
-                                  : *reinterpret_cast<const float4*>(static_cast<const float*>(p.gate) + gi);
-            gv[0] = bf16_round(gr.x); gv[1] = bf16_round(gr.y); gv[2] = bf16_round(gr.z); gv[3] = bf16_round(gr.w);
-          }
+          const float4 gr = rl == row0 ? gate_pf : gate_of_again(p.gate, p.gate_bf16, p.ldgate, p.rows_per_gate, m, n);
+          const float gv[4] = {gr.x, gr.y, gr.z, gr.w};
 #pragma unroll
           for (int e = 0; e < 4; ++e) o[e] = bf16_round(o[e] * gv[e]);
         }
