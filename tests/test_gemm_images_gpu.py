@@ -23,7 +23,8 @@ def _same(a, b):
 # one token, odd counts, a tile's last row pair half empty, fewer row pairs than CTAs, two tiles of which the second is shorter
 @pytest.mark.parametrize("m", [1, 7, 17, 21, 33, 50, 64, 79, 81, 106, 127])
 @pytest.mark.parametrize("splits", [1, 2, 3, 5, 8])
-def test_same_bits_as_a_forced_tile_and_the_general_image(m, splits):
+@pytest.mark.parametrize("planes", [2, 3])
+def test_same_bits_as_a_forced_tile_and_the_general_image(m, splits, planes):
     from tybok_b200 import ops
 
     n, k = 640, 1152  # a channel tile count that is odd, nine K blocks
@@ -31,16 +32,20 @@ def test_same_bits_as_a_forced_tile_and_the_general_image(m, splits):
     rnd = lambda *s: torch.empty(*s, device="cuda").normal_(0, 1, generator=g).to(torch.bfloat16)  # noqa: E731
     xp, (w8, sc) = ops.split3(rnd(m, k), 4), _weights(n, k, 3)
     res, gate, bias = rnd(m, n), rnd(m, n), rnd(n)
-    calls = [lambda t: ops.w8x3_linear(xp, 4, w8, sc, bias, token_tile=t, splits=splits),
-             lambda t: ops.w8x3_linear(xp, 4, w8, sc, epilogue=ops.EPI_GELU, out_planes=True, token_tile=t, splits=splits),
-             lambda t: ops.w8x3_linear(xp, 4, w8, sc, epilogue=ops.EPI_RESIDUAL, residual=res, gate=gate.float(), rows_per_gate=1, token_tile=t,
-                                       splits=splits),
-             lambda t: ops.w8x3_geglu_packed(xp, 4, w8, sc, out_planes=True, token_tile=t, splits=splits)]
+    xp2, rs = ops.norm_planes2(rnd(m, k), ops.NORM_RMS, torch.zeros(k, device="cuda"))
+    lin = (lambda **kw: ops.w8x3_linear(xp, 4, w8, sc, **kw)) if planes == 3 else (lambda **kw: ops.w8x2_gemm(xp2, rs, w8, sc, **kw))
+    gated = (lambda **kw: ops.w8x3_geglu_packed(xp, 4, w8, sc, **kw)) if planes == 3 else (
+        lambda **kw: ops.w8x2_gemm(xp2, rs, w8, sc, epilogue=ops.EPI_GEGLU_PACKED, **kw))
+    calls = [lambda t: lin(bias=bias, token_tile=t, splits=splits),
+             lambda t: lin(epilogue=ops.EPI_GELU, out_planes=True, token_tile=t, splits=splits),
+             lambda t: lin(epilogue=ops.EPI_RESIDUAL, residual=res, gate=gate.float(), rows_per_gate=1, token_tile=t, splits=splits),
+             lambda t: gated(out_planes=True, token_tile=t, splits=splits)]
     counters = torch.zeros(16 * 8, dtype=torch.int32, device="cuda")
     lib = ops._lib.load()
     for call in calls:
         y = call(0)
-        assert _same(y, call(64 if m > 64 else (m + 15) // 16 * 16))
+        cap = 64 if planes == 3 else 128
+        assert _same(y, call(cap if m > cap else (m + 15) // 16 * 16))
         lib.tybok_debug_set_counters(counters.data_ptr())
         try:
             general = call(0)

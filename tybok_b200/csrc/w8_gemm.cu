@@ -188,12 +188,12 @@ __device__ __noinline__ float deferred_rstd_again(const float* part, int tiles, 
 // (accumulator groups to push, rows to finish): sixteen warps halve both.
 // FORM, EPI: what an image is compiled for.  A CTA runs this code once, so a launch waits for its instructions (over 2000 of a
 // launch's 10000 clk), and chains of small launches alternate between images that should all stay in the instruction cache.
-// So the forms that such chains consist of (one weight matrix, three planes in columns of their own; and the one that makes its
-// planes) have images of a third to a half of the size, without the others' code and the tuning aids, which run in the image that
+// So the forms that such chains consist of (one weight matrix, three or two planes in columns of their own; and the one that makes
+// its planes) have images of a third to a half of the size, without the others' code and the tuning aids, which run in the image that
 // takes every form.  One image per epilogue is no better than one for none, GELU and residual together: 50-token MLP 12.7
 // against 12.9 us, but DiT block chains 3.84 against 3.71 ms.  With the row pairs and tiles below, batch-1 chunk 9.90 -> 9.22 ms,
 // 50-token MLP 14.6 -> 12.9 us, DiT runner 4.00 -> 3.72 ms, denoiser at 106 tokens 16.2 -> 14.6 ms, 1 x 2560 x 2048 6.5 -> 5.4 us.
-enum : int { FORM_ANY = 0, FORM_PLANES3 = 1, FORM_BF16 = 2, EPI_ANY = -1, EPI_LINEAR = -2 };  // (LINEAR: none, GELU or residual)
+enum : int { FORM_ANY = 0, FORM_PLANES3 = 1, FORM_BF16 = 2, FORM_PLANES2 = 3, EPI_ANY = -1, EPI_LINEAR = -2 };  // (LINEAR: none, GELU or residual)
 template <int EW, int FORM, int EPI>
 __global__ void __launch_bounds__(32 * (2 + EW), EW == EPI_WARPS ? 2 : 1)
 w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
@@ -203,7 +203,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
 
   constexpr bool ANY = FORM == FORM_ANY;
   auto is = [&](int e) { return EPI == EPI_ANY ? p.epi == e : EPI == EPI_LINEAR ? e <= EPI_RESIDUAL && p.epi == e : e == EPI; };
-  const int np = ANY ? p.np : 3, nw = ANY ? p.nw : 1;
+  const int np = ANY ? p.np : FORM == FORM_PLANES2 ? 2 : 3, nw = ANY ? p.nw : 1;
   const bool merge = ANY ? p.merge : true, xb = ANY ? p.xb != nullptr : FORM == FORM_BF16;
   const long long t_start = ANY ? clock64() : 0;
   const int tid = threadIdx.x;
@@ -276,7 +276,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   const int rpr = 2 * (((nvalid + 1) / 2 + p.splits - 1) / p.splits);
   const int rank = p.splits > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   auto token_of = [&](int rl) { return 2 * ((rl >> 1) * p.splits + rank) + (rl & 1); };
-  const float* const row_scale = ANY ? p.row_scale : nullptr;
+  const float* const row_scale = ANY || FORM == FORM_PLANES2 ? p.row_scale : nullptr;
   long long* tr = ANY && p.trace ? p.trace + 16ll * ((blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) : nullptr;
   if (tr && tid == 0) { tr[0] = t_start; tr[1] = clock64(); }
 
@@ -948,13 +948,15 @@ struct NormFold {
 };
 
 using GemmKernel = void(const CUtensorMap, const CUtensorMap, const CUtensorMap, const GemmParams);
-static GemmKernel* lean_kernel(int epi) {
+template <int FORM>
+static GemmKernel* lean_kernel_of(int epi) {
   switch (epi) {
-    case EPI_GEGLU_PACKED: return w8_gemm_kernel<EPI_WARPS_WIDE, FORM_PLANES3, EPI_GEGLU_PACKED>;
-    case EPI_QKV_ROPE: return w8_gemm_kernel<EPI_WARPS_WIDE, FORM_PLANES3, EPI_QKV_ROPE>;
-    default: return w8_gemm_kernel<EPI_WARPS_WIDE, FORM_PLANES3, EPI_LINEAR>;
+    case EPI_GEGLU_PACKED: return w8_gemm_kernel<EPI_WARPS_WIDE, FORM, EPI_GEGLU_PACKED>;
+    case EPI_QKV_ROPE: return w8_gemm_kernel<EPI_WARPS_WIDE, FORM, EPI_QKV_ROPE>;
+    default: return w8_gemm_kernel<EPI_WARPS_WIDE, FORM, EPI_LINEAR>;
   }
 }
+static GemmKernel* lean_kernel(int epi, int np) { return np == 2 ? lean_kernel_of<FORM_PLANES2>(epi) : lean_kernel_of<FORM_PLANES3>(epi); }
 
 static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, const float* s0, const float* s1,
                        const void* bias, void* y, void* y_planes, int M, int N, int K, long long ldy, int epi,
@@ -1069,7 +1071,9 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   if (!host::per_device(attr_set, [] {
         for (GemmKernel* k : {w8_gemm_kernel<EPI_WARPS, FORM_ANY, EPI_ANY>, w8_gemm_kernel<EPI_WARPS_WIDE, FORM_ANY, EPI_ANY>,
                               w8_gemm_kernel<EPI_WARPS_WIDE, FORM_BF16, EPI_LINEAR>,
-                              w8_gemm_kernel<EPI_WARPS_WIDE, FORM_BF16, EPI_GEGLU_PACKED>, lean_kernel(EPI_NONE), lean_kernel(EPI_GEGLU_PACKED), lean_kernel(EPI_QKV_ROPE)})
+                              w8_gemm_kernel<EPI_WARPS_WIDE, FORM_BF16, EPI_GEGLU_PACKED>, lean_kernel(EPI_NONE, 3),
+                              lean_kernel(EPI_GEGLU_PACKED, 3), lean_kernel(EPI_QKV_ROPE, 3), lean_kernel(EPI_NONE, 2),
+                              lean_kernel(EPI_GEGLU_PACKED, 2), lean_kernel(EPI_QKV_ROPE, 2)})
           if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, DYN_SMEM_MAX) != cudaSuccess) return 0;
         return 1;
       }))
@@ -1098,10 +1102,10 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   }
   cfg.attrs = attr;
   cfg.numAttrs = na;
-  const bool plain = nw == 1 && np == 3 && pl.merge && !p.trace && !p.dbg;
+  const bool plain = nw == 1 && pl.merge && !p.trace && !p.dbg;
   GemmKernel* k = !wide ? w8_gemm_kernel<EPI_WARPS, FORM_ANY, EPI_ANY>
                   : !plain ? w8_gemm_kernel<EPI_WARPS_WIDE, FORM_ANY, EPI_ANY>
-                  : !x_bf16 ? lean_kernel(epi)
+                  : !x_bf16 ? lean_kernel(epi, np)
                   : epi == EPI_GEGLU_PACKED ? w8_gemm_kernel<EPI_WARPS_WIDE, FORM_BF16, EPI_GEGLU_PACKED>
                                             : w8_gemm_kernel<EPI_WARPS_WIDE, FORM_BF16, EPI_LINEAR>;
   if (cudaLaunchKernelEx(&cfg, k, tm_w0, tm_w1, tm_x, p) != cudaSuccess)
