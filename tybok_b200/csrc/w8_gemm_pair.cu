@@ -318,6 +318,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
         const int a = it & 1;
         const uint32_t plane16 = static_cast<uint32_t>(tl.bt * (P_BK / 2)) >> 4;
         const uint32_t idesc = p.np == 2 ? idesc_e4m3_e4m3_f32(256, tl.bt) : idesc_e4m3_e5m2_f32(256, tl.bt);
+        const uint32_t mx_desc = idesc_mx_e4m3(256, tl.bt, 0), sf_ones = smem_u32(smem) + p.sf_off;
         ok = __all_sync(0xffffffffu, wait_or_abort(&bars.acc_empty[a], ((it >> 1) & 1) ^ 1, &bars.abort));
         tc_fence_after();
         for (int k = 0; k < nkb && ok; ++k) {
@@ -327,26 +328,34 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
           tc_fence_after();
           const uint32_t st16 = (smem_u32(smem + s * p.stage_bytes) & 0x3FFFFu) >> 4;
           const uint32_t x16 = st16 + NA * (P_WTILE >> 4);
-          if (MX && leader) {
-            const uint32_t ones = smem_u32(smem) + p.sf_off, words = ones + 512 + (slot * MX_BATCH + k % MX_BATCH) * 1024;
-            if (k == 0 && it == 0) tc_copy_scales_pair(tmem + sfa, ones);
-            tc_copy_scales_pair(tmem + sfb + buf * 8, words);
-            if (tl.bt > 128) tc_copy_scales_pair(tmem + sfb + buf * 8 + 4, words + 512);
+          if constexpr (MX) {  // (a predicate for every instruction: in a branch their operands leave the uniform registers, 60-100 ns a K block)
+            const uint32_t words = sf_ones + 512 + (slot * MX_BATCH + k % MX_BATCH) * 1024, to = tmem + sfb + buf * 8;
+            if ((k | it) == 0)
+              if (leader) tc_copy_scales_pair(tmem + sfa, sf_ones);
+            if (leader) tc_copy_scales_pair(to, words);
+            if (tl.bt > 128)
+              if (leader) tc_copy_scales_pair(to + 4, words + 512);
+#pragma unroll
+            for (int pl = 0; pl < 2; ++pl)
+#pragma unroll
+              for (int w = 0; w < NA; ++w)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  const uint64_t ad = dk | (st16 + w * (P_WTILE >> 4) + j * 2);
+                  const uint64_t bd = dk | (x16 + pl * plane16 + j * 2);
+                  if (leader) umma_ss_mx_pair(tmem + a * acc_cols + w * tl.bt, ad, bd, mx_desc + ((pl << 10) | (j << 4)), tmem + sfa, to,
+                                              (k | pl | j) ? 1u : 0u);
+                }
           }
-          for (int pl = 0; pl < p.np; ++pl) {
+          for (int pl = 0; pl < (MX ? 0 : p.np); ++pl) {
 #pragma unroll
             for (int w = 0; w < NA; ++w) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 const uint64_t ad = dk | (st16 + w * (P_WTILE >> 4) + j * 2);
                 const uint64_t bd = dk | (x16 + pl * plane16 + j * 2);
-                if constexpr (MX) {
-                  if (leader) umma_ss_mx_pair(tmem + a * acc_cols + w * tl.bt, ad, bd, idesc_mx_e4m3(256, tl.bt, pl) | (j << 4), tmem + sfa,
-                                              tmem + sfb + buf * 8, (k | pl | j) ? 1u : 0u);
-                } else {
-                  if (leader) umma_ss_f8_pair(tmem + a * acc_cols + (p.merge ? pl : w) * tl.bt, ad, bd, idesc,
-                                              (k | (p.merge ? 0 : pl) | j) ? 1u : 0u);
-                }
+                if (leader) umma_ss_f8_pair(tmem + a * acc_cols + (p.merge ? pl : w) * tl.bt, ad, bd, idesc,
+                                            (k | (p.merge ? 0 : pl) | j) ? 1u : 0u);
               }
             }
           }
@@ -757,8 +766,8 @@ int ring_bytes(bool mx) { return P_SMEM - 1024 - (mx ? MX_SMEM : 0); }
 
 // Token tiles are whole steps of 32 tokens, at most 256 / na, and differ by one step (block-scaled form: steps of 16, at most
 // 240 / na).  Cost of a tile and K block: tensor time against operand fill at 52 bytes per clock and SM (measured for this
-// kernel's access pattern; 36 where no pair has a second tile, so that latency shows).  A K block of the block-scaled form takes
-// 850 clk at least.
+// kernel's access pattern; 36 where no pair has a second tile, so that latency shows).  A K block of the block-scaled form counts
+// 850 clk at least (it takes some 700; counted so, finer tiles win here and lose on the device: 233 x 16384 x 2048 22.5 -> 25.0 us).
 constexpr double MX_MIN_BLOCK = 850.0;
 PairPlan plan_pair(int M, int rows, int K, int na, int np, bool mx) {
   PairPlan best{};
