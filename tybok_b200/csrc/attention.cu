@@ -1017,21 +1017,23 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     }
   } else if (warp == 1) {
     const bool leader = elect_one();
-    const uint64_t dk = smem_desc_sw128(0);
     const uint32_t idesc_s = idesc_bf16_f32(AT_BQ, PF_BK);
     const uint32_t idesc_o = idesc_bf16_f32(AT_BQ, HD) | (1u << 16);
-    const uint32_t q16 = (smem_u32(sq) & 0x3FFFFu) >> 4;
+    // One descriptor per block, its steps add constants to it (addresses end below 2^14 units of 16 bytes, so no carry
+    // leaves the field): fewer instructions to fetch in a launch that waits for them. The runner of 30 DiT blocks at
+    // 50 tokens: 3643 -> 3628 us a call; the engine at batch 1 is the same.
+    const uint64_t qd = smem_desc_sw128(smem_u32(sq));
     bool ok = __all_sync(0xffffffffu, wait_or_abort(&bars.q_full, 0, &bars.abort));
     auto issue_s = [&](int j) {  // S_j = Q K_j^T into columns PF_BK * (j & 1); frees the K slot when done
       const int s = j & 1;
       ok = ok && __all_sync(0xffffffffu, wait_or_abort(&bars.k_full[s], (j >> 1) & 1, &bars.abort));
       if (!ok) return;
       tc_fence_after();
-      const uint32_t k16 = (smem_u32(sk + s * PF_KV) & 0x3FFFFu) >> 4;
+      const uint64_t kd = smem_desc_sw128(smem_u32(sk + s * PF_KV));
 #pragma unroll
       for (int ks = 0; ks < HD / 16; ++ks) {  // the head dimension in steps of 16: chunk ks / 4, 32 bytes per step
         const uint32_t qo = (ks >> 2) * (AT_CHUNK >> 4) + (ks & 3) * 2, ko = (ks >> 2) * (PF_KCHUNK >> 4) + (ks & 3) * 2;
-        if (leader) umma_ss_bf16(tmem + s * PF_BK, dk | (q16 + qo), dk | (k16 + ko), idesc_s, ks > 0 ? 1u : 0u);
+        if (leader) umma_ss_bf16(tmem + s * PF_BK, qd + qo, kd + ko, idesc_s, ks > 0 ? 1u : 0u);
       }
       if (leader) {
         tc_commit(&bars.k_empty[s]);
@@ -1047,13 +1049,13 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         ok = __all_sync(0xffffffffu, wait_or_abort(&bars.p_full[s], par, &bars.abort) && wait_or_abort(&bars.v_full[s], par, &bars.abort));
         if (!ok) break;
         tc_fence_after();
-        const uint32_t v_addr = smem_u32(sv + s * PF_KV);
+        const uint64_t vd = smem_desc_sw128_mn(smem_u32(sv + s * PF_KV), PF_KCHUNK);
+        const uint64_t pd = smem_desc_sw128(smem_u32(spk + s * AT_CHUNK));
 #pragma unroll
         for (int ks = 0; ks < PF_BK / 16; ++ks) {  // 16 keys per step: 16 rows x 128 bytes inside every chunk
-          const uint64_t bd = smem_desc_sw128_mn(v_addr + ks * 2048, PF_KCHUNK);
+          const uint64_t bd = vd + ks * (2048 >> 4);
           if (SHORT && ks >= PF_BK / 32) {
-            const uint32_t p16 = (smem_u32(spk + s * AT_CHUNK) & 0x3FFFFu) >> 4;
-            if (leader) umma_ss_bf16(t_o, dk | (p16 + (ks & 3) * 2), bd, idesc_o, 1u);
+            if (leader) umma_ss_bf16(t_o, pd + (ks & 3) * 2, bd, idesc_o, 1u);
           } else {
             if (leader) umma_ts_bf16(t_o, tmem + s * PF_BK + ks * 8, bd, idesc_o, (j > 0 || ks > 0) ? 1u : 0u);
           }
