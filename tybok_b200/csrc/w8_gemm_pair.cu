@@ -310,7 +310,6 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     const bool leader = elect_one();
     bool ok = true;
     if (rank == 0) {
-      const uint64_t dk = smem_desc_sw128(0);
       int s = 0, it = 0, slot = 0, buf = 0;
       uint32_t par = 0, sf_par = 0;
       for (int t = pair; t < tiles && ok; t += npairs, ++it) {
@@ -326,8 +325,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
                                            wait_or_abort(&bars.full[s], par, &bars.abort));
           if (!ok) break;
           tc_fence_after();
-          const uint32_t st16 = (smem_u32(smem + s * p.stage_bytes) & 0x3FFFFu) >> 4;
-          const uint32_t x16 = st16 + NA * (P_WTILE >> 4);
+          const uint64_t wd = smem_desc_sw128(smem_u32(smem + s * p.stage_bytes)), xd = wd + NA * (P_WTILE >> 4);
           if constexpr (MX) {  // (a predicate for every instruction: in a branch their operands leave the uniform registers, 60-100 ns a K block)
             const uint32_t words = sf_ones + 512 + (slot * MX_BATCH + k % MX_BATCH) * 1024, to = tmem + sfb + buf * 8;
             if ((k | it) == 0)
@@ -341,8 +339,8 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
               for (int w = 0; w < NA; ++w)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                  const uint64_t ad = dk | (st16 + w * (P_WTILE >> 4) + j * 2);
-                  const uint64_t bd = dk | (x16 + pl * plane16 + j * 2);
+                  const uint64_t ad = wd + w * (P_WTILE >> 4) + j * 2;
+                  const uint64_t bd = xd + pl * plane16 + j * 2;
                   if (leader) umma_ss_mx_pair(tmem + a * acc_cols + w * tl.bt, ad, bd, mx_desc + ((pl << 10) | (j << 4)), tmem + sfa, to,
                                               (k | pl | j) ? 1u : 0u);
                 }
@@ -352,8 +350,8 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
             for (int w = 0; w < NA; ++w) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const uint64_t ad = dk | (st16 + w * (P_WTILE >> 4) + j * 2);
-                const uint64_t bd = dk | (x16 + pl * plane16 + j * 2);
+                const uint64_t ad = wd + w * (P_WTILE >> 4) + j * 2;
+                const uint64_t bd = xd + pl * plane16 + j * 2;
                 if (leader) umma_ss_f8_pair(tmem + a * acc_cols + (p.merge ? pl : w) * tl.bt, ad, bd, idesc,
                                             (k | (p.merge ? 0 : pl) | j) ? 1u : 0u);
               }
