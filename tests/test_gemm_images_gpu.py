@@ -76,3 +76,20 @@ def test_few_tokens_in_both_images(m):
             lib.tybok_debug_set_counters(None)
         assert torch.equal(y, general)
     ops.check_status()
+
+
+# Over 64 tokens in a tile an epilogue warp sends two groups of 16 rows per matrix, in turn: 65 (one row in the second group), odd,
+# a full tile, and two tiles of which one is forced.
+@pytest.mark.parametrize("m,tile", [(64, 0), (65, 0), (70, 0), (79, 0), (80, 0), (150, 80)])
+@pytest.mark.parametrize("splits", [0, 2, 3, 4, 8])
+def test_two_matrices_with_k_over_a_cluster(m, tile, splits):
+    from tybok_b200 import ops
+
+    i, k = 640, 1024
+    g = torch.Generator(device="cuda").manual_seed(m)
+    xp = ops.split3(torch.empty(m, k, device="cuda").normal_(0, 1, generator=g).to(torch.bfloat16), 4)
+    (g8, gs), (u8, us) = _weights(i, k, 3), _weights(i, k, 4)
+    two = ops.w8x3_geglu(xp, 4, g8, gs, u8, us, out_planes=True, token_tile=tile, splits=splits)
+    one = ops.w8x3_geglu_packed(xp, 4, *ops.pack_gate_up(g8, gs, u8, us), out_planes=True, token_tile=tile, splits=splits)
+    ops.check_status()
+    assert _same(two, one)

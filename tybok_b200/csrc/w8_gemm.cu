@@ -523,7 +523,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
     // this phase of the cluster barrier says so.  Each warp arrives where it waits for something else anyway, and the
     // accumulator is not complete yet here.  (50-token MLP 14.59 -> 14.64 us; 1 x 2560 x 2048, whose epilogue warps are
     // busy until here, 6.39 -> 6.52 us; arrivals at the kernel's start cost twice that.)
-    // Where this warp's first 16 rows go: pairs of them to the owners in turn (0: past the tile's end).
+    // Where 16 rows of this warp go: pairs of them to the owners in turn (0: past the tile's end).  The first 16 are looked up here.
     const uint32_t stage_addr = smem_u32(smem + p.stage_off);
     uint32_t peer[8];
     auto peers = [&](int g) {
@@ -581,7 +581,7 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
             for (int e = 0; e < 16; ++e)
               if (g * 16 + e < nvalid) dst[e * BN] = __uint_as_float(v[e]);
           } else {
-            if (!AHEAD || g != half) peers(g);
+            if (!AHEAD || w > 0 || g != half) peers(g);  // (the second matrix starts over at `half` after other rows)
 #pragma unroll
             for (int e = 0; e < 8; ++e) {
               const uint32_t dst = peer[e] + w * rpr * (BN * 4);
