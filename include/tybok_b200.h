@@ -163,25 +163,6 @@ int tybok_w8x2_qkv_rope(const void* x_planes2, const float* row_scale, const voi
                         void* v_cache, int B, int L, int H, int G, int D, int Lcap, int key_off, int K, int token_tile,
                         int splits, int* status_word, void* stream);
 
-/* ---- block-scaled two-plane activations ---------------------------------------------------
- * Two planes [2][M][K], e4m3 and e5m2, of x * 2^k with one k per token and 32 channels (the block's largest magnitude in
- * (224, 448]) and the scale words [K / 128][M] of four UE8M0 bytes 2^-k, which the MMA applies (kind mxf8f6f4).  Exact within
- * 2^-14.8 of the block maximum, 2.8e-7 of it below: no coarser than three e5m2 planes, for a third less tensor work.  A block
- * is local to an epilogue warp, so a GEMM can write the form for the next one.  K a multiple of 128.
- *   tybok_w8mx_suits whether this form is the faster one for a product of M tokens.
- *   tybok_split_mx   bf16 rows -> that form; tybok_layernorm_modulate_mx: tybok_layernorm_modulate_groups into it (W a multiple of 128).
- *   tybok_w8mx_gemm  tybok_w8x2_gemm on it (x_sf), or on the row-scaled form (row_scale) where only the output is block-scaled:
- *                    y_planes [2][M][n_out] with y_sf [n_out / 128][M], n_out a multiple of 128.  splits: 0 = chosen here,
- *                    1 = whole K per tile, more = K over a cluster. */
-int tybok_w8mx_suits(int M, int N, int K);
-int tybok_layernorm_modulate_mx(const void* x, int64_t ldx, const void* shift, const void* scale, int64_t ldmod, int rows_per_group, int M,
-                                int W, float eps, void* planes, void* sf, void* stream);
-int tybok_split_mx(const void* x, int64_t ldx, void* planes, void* sf, int M, int K, void* stream);
-int tybok_w8mx_gemm(const void* x_planes, const void* x_sf, const float* row_scale, const void* w8, const float* scale, const void* bias,
-                    void* y, int64_t ldy, void* y_planes, void* y_sf, int M, int N, int K, int epilogue, const void* residual,
-                    int64_t ldres, const void* gate, int64_t ldgate, int rows_per_gate, int gate_is_bf16, int splits, int* status_word,
-                    void* stream);
-
 /* RMS normalisation feeding a W8 GEMM (fp32 statistics, one warp per row).
  *   weight != NULL: plain Gemma norm    y = bf16(x * rsqrt(mean(x^2)+eps) * (1 + weight))
  *   mod    != NULL: AdaRMS norm         y = bf16(x * rsqrt(mean(x^2)+eps) * (1 + scale) + shift),

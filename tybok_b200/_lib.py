@@ -81,15 +81,6 @@ SIGNATURES = {
         [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_i64, c_void_p, c_int, c_int, c_int, c_int, c_int,
          c_void_p, c_i64, c_void_p, c_i64, c_int, c_int, c_int, c_int, c_void_p, c_void_p],
     ),
-    "tybok_w8mx_suits": (c_int, [c_int, c_int, c_int]),
-    "tybok_layernorm_modulate_mx": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_i64, c_int, c_int, c_int, ctypes.c_float, c_void_p,
-                                            c_void_p, c_void_p]),
-    "tybok_split_mx": (c_int, [c_void_p, c_i64, c_void_p, c_void_p, c_int, c_int, c_void_p]),
-    "tybok_w8mx_gemm": (
-        c_int,
-        [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_i64, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
-         c_void_p, c_i64, c_void_p, c_i64, c_int, c_int, c_int, c_void_p, c_void_p],
-    ),
     "tybok_w8x2_qkv_rope": (
         c_int,
         [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int,

@@ -112,11 +112,9 @@ class GemmaStack {
     const bool folds = mods && fold && m < TWO_PLANE_MIN_TOKENS && any_packed;
     const size_t at_ws = tybok_attention_workspace_needed(b, l, heads_, kv_, hd_, keys);
     const size_t u = folds ? size_t(3) * m * w_ : 0, part = folds ? size_t(4) * m * (w_ / 128 + 1) : 0;
-    // Where the block-scaled form is the faster one for the down projection, the gate / up GEMM writes its planes in it.
-    const bool mx_down = packed && m >= TWO_PLANE_MIN_TOKENS && inner % 128 == 0 && tybok_w8mx_suits(m, w_, inner);
     Arena ar;
     const size_t np = ar.add(size_t(packed && m >= TWO_PLANE_MIN_TOKENS ? 2 : 3) * m * w_), rs = ar.add(size_t(4) * m);
-    const size_t q = ar.add(size_t(2) * m * a), ap = ar.add(size_t(3) * m * a), hp = ar.add(size_t(mx_down ? 2 : 3) * m * inner), hs = ar.add(mx_down ? size_t(m) * inner / 32 : 0);
+    const size_t q = ar.add(size_t(2) * m * a), ap = ar.add(size_t(3) * m * a), hp = ar.add(size_t(3) * m * inner);
     const size_t x1 = ar.add(size_t(2) * m * w_), xa = ar.add(size_t(2) * m * w_), xb = ar.add(size_t(2) * m * w_), ws = ar.add(at_ws);
     const size_t up0 = ar.add(u), up1 = ar.add(u), part0 = ar.add(part), part1 = ar.add(part);
     ar.allocate(x0);
@@ -183,19 +181,6 @@ class GemmaStack {
       } else {
         residual(ar.at(ap), SHIFT_ATTN, lay.o, ar.at(x1), cur, ld, mi ? mi + 2 * w_ : nullptr, m, status, st);
         norm(two, ar.at(x1), w_, lay.norm_post, mp, m, eps, ar.at(np), ar.at(rs), st);
-        if (mx_down) {
-          check(tybok_w8mx_gemm(ar.at(np), nullptr, static_cast<float*>(ar.at(rs)), lay.gate_up.wp(), lay.gate_up.sp(), nullptr, nullptr, inner,
-                                ar.at(hp), ar.at(hs), m, 2 * inner, w_, TYBOK_EPI_GEGLU_PACKED, nullptr, 0, nullptr, 0, 1, 0, 0, status, st),
-                "tybok_w8mx_gemm");
-          check(tybok_w8mx_gemm(ar.at(hp), ar.at(hs), nullptr, lay.down.wp(), lay.down.sp(), nullptr, out, w_, nullptr, nullptr, m, w_, inner,
-                                TYBOK_EPI_RESIDUAL, ar.at(x1), w_, mp ? mp + 2 * w_ : nullptr, w_, m, 0, 0, status, st),
-                "tybok_w8mx_gemm");
-          cur = out;
-          ld = w_;
-          carried = false;
-          record_event(record, i, st);
-          continue;
-        }
         if (two)
           check(tybok_w8x2_gemm(ar.at(np), static_cast<float*>(ar.at(rs)), lay.gate_up.wp(), lay.gate_up.sp(), nullptr, nullptr, inner, ar.at(hp),
                                 SHIFT_FFN, m, 2 * inner, w_, TYBOK_EPI_GEGLU_PACKED, nullptr, 0, nullptr, 0, 1, 0, 0, 0, status, st),

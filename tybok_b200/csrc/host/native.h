@@ -111,16 +111,6 @@ class Arena {
   char* base_ = nullptr;
 };
 
-// The block-scaled form of M rows of K values in an arena: two planes and the scale words.
-struct MxPlanes {
-  size_t planes = 0, sf = 0;
-  MxPlanes(Arena& a, bool used, size_t m, size_t k) {
-    if (!used) return;
-    planes = a.add(2 * m * k);
-    sf = a.add(m * k / 32);
-  }
-};
-
 void bind_ops(py::module_& m);
 void bind_dit(py::module_& m);
 void bind_gemma(py::module_& m);

@@ -113,17 +113,6 @@ static Tensor w8a16_linear(const Tensor& x, const Tensor& w8, const Tensor& scal
       return y;
     }
   }
-  if (shift == TYBOK_DEFAULT_X_SHIFT && token_tile <= 0 && splits <= 0 && tybok_w8mx_suits(m, n, k)) {
-    Arena a;
-    const MxPlanes p(a, true, m, k);
-    a.allocate(x2);
-    check(tybok_split_mx(ptr(x2), x2.stride(0), a.at(p.planes), a.at(p.sf), m, k, st), "tybok_split_mx");
-    check(tybok_w8mx_gemm(a.at(p.planes), a.at(p.sf), nullptr, ptr(w8), f32(scale), ptr(bias), ptr(y), n, nullptr, nullptr, m, n, k, epilogue,
-                          residual ? ptr(res) : nullptr, residual ? res.stride(0) : 0, ptr(gate), ldgate, rows_per_gate, gate_bf16, 0,
-                          status_ptr(x.get_device()), st),
-          "tybok_w8mx_gemm");
-    return y;
-  }
   const Tensor planes = at::empty({3 * m * k}, x.options().dtype(at::kByte));
   check(tybok_split3(ptr(x2), x2.stride(0), ptr(planes), m, k, shift, st), "tybok_split3");
   check(tybok_w8x3_linear(ptr(planes), shift, ptr(w8), f32(scale), ptr(bias), ptr(y), n, nullptr, 0, m, n, k, epilogue,
@@ -181,25 +170,11 @@ class Mlp {
     std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
     shape.back() = down_.n;
     Tensor y = at::empty(shape, x2.options());
-    void* st = stream_of(x);
-    int* status = status_ptr(x.get_device());
     Arena a;
-    // Block-scaled planes where they are the faster form for both products (the gate / up GEMM then writes them for the other).
-    const bool mx = packed_ && i % 128 == 0 && tybok_w8mx_suits(m, 2 * i, k) && tybok_w8mx_suits(m, down_.n, i);
-    const MxPlanes xm(a, mx, m, k), hm(a, mx, m, i);
-    if (mx) {
-      a.allocate(x2);
-      check(tybok_split_mx(ptr(x2), x2.stride(0), a.at(xm.planes), a.at(xm.sf), m, k, st), "tybok_split_mx");
-      check(tybok_w8mx_gemm(a.at(xm.planes), a.at(xm.sf), nullptr, gu_.wp(), gu_.sp(), nullptr, nullptr, i, a.at(hm.planes), a.at(hm.sf), m, 2 * i,
-                            k, TYBOK_EPI_GEGLU_PACKED, nullptr, 0, nullptr, 0, 1, 0, 0, status, st),
-            "tybok_w8mx_gemm");
-      check(tybok_w8mx_gemm(a.at(hm.planes), a.at(hm.sf), nullptr, down_.wp(), down_.sp(), nullptr, ptr(y), down_.n, nullptr, nullptr, m,
-                            down_.n, i, TYBOK_EPI_NONE, nullptr, 0, nullptr, 0, 1, 0, 0, status, st),
-            "tybok_w8mx_gemm");
-      return y.scalar_type() == x.scalar_type() ? y : y.to(x.scalar_type());
-    }
     const size_t xp = a.add(size_t(3) * m * k), hp = a.add(size_t(3) * m * i);
     a.allocate(x2);
+    void* st = stream_of(x);
+    int* status = status_ptr(x.get_device());
     bool direct = false;  // few tokens: the gate/up GEMM makes its own planes
     if (m <= 16 && packed_) {
       const int rc = tybok_w8a16_geglu_packed_direct(ptr(x2), x2.stride(0), gu_.wp(), gu_.sp(), a.at(hp), SHIFT_FFN, m, i, k, status, st);
@@ -253,26 +228,11 @@ class FfnTail {
     const int64_t ldm = sh.size(0) > 1 ? sh.stride(0) : 0;
     Tensor y = at::empty(x.sizes(), x2.options());
     if (m == 0) return y.to(x.scalar_type());
-    void* st = stream_of(x);
-    int* status = status_ptr(x.get_device());
     Arena a;
-    const bool mx = h <= 4096 && f % 128 == 0 && tybok_w8mx_suits(m, f, h) && tybok_w8mx_suits(m, h, f);
-    const MxPlanes xm(a, mx, m, h), hm(a, mx, m, f);
-    if (mx) {  // block-scaled planes: a third less tensor work in both products, LayerNorm with a warp per row
-      a.allocate(x2);
-      check(tybok_layernorm_modulate_mx(ptr(x2), x2.stride(0), ptr(sh), ptr(sc), ldm, per, m, h, eps_, a.at(xm.planes), a.at(xm.sf), st),
-            "tybok_layernorm_modulate_mx");
-      check(tybok_w8mx_gemm(a.at(xm.planes), a.at(xm.sf), nullptr, up_.wp(), up_.sp(), up_.bp(), nullptr, f, a.at(hm.planes), a.at(hm.sf), m, f, h,
-                            TYBOK_EPI_GELU, nullptr, 0, nullptr, 0, 1, 0, 0, status, st),
-            "tybok_w8mx_gemm");
-      check(tybok_w8mx_gemm(a.at(hm.planes), a.at(hm.sf), nullptr, down_.wp(), down_.sp(), down_.bp(), ptr(y), h, nullptr, nullptr, m, h, f,
-                            TYBOK_EPI_RESIDUAL, ptr(x2), x2.stride(0), ptr(gt), gt.size(0) > 1 ? gt.stride(0) : 0, gt.size(0) > 1 ? per : m, 1, 0,
-                            status, st),
-            "tybok_w8mx_gemm");
-      return y.scalar_type() == x.scalar_type() ? y : y.to(x.scalar_type());
-    }
     const size_t xp = a.add(size_t(3) * m * h), hp = a.add(size_t(3) * m * f);
     a.allocate(x2);
+    void* st = stream_of(x);
+    int* status = status_ptr(x.get_device());
     check(tybok_layernorm_modulate_groups(ptr(x2), x2.stride(0), ptr(sh), ptr(sc), ldm, per, m, h, eps_, nullptr, h, a.at(xp),
                                           SHIFT_NORMED, st),
           "tybok_layernorm_modulate");

@@ -420,103 +420,6 @@ __global__ void __launch_bounds__(512) layernorm_row_kernel(const NormParams p) 
   }
 }
 
-// LayerNorm and modulation, out as the block-scaled planes (split3.cuh): one CTA per row, two vectors of eight elements per
-// thread, everything the row needs in flight at once, both sums over all warps.  (The row kernel above keeps one warp's order of
-// summation for the DiT chain, and that warp sets its pace: 4146 x 3072 31 us, here 21; 140 rows 4.0, here 2.9.)  Four lanes hold a block
-// of 32 channels, sixteen a scale word.
-constexpr int LN_MX_V = 2;
-__global__ void __launch_bounds__(256, 6) layernorm_mx_kernel(const NormParams p, uint32_t* __restrict__ sf) {
-  __shared__ float red[2][8];
-  if (p.pdl) pdl_launch_dependents();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5, m = blockIdx.x, nvec = p.W / 8;
-  const long long plane = static_cast<long long>(p.M) * p.W, go = static_cast<long long>(m / p.rows_per_group) * p.ldmod;
-  if (p.pdl) pdl_wait();
-  uint4 raw[LN_MX_V], rs[LN_MX_V], rh[LN_MX_V];
-#pragma unroll
-  for (int i = 0; i < LN_MX_V; ++i) {
-    const int c = threadIdx.x + i * blockDim.x;
-    raw[i] = rs[i] = rh[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (c < nvec) {
-      raw[i] = *reinterpret_cast<const uint4*>(p.x + m * p.ldx + c * 8);
-      rs[i] = *reinterpret_cast<const uint4*>(p.ln_scale + go + c * 8);
-      rh[i] = *reinterpret_cast<const uint4*>(p.ln_shift + go + c * 8);
-    }
-  }
-  float sum = 0.f;
-#pragma unroll
-  for (int i = 0; i < LN_MX_V; ++i) {
-    const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) sum += __uint_as_float(w[e] << 16) + __uint_as_float(w[e] & 0xffff0000u);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if (lane == 0) red[0][warp] = sum;
-  __syncthreads();
-  sum = 0.f;
-  for (int w = 0; w < nwarps; ++w) sum += red[0][w];
-  const float mean = sum / static_cast<float>(p.W);
-  float ss = 0.f;
-#pragma unroll
-  for (int i = 0; i < LN_MX_V; ++i) {
-    if (threadIdx.x + i * blockDim.x >= nvec) continue;
-    const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float a = __uint_as_float(w[e] << 16) - mean, b = __uint_as_float(w[e] & 0xffff0000u) - mean;
-      ss = fmaf(a, a, ss);
-      ss = fmaf(b, b, ss);
-    }
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-  if (lane == 0) red[1][warp] = ss;
-  __syncthreads();
-  ss = 0.f;
-  for (int w = 0; w < nwarps; ++w) ss += red[1][w];
-  const float rstd = rsqrtf(ss / static_cast<float>(p.W) + p.eps);
-#pragma unroll
-  for (int i = 0; i < LN_MX_V; ++i) {
-    const int c = threadIdx.x + i * blockDim.x;
-    const bool live = c < nvec;  // the same for sixteen lanes (W % 128 == 0)
-    const uint32_t wx[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w}, ws[4] = {rs[i].x, rs[i].y, rs[i].z, rs[i].w}, wh[4] = {rh[i].x, rh[i].y, rh[i].z, rh[i].w};
-    uint32_t o[4];
-    // modulate(LN(x)) with every step rounded to bf16, as layernorm_row_kernel has it
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float v[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const uint32_t mask = u ? 0xffff0000u : 0xffffffffu;
-        const int sh = u ? 0 : 16;
-        const float nrm = bf16_round((__uint_as_float((wx[e] << sh) & mask) - mean) * rstd);
-        v[u] = bf16_round(nrm * bf16_round(1.0f + __uint_as_float((ws[e] << sh) & mask))) + __uint_as_float((wh[e] << sh) & mask);
-      }
-      const __nv_bfloat162 b = __floats2bfloat162_rn(v[0], v[1]);
-      o[e] = *reinterpret_cast<const uint32_t*>(&b);
-    }
-    uint32_t am = __vmaxu2(absmax4_bf16(o[0], o[1]), absmax4_bf16(o[2], o[3]));
-    am = __vmaxu2(am, __shfl_xor_sync(0xffffffffu, am, 1));
-    am = __vmaxu2(am, __shfl_xor_sync(0xffffffffu, am, 2));
-    float up;
-    uint32_t word = block_pow2(absmax_of_pair(am), up) << (8 * ((lane >> 2) & 3));
-    word |= __shfl_xor_sync(0xffffffffu, word, 4);
-    word |= __shfl_xor_sync(0xffffffffu, word, 8);
-    if (!live) continue;
-    const float lo[4] = {__uint_as_float(o[0] << 16) * up, __uint_as_float(o[0] & 0xffff0000u) * up, __uint_as_float(o[1] << 16) * up,
-                         __uint_as_float(o[1] & 0xffff0000u) * up};
-    const float hi[4] = {__uint_as_float(o[2] << 16) * up, __uint_as_float(o[2] & 0xffff0000u) * up, __uint_as_float(o[3] << 16) * up,
-                         __uint_as_float(o[3] & 0xffff0000u) * up};
-    uint2 w1, w2;
-    split_mx_quad(lo, w1.x, w2.x);
-    split_mx_quad(hi, w1.y, w2.y);
-    uint8_t* dst = p.planes2 + static_cast<long long>(m) * p.W + c * 8;
-    *reinterpret_cast<uint2*>(dst) = w1;
-    *reinterpret_cast<uint2*>(dst + plane) = w2;
-    if ((lane & 15) == 0) sf[static_cast<long long>(c >> 4) * p.M + m] = word;
-  }
-}
-
 // ------------------------------------------------------------------------------------------
 // Residual add + affine LayerNorm of the vision tower (tybok/policies/pi05/models/vision.py:
 // x = x + sublayer(x); h = LayerNorm(x)): x_out = bf16(x + y), h = bf16(LN_fp32(x_out) * w + b).
@@ -986,34 +889,6 @@ int tybok_layernorm_modulate_groups(const void* x, int64_t ldx, const void* shif
   if (((reinterpret_cast<uintptr_t>(shift) | reinterpret_cast<uintptr_t>(scale)) & 15) || ldmod % 8 != 0 || rows_per_group <= 0)
     return tb::host::fail(TYBOK_ERR_ARG, "layernorm_modulate: shift/scale rows must be 16-byte aligned, rows_per_group positive");
   return tb::launch_norm(x, ldx, nullptr, nullptr, ldmod, rows_per_group, scale, shift, M, W, eps, y, ldy, y_planes, out_shift, stream);
-}
-
-int tybok_layernorm_modulate_mx(const void* x, int64_t ldx, const void* shift, const void* scale, int64_t ldmod, int rows_per_group, int M,
-                                int W, float eps, void* planes, void* sf, void* stream) {
-  using namespace tb;
-  if (!x || !shift || !scale || !planes || !sf) return host::fail(TYBOK_ERR_ARG, "layernorm_modulate_mx: null pointer argument");
-  if (M <= 0 || W <= 0 || W % 128 != 0 || W > NORM_MAX_W || rows_per_group <= 0)
-    return host::fail(TYBOK_ERR_ARG, "layernorm_modulate_mx: W must be a multiple of 128 and <= 4096, rows_per_group positive");
-  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(shift) | reinterpret_cast<uintptr_t>(scale)) & 15) || ldx % 8 != 0 ||
-      ldmod % 8 != 0 || (reinterpret_cast<uintptr_t>(planes) & 15) || (reinterpret_cast<uintptr_t>(sf) & 3))
-    return host::fail(TYBOK_ERR_ARG, "layernorm_modulate_mx: rows and planes must be 16-byte aligned, the scales 4-byte");
-  if (int rc = host::require_sm100()) return rc;
-  NormParams p{};
-  p.x = static_cast<const __nv_bfloat16*>(x); p.ldx = ldx; p.ln_shift = static_cast<const __nv_bfloat16*>(shift);
-  p.ln_scale = static_cast<const __nv_bfloat16*>(scale); p.ldmod = ldmod; p.rows_per_group = rows_per_group; p.M = M; p.W = W; p.eps = eps;
-  p.planes2 = static_cast<uint8_t*>(planes); p.pdl = host::pdl_enabled() ? 1 : 0;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(M);
-  cfg.blockDim = dim3(((W / 8 + LN_MX_V - 1) / LN_MX_V + 31) / 32 * 32);
-  cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = p.pdl;
-  if (cudaLaunchKernelEx(&cfg, layernorm_mx_kernel, p, static_cast<uint32_t*>(sf)) != cudaSuccess) return host::fail_cuda("launch layernorm_mx_kernel");
-  host::count_launch();
-  return TYBOK_OK;
 }
 
 int tybok_layernorm_affine(const void* x, int64_t ldx, const void* weight, const void* bias, int M, int W, float eps,

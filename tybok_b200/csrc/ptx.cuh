@@ -275,31 +275,6 @@ __device__ __forceinline__ void umma_ss_f8_pair(uint32_t d_tmem, uint64_t a_desc
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Instruction descriptor for kind::mxf8f6f4 with A = e4m3 and B = e4m3 (format 0) or e5m2 (format 1), both K-major, one UE8M0
-// scale per row and 32-wide K slice: [4,6) byte of the B scale word, [7,10) A format, [10,13) B format, [17,23) N >> 3,
-// [23] 1 = UE8M0, [24,29) M >> 4, [29,31) byte of the A scale word.
-__host__ __device__ constexpr uint32_t idesc_mx_e4m3(int m, int n, int b_format) {
-  return (static_cast<uint32_t>(b_format) << 10) | (static_cast<uint32_t>(n >> 3) << 17) | (1u << 23) | (static_cast<uint32_t>(m >> 4) << 24);
-}
-// The pair's product with block scales: the scale words of A's 128 rows of each CTA and of all N rows of B lie in that
-// CTA's tensor memory, row r in lane r % 32 of column r / 32, the same in all four lane quadrants.
-__device__ __forceinline__ void umma_ss_mx_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t sfa_tmem,
-                                                uint32_t sfb_tmem, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %6, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale.scale_vec::1X [%0], %1, %2, %3, [%4], [%5], p;\n\t}\n" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(sfa_tmem), "r"(sfb_tmem), "r"(accumulate)
-      : "memory");
-}
-// Scale words of 128 rows (32 rows of 16 bytes in shared memory, row l: rows l, l + 32, l + 64, l + 96) -> four columns of tensor
-// memory, in all four lane quadrants, in both CTAs of the pair from the same offset of each one's shared memory.  In order with
-// the products that the same thread issues.  Descriptor: no swizzle, groups of 8 rows 128 bytes apart, version 1.
-__device__ __forceinline__ void tc_copy_scales_pair(uint32_t taddr, uint32_t smem_addr) {
-  const uint64_t desc = static_cast<uint64_t>((smem_addr & 0x3FFFF) >> 4) | (static_cast<uint64_t>(128 >> 4) << 16) |
-                        (static_cast<uint64_t>(128 >> 4) << 32) | (static_cast<uint64_t>(1) << 46);
-  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
-}
 // Arrive on the barrier at the same shared-memory offset in every CTA of `cta_mask` once the
 // pair's tcgen05 operations issued so far have retired.
 __device__ __forceinline__ void tc_commit_pair(uint64_t* bar, uint16_t cta_mask) {

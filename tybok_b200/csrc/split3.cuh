@@ -95,37 +95,4 @@ __device__ __forceinline__ void row_pow2(float amax, float& up, float& down) {
   down = __uint_as_float(static_cast<uint32_t>(127 - k) << 23);
 }
 
-// ------------------------------------------------------------------------------------------
-// Two terms with one power-of-two scale per BLOCK of 32 channels of a token, for the block-scaled MMA kind, which applies
-// that scale itself (one UE8M0 byte per row and 32-wide K slice): x * 2^k = g1 + g2, g1 = rn_e4m3(x'), g2 = rn_e5m2(x' - g1),
-// k puts the block's largest magnitude into (224, 448].  g1 carries 4 significant bits and leaves a residual of at most
-// 2^-4 of its leading bit in steps of the bf16 value's last bit: a signed multiple of up to 8, which the 3 bits of e5m2 hold.
-// So the sum is exact wherever g1 is a normal number, |x'| >= 2^-6 (within 2^-14.8 of the block maximum), and below that the
-// error is at most 2^-14 scaled units, 2.8e-7 of the block maximum.  (Three e5m2 terms with a fixed shift of 4 are exact
-// from 4.9e-4 and err by up to 5e-7 below.)  No producer has to see a whole row: an epilogue warp holds a block.
-__device__ __forceinline__ void split_mx_quad(const float (&x)[4], uint32_t& w1, uint32_t& w2) {
-  uint32_t a = f16x2_from_floats(x[0], x[1]), b = f16x2_from_floats(x[2], x[3]);
-  const uint32_t a1 = e4m3x2_from_f16x2(a), b1 = e4m3x2_from_f16x2(b);
-  a = f16x2_sub(a, f16x2_from_e4m3x2(a1));
-  b = f16x2_sub(b, f16x2_from_e4m3x2(b1));
-  w1 = a1 | (b1 << 16);
-  w2 = e5m2x2_from_f16x2(a) | (e5m2x2_from_f16x2(b) << 16);
-}
-// up = 2^k for the producer and the UE8M0 byte of 2^-k for the MMA.  Blocks below 2^-118 keep k = 126 (their scaled values
-// are smaller, the bytes valid); an infinity or NaN in the block gives the byte that means NaN, so it shows in the result.
-__device__ __forceinline__ uint32_t block_pow2(float amax, float& up) {
-  const uint32_t bits = __float_as_uint(amax);
-  const int e = static_cast<int>(bits >> 23) - 127;
-  const int k = min(126, 8 - e - ((bits & 0x7fffffu) > 0x600000u ? 1 : 0));
-  up = __uint_as_float(static_cast<uint32_t>(k + 127) << 23);
-  return bits >= 0x7f800000u ? 0xffu : static_cast<uint32_t>(127 - k);
-}
-// Largest magnitude of four packed bf16 values, as two bf16 lanes (a NaN is kept: fmax drops it, its bits are the largest).
-__device__ __forceinline__ uint32_t absmax4_bf16(uint32_t a, uint32_t b) {
-  return __vmaxu2(a & 0x7fff7fffu, b & 0x7fff7fffu);
-}
-__device__ __forceinline__ float absmax_of_pair(uint32_t v) {
-  return __uint_as_float(max(v << 16, v & 0xffff0000u));
-}
-
 }  // namespace tb

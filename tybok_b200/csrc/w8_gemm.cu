@@ -787,45 +787,6 @@ __global__ void split3_kernel(const __nv_bfloat16* __restrict__ x, long long ldx
   }
 }
 
-// x[M,K] (bf16, row stride ldx) -> the two planes [2][M][K] of the block-scaled form and its scale words [K / 128][M].
-// Bound by memory: 2 bytes in and 2.03 out per element (three planes write 3).  Sixteen threads of eight elements each make
-// a 128-wide K block of a token, four of them a block of 32.
-__global__ void __launch_bounds__(256) split_mx_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ planes,
-                                                       uint32_t* __restrict__ sf, int M, int K, int pdl) {
-  if (pdl) pdl_launch_dependents();
-  if (pdl) pdl_wait();
-  const long long plane = static_cast<long long>(M) * K;
-  const int kv = K / 8, lane = threadIdx.x & 31;
-  const long long total = static_cast<long long>(M) * kv;  // a multiple of 16: half warps are whole
-  for (long long i0 = blockIdx.x * static_cast<long long>(blockDim.x) + (threadIdx.x & ~31); i0 < total;
-       i0 += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const long long i = i0 + lane;
-    const bool live = i < total;
-    const int m = static_cast<int>((live ? i : i0) / kv), c = static_cast<int>((live ? i : i0) % kv);
-    uint4 raw = make_uint4(0u, 0u, 0u, 0u);
-    if (live) raw = *reinterpret_cast<const uint4*>(x + m * ldx + c * 8);
-    uint32_t am = __vmaxu2(absmax4_bf16(raw.x, raw.y), absmax4_bf16(raw.z, raw.w));
-    am = __vmaxu2(am, __shfl_xor_sync(0xffffffffu, am, 1));
-    am = __vmaxu2(am, __shfl_xor_sync(0xffffffffu, am, 2));
-    float up;
-    uint32_t word = block_pow2(absmax_of_pair(am), up) << (8 * ((lane >> 2) & 3));
-    word |= __shfl_xor_sync(0xffffffffu, word, 4);
-    word |= __shfl_xor_sync(0xffffffffu, word, 8);
-    if (!live) continue;
-    const float lo[4] = {__uint_as_float(raw.x << 16) * up, __uint_as_float(raw.x & 0xffff0000u) * up, __uint_as_float(raw.y << 16) * up,
-                         __uint_as_float(raw.y & 0xffff0000u) * up};
-    const float hi[4] = {__uint_as_float(raw.z << 16) * up, __uint_as_float(raw.z & 0xffff0000u) * up, __uint_as_float(raw.w << 16) * up,
-                         __uint_as_float(raw.w & 0xffff0000u) * up};
-    uint2 w1, w2;
-    split_mx_quad(lo, w1.x, w2.x);
-    split_mx_quad(hi, w1.y, w2.y);
-    uint8_t* dst = planes + static_cast<long long>(m) * K + c * 8;
-    *reinterpret_cast<uint2*>(dst) = w1;
-    *reinterpret_cast<uint2*>(dst + plane) = w2;
-    if ((lane & 15) == 0) sf[static_cast<long long>(c >> 4) * M + m] = word;
-  }
-}
-
 // ------------------------------------------------------------------------------------ host
 struct Plan {
   int bt, t_tiles, n_tiles, splits, kb_total, kb_per_split, nstages, smem_bytes, tmem_cols, merge, mma_n, stage_bytes, stage_off;
@@ -940,12 +901,6 @@ static bool make_plan(int M, int N, int K, int nw, int force_bt, int force_split
   return true;
 }
 
-// Estimated SM clocks of one wave of this plan: a K block costs the slower of its products and its operand fill at 50 bytes per
-// clock; set-up and exchange on top.
-static double one_tile_cost(const Plan& pl, int np) {
-  return pl.kb_per_split * std::max(2.0 * np * pl.bt, (16384.0 + np * 128.0 * pl.bt) / 50.0) + (pl.splits > 1 ? 3000.0 : 0.0);
-}
-
 // AdaRMS norm folded into the GEMMs on either side of it (see GemmParams).
 struct NormFold {
   const float* next_scale = nullptr;  // producer
@@ -1017,12 +972,14 @@ static int launch_gemm(const uint8_t* planes, const void* w0, const void* w1, co
   if (pl.n_tiles > 65535) return host::fail(TYBOK_ERR_ARG, "w8 gemm: grid too large");
   if (check_only) return TYBOK_OK;  // every argument check has passed; nothing was launched
   const bool free_form = force_bt <= 0 && force_splits <= 0 && !fold;
-  // Within one wave of tiles: K over the pairs of a cluster where that is estimated to be clearly ahead of this plan.  Those are the long K whose tile count leaves a third of the SMs idle but is too high for this kernel's own split:
+  // Within one wave of tiles: K over the pairs of a cluster where that is estimated to be clearly ahead of this plan
+  // (a K block costs the slower of its products and its operand fill at 50 bytes per clock; set-up and exchange on top).
+  // Those are the long K whose tile count leaves a third of the SMs idle but is too high for this kernel's own split:
   // 333 x 2048 x 16384 48.9 -> 35.7 us, 400 tokens 49.1 -> 38.7, 200 x 3072 x 14336 43.6 -> 36.2; 544 x 2048 x 16384
   // would stay at 51.
   bool split = false;
   if (free_form && M > 128 && !rope && (epi == EPI_NONE || epi == EPI_GELU || epi == EPI_RESIDUAL) && !gemm_pair_suits(M, N, nw, np)) {
-    const double here = one_tile_cost(pl, np);
+    const double here = pl.kb_per_split * std::max(2.0 * np * pl.bt, (16384.0 + np * 128.0 * pl.bt) / 50.0) + (pl.splits > 1 ? 3000.0 : 0.0);
     const double there = gemm_pair_split_cost(M, N, K, np);
     split = there > 0 && there + 6000.0 < 0.85 * here;
   }
@@ -1160,30 +1117,6 @@ static int launch_split3(const void* x, long long ldx, void* planes, int M, int 
   return TYBOK_OK;
 }
 
-static int launch_split_mx(const void* x, long long ldx, void* planes, void* sf, int M, int K, cudaStream_t stream) {
-  if (!x || !planes || !sf) return host::fail(TYBOK_ERR_ARG, "split_mx: null pointer argument");
-  if (M <= 0 || K <= 0 || K % 128 != 0 || ldx % 8 != 0 || ldx < K)
-    return host::fail(TYBOK_ERR_ARG, "split_mx: K must be a multiple of 128, ldx of 8, ldx >= K");
-  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(planes)) & 15) || (reinterpret_cast<uintptr_t>(sf) & 3))
-    return host::fail(TYBOK_ERR_ARG, "split_mx: x and planes must be 16-byte aligned, the scales 4-byte");
-  const long long total = static_cast<long long>(M) * (K / 8);
-  const int pdl = host::pdl_enabled() ? 1 : 0;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(static_cast<unsigned>(std::min<long long>((total + 255) / 256, 8 * host::sm_count())));
-  cfg.blockDim = dim3(256);
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl;
-  if (cudaLaunchKernelEx(&cfg, split_mx_kernel, static_cast<const __nv_bfloat16*>(x), ldx, static_cast<uint8_t*>(planes),
-                         static_cast<uint32_t*>(sf), M, K, pdl) != cudaSuccess)
-    return host::fail_cuda("launch split_mx_kernel");
-  host::count_launch();
-  return TYBOK_OK;
-}
-
 // The argument checks of tybok_w8x3_linear without its launch (for the two-launch entry points,
 // which must not start their first kernel when the second would be refused).
 static int check_linear_args(const void* planes, const void* w8, const float* scale, const void* bias, void* y,
@@ -1273,59 +1206,6 @@ int tybok_w8x2_gemm(const void* x_planes2, const float* row_scale, const void* w
                          ldy, epilogue == TYBOK_EPI_GEGLU_PACKED ? tb::EPI_GEGLU_PACKED : epilogue, residual, ldres, gate,
                          ldgate, rows_per_gate, gate_is_bf16, 0, out_shift, token_tile, splits, status_word,
                          static_cast<cudaStream_t>(stream), nullptr, false, row_scale);
-}
-
-// Where the block-scaled form is the faster one: enough work to fill the pair kernel (below 12 GFLOP the one-tile kernel's shorter
-// launch wins: 544 x 2560 x 2048 11.6 against 14.9 us), K long enough that its epilogue hides (K = 1024 gains nothing: 3200 x 4096
-// 32.1 against 34.1 us), and an estimate ahead of the three-plane plan's, which its steps of 16 tokens or one tile too many
-// for the pairs can spoil (4352 x 1024 x 4096 37.8 against 40.5 us).  A FFN tail of 150 tokens takes 59.4 us with three planes
-// and 62.2 with this form, one of 185 65.3 against 64.6, of 200 96.5 against 68.2.
-int tybok_w8mx_suits(int M, int N, int K) {
-  using namespace tb;
-  if (M <= 160 || N <= 0 || K % 128 != 0 || K < 1536 || 2.0 * M * N * K < 12e9) return 0;
-  double three = gemm_pair_cost(M, N, K, 3);
-  if (!gemm_pair_suits(M, N, 1, 3)) {
-    Plan pl;
-    if (!make_plan(M, N, K, 1, 0, 0, pl)) return 0;
-    three = one_tile_cost(pl, 3);
-    const double split = gemm_pair_split_cost(M, N, K, 3);
-    if (split > 0 && split + 6000.0 < 0.85 * three) three = split;
-  }
-  return gemm_pair_mx_cost(M, N, K) < 0.95 * three ? 1 : 0;
-}
-
-int tybok_split_mx(const void* x, int64_t ldx, void* planes, void* sf, int M, int K, void* stream) {
-  return tb::launch_split_mx(x, ldx, planes, sf, M, K, static_cast<cudaStream_t>(stream));
-}
-
-int tybok_w8mx_gemm(const void* x_planes, const void* x_sf, const float* row_scale, const void* w8, const float* scale, const void* bias,
-                    void* y, int64_t ldy, void* y_planes, void* y_sf, int M, int N, int K, int epilogue, const void* residual,
-                    int64_t ldres, const void* gate, int64_t ldgate, int rows_per_gate, int gate_is_bf16, int splits, int* status_word,
-                    void* stream) {
-  using namespace tb;
-  const bool gated = epilogue == TYBOK_EPI_GEGLU_PACKED;
-  if (epilogue != TYBOK_EPI_NONE && epilogue != TYBOK_EPI_GELU && epilogue != TYBOK_EPI_RESIDUAL && !gated)
-    return host::fail(TYBOK_ERR_ARG, "w8mx_gemm: unknown epilogue");
-  if ((x_sf != nullptr) == (row_scale != nullptr)) return host::fail(TYBOK_ERR_ARG, "w8mx_gemm: block scales or row scales, not both");
-  if ((y_planes != nullptr) != (y_sf != nullptr)) return host::fail(TYBOK_ERR_ARG, "w8mx_gemm: output planes come with their scales");
-  if (y_sf && epilogue == TYBOK_EPI_RESIDUAL) return host::fail(TYBOK_ERR_ARG, "w8mx_gemm: the residual form has no output planes");
-  const int n_out = gated ? N / 2 : N;
-  if ((x_sf && K % 128 != 0) || (y_sf && n_out % 128 != 0))
-    return host::fail(TYBOK_ERR_ARG, "w8mx_gemm: the block-scaled form needs widths that are multiples of 128");
-  if (reinterpret_cast<uintptr_t>(x_sf) & 3) return host::fail(TYBOK_ERR_ARG, "w8mx_gemm: scale words must be 4-byte aligned");
-  const int epi = gated ? EPI_GEGLU_PACKED : epilogue;
-  if (int rc = launch_gemm(static_cast<const uint8_t*>(x_planes), w8, nullptr, scale, nullptr, bias, y, y_planes, M, N, K, ldy, epi, residual,
-                           ldres, gate, ldgate, rows_per_gate, gate_is_bf16, 0, 0, 0, 0, status_word, static_cast<cudaStream_t>(stream),
-                           nullptr, true))
-    return rc;
-  GemmCall c{};
-  c.planes = static_cast<const uint8_t*>(x_planes); c.np = 2; c.row_scale = row_scale; c.sf = static_cast<const uint32_t*>(x_sf);
-  c.w0 = w8; c.s0 = scale; c.bias = static_cast<const __nv_bfloat16*>(bias); c.y = static_cast<__nv_bfloat16*>(y); c.ldy = ldy;
-  c.y_planes = static_cast<uint8_t*>(y_planes); c.y_sf = static_cast<uint8_t*>(y_sf); c.M = M; c.N = N; c.K = K; c.n_out = n_out; c.epi = epi;
-  c.res = static_cast<const __nv_bfloat16*>(residual); c.ldres = ldres; c.gate = gate; c.ldgate = ldgate; c.rows_per_gate = rows_per_gate;
-  c.gate_bf16 = gate_is_bf16; c.out_scale = 1.0f; c.plane_scale = 1.0f; c.status = status_word; c.stream = static_cast<cudaStream_t>(stream);
-  c.split = !gated && (splits > 1 || (splits <= 0 && gemm_pair_mx_splits(M, N, K)));
-  return launch_gemm_pair(c);
 }
 
 int tybok_w8x2_qkv_rope(const void* x_planes2, const float* row_scale, const void* w8_paired, const float* scale_paired,

@@ -28,7 +28,6 @@ struct GemmCall {
   const uint8_t* planes;   // [np][M][K]
   int np;                  // 3 e5m2 planes (fixed exponent shift) or 2 e4m3 planes with row_scale
   const float* row_scale;  // [M], two-plane form
-  const uint32_t* sf;      // block-scaled two-plane form: [K / 128][M] words of four UE8M0 bytes, else NULL
   const void* w0;          // [N][K] e4m3 (packed forms: the interleaved matrix)
   const void* w1;          // second matrix of EPI_GEGLU, else NULL
   const float* s0;
@@ -36,8 +35,7 @@ struct GemmCall {
   const __nv_bfloat16* bias;
   __nv_bfloat16* y;
   long long ldy;
-  uint8_t* y_planes;       // three e5m2 planes, or with y_sf the two planes of the block-scaled form
-  uint8_t* y_sf;           // [n_out / 128][M][4] UE8M0 bytes, or NULL
+  uint8_t* y_planes;
   int M, N, K, n_out;
   int epi;
   const __nv_bfloat16* res;
@@ -56,12 +54,6 @@ struct GemmCall {
 bool gemm_pair_suits(int M, int N, int nw, int np);
 // Estimated SM clocks of the split form (a cluster of pairs per tile) for one wave of clusters; negative: does not apply.
 double gemm_pair_split_cost(int M, int N, int K, int np);
-// Whether the block-scaled form runs this product with K over the pairs of a cluster.
-bool gemm_pair_mx_splits(int M, int N, int K);
-// Estimated SM clocks of the pair kernel for a product with one weight matrix: the block-scaled form (split or not), and three
-// planes with whole K per tile.
-double gemm_pair_mx_cost(int M, int N, int K);
-double gemm_pair_cost(int M, int N, int K, int np);
 int launch_gemm_pair(const GemmCall& c);
 
 }  // namespace tb

@@ -19,9 +19,6 @@
 //   * one CTA per SM that takes all 512 tensor-memory columns: nothing else that allocates tensor memory
 //     can be resident beside it (its shared memory leaves no room), so allocation never waits.
 // Token tiles differ by 32 tokens at most (two tensor maps), so ragged token counts waste under one step.
-// The MX instances take activation planes with block scales, for operands whose producer does not see a whole row: two planes
-// instead of three, at the rate of the row-scaled form (4146 x 3072 x 14336 343 -> 250 us, 544 x 2048 x 16384 49 -> 37 us,
-// 16384 x 2048 from 800 rows 55 -> 45 us).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -47,13 +44,6 @@ constexpr int P_CHUNK = 16;           // tokens that an epilogue warp finishes a
 constexpr int P_THREADS = 32 * (2 + P_EPI_WARPS);
 constexpr int P_SMEM = 226 * 1024;
 constexpr int P_ACC_COLS = 256;       // tensor-memory columns of one accumulator (two per CTA)
-// Block-scaled form: the scale words of the products take tensor memory beside the accumulators: four columns of ones for the
-// weights, then three buffers of eight columns (one per 32 tokens), each with the words of a K block.
-constexpr int MX_MAX_TOK = 240;       // accumulator columns: 2 x 240 + 4 + 3 x 8 of 512
-constexpr int MX_BUFS = 3;
-constexpr int MX_BATCH = 4;           // K blocks per shared-memory slot (1 KB each) that the scale warp fills
-constexpr int MX_SLOTS = 2;           // each filled by a warp of its own
-constexpr int MX_SMEM = 512 + 1024 * MX_BATCH * MX_SLOTS;  // the ones for the weights first
 
 struct PairParams {
   int M, N, K, n_out;
@@ -68,10 +58,6 @@ struct PairParams {
   int pdl;
   float out_scale, plane_scale;
   const float* row_scale;
-  const uint32_t* sf;    // block-scaled form: [kb][M] scale words of the activation planes
-  int acc_cols;                    // columns of one accumulator
-  int sf_off;                      // byte offset of the scale words in shared memory, behind the operand ring
-  uint8_t* y_sf;         // scale bytes [n_out / 128][M][4] of block-scaled output planes, or NULL (three e5m2 planes)
   const float* s0;
   const float* s1;
   const __nv_bfloat16* bias;
@@ -94,9 +80,6 @@ struct __align__(8) PairBars {
   uint64_t acc_full[2];          // each CTA: accumulator complete
   uint64_t acc_empty[2];         // even CTA: the epilogue warps of both CTAs have read the accumulator
   uint64_t mma_done;             // every product this pair issued has retired
-  uint64_t sf_full[MX_SLOTS];    // even CTA: both CTAs have the scale words of four K blocks in shared memory
-  uint64_t sf_odd[MX_SLOTS];     // odd CTA: it has them (its idle MMA warp tells the even CTA)
-  uint64_t sf_empty[MX_SLOTS];   // each CTA: the pair's products have read them
   uint32_t tmem_base;
   volatile int issued;           // stages whose copies this CTA's producer has requested, once it is through; -1 before
   volatile int abort;
@@ -187,22 +170,14 @@ __device__ __forceinline__ uint2 quad_transpose(uint32_t a, uint32_t b, int lane
 // SPLIT: long K and too few tiles for the device: a cluster of 2 * splits CTAs works on ONE tile, each pair on its part of
 // K.  Once all of them are through (their rings are idle then), every pair sends the token chunks it does not own
 // into the owners' shared memory, and a chunk's owner adds the parts in split order and finishes it.
-// MX: the planes are e4m3 + e5m2 with a UE8M0 scale per token and 32 channels (split3.cuh), which the block-scaled MMA
-// applies.  One more warp reads the scale words, four K blocks at a time and four ahead, and lays them out in a shared-memory slot
-// as the copy to tensor memory wants them (word of token 32 c + l in row l, column c); the MMA warp issues that copy in order
-// with the products.  So a token tile may start anywhere.  What a hand-over costs is its release at cluster scope, about
-// 1000 clk with the loads in flight: one for every K block was the pace of the whole kernel (18944 x 16384 x 240 tokens, one tile
-// per pair, 137 us; four warps that stored to tensor memory and handed over single blocks 144 us).
-template <int EPI, bool SPLIT, bool MX>
-__global__ void __launch_bounds__(P_THREADS + (MX ? 32 * MX_SLOTS : 0), 1)
+template <int EPI, bool SPLIT>
+__global__ void __launch_bounds__(P_THREADS, 1)
 w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w1,
                     const __grid_constant__ CUtensorMap tm_big, const __grid_constant__ CUtensorMap tm_small,
                     const PairParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ PairBars bars;
-  constexpr int NA = (EPI == EPI_GEGLU || EPI == EPI_QKV_ROPE) ? 2 : 1;  // accumulators (of <= ACC / NA tokens) per tile
-  const int acc_cols = MX ? p.acc_cols : P_ACC_COLS;
-  const int sfa = 2 * acc_cols, sfb = sfa + 4;
+  constexpr int NA = (EPI == EPI_GEGLU || EPI == EPI_QKV_ROPE) ? 2 : 1;  // accumulators (of <= 256 / NA tokens) per tile
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t crank = cluster_ctarank(), rank = crank & 1u, lead = crank & ~1u;  // the even CTA issues the pair's products
@@ -222,11 +197,6 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
       mbar_init(&bars.acc_empty[i], 2 * P_EPI_WARPS);
     }
     mbar_init(&bars.mma_done, 1);
-    for (int i = 0; MX && i < MX_SLOTS; ++i) {
-      mbar_init(&bars.sf_full[i], 2);
-      mbar_init(&bars.sf_odd[i], 1);
-      mbar_init(&bars.sf_empty[i], 1);
-    }
     bars.abort = 0;
     bars.issued = -1;
     fence_barrier_init();
@@ -310,62 +280,33 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     const bool leader = elect_one();
     bool ok = true;
     if (rank == 0) {
-      int s = 0, it = 0, slot = 0, buf = 0;
-      uint32_t par = 0, sf_par = 0;
+      int s = 0, it = 0;
+      uint32_t par = 0;
       for (int t = pair; t < tiles && ok; t += npairs, ++it) {
         const Tile tl = tile_at(p, t);
         const int a = it & 1;
         const uint32_t plane16 = static_cast<uint32_t>(tl.bt * (P_BK / 2)) >> 4;
         const uint32_t idesc = p.np == 2 ? idesc_e4m3_e4m3_f32(256, tl.bt) : idesc_e4m3_e5m2_f32(256, tl.bt);
-        const uint32_t mx_desc = idesc_mx_e4m3(256, tl.bt, 0), sf_ones = smem_u32(smem) + p.sf_off;
         ok = __all_sync(0xffffffffu, wait_or_abort(&bars.acc_empty[a], ((it >> 1) & 1) ^ 1, &bars.abort));
         tc_fence_after();
         for (int k = 0; k < nkb && ok; ++k) {
-          ok = __all_sync(0xffffffffu, (!MX || k % MX_BATCH || wait_or_abort(&bars.sf_full[slot], sf_par, &bars.abort)) &&
-                                           wait_or_abort(&bars.full[s], par, &bars.abort));
+          ok = __all_sync(0xffffffffu, wait_or_abort(&bars.full[s], par, &bars.abort));
           if (!ok) break;
           tc_fence_after();
           const uint64_t wd = smem_desc_sw128(smem_u32(smem + s * p.stage_bytes)), xd = wd + NA * (P_WTILE >> 4);
-          if constexpr (MX) {  // (a predicate for every instruction: in a branch their operands leave the uniform registers, 60-100 ns a K block)
-            const uint32_t words = sf_ones + 512 + (slot * MX_BATCH + k % MX_BATCH) * 1024, to = tmem + sfb + buf * 8;
-            if ((k | it) == 0)
-              if (leader) tc_copy_scales_pair(tmem + sfa, sf_ones);
-            if (leader) tc_copy_scales_pair(to, words);
-            if (tl.bt > 128)
-              if (leader) tc_copy_scales_pair(to + 4, words + 512);
-#pragma unroll
-            for (int pl = 0; pl < 2; ++pl)
-#pragma unroll
-              for (int w = 0; w < NA; ++w)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const uint64_t ad = wd + w * (P_WTILE >> 4) + j * 2;
-                  const uint64_t bd = xd + pl * plane16 + j * 2;
-                  if (leader) umma_ss_mx_pair(tmem + a * acc_cols + w * tl.bt, ad, bd, mx_desc + ((pl << 10) | (j << 4)), tmem + sfa, to,
-                                              (k | pl | j) ? 1u : 0u);
-                }
-          }
-          for (int pl = 0; pl < (MX ? 0 : p.np); ++pl) {
+          for (int pl = 0; pl < p.np; ++pl) {
 #pragma unroll
             for (int w = 0; w < NA; ++w) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
                 const uint64_t ad = wd + w * (P_WTILE >> 4) + j * 2;
                 const uint64_t bd = xd + pl * plane16 + j * 2;
-                if (leader) umma_ss_f8_pair(tmem + a * acc_cols + (p.merge ? pl : w) * tl.bt, ad, bd, idesc,
+                if (leader) umma_ss_f8_pair(tmem + a * P_ACC_COLS + (p.merge ? pl : w) * tl.bt, ad, bd, idesc,
                                             (k | (p.merge ? 0 : pl) | j) ? 1u : 0u);
               }
             }
           }
           if (leader) tc_commit_pair(&bars.empty[s], both);
-          if (MX) {
-            buf = buf == MX_BUFS - 1 ? 0 : buf + 1;
-            if (k % MX_BATCH == MX_BATCH - 1 || k == nkb - 1) {
-              if (leader) tc_commit_pair(&bars.sf_empty[slot], both);
-              sf_par ^= slot;
-              slot ^= 1;
-            }
-          }
           __syncwarp();
           if (++s == p.nstages) {
             s = 0;
@@ -385,20 +326,6 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
       }
       __syncwarp();
     }
-    if (MX && rank == 1) {  // pass the scale warp's hand-overs on
-      const uint32_t sf_full0 = dsmem_addr(smem_u32(&bars.sf_full[0]), lead);
-      int slot = 0;
-      uint32_t par = 0;
-      for (int t = pair; t < tiles && ok; t += npairs)
-        for (int k = 0; k < nkb && ok; k += MX_BATCH) {
-          ok = __all_sync(0xffffffffu, wait_or_abort(&bars.sf_odd[slot], par, &bars.abort));
-          if (ok && lane == 0) mbar_arrive_cluster(sf_full0 + slot * 8);
-          __syncwarp();
-          par ^= slot;
-          slot ^= 1;
-        }
-      if (!ok && lane == 0) pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
-    }
     // The odd CTA's wait spans the whole launch: it only gives up once something else has failed.
     bool done = false;
     for (int tries = 0; tries < 16 && !done; ++tries) {
@@ -407,55 +334,6 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     }
     if (!done) done = mbar_wait(&bars.mma_done, 0);
     if (!done && lane == 0) pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_MMA);
-  } else if (MX && warp >= 2 + P_EPI_WARPS) {
-    // ------------------------------------------------------------ scale words -> shared memory
-    const int slot = warp - 2 - P_EPI_WARPS;  // this warp's: it takes every other batch of K blocks
-    uint64_t* const done = rank == 0 ? &bars.sf_full[slot] : &bars.sf_odd[slot];
-    uint4* ones = reinterpret_cast<uint4*>(smem + p.sf_off);
-    ones[lane] = make_uint4(0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu, 0x7f7f7f7fu);  // 2^0: the weights' scales are the epilogue's
-    if (p.pdl) pdl_wait();
-    auto load = [&](const Tile& tl, int k0, uint32_t (&v)[MX_BATCH][8]) {
-#pragma unroll
-      for (int b = 0; b < MX_BATCH; ++b) {
-        const uint32_t* src = p.sf + static_cast<long long>(kb0 + min(k0 + b, nkb - 1)) * p.M;
-#pragma unroll
-        for (int c = 0; c < 8; ++c) v[b][c] = c * 32 < tl.bt ? __ldcg(src + min(tl.m0 + c * 32 + lane, p.M - 1)) : 0u;
-      }
-    };
-    auto next = [&](int& t, int& k0) {
-      if ((k0 += MX_BATCH) >= nkb) {
-        k0 = 0;
-        t += npairs;
-      }
-    };
-    uint32_t par = 1, cur[MX_BATCH][8], nxt[MX_BATCH][8];
-    bool ok = true;
-    int t = pair, k0 = 0;
-    if (slot) next(t, k0);
-    if (t < tiles) load(tile_at(p, t), k0, nxt);
-    while (t < tiles) {
-      const bool two = tile_at(p, t).bt > 128;
-#pragma unroll
-      for (int b = 0; b < MX_BATCH; ++b)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) cur[b][c] = nxt[b][c];
-      next(t, k0);
-      next(t, k0);
-      if (t < tiles) load(tile_at(p, t), k0, nxt);
-      ok = __all_sync(0xffffffffu, wait_or_abort(&bars.sf_empty[slot], par, &bars.abort));
-      if (!ok) break;
-#pragma unroll
-      for (int b = 0; b < MX_BATCH; ++b) {
-        uint4* dst = ones + 32 + (slot * MX_BATCH + b) * 64;
-        dst[lane] = make_uint4(cur[b][0], cur[b][1], cur[b][2], cur[b][3]);
-        if (two) dst[lane + 32] = make_uint4(cur[b][4], cur[b][5], cur[b][6], cur[b][7]);
-      }
-      fence_proxy_async();  // the copy reads them through the async proxy
-      __syncwarp();
-      if (lane == 0) mbar_arrive(done);
-      par ^= 1;
-    }
-    if (!ok && lane == 0) pair_fail(&bars, p.status, TYBOK_DEV_TIMEOUT_PRODUCER);
   } else {
     // ------------------------------------------------------------ epilogue
     const int q = warp & 3, part = (warp - 2) >> 2;  // tensor-memory lane quadrant; which of its four warps
@@ -527,7 +405,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
       };
       auto finish = [&](int mc, uint32_t (&v)[16], uint32_t (&u)[NA == 2 ? 16 : 1], uint2 (&rr)[EPI == EPI_RESIDUAL ? 4 : 1]) {
         float rs = 1.0f;
-        if (!MX && p.row_scale) rs = p.row_scale[min(mc + (lane & 15), p.M - 1)];
+        if (p.row_scale) rs = p.row_scale[min(mc + (lane & 15), p.M - 1)];
         uint32_t pk[8], pw[EPI == EPI_QKV_ROPE ? 8 : 1];  // bf16 results of two tokens each (and of the rotary partners)
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
@@ -537,7 +415,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
             const int i = 2 * k + e;
             float x = __uint_as_float(v[i]);
             float r = 1.0f;
-            if (!MX && p.row_scale) {
+            if (p.row_scale) {
               r = __shfl_sync(0xffffffffu, rs, i);
               x *= r;
             }
@@ -573,32 +451,6 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
           }
           pk[k] = pack_bf16(o[0], o[1]);
           if constexpr (EPI == EPI_QKV_ROPE) pw[k] = pack_bf16(w[0], w[1]);
-        }
-        // Block-scaled output: the warp's 32 channels are one block of each of its 16 tokens.  Three steps that halve the tokens a
-        // lane keeps, two over the rest: lane l then has the maxima of tokens 2 (l >> 2) and the next.
-        uint32_t scales = 0;
-        const bool block_scaled = (EPI == EPI_NONE || EPI == EPI_GELU || EPI == EPI_GEGLU) && p.y_sf;
-        if (block_scaled) {
-          uint32_t a[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) a[k] = pk[k] & 0x7fff7fffu;
-#pragma unroll
-          for (int h = 4; h > 0; h >>= 1) {
-            const bool up_half = lane & (4 * h);
-#pragma unroll
-            for (int k = 0; k < h; ++k) {
-              const uint32_t theirs = __shfl_xor_sync(0xffffffffu, up_half ? a[k] : a[k + h], 4 * h);
-              a[k] = __vmaxu2(up_half ? a[k + h] : a[k], theirs);
-            }
-          }
-          a[0] = __vmaxu2(a[0], __shfl_xor_sync(0xffffffffu, a[0], 2));
-          a[0] = __vmaxu2(a[0], __shfl_xor_sync(0xffffffffu, a[0], 1));
-          float up0, up1;
-          const uint32_t b0 = block_pow2(__uint_as_float(a[0] << 16), up0), b1 = block_pow2(__uint_as_float(a[0] & 0xffff0000u), up1);
-          scales = (__float_as_uint(up0) >> 23) | (__float_as_uint(up1) >> 7);  // exponents of the two factors
-          const int m = mc + 2 * (lane >> 2) + (lane & 1);
-          if ((lane & 2) == 0 && m < m_end && live)
-            p.y_sf[(static_cast<long long>(n_first >> 7) * p.M + m) * 4 + ((n_first >> 5) & 3)] = static_cast<uint8_t>(lane & 1 ? b1 : b0);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
@@ -643,11 +495,6 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
               *reinterpret_cast<uint2*>(dst + hd2 + d) = hi;
             }
           } else {
-            float up = p.plane_scale;
-            if (block_scaled) {
-              const uint32_t sc = __shfl_sync(0xffffffffu, scales, (4 * k + j4) >> 1 << 2);
-              up = __uint_as_float((j4 & 1 ? sc >> 16 : sc & 0xffffu) << 23);
-            }
             if (m < m_end && quad_live) {
               if (EPI == EPI_RESIDUAL) {
                 const uint2 r2 = rr[EPI == EPI_RESIDUAL ? k : 0];
@@ -656,18 +503,14 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
               }
               if (p.y) *reinterpret_cast<uint2*>(p.y + m * p.ldy + n_first) = t0;
               if (p.y_planes) {
-                const float xs[4] = {bf16_lo(t0.x) * up, bf16_hi(t0.x) * up, bf16_lo(t0.y) * up, bf16_hi(t0.y) * up};
-                uint32_t w1, w2;
+                const float xs[4] = {bf16_lo(t0.x) * p.plane_scale, bf16_hi(t0.x) * p.plane_scale,
+                                     bf16_lo(t0.y) * p.plane_scale, bf16_hi(t0.y) * p.plane_scale};
+                uint32_t w1, w2, w3;
+                split3_quad(xs, w1, w2, w3);
                 uint8_t* dst = p.y_planes + static_cast<long long>(m) * p.n_out + n_first;
-                if (block_scaled) {
-                  split_mx_quad(xs, w1, w2);
-                } else {
-                  uint32_t w3;
-                  split3_quad(xs, w1, w2, w3);
-                  *reinterpret_cast<uint32_t*>(dst + 2 * plane) = w3;
-                }
                 *reinterpret_cast<uint32_t*>(dst) = w1;
                 *reinterpret_cast<uint32_t*>(dst + plane) = w2;
+                *reinterpret_cast<uint32_t*>(dst + 2 * plane) = w3;
               }
             }
           }
@@ -716,15 +559,15 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
           if (mc >= m_end) break;
           uint32_t v[16];
           uint32_t u[NA == 2 ? 16 : 1];
-          tmem_ld16(tmem + a * acc_cols + lane_addr + c * P_CHUNK, v);
-          if constexpr (NA == 2) tmem_ld16(tmem + a * acc_cols + lane_addr + tl.bt + c * P_CHUNK, u);
+          tmem_ld16(tmem + a * P_ACC_COLS + lane_addr + c * P_CHUNK, v);
+          if constexpr (NA == 2) tmem_ld16(tmem + a * P_ACC_COLS + lane_addr + tl.bt + c * P_CHUNK, u);
           uint2 rr[EPI == EPI_RESIDUAL ? 4 : 1];
           residual_rows(mc, rr);
           tc_wait_ld();
-          if (NA == 1 && !MX && p.merge) {
+          if (NA == 1 && p.merge) {
             for (int pl = 1; pl < p.np; ++pl) {
               uint32_t v2[16];
-              tmem_ld16(tmem + a * acc_cols + lane_addr + pl * tl.bt + c * P_CHUNK, v2);
+              tmem_ld16(tmem + a * P_ACC_COLS + lane_addr + pl * tl.bt + c * P_CHUNK, v2);
               tc_wait_ld();
 #pragma unroll
               for (int e = 0; e < 16; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(v2[e]));
@@ -739,7 +582,7 @@ w8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_cons
     }
   }
 
-  if (SPLIT && (warp < 2 || warp >= 2 + P_EPI_WARPS)) {  // the two meeting points of the epilogue warps' exchange
+  if (SPLIT && warp < 2) {  // the two meeting points of the epilogue warps' exchange
     __syncwarp();
     cluster_sync_all();
     cluster_sync_all();
@@ -759,50 +602,41 @@ struct PairPlan {
   double cost;  // SM clocks
 };
 
-// Shared memory for the operand ring: 1 KB goes to alignment, the block-scaled form keeps its scale slots behind the ring.
-int ring_bytes(bool mx) { return P_SMEM - 1024 - (mx ? MX_SMEM : 0); }
-
-// Token tiles are whole steps of 32 tokens, at most 256 / na, and differ by one step (block-scaled form: steps of 16, at most
-// 240 / na).  Cost of a tile and K block: tensor time against operand fill at 52 bytes per clock and SM (measured for this
-// kernel's access pattern; 36 where no pair has a second tile, so that latency shows).  A K block of the block-scaled form counts
-// 850 clk at least (it takes some 700; counted so, finer tiles win here and lose on the device: 233 x 16384 x 2048 22.5 -> 25.0 us).
-constexpr double MX_MIN_BLOCK = 850.0;
-PairPlan plan_pair(int M, int rows, int K, int na, int np, bool mx) {
+// Token tiles are whole steps of 32 tokens, at most 256 / na, and differ by one step.  Cost of a tile and K block:
+// tensor time against operand fill at 52 bytes per clock and SM (measured for this kernel's access pattern).
+PairPlan plan_pair(int M, int rows, int K, int na, int np) {
   PairPlan best{};
   best.cost = -1.0;
   // Up to 128 tokens the planes keep their own columns, as in the one-tile kernel: the sum over K and planes then has
   // the same order in both, so such a call's result does not depend on which of them the tile count selects.
-  best.merge = (na == 1 && M <= 128 && !mx) ? 1 : 0;
+  best.merge = (na == 1 && M <= 128) ? 1 : 0;
   const int pairs = std::max(1, host::sm_count() / 2);
   const int ch = (rows + 256 * na - 1) / (256 * na);
-  const int step = mx ? 16 : 32, units = (M + step - 1) / step;
+  const int units = (M + 31) / 32;
   // Those columns are a token tile's planes times its tokens: one accumulator takes 256 of them, and the whole of tensor
   // memory (384 for three planes of 128 tokens) where no pair has a second tile.  One token tile reads the weights once
   // (106 x 14336 x 3072: two tiles of 64 tokens 25.2 us, one of 128 20.7 us).
-  const int umax = mx ? MX_MAX_TOK / 16 / na : best.merge ? (ch <= pairs ? 16 / np : 8 / np) : 8 / na;
+  const int umax = best.merge ? (ch <= pairs ? 16 / np : 8 / np) : 8 / na;
   const int kb = (K + P_BK - 1) / P_BK;
-  auto tile_cost = [&](int u, bool one_wave) {
-    const double tok = static_cast<double>(step) * u, mma = 2.0 * tok * na * np;
-    const double fill = (na * 16384.0 + np * 64.0 * tok) / (mx && one_wave ? 36.0 : 52.0);
-    return std::max(kb * std::max(std::max(mma, fill), mx ? MX_MIN_BLOCK : 0.0), 700.0 + tok * 24.0 * na) + (mx && one_wave ? 4000.0 : 0.0);
+  auto tile_cost = [&](int u) {
+    const double mma = 64.0 * u * na * np, fill = (na * 16384.0 + np * 2048.0 * u) / 52.0;
+    return std::max(kb * std::max(mma, fill), 700.0 + 32.0 * u * 24.0 * na);
   };
-  const int tt0 = (units + umax - 1) / umax, tt1 = mx ? std::min(units, 2 * tt0 + 16) : units;  // (no finer tiles pay)
-  for (int tt = tt0; tt <= tt1; ++tt) {
+  for (int tt = (units + umax - 1) / umax; tt <= units; ++tt) {
     const int ub = (units + tt - 1) / tt, us = units % tt == 0 ? ub : ub - 1;
     const int nb = units % tt == 0 ? tt : units % tt;
     const long long tiles = static_cast<long long>(ch) * tt;
-    const bool one = tiles <= pairs;
-    const double avg = (nb * tile_cost(ub, one) + (tt - nb) * tile_cost(us, one)) / tt;
-    const double cost = static_cast<double>(tiles / pairs) * avg + (tiles % pairs ? tile_cost(ub, one) : 0.0);
+    const double avg = (nb * tile_cost(ub) + (tt - nb) * tile_cost(us)) / tt;
+    const double cost = static_cast<double>(tiles / pairs) * avg + (tiles % pairs ? tile_cost(ub) : 0.0);
     if (best.cost < 0 || cost < best.cost) {
       best.cost = cost;
-      best.ch_tiles = ch; best.tok_tiles = tt; best.n_big = nb; best.bt_big = step * ub; best.bt_small = step * us; best.kb = kb;
+      best.ch_tiles = ch; best.tok_tiles = tt; best.n_big = nb; best.bt_big = 32 * ub; best.bt_small = 32 * us; best.kb = kb;
     }
   }
   best.splits = 1;
   best.kb_split = best.kb;
   best.stage_bytes = na * P_WTILE + np * (best.bt_big / 2) * P_BK;
-  best.nstages = std::min(P_MAX_STAGES, ring_bytes(mx) / best.stage_bytes);
+  best.nstages = std::min(P_MAX_STAGES, (P_SMEM - 1024) / best.stage_bytes);
   // L2 groups: as many token tiles as keep the group's planes within a quarter of L2
   const double tile_bytes = static_cast<double>(best.bt_big) * K * np;
   best.group = std::max(1, std::min(best.tok_tiles, static_cast<int>(32.0e6 / tile_bytes)));
@@ -813,7 +647,7 @@ PairPlan plan_pair(int M, int rows, int K, int na, int np, bool mx) {
 int resident_clusters(int splits) {
   static host::DeviceCache cache[5];
   return host::per_device(cache[splits], [splits] {
-    auto* k = w8_gemm_pair_kernel<EPI_RESIDUAL, true, false>;
+    auto* k = w8_gemm_pair_kernel<EPI_RESIDUAL, true>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM);
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(2 * splits);
@@ -837,26 +671,25 @@ int resident_clusters(int splits) {
 
 // Split form: one wave of clusters.  The exchange moves (splits - 1) / splits of a 128-channel fp32 tile through
 // distributed shared memory (about 18 bytes per clock and SM) between two cluster meetings.
-PairPlan plan_split(int M, int rows, int K, int np, bool mx) {
+PairPlan plan_split(int M, int rows, int K, int np) {
   PairPlan best{};
   best.cost = -1.0;
-  const int step = mx ? 16 : 32, umax = mx ? MX_MAX_TOK / 16 : 8;
-  const int units = (M + step - 1) / step, ch = (rows + 255) / 256, kb = (K + P_BK - 1) / P_BK;
+  const int units = (M + 31) / 32, ch = (rows + 255) / 256, kb = (K + P_BK - 1) / P_BK;
   for (int sp = 2; sp <= 4; ++sp) {
     const int cap = resident_clusters(sp), kbs = (kb + sp - 1) / sp;
     if ((sp - 1) * kbs >= kb) continue;  // no empty split
-    for (int tt = (units + umax - 1) / umax; tt <= units && static_cast<long long>(ch) * tt <= cap; ++tt) {
-      const int ub = (units + tt - 1) / tt, tok = step * ub, chunks = (tok + P_CHUNK - 1) / P_CHUNK;
-      const int stage = P_WTILE + np * (tok / 2) * P_BK, ns = std::min(P_MAX_STAGES, ring_bytes(mx) / stage);
-      if (sp * ((chunks + sp - 1) / sp) * P_CHUNK * 512 > ns * stage) continue;  // the parts land in the idle ring
-      const double mma = 2.0 * tok * np, fill = (16384.0 + np * 64.0 * tok) / 36.0;  // one tile per pair: latency shows
-      const double cost = kbs * std::max(std::max(mma, fill), mx ? MX_MIN_BLOCK : 0.0) + tok * 512.0 * (sp - 1) / sp / 18.0 + 4000.0;
+    for (int tt = (units + 7) / 8; tt <= units && static_cast<long long>(ch) * tt <= cap; ++tt) {
+      const int ub = (units + tt - 1) / tt;
+      const int stage = P_WTILE + np * 16 * ub * P_BK, ns = std::min(P_MAX_STAGES, (P_SMEM - 1024) / stage);
+      if (sp * ((2 * ub + sp - 1) / sp) * P_CHUNK * 512 > ns * stage) continue;  // the parts land in the idle ring
+      const double mma = 64.0 * ub * np, fill = (16384.0 + np * 2048.0 * ub) / 36.0;  // one tile per pair: latency shows
+      const double cost = kbs * std::max(mma, fill) + 32.0 * ub * 512.0 * (sp - 1) / sp / 18.0 + 4000.0;
       if (best.cost < 0 || cost < best.cost) {
         best.cost = cost;
         best.ch_tiles = ch; best.tok_tiles = tt; best.kb = kb; best.splits = sp; best.kb_split = kbs;
         best.n_big = units % tt == 0 ? tt : units % tt;
-        best.bt_big = step * ub;
-        best.bt_small = units % tt == 0 ? step * ub : step * (ub - 1);
+        best.bt_big = 32 * ub;
+        best.bt_small = units % tt == 0 ? 32 * ub : 32 * (ub - 1);
         best.stage_bytes = stage;
         best.nstages = ns;
         best.group = tt;
@@ -866,44 +699,9 @@ PairPlan plan_split(int M, int rows, int K, int np, bool mx) {
   return best;
 }
 
-using PairKernel = void(const CUtensorMap, const CUtensorMap, const CUtensorMap, const CUtensorMap, const PairParams);
-// The instance for an epilogue (NULL: not built).
-PairKernel* pair_kernel(int epi, bool split, bool mx) {
-  switch (epi) {
-    case EPI_NONE:
-      return mx ? (split ? w8_gemm_pair_kernel<EPI_NONE, true, true> : w8_gemm_pair_kernel<EPI_NONE, false, true>)
-                : (split ? w8_gemm_pair_kernel<EPI_NONE, true, false> : w8_gemm_pair_kernel<EPI_NONE, false, false>);
-    case EPI_GELU:
-      return mx ? (split ? w8_gemm_pair_kernel<EPI_GELU, true, true> : w8_gemm_pair_kernel<EPI_GELU, false, true>)
-                : (split ? w8_gemm_pair_kernel<EPI_GELU, true, false> : w8_gemm_pair_kernel<EPI_GELU, false, false>);
-    case EPI_RESIDUAL:
-      return mx ? (split ? w8_gemm_pair_kernel<EPI_RESIDUAL, true, true> : w8_gemm_pair_kernel<EPI_RESIDUAL, false, true>)
-                : (split ? w8_gemm_pair_kernel<EPI_RESIDUAL, true, false> : w8_gemm_pair_kernel<EPI_RESIDUAL, false, false>);
-    case EPI_GEGLU:
-    case EPI_GEGLU_PACKED:
-      return split ? nullptr : mx ? w8_gemm_pair_kernel<EPI_GEGLU, false, true> : w8_gemm_pair_kernel<EPI_GEGLU, false, false>;
-    default:
-      return split || mx ? nullptr : w8_gemm_pair_kernel<EPI_QKV_ROPE, false, false>;
-  }
-}
-
 }  // namespace
 
-double gemm_pair_split_cost(int M, int N, int K, int np) { return plan_split(M, N, K, np, false).cost; }
-
-double gemm_pair_cost(int M, int N, int K, int np) {
-  const PairPlan pl = plan_pair(M, N, K, 1, np, false);
-  if (pl.ch_tiles * pl.tok_tiles > host::sm_count() / 2) return pl.cost;
-  return pl.kb * std::max(2.0 * pl.bt_big * np, (16384.0 + np * 64.0 * pl.bt_big) / 36.0) + 4000.0;  // latency shows
-}
-double gemm_pair_mx_cost(int M, int N, int K) {
-  return gemm_pair_mx_splits(M, N, K) ? plan_split(M, N, K, 2, true).cost : plan_pair(M, N, K, 1, 2, true).cost;
-}
-
-bool gemm_pair_mx_splits(int M, int N, int K) {
-  const PairPlan one = plan_pair(M, N, K, 1, 2, true), sp = plan_split(M, N, K, 2, true);
-  return sp.cost > 0 && sp.cost < one.cost;
-}
+double gemm_pair_split_cost(int M, int N, int K, int np) { return plan_split(M, N, K, np).cost; }
 
 // The pair form takes what the one-tile-per-CTA form (w8_gemm.cu) would run in more than one wave: more than one
 // 128-row x 80-token (three planes) or 128-token (two planes) tile per SM.  Within one wave that form is ahead, since
@@ -918,8 +716,7 @@ bool gemm_pair_suits(int M, int N, int nw, int np) {
 int launch_gemm_pair(const GemmCall& c) {
   const int na = (c.epi == EPI_QKV_ROPE || c.epi == EPI_GEGLU || c.epi == EPI_GEGLU_PACKED) ? 2 : 1;
   const bool packed = c.epi == EPI_GEGLU_PACKED || c.epi == EPI_QKV_ROPE;
-  const bool mx = c.sf != nullptr;
-  const PairPlan pl = c.split ? plan_split(c.M, c.N, c.K, c.np, mx) : plan_pair(c.M, c.w1 ? 2 * c.N : c.N, c.K, na, c.np, mx);
+  const PairPlan pl = c.split ? plan_split(c.M, c.N, c.K, c.np) : plan_pair(c.M, c.w1 ? 2 * c.N : c.N, c.K, na, c.np);
 
   CUtensorMap tm_w0, tm_w1, tm_big, tm_small;
   if (int rc = host::tensor_map_2d(&tm_w0, c.w0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, c.K, c.N, c.K, P_BK, packed ? 64 : 128)) return rc;
@@ -939,11 +736,6 @@ int launch_gemm_pair(const GemmCall& c) {
   p.n_big = pl.n_big; p.bt_big = pl.bt_big; p.bt_small = pl.bt_small;
   p.pdl = host::pdl_enabled() ? 1 : 0;
   p.out_scale = c.out_scale; p.plane_scale = c.plane_scale; p.row_scale = c.row_scale;
-  p.sf = c.sf; p.y_sf = c.y_sf;
-  if (mx) {
-    p.acc_cols = na * pl.bt_big;
-    p.sf_off = pl.nstages * pl.stage_bytes;
-  }
   p.s0 = c.s0; p.s1 = c.s1; p.bias = c.bias; p.y = c.y; p.ldy = c.ldy; p.y_planes = c.y_planes;
   p.res = c.res; p.ldres = c.ldres; p.gate = c.gate; p.ldgate = c.ldgate;
   p.rows_per_gate = c.rows_per_gate > 0 ? c.rows_per_gate : 1; p.gate_bf16 = c.gate_bf16;
@@ -953,11 +745,10 @@ int launch_gemm_pair(const GemmCall& c) {
 
   static host::DeviceCache attr_set;
   if (!host::per_device(attr_set, [] {
-        for (int i = 0; i < 24; ++i) {
-          PairKernel* k = pair_kernel(i % 6, i / 6 % 2, i / 12);
-          if (!k) continue;
+        for (auto* k : {w8_gemm_pair_kernel<EPI_NONE, false>, w8_gemm_pair_kernel<EPI_GELU, false>, w8_gemm_pair_kernel<EPI_RESIDUAL, false>,
+                        w8_gemm_pair_kernel<EPI_GEGLU, false>, w8_gemm_pair_kernel<EPI_QKV_ROPE, false>, w8_gemm_pair_kernel<EPI_NONE, true>,
+                        w8_gemm_pair_kernel<EPI_GELU, true>, w8_gemm_pair_kernel<EPI_RESIDUAL, true>})
           if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, P_SMEM) != cudaSuccess) return 0;
-        }
         return 1;
       }))
     return host::fail_cuda("cudaFuncSetAttribute(w8_gemm_pair_kernel)");
@@ -965,7 +756,7 @@ int launch_gemm_pair(const GemmCall& c) {
   const int tiles = pl.ch_tiles * pl.tok_tiles;
   const int pairs = c.split ? tiles * pl.splits : std::min(tiles, std::max(1, host::sm_count() / 2));
   cfg.gridDim = dim3(2 * pairs);
-  cfg.blockDim = dim3(P_THREADS + (mx ? 32 * MX_SLOTS : 0));
+  cfg.blockDim = dim3(P_THREADS);
   cfg.dynamicSmemBytes = P_SMEM;  // always the whole SM: no other user of tensor memory beside this CTA
   cfg.stream = c.stream;
   cudaLaunchAttribute attr[2];
@@ -982,8 +773,15 @@ int launch_gemm_pair(const GemmCall& c) {
   ++n_attr;
   cfg.attrs = attr;
   cfg.numAttrs = n_attr;
-  PairKernel* k = pair_kernel(c.epi, c.split, mx);
-  if (!k) return host::fail(TYBOK_ERR_ARG, "w8 gemm: this epilogue has no such form");
+  auto* k = c.split ? w8_gemm_pair_kernel<EPI_NONE, true> : w8_gemm_pair_kernel<EPI_NONE, false>;
+  switch (c.epi) {
+    case EPI_GELU: k = c.split ? w8_gemm_pair_kernel<EPI_GELU, true> : w8_gemm_pair_kernel<EPI_GELU, false>; break;
+    case EPI_RESIDUAL: k = c.split ? w8_gemm_pair_kernel<EPI_RESIDUAL, true> : w8_gemm_pair_kernel<EPI_RESIDUAL, false>; break;
+    case EPI_GEGLU:
+    case EPI_GEGLU_PACKED: k = w8_gemm_pair_kernel<EPI_GEGLU, false>; break;
+    case EPI_QKV_ROPE: k = w8_gemm_pair_kernel<EPI_QKV_ROPE, false>; break;
+    default: break;
+  }
   if (cudaLaunchKernelEx(&cfg, k, tm_w0, tm_w1, tm_big, tm_small, p) != cudaSuccess) return host::fail_cuda("launch w8_gemm_pair_kernel");
   host::count_launch();
   return TYBOK_OK;
