@@ -44,3 +44,12 @@ def test_masked_blocks(b, l, keys, h, g, d, scale, first, last):
     finally:
         lib.tybok_debug_set_trace(None)
     assert torch.equal(y, y1) and torch.equal(yp, yp1)
+
+
+# Scales that no model uses but the entry takes: zero (the mean of the valid values), below zero, and so small that a finite stand-in for a
+# masked score would not be small beside the others.  Keys past the last one count as masked, so the unmasked call is a case too.
+@pytest.mark.parametrize("b,l,keys,h,g,d", FORMS)
+@pytest.mark.parametrize("scale", [0.0, 1e-30, -0.002, -0.0625])
+@pytest.mark.parametrize("first,last", [(0, 0), (128, 37)])
+def test_masked_keys_count_for_nothing_at_any_scale(b, l, keys, h, g, d, scale, first, last):
+    test_masked_blocks(b, l, keys, h, g, d, scale, min(first, keys // 2), last)

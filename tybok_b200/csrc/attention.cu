@@ -26,6 +26,9 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
+#include <limits>
+
 #include "../../include/tybok_b200.h"
 #include "host_util.h"
 #include "ptx.cuh"
@@ -233,7 +236,8 @@ struct AttnParams {
   int B, L, H, G, Lk, Lcap;
   int nsplit;
   int rows_per_rank;  // push form: query rows that each CTA of a cluster merges
-  float scale_log2e;  // softmax scale * log2(e)
+  float scale_log2e;     // |softmax scale| * log2(e), above zero
+  uint32_t negate_q;     // bit of the scores' instruction descriptor that negates Q: a scale below zero
   const uint8_t* key_valid;  // [B][Lk] or NULL (all keys valid)
   __nv_bfloat16* out;        // [B*L][H*D] or NULL
   uint8_t* out_planes;       // [3][B*L][H*D] or NULL
@@ -268,9 +272,9 @@ struct __align__(16) AttnBars {
   float wn[AT_MAX_SPLITS][AT_BQ];  // merge weights of the rows this CTA owns: exp2(m_s - m) / denominator
 };
 
-// Score of a masked key: so small that its exponential is zero beside any other (and beside half of itself, which stands in for
-// the reference maximum of a row that has seen masked keys only).
-constexpr float PF_MASKED = -1e30f;
+// Score of a masked key, and of the rows past the last key: its exponential is zero at every scale.  Maxima start from -1e30, so
+// the reference of a row that has seen masked keys only is finite.
+#define AT_MASKED 0xff800000u  // -infinity
 // 2^x by the special-function unit alone (results below 2^-126 flush to zero).
 __device__ __forceinline__ float pf_exp2(float x) {
   float y;
@@ -411,7 +415,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const bool leader = elect_one();
     bool ok = true;
     {
-      const uint32_t idesc_s = idesc_bf16_f32(AT_BQ, AT_BK);
+      const uint32_t idesc_s = idesc_bf16_f32(AT_BQ, AT_BK) | p.negate_q;
       // (descriptors once, steps add constants; with the GEMM's other loops, batch-1 chunk 8.96 -> 8.94 ms, three runs each)
       const uint64_t qd = smem_desc_sw128(smem_u32(sq)), kd = smem_desc_sw128(smem_u32(sk));
 #pragma unroll 4
@@ -475,11 +479,11 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       tmem_ld32(t_s + lane_addr + (hf * 2 + 1) * 32, v1);
       tc_wait_ld();
       const uint32_t b0 = bars.valid[hf * 2], b1 = bars.valid[hf * 2 + 1];
-      if ((b0 & b1) != 0xffffffffu) {  // a masked score becomes so small that its exponential is zero
+      if ((b0 & b1) != 0xffffffffu) {
 #pragma unroll
         for (int e = 0; e < 32; ++e) {
-          if (!((b0 >> e) & 1u)) v0[e] = __float_as_uint(PF_MASKED);
-          if (!((b1 >> e) & 1u)) v1[e] = __float_as_uint(PF_MASKED);
+          if (!((b0 >> e) & 1u)) v0[e] = AT_MASKED;
+          if (!((b1 >> e) & 1u)) v1[e] = AT_MASKED;
         }
       }
 #pragma unroll
@@ -493,14 +497,13 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     const float m2 = fmaxf(bars.hmax[0][row], bars.hmax[1][row]) * p.scale_log2e;  // scale > 0
     float sum = 0.f;
     if (ok && live) {
-      const float base = fmaxf(m2, 0.5f * PF_MASKED * p.scale_log2e);  // a row whose keys are all masked: its exponentials stay zero
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t pk[16];
 #pragma unroll
         for (int e = 0; e < 32; e += 2) {
           const float s0 = __uint_as_float(c == 0 ? v0[e] : v1[e]), s1 = __uint_as_float(c == 0 ? v0[e + 1] : v1[e + 1]);
-          const float p0 = pf_exp2(s0 * p.scale_log2e - base), p1 = pf_exp2(s1 * p.scale_log2e - base);
+          const float p0 = pf_exp2(s0 * p.scale_log2e - m2), p1 = pf_exp2(s1 * p.scale_log2e - m2);
           sum += p0 + p1;
           const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
           pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
@@ -1021,7 +1024,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
     }
   } else if (warp == 1) {
     const bool leader = elect_one();
-    const uint32_t idesc_s = idesc_bf16_f32(AT_BQ, PF_BK);
+    const uint32_t idesc_s = idesc_bf16_f32(AT_BQ, PF_BK) | p.negate_q;
     const uint32_t idesc_o = idesc_bf16_f32(AT_BQ, HD) | (1u << 16);
     // One descriptor per block, its steps add constants to it (addresses end below 2^14 units of 16 bytes, so no carry
     // leaves the field): fewer instructions to fetch in a launch that waits for them. The runner of 30 DiT blocks at
@@ -1138,7 +1141,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
           if (bits[w] != 0xffffffffu) {
 #pragma unroll
             for (int e = 0; e < 32; ++e)
-              if (!((bits[w] >> e) & 1u)) v[w][e] = __float_as_uint(PF_MASKED);
+              if (!((bits[w] >> e) & 1u)) v[w][e] = AT_MASKED;
           }
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {  // two chains of three-way maxima: the warp has nothing else to do meanwhile
@@ -1188,7 +1191,6 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         }
       }
       if (ok && slive) {
-        const float base = fmaxf(m_ref, 0.5f * PF_MASKED * p.scale_log2e);
         float sum = 0.f;
         auto add = [&](int e, float two) {
           if (SHORT && hf) tail[SHORT ? e >> 1 : 0] = two;
@@ -1199,8 +1201,8 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
           uint32_t pk[16];
 #pragma unroll
           for (int e = 0; e < 32; e += 2) {
-            const float p0 = pf_exp2(__uint_as_float(v[w][e]) * p.scale_log2e - base);
-            const float p1 = pf_exp2(__uint_as_float(v[w][e + 1]) * p.scale_log2e - base);
+            const float p0 = pf_exp2(__uint_as_float(v[w][e]) * p.scale_log2e - m_ref);
+            const float p1 = pf_exp2(__uint_as_float(v[w][e + 1]) * p.scale_log2e - m_ref);
             add(e, p0 + p1);
             const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
             pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
@@ -1433,7 +1435,7 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
     }
   } else if (warp == 1) {
     const bool leader = elect_one();
-    const uint32_t idesc_s = idesc_bf16_f32(128, BK), idesc_o = idesc_bf16_f32(128, HD) | (1u << 16);
+    const uint32_t idesc_s = idesc_bf16_f32(128, BK) | p.negate_q, idesc_o = idesc_bf16_f32(128, HD) | (1u << 16);
     auto issue_s = [&](int t, int j) {
       const uint64_t qd = smem_desc_sw128(smem_u32(sq + t * 32768)), kd = smem_desc_sw128(smem_u32(sk + (j & 1) * KV));
 #pragma unroll
@@ -1516,12 +1518,12 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
           const uint32_t bits[4] = {b0, b1, b2, b3};
           const bool all = (b0 & b1 & b2 & b3) == 0xffffffffu;
           tc_wait_ld();
-          if (!all) {  // a masked score becomes so small that its exponential is zero
+          if (!all) {
 #pragma unroll
             for (int w = 0; w < 4; ++w)
 #pragma unroll
               for (int e = 0; e < 32; ++e)
-                if (!((bits[w] >> e) & 1u)) v[w][e] = __float_as_uint(PF_MASKED);
+                if (!((bits[w] >> e) & 1u)) v[w][e] = AT_MASKED;
           }
           float mx0 = -1e30f, mx1 = -1e30f, mx2 = -1e30f, mx3 = -1e30f;
 #pragma unroll
@@ -1550,8 +1552,7 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
             }
             if (grow) m_ref = m_blk;
           }
-          const float base = fmaxf(m_ref, 0.5f * PF_MASKED * p.scale_log2e);  // (a row that has seen masked keys only)
-          const uint64_t nm = f32x2(-base, -base);
+          const uint64_t nm = f32x2(-m_ref, -m_ref);
           uint64_t sum0 = f32x2(0.f, 0.f), sum1 = sum0;
 #pragma unroll
           for (int w = 0; w < 4; ++w) {
@@ -1643,6 +1644,13 @@ attention_two_tile_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid
 }  // namespace tb
 
 namespace tb {
+// The kernels want a scale above zero: the scores' maximum is that of the scaled ones, and a masked score stays -infinity under it.
+// Softmax at a scale below zero is that of the negated scores; at zero it is uniform, as at one that no score brings above 2^-22.
+static void at_set_scale(AttnParams& p, float scale) {
+  p.scale_log2e = fabsf(scale) * 1.4426950408889634f;
+  if (p.scale_log2e == 0.f) p.scale_log2e = std::numeric_limits<float>::denorm_min();
+  p.negate_q = scale < 0.f ? 1u << 13 : 0u;
+}
 using AtKernel = void(const CUtensorMap, const CUtensorMap, const CUtensorMap, const AttnParams);
 static AtKernel* at_kernel(bool push, bool aids) {
   return push ? (aids ? attention_kernel<true, true> : attention_kernel<true, false>)
@@ -1848,7 +1856,7 @@ int tybok_attention(const void* q, const void* k_cache, const void* v_cache, con
 
   AttnParams p{};
   p.B = B; p.L = L; p.H = H; p.G = G; p.Lk = Lk; p.Lcap = Lcap; p.nsplit = nsplit;
-  p.scale_log2e = scale * 1.4426950408889634f;
+  at_set_scale(p, scale);
   p.key_valid = static_cast<const uint8_t*>(key_valid);
   p.out = static_cast<__nv_bfloat16*>(out);
   p.out_planes = static_cast<uint8_t*>(out_planes);
@@ -1943,7 +1951,7 @@ int tybok_attention_rows(const void* q, const void* k_rows, const void* v_rows, 
   }
   AttnParams p{};
   p.B = 1; p.L = L; p.H = H; p.G = H; p.Lk = Lk; p.Lcap = tail_cap; p.nsplit = 1; p.nb_rows = nb;
-  p.scale_log2e = scale * 1.4426950408889634f;
+  at_set_scale(p, scale);
   p.key_valid = static_cast<const uint8_t*>(key_valid);
   p.out = static_cast<__nv_bfloat16*>(out); p.out_planes = static_cast<uint8_t*>(out_planes); p.plane_scale = ldexpf(1.0f, out_shift);
   p.wide_out = ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(out_planes)) & 31) == 0;

@@ -320,7 +320,7 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr) {
 
 // Instruction descriptor for kind::f16 with bf16 A and B (both K-major) and fp32 accumulation:
 // [4,6) D format 1 = f32, [7,10) A format 1 = bf16, [10,13) B format 1 = bf16,
-// [17,23) N >> 3, [24,29) M >> 4.
+// [13] negate A, [16] B is MN-major, [17,23) N >> 3, [24,29) M >> 4.
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
          (static_cast<uint32_t>(m >> 4) << 24);
