@@ -1138,6 +1138,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         tc_wait_ld();
 #pragma unroll
         for (int w = 0; w < KW; ++w) {
+          if (!SHORT && bits[w] == 0u) continue;
           if (bits[w] != 0xffffffffu) {
 #pragma unroll
             for (int e = 0; e < 32; ++e)
@@ -1198,14 +1199,19 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_
         };
 #pragma unroll
         for (int w = 0; w < KW; ++w) {
-          uint32_t pk[16];
+          // A word of 32 masked keys, as padding has them and the last block of a ragged key count, costs no maxima and exponentials:
+          // 106 queries over 129 keys and 24 heads 7.9 -> 7.4 us (with 13 masked keys 7.2), 968 over 968 with 69 masked 23.9 -> 23.4 us.
+          // Not in the SHORT form, whose one word per thread is then a branch on its chain: 50 x 4146 keys 39.8 -> 42.3 us.
+          uint32_t pk[16] = {};
+          if (SHORT || bits[w] != 0u) {
 #pragma unroll
-          for (int e = 0; e < 32; e += 2) {
-            const float p0 = pf_exp2(__uint_as_float(v[w][e]) * p.scale_log2e - m_ref);
-            const float p1 = pf_exp2(__uint_as_float(v[w][e + 1]) * p.scale_log2e - m_ref);
-            add(e, p0 + p1);
-            const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
-            pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
+            for (int e = 0; e < 32; e += 2) {
+              const float p0 = pf_exp2(__uint_as_float(v[w][e]) * p.scale_log2e - m_ref);
+              const float p1 = pf_exp2(__uint_as_float(v[w][e + 1]) * p.scale_log2e - m_ref);
+              add(e, p0 + p1);
+              const __nv_bfloat162 pp = __floats2bfloat162_rn(p0, p1);
+              pk[e >> 1] = *reinterpret_cast<const uint32_t*>(&pp);
+            }
           }
           // P_j as bf16 pairs over the start of S_j: 16 columns per 32 keys (every thread of the row
           // has read its scores before the named barrier above)
