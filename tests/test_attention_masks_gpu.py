@@ -1,5 +1,5 @@
-"""Rows that meet masked keys only, for a block or for all of them, in every attention form and at scales on both sides of the usual
-one; and the images with the tuning aids against those without: the same bits."""
+"""Masked keys in every attention form: rows that meet masked keys only, for a block or for all of them, at every scale that the entry
+takes; the images with the tuning aids against those without, the same bits; and blocks of small weight in the merge."""
 
 import pytest
 import torch
@@ -53,3 +53,21 @@ def test_masked_blocks(b, l, keys, h, g, d, scale, first, last):
 @pytest.mark.parametrize("first,last", [(0, 0), (128, 37)])
 def test_masked_keys_count_for_nothing_at_any_scale(b, l, keys, h, g, d, scale, first, last):
     test_masked_blocks(b, l, keys, h, g, d, scale, min(first, keys // 2), last)
+
+
+# Two blocks of keys that are merged: one of weight about 2^-130 whose single valid key has values that its weight brings back to order 1.
+@pytest.mark.parametrize("b,h,g,keys", [(1, 8, 1, 256), (2, 8, 2, 256), (1, 8, 1, 1024)])  # rows pushed, one more group, staged in L2
+def test_a_blocks_small_weight_counts(b, h, g, keys):
+    from tybok_b200 import ops
+
+    q = torch.zeros(b * 50, h, 256, device="cuda", dtype=torch.bfloat16)
+    k, v = (torch.zeros(b, g, keys, 256, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    q[..., 0], k[:, :, 128, 0] = 1.0, -90.0
+    v[:, :, 128] = 3e38
+    valid = torch.zeros(b, keys, dtype=torch.uint8, device="cuda")
+    valid[:, :129] = 1
+    y = ops.attention(q.view(b * 50, h * 256), k, v, valid, tokens=50, keys=keys, scale=1.0)[0]
+    ops.check_status()
+    want = float(torch.exp(torch.tensor(-90.0).double()) * v[0, 0, 128, 0].double() / 128)
+    # weight 2^-130 / 128 has 12 bits left; bf16 result
+    assert bool(((y.double() - want).abs() <= (2.0**-9 + 2.0**-11) * want).all()), (float(y.min()), float(y.max()), want)

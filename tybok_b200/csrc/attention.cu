@@ -665,7 +665,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
     float denom = 0.f;
 #pragma unroll
     for (int s = 0; s < AT_MAX_SPLITS; ++s) {
-      w[s] = s < p.nsplit ? pf_exp2(w_in[s] - mx) : 0.f;  // 0 for a block without valid keys
+      w[s] = s < p.nsplit ? exp2f(w_in[s] - mx) : 0.f;  // 0 for a block without valid keys; below 2^-126 it still counts
       denom += w[s] * l[s];
     }
     const float inv = denom > 0.f ? 1.0f / denom : 0.f;
@@ -786,7 +786,7 @@ attention_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant
       float denom = 0.f;
 #pragma unroll
       for (int s = 0; s < AT_MAX_SPLITS; ++s) {
-        w[s] = s < p.nsplit ? pf_exp2(w[s] - mx) : 0.f;  // 0 for a block without valid keys
+        w[s] = s < p.nsplit ? exp2f(w[s] - mx) : 0.f;  // as in merge_weights
         denom += w[s] * l[s];
       }
       const float inv = denom > 0.f ? 1.0f / denom : 0.f;
