@@ -174,3 +174,45 @@ def test_gate_off_its_alignment(m, n, dtype):
         else:
             assert torch.equal(run(t), want)
     ops.check_status()
+
+
+# tokens on both sides of the two-plane threshold; interleaved gate / up weights and, at a width that is no multiple of 64, two matrices
+@pytest.mark.parametrize("b,l,inner", [(1, 33, 256), (2, 70, 256), (2, 150, 256), (1, 70, 336)])
+def test_filling_the_caches_equals_the_whole_pass(b, l, inner):
+    """Keys and values of every layer bit for bit, and a stream that waits for a layer's event finds them written."""
+    from tybok_b200 import _lib, ops
+
+    w, d, heads, layers = 256, 256, 2, 3
+    g = torch.Generator(device="cuda").manual_seed(l)
+    lin = lambda n, k: quantize_w8(_rnd(g, n, k, std=0.02))  # noqa: E731
+    rows = []
+    for _ in range(layers):
+        gate, up = lin(inner, w), lin(inner, w)
+        ffn = (ops.pack_gate_up(*gate, *up), None) if inner % 64 == 0 else (gate, up)
+        norms = [_rnd(g, w, std=0.1).float() for _ in range(2)]
+        rows.append((lin((heads + 2) * d, w), lin(w, heads * d), *ffn, lin(w, inner), *norms))
+    stack = _lib.native().GemmaStack(w, heads, 1, d, rows)
+    x, valid = _rnd(g, b * l, w), torch.ones(b, l, dtype=torch.uint8, device="cuda")
+    valid[:, l // 2 : l // 2 + 5] = 0
+    pos = torch.arange(l, dtype=torch.int32, device="cuda").repeat(b)
+    cos, sin = _rnd(g, l, d), _rnd(g, l, d)
+    caches = lambda: ([torch.zeros(b, 1, l + 7, d, dtype=torch.bfloat16, device="cuda") for _ in range(layers)] for _ in range(2))  # noqa: E731
+    (kc, vc), (k1, v1) = caches(), caches()
+    stack.forward(x, b, l, pos, cos, sin, kc, vc, 0, valid, None, None, 0, layers, [], [])
+    done, side = [torch.cuda.Event() for _ in range(layers)], torch.cuda.Stream()
+    for ev in done:
+        ev.record()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(20_000_000)  # ten milliseconds in which an event that is not recorded again lets the side stream pass
+    stack.fill_caches(x, b, l, pos, cos, sin, k1, v1, valid, [ev.cuda_event for ev in done])
+    seen = []
+    with torch.cuda.stream(side):
+        for i, ev in enumerate(done):
+            side.wait_event(ev)
+            seen.append((k1[i].clone(), v1[i].clone()))
+    torch.cuda.synchronize()
+    ops.check_status()
+    for i in range(layers):
+        assert bool(kc[i][:, :, :l].any()) and not bool(k1[i][:, :, l:].any())
+        assert torch.equal(seen[i][0], kc[i]) and torch.equal(seen[i][1], vc[i])
+        assert torch.equal(k1[i], kc[i]) and torch.equal(v1[i], vc[i])

@@ -51,8 +51,7 @@ class GemmaStack {
     return run(x, b, l, pos, cos, sin, kc, vc, key_off, key_valid, mods, fold, first, count, wait, record, false);
   }
   // The same for the caches alone: a prefix whose output nobody reads ends with its last layer's keys and values.  That layer's
-  // attention, output projection and FFN are nearly an eighteenth of the pass (chunk 10.06 -> 9.94 ms at batch 1, 101.3 -> 97.6 ms
-  // at batch 32).
+  // attention, output projection and FFN are nearly an eighteenth of the pass (66.3 -> 62.8 ms at batch 32).
   void fill_caches(const Tensor& x, int b, int l, const Tensor& pos, const Tensor& cos, const Tensor& sin, const std::vector<Tensor>& kc,
                    const std::vector<Tensor>& vc, const Tensor& key_valid, const std::vector<uint64_t>& record) const {
     run(x, b, l, pos, cos, sin, kc, vc, 0, key_valid, std::nullopt, std::nullopt, 0, static_cast<int>(layers_.size()), {}, record, true);

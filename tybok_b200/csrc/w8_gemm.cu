@@ -616,8 +616,8 @@ w8_gemm_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant_
   }
   if (warp >= 2 && !bars.abort) {
     // ---------------------------------------------------------- epilogue, phase B
-    // 4 consecutive channels per thread, 8 token rows per pass; with split-K, rank r owns token
-    // rows [r*R, (r+1)*R) and sums them over all ranks in rank order.
+    // 4 consecutive channels per thread, EW token rows per pass (twice as many in the packed forms); with split-K, pairs of token
+    // rows go round the ranks (token_of), and a row's owner sums it over all ranks in rank order.
     if (tr && tid == 64) tr[9] = clock64();
     const int et = tid - 64;
     const int v4 = et & 31;

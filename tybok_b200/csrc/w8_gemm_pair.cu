@@ -11,7 +11,7 @@
 //   * two accumulators of 256 columns take turns: sixteen epilogue warps, 16 tokens at a time, empty one while the next
 //     tile's products fill the other.  (Eight warps with 32 tokens each did not keep up where a tile's K is short and its epilogue
 //     long: four warps per scheduler instead of two hide the latencies of its chains, results are rounded to bf16 in
-//     pairs, and half the registers do.  DiT denoiser at 106 tokens 16.48 -> 16.15 ms, same bits.)  Before, each tile's epilogue ran on a second resident CTA, which halved the
+//     pairs, and half the registers do.  DiT denoiser at 106 tokens 16.65 -> 16.21 ms, same bits.)  Before, each tile's epilogue ran on a second resident CTA, which halved the
 //     ring (two 46 KB stages in flight per CTA).  Now the ring has 4 (np = 2) or 3 stages of 48 / 64 KB.
 //   * an epilogue thread holds one channel (its tensor-memory lane) of 16 tokens, so scale, bias and gate
 //     are per-thread scalars; results turn into four channels per thread by a 4 x 4 transpose across
