@@ -260,7 +260,7 @@ int tybok_w8x3_qkv_rope(const void* x_planes, int x_shift, const void* w8_paired
 /* GQA/MQA attention of L query tokens per batch element over the first Lk keys of the caches
  * (head_dim 256: Lk <= 1024 for L <= 128, Lk <= 8192 for longer query sequences; head_dim 128: any L,
  * Lk <= 8192):
- * softmax(q k^T * scale + mask) v with fp32 softmax, bf16 P.
+ * softmax(q k^T * scale + mask) v with fp32 softmax, bf16 P, at any finite scale; a query without a valid key gives zeros.
  *   q          [B*L, H*D] bf16 (already rotated);  k_cache / v_cache  [B, G, Lcap, D] bf16, finite
  *   key_valid  NULL or uint8 [B, Lk]: 0 masks a key for every query of that batch element
  *   out        bf16 [B*L, H*D] and/or out_planes [3][B*L][H*D] planes of out * 2^out_shift
